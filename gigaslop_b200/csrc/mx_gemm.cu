@@ -377,18 +377,27 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, MX_TMEM_COLS); }
 }
 
-// ---- row-major [rows, K/32] scales -> the 128 x 4 tile order (one thread per output byte) -------------------
-__global__ void mx_scales_to_tiled_kernel(const uint8_t* __restrict__ src, long long ld, long long rows, int k32,
-                                          uint8_t* __restrict__ dst, long long total) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int kt = k32 / 4;                                  // 128-wide K tiles
-  const long long tile = i / 512; const int in = (int)(i % 512);
-  const long long rb = tile / kt; const int kb = (int)(tile % kt);
-  const int r = (in / 16) + 32 * ((in % 16) / 4);          // row inside the 128-row block
-  const int b = kb * 4 + (in % 4);
-  const long long row = rb * 128 + r;
-  dst[i] = (row < rows) ? src[row * ld + b] : (uint8_t)127;   // padding rows: scale 1.0 on zero data
+// ---- row-major [rows, K/32] scales -> the 128 x 4 tile order --------------------------------------------------
+// A thread moves the four scales of one row and one 128-wide K tile: one word of the tile, four neighbouring source bytes
+// (K % 128 == 0, so a row holds whole groups of four).  Consecutive threads write consecutive words; the 32 rows of a
+// lane group lie ld bytes apart, and the other words of their sectors are picked up from L1 by the threads of the
+// neighbouring tiles.  With a thread per byte the launch took 10.5 us (mean of 65536 x 512 and x 2048; 4.3 us now).
+__global__ void mx_scales_to_tiled_kernel(const uint8_t* __restrict__ src, long long ld, long long rows, int kt,
+                                          uint8_t* __restrict__ dst, unsigned words, bool word_loads, bool word_stores) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= words) return;
+  const unsigned tile = i >> 7, in = i & 127;              // 128 words per tile
+  const unsigned rb = tile / (unsigned)kt, kb = tile % (unsigned)kt;
+  const long long row = (long long)rb * 128 + (in >> 2) + 32 * (in & 3);
+  uint32_t v = 0x7f7f7f7fu;                                // padding rows: scale 1.0 on zero data
+  if (row < rows) {
+    const uint8_t* s = src + row * ld + kb * 4;
+    if (word_loads) v = __ldg(reinterpret_cast<const uint32_t*>(s));
+    else v = s[0] | (uint32_t)s[1] << 8 | (uint32_t)s[2] << 16 | (uint32_t)s[3] << 24;
+  }
+  uint8_t* d = dst + (size_t)i * 4;
+  if (word_stores) *reinterpret_cast<uint32_t*>(d) = v;
+  else { d[0] = (uint8_t)v; d[1] = (uint8_t)(v >> 8); d[2] = (uint8_t)(v >> 16); d[3] = (uint8_t)(v >> 24); }
 }
 
 size_t mx_tiled_scale_bytes(long long rows, int K) {
@@ -398,10 +407,12 @@ size_t mx_tiled_scale_bytes(long long rows, int K) {
 int32_t launch_mx_scales_to_tiled(const uint8_t* src, long long ld, long long rows, int K, uint8_t* dst, cudaStream_t st) {
   if (rows == 0) return GSB200_OK;
   if (!src || !dst || rows < 0 || K <= 0 || K % 128 != 0 || ld < K / 32) return GSB200_ERR_BAD_ARG;
-  const long long total = (long long)mx_tiled_scale_bytes(rows, K);
-  const long long blocks = (total + 255) / 256;
-  if (blocks > 0x7fffffffll) return GSB200_ERR_BAD_ARG;
-  mx_scales_to_tiled_kernel<<<(unsigned)blocks, 256, 0, st>>>(src, ld, rows, K / 32, dst, total);
+  const long long words = (long long)mx_tiled_scale_bytes(rows, K) / 4;
+  if (words > 0xffffff00ll) return GSB200_ERR_BAD_ARG;
+  const bool word_loads = ld % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 3) == 0;
+  const bool word_stores = (reinterpret_cast<uintptr_t>(dst) & 3) == 0;
+  mx_scales_to_tiled_kernel<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(src, ld, rows, K / 128, dst, (unsigned)words,
+                                                                          word_loads, word_stores);
   return cuda_status(cudaGetLastError(), "mx scale re-tiling launch");
 }
 

@@ -71,6 +71,28 @@ def test_fp8_quantiser_bitexact(M, K, torch_form):
     assert_bitexact(q, q_ref, "fp8 bytes")
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("K", [256, 768, 2048, 2304])
+def test_fp8_quantiser_quotients_bitexact(dtype, K):
+    """The torch formulation divides every element by the row scale: every finite fp16 value (both zeros and the
+    subnormals among them) under row maxima from 2^-24 to 65504, bit for bit."""
+    g = need_lib()
+    every = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.float16)
+    every = every[torch.isfinite(every)]
+    every = every[torch.argsort(every.abs().float())]           # rows of like magnitude, so that every E4M3 binade is met
+    M = (every.numel() + K - 1) // K
+    x = torch.zeros(M * K, dtype=torch.float16)
+    x[: every.numel()] = every
+    x = x.view(M, K).to(dtype)
+    gen = torch.Generator().manual_seed(K)
+    mixed = torch.randn(64, K, generator=gen) * torch.logspace(-6, 3, 64)[:, None]
+    x = torch.cat([x, mixed.to(dtype)])
+    q_ref, s_ref = oracle.fp8_quantize_per_token(x.float())
+    q, s = g.fp8_quantize_per_token(x.cuda())
+    assert_bitexact(s, s_ref, "fp8 scale")
+    assert_bitexact(q, q_ref, "fp8 bytes")
+
+
 def test_fp8_quantiser_golden():
     g = need_lib()
     gold = load_golden("fp8_quant")
