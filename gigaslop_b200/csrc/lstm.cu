@@ -6,17 +6,24 @@
 // this library); h feeds the recurrent GEMM as E4M3 at the fixed scale 1/448 (the reference's convention for a
 // value bounded by 1, fly/rdna_fp8_factored_lstm.py:321-326); c and the emitted h are fp16.
 //
-// Decomposition: CTA (g, s) owns 128 batch rows (row group g) x 32 hidden units (slice s) = 128 gate columns.
+// Three kernels with the same arithmetic, and the same order of the K blocks, so that they give the same bytes:
+//   lstm_tmem_kernel       what runs: W_hh in tensor memory, gates^T = W_hh . h^T, h exchanged between at most four CTAs
+//   lstm_cluster_kernel    H <= 384, 128 batch rows x 32 hidden units per CTA, h through distributed shared memory
+//   lstm_recurrent_kernel  H <= 512, the same tile, h through global memory (cooperative launch)
+// The last two are for a device that cannot host the first one's clusters and can be selected by environment variables.
+//
+// In these two, CTA (g, s) owns 128 batch rows (row group g) x 32 hidden units (slice s) = 128 gate columns.
 // Its W_hh slice (128 rows x H bytes) stays in shared memory for the whole layer, c_t stays in registers.
-// Batch rows are independent, so only the H/32 CTAs of a row group exchange data: each step every CTA
-// writes its 128 x 32 piece of h_t (E4M3) to a double-buffered global scratch and bumps its step counter;
+// Batch rows are independent, so only the H/32 CTAs of a row group exchange data: each step every CTA of the cooperative
+// kernel writes its 128 x 32 piece of h_t (E4M3) to a double-buffered global scratch and bumps its step counter;
 // the others poll the counters (bounded), pull the full 128 x H tile into 128B-swizzled shared memory and
 // run 128 x 128 x H on the tensor core (tcgen05 kind::f8f6f4, fp32 accumulators in TMEM).  The next step's ih tile
-// is prefetched by TMA while the current step computes.  The step is latency-bound (0.3 us of tensor time).
+// is prefetched by TMA while the current step computes.
 #include <cooperative_groups.h>
 #include <cuda_fp8.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "capi_internal.h"
 #include "ptx.cuh"
@@ -27,10 +34,8 @@ namespace gsb {
 // Tuning aid (never in the shipped library): SM clock stamps of one step of CTA 0, threads 0 and 128.
 __device__ long long g_lstm_prof[2][16];
 #define LPROF(slot) do { if (blockIdx.x == 0 && s == 100 && (tid == 0 || tid == 128)) g_lstm_prof[tid == 128][slot] = clock64(); } while (0)
-#define LPROF2(who, slot) do { if (blockIdx.x == 0 && (s == 100 || s == 101)) g_lstm_prof[who][(slot) + 8 * (s - 100)] = clock64(); } while (0)
 #else
 #define LPROF(slot) do { } while (0)
-#define LPROF2(who, slot) do { } while (0)
 #endif
 
 constexpr int LSTM_THREADS = 256;            // 8 warps: all load / do gate math; warp 0 lane 0 also issues TMA + MMA
@@ -202,11 +207,12 @@ lstm_recurrent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     if (tid == 0) {
       tc_fence_after();
       constexpr uint32_t idesc = umma_idesc(1, 0, 0, LSTM_ROWS, LSTM_NCOL);
-      for (int kb = 0; kb < p.k_blocks; ++kb) {
+      for (int n = 0, kb = hid0 >> 7; n < p.k_blocks; ++n) {        // (the K order of the transposed form)
         const uint64_t a_desc = umma_smem_desc_sw128(smem_u32(h_s + kb * LSTM_KB_BYTES));
         const uint64_t b_desc = umma_smem_desc_sw128(smem_u32(w_s + kb * LSTM_KB_BYTES));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) umma_f8(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
+        for (int k = 0; k < 4; ++k) umma_f8(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (n | k) != 0);
+        if (++kb == p.k_blocks) kb = 0;
       }
       umma_commit(mma_done);
     }
@@ -427,9 +433,11 @@ lstm_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     const uint64_t a_desc = buf ? a_base[1] : a_base[0];
     const int ksteps = H >> 5;                        // 32 bytes of K per MMA
     tc_fence_after();
-    for (int ks = 0; ks < ksteps; ++ks)
+    for (int n = 0, ks = (hid0 >> 7) * 4; n < ksteps; ++n) {         // (the K order of the transposed form)
       umma_f8(tmem_base, a_desc + (uint64_t)(ks * (2 * LSTMC_CHUNK >> 4)),
-              b_base + (uint64_t)((ks >> 2) * (LSTM_KB_BYTES >> 4) + 2 * (ks & 3)), idesc, ks != 0);
+              b_base + (uint64_t)((ks >> 2) * (LSTM_KB_BYTES >> 4) + 2 * (ks & 3)), idesc, n != 0);
+      if (++ks == ksteps) ks = 0;
+    }
     umma_commit(mma_done);
   };
   if (tid == LSTMC_MMA_TID && ok && p.T > 0) issue_mmas(1);       // step 0 reads buffer 1
@@ -544,317 +552,450 @@ lstm_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   cluster_sync_all();                    // nobody leaves while another CTA of the cluster may still store into it
 }
 
-// ---- cluster form, two interleaved 64-row halves per CTA -----------------------------------------------------------
-// The step of the kernel above is one serial chain per CTA: gather h (about 1700 clocks from the CTA barrier until the
-// last slice's piece has crossed the cluster), issue the MMAs (about 100 clocks each), wait for the accumulator, gate
-// math, stage, barrier, send.  Nothing in it is busy for long; it is latency end to end.  Here a CTA still owns 128
-// batch rows x 32 hidden units, but as TWO independent halves of 64 rows that take turns: while the pieces of one half
-// are in flight and its MMAs run, the eight compute warps do the gate math of the other half.  What makes that work:
-//  * M = 64 MMAs.  Their accumulator sits in the lower 16 lanes of each TMEM lane quarter, and tcgen05.ld.16x256b hands
-//    a warp 16 rows x 16 columns as 2 rows x (2 + 2) column pairs per thread, so all 256 compute threads share a half's
-//    64 x 128 gate values evenly: 8 cells each (2 rows x 4 hidden units, all four gates of a cell in one thread).
-//  * a ninth warp that only issues MMAs (and the TMA loads of the ih tiles), so no compute thread ever waits for a gather;
-//  * one mbarrier per (half, buffer, source slice): the K step that reads slice k's 32 bytes of h is issued as soon as
-//    that slice's piece has landed, so the MMA issue overlaps the gather instead of following it.
-// The outputs leave through the staged images of the piece (whole 32-byte / 64-byte runs per row, written by
-// cooperating threads) instead of 16-byte slivers per row.  Arithmetic per cell is that of the other two kernels (a test
-// holds all three to the same bytes).
-constexpr int L64_ROWS = 64;
-constexpr int L2_THREADS = 320;                                // 8 compute warps + the MMA warp + the send warp
-constexpr int L2_COMPUTE = 256;
-constexpr int L64_CHUNK = L64_ROWS * 16;                       // one 16-byte K chunk of all 64 rows
-constexpr int L64_PIECE = L64_ROWS * LSTM_HS;                  // 2 KiB: this CTA's piece of a half's h (two chunks = one K step)
-constexpr int L64_HBUF = LSTMC_MAX_KB * 8 * L64_CHUNK;         // 24 KiB: a half's 64 x 384 tile of h as 24 chunks
-constexpr int L64_IH_GATE = L64_ROWS * LSTM_HS * 2;            // 4 KiB: one gate's 64 x 32 fp16 box
-constexpr int L64_IH_BYTES = 4 * L64_IH_GATE;                  // 16 KiB
-constexpr int L64_H16_BYTES = L64_ROWS * LSTM_HS * 2;          // 4 KiB: fp16 image of the piece (layer output)
-constexpr int L2_MAX_SLICES = 12;
-constexpr int L2_SMEM_W = 0;
-constexpr int L2_SMEM_H = L2_SMEM_W + LSTMC_MAX_KB * LSTM_KB_BYTES;          // [half][buffer]
-constexpr int L2_SMEM_IH = L2_SMEM_H + 4 * L64_HBUF;                         // [half][buffer]
-constexpr int L2_SMEM_STG = L2_SMEM_IH + 4 * L64_IH_BYTES;                   // [half][buffer]
-constexpr int L2_SMEM_H16 = L2_SMEM_STG + 4 * L64_PIECE;                     // [half]
-constexpr int L2_SMEM_SC = L2_SMEM_H16 + 2 * L64_H16_BYTES;
-constexpr int L2_SMEM_BAR = L2_SMEM_SC + 1024;
-constexpr int L2_SMEM_USED = L2_SMEM_BAR + 512;
-constexpr int L2_SMEM_BYTES = L2_SMEM_USED + 1024;
-static_assert(L2_SMEM_BYTES <= 227 * 1024 && L2_SMEM_BYTES > 116 * 1024, "one CTA per SM");
+// ---- transposed form: W_hh in tensor memory, the batch as the N dimension ------------------------------------------
+// gates^T = W_hh . h^T: a CTA owns 128 hidden units and G = 8, 12, 16 or 32 batch rows (N = R = 16 or 32 columns of the
+// MMA; columns without a row multiply zeros).  The four gates of its hidden units are four M = 128 x N = R accumulators, so
+// a cell's four gate values sit in one TMEM lane and one thread has them all.  The A operand, W_hh (4 x 128 rows x up to
+// 384 bytes), is written to tensor memory once per launch (384 of its 512 columns; a fourth K block, H > 384, stays in
+// shared memory).
+//
+// A step is latency end to end: MMAs (issue-bound: 12 per gate at H = 384), accumulator to registers, gate math, h to the
+// other CTAs of the row group, MMAs.  What the split buys:
+//  * a row group is ceil(H / 128) CTAs instead of H / 32, so h goes to at most three other CTAs.  (With 32 units per CTA a
+//    step's all-gather was twelve bulk copies per CTA and half at 220 clocks each, all of the step's 2.7 us.)  It leaves
+//    with st.async straight after the gate math, half of a warp's rows at a time, 16 bytes per lane, and reports to the
+//    receiver's mbarrier; a bulk copy from a warp of its own is as fast for two receivers (1.62 us per step) and slower
+//    for one, plain remote stores with a releasing arrive cost 1300 clocks (2.10 us).
+//  * the batch is the small dimension, so B = 512 spreads over 129 SMs (G = 12) instead of 48: the gate math, five
+//    special-function instructions per cell, is 1000 clocks for 2048 cells (G = 16), 600 for 1024.
+//  * W_hh in tensor memory: an MMA from a shared-memory A operand of 128 rows takes 40 clocks, from TMEM 16.
+// B = 512, H = 384: 1.27 us per step (2.57 before), H = 512: 1.83 (4.8), H = 256: 0.96 (2.29), H = 128: 0.73 (2.27).
+// Clocks of a step (G = 16, H = 384, of ~2650): own K block's MMAs 340, wait for the others' h 300, their MMAs 560, commit
+// to registers 300, gate math and sending 1000, hand-over to the MMA warps 130.
+//   warps 0 .. CW-1   gate math.  Warp w: TMEM lane quarter w % 4 (32 hidden units, one per lane), G / (CW / 4) batch rows
+//   last four warps   one MMA-issuing thread per gate (an MMA costs the thread that issues it 60 to 70 clocks); the last
+//                     one also issues the TMA loads of the ih tiles
+// h is kept as K-major rows of 128 bytes with the 128-byte swizzle, one K block per CTA of the row group: a CTA's piece is
+// one K block, written by its own gate warps where its own MMAs read it and sent from there to the others.
+// h_t goes to buffer t & 1; the MMAs of step t read buffer (t + 1) & 1.  Buffer t & 1 may be written in step t: the MMAs of
+// step t - 1 that read it are complete (here: this CTA has waited for them; there: the sender got our h_{t-1}, sent after
+// them).
+constexpr int LT_HS = 128;                                     // hidden units per CTA (UMMA M)
+constexpr int LT_TMEM_KB = 3;                                  // K blocks of W_hh in tensor memory
+constexpr int LT_ACC_COL = 4 * LT_TMEM_KB * 32;                // accumulator columns start here (gate g: + g * R)
+constexpr int LT_MAX_SLICES = 4;                               // H <= 512
+constexpr int LT_STAGES = 3;                                   // ih tiles in flight
 
-__global__ void __launch_bounds__(L2_THREADS, 1)
-lstm_cluster2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_ih,
-                     const LstmParams p) {
+template <int R, int G>
+struct LtSmem {
+  static constexpr int KB_BYTES = R * 128;                     // one K block of h
+  static constexpr int HBUF = LT_MAX_SLICES * KB_BYTES;
+  static constexpr int IH_GATE = G * LT_HS * 2;
+  static constexpr int IH_BYTES = 4 * IH_GATE;
+  static constexpr int H = 0;                                  // [2][HBUF]
+  static constexpr int IH = H + 2 * HBUF;                      // [LT_STAGES][IH_BYTES]
+  static constexpr int BAR = IH + LT_STAGES * IH_BYTES;
+  static constexpr int W = BAR + 1024;                         // fourth K block of W_hh: four gates x 16 KiB (H > 384 only)
+  static constexpr int bytes(int slices) { return W + (slices > LT_TMEM_KB ? 4 * LSTM_KB_BYTES : 0) + 1024; }
+};
+static_assert(LtSmem<32, 32>::bytes(4) <= 227 * 1024, "shared memory budget");
+
+template <int R, int G, int CW>
+__global__ void __launch_bounds__(32 * (CW + 4), 1)
+lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_ih, const uint8_t* __restrict__ w_hh,
+                 long long ld_w, const LstmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* w_s = smem + L2_SMEM_W;
-  uint8_t* h_s = smem + L2_SMEM_H;                 // + (2 * half + buffer) * L64_HBUF
-  uint8_t* ih_s = smem + L2_SMEM_IH;               // + (2 * half + buffer) * L64_IH_BYTES
-  uint8_t* stg_s = smem + L2_SMEM_STG;             // + (2 * half + buffer) * L64_PIECE
-  uint8_t* h16_base = smem + L2_SMEM_H16;          // + half * L64_H16_BYTES
-  float* sc_s = reinterpret_cast<float*>(smem + L2_SMEM_SC);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L2_SMEM_BAR);
-  uint64_t* w_full = bars;
-  uint64_t* ih_full = bars + 1;                    // [half][buffer]
-  uint64_t* mma_done = bars + 5;                   // [half]
-  uint64_t* staged = bars + 7;                     // [half]: this CTA's piece of the step's h is staged, the send warp may copy it
-  uint64_t* h_ready = bars + 9;                    // [half][buffer]: every slice's piece of h has landed (bytes counted)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  using L = LtSmem<R, G>;
+  constexpr int RPT = G / (CW / 4);                // batch rows per gate thread
+  static_assert(RPT == 4 || RPT == 8, "rows per thread");
+  uint8_t* h_s = smem + L::H;
+  uint8_t* ih_s = smem + L::IH;
+  uint8_t* w_s = smem + L::W;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
+  uint64_t* ih_full = bars;                        // [LT_STAGES]
+  uint64_t* own_ready = ih_full + LT_STAGES;      // [2] this CTA's piece of h is in the buffer, its accumulators have been read
+  uint64_t* h_ready = own_ready + 2;               // [2] the other CTAs' pieces have landed (bytes counted)
+  uint64_t* mma_done = h_ready + 2;                // the four gates' accumulators are complete
+  uint64_t* w_full = mma_done + 1;                 // the fourth K block of W_hh has landed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(w_full + 1);
   const AbortFlag abort_flag{smem_u32(tmem_slot + 1)};
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int grp = blockIdx.x / p.slices;        // 128-row group = cluster
-  const int slc = blockIdx.x % p.slices;        // hidden slice = rank inside the cluster
-  const int row0 = grp * LSTM_ROWS;
-  const int hid0 = slc * LSTM_HS;
+  const int grp = blockIdx.x / p.slices;           // row group = cluster
+  const int slc = blockIdx.x % p.slices;           // hidden slice = rank inside the cluster = its K block of h
+  const int row0 = grp * G, hid0 = slc * LT_HS;
   const int H = p.H, B = p.B;
-  const int halves = (B - row0 > L64_ROWS) ? 2 : 1;     // the last group may have rows for one half only
+  const int kb_tmem = p.k_blocks < LT_TMEM_KB ? p.k_blocks : LT_TMEM_KB;
+  const uint32_t peer_bytes = (uint32_t)(p.slices - 1) * G * LT_HS;
 
   if (tid == 0) {
-    mbar_init(w_full, 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&ih_full[i], 1);
-    mbar_init(&mma_done[0], 1); mbar_init(&mma_done[1], 1);
-    mbar_init(&staged[0], 1); mbar_init(&staged[1], 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&h_ready[i], 1);
-    // arm the first use of each tile barrier: h_0 arrives in buffer 0 (if there is a step 1), h_1 in buffer 1
-    for (int hf = 0; hf < halves; ++hf) {
-      if (p.T > 1) mbar_arrive_expect_tx(&h_ready[2 * hf + 0], p.slices * L64_PIECE);
-      if (p.T > 2) mbar_arrive_expect_tx(&h_ready[2 * hf + 1], p.slices * L64_PIECE);
-    }
+    for (int i = 0; i < LT_STAGES; ++i) mbar_init(&ih_full[i], 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&own_ready[i], CW); mbar_init(&h_ready[i], 1); }
+    mbar_init(mma_done, 4); mbar_init(w_full, 1);
+    // arm the first use of each buffer: h_0 arrives in buffer 0 (if there is a step 1), h_1 in buffer 1
+    if (p.slices > 1 && p.T > 1) mbar_arrive_expect_tx(&h_ready[0], peer_bytes);
+    if (p.slices > 1 && p.T > 2) mbar_arrive_expect_tx(&h_ready[1], peer_bytes);
     abort_flag.set(0);
     fence_mbar_init();
     prefetch_tmap(&tm_w); prefetch_tmap(&tm_ih);
   }
-  if (warp == 8) { tmem_alloc(tmem_slot, 2 * LSTM_NCOL); tmem_relinquish(); }
-  if (tid < LSTM_NCOL) {
-    const int n = (tid >> 5) * H + hid0 + (tid & 31);
-    sc_s[tid] = __ldg(p.s_hh + n) * (1.0f / 448.0f);
-    sc_s[LSTM_NCOL + tid] = p.bias ? __ldg(p.bias + n) : 0.f;
-  }
+  if (warp == CW) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  cluster_sync_all();                    // every CTA's barriers exist (and are armed) before anyone sends to them
+  cluster_sync_all();                              // every CTA's barriers exist (and are armed) before anyone sends to them
   const uint32_t tmem_base = *tmem_slot;
   const unsigned int budget = spin_budget();
   const bool rank_ok = cluster_ctarank() == (uint32_t)slc;
   if (!rank_ok && tid == 0) { abort_flag.set(1); atomicOr(&g_status[0], ST_TIMEOUT_LSTM); g_status[1] = 0x50; }
 
   auto step_t = [&](int s) { return p.reverse ? p.T - 1 - s : s; };
-  auto issue_ih = [&](int hf, int s) {     // one thread: TMA the four gate boxes of step s, half hf
-    const int ib = 2 * hf + (s & 1);
-    uint8_t* dst = ih_s + ib * L64_IH_BYTES;
-    mbar_arrive_expect_tx(&ih_full[ib], L64_IH_BYTES);
-    const int r = step_t(s) * B + row0 + hf * L64_ROWS;
+  auto issue_ih = [&](int s, int st) {             // one thread: the four gate boxes of step s into stage st
+    mbar_arrive_expect_tx(&ih_full[st], L::IH_BYTES);
+    const int r = step_t(s) * B + row0;
 #pragma unroll
-    for (int g = 0; g < 4; ++g) tma_load_2d(dst + g * L64_IH_GATE, &tm_ih, &ih_full[ib], g * H + hid0, r);
+    for (int g = 0; g < 4; ++g) tma_load_2d(ih_s + st * L::IH_BYTES + g * L::IH_GATE, &tm_ih, &ih_full[st], g * H + hid0, r);
   };
 
-  // this thread's cells of a half (compute warps): rows ra and ra + 8, hidden units u0 + {0, 1} and u0 + 8 + {0, 1} of
-  // the slice; cell index = 4 * k + 2 * rowsel + j, the order in which tcgen05.ld.16x256b.x2 delivers them
-  const int q = warp & 3, hh = (warp >> 2) & 1;
-  const int ra = 16 * q + (lane >> 2);
-  const int u0 = 16 * hh + 2 * (lane & 3);
-  auto cell_row = [&](int i) { return ra + ((i >> 1) & 1) * 8; };
-  auto cell_u = [&](int i) { return u0 + (i >> 2) * 8 + (i & 1); };
-  float c[2][8];
-  float2 sc2[4][2], bi2[4][2];
-  int ih_off[4];
-  if (warp >= 8) {
-    if (warp == 8 && lane == 0) {         // W slice and the first two ih tiles of each half
-      mbar_arrive_expect_tx(w_full, p.k_blocks * LSTM_KB_BYTES);
-      for (int kb = 0; kb < p.k_blocks; ++kb)
-#pragma unroll
-        for (int g = 0; g < 4; ++g)
-          tma_load_2d(w_s + kb * LSTM_KB_BYTES + g * (LSTM_HS * 128), &tm_w, w_full, kb * 128, g * H + hid0);
-      for (int hf = 0; hf < halves; ++hf) { issue_ih(hf, 0); if (p.T > 1) issue_ih(hf, 1); }
-    }
-  } else {
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf)
+  // gate threads: hidden unit hid, batch rows r_lo .. r_lo + RPT - 1 of the group
+  const int q = warp & 3;
+  const int u = q * 32 + lane, hid = hid0 + u;
+  const bool hid_ok = hid < H;
+  const int r_lo = (warp >> 2) * RPT;
+  const int rows_live = min(RPT, max(0, B - (row0 + r_lo)));          // rows of this thread that exist
+  float c[RPT];
+  if (warp < CW) {
+    // W_hh -> tensor memory: lane = hidden unit, 32 columns = 128 bytes of K; the warps of a lane quarter share the K blocks
+    for (int blk = warp >> 2; blk < 4 * kb_tmem; blk += CW / 4) {
+      const int g = blk / kb_tmem, kb = blk % kb_tmem;
+      uint32_t v[32];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int row = row0 + hf * L64_ROWS + cell_row(i);
-        c[hf][i] = (p.c0 && row < B) ? __half2float(p.c0[(long long)row * H + hid0 + cell_u(i)]) : 0.f;
+        uint4 w = make_uint4(0, 0, 0, 0);
+        if (hid_ok && kb * 128 + i * 16 < H) w = __ldg(reinterpret_cast<const uint4*>(w_hh + (long long)(g * H + hid) * ld_w + kb * 128 + i * 16));
+        v[4 * i] = w.x; v[4 * i + 1] = w.y; v[4 * i + 2] = w.z; v[4 * i + 3] = w.w;
       }
-#pragma unroll
-    for (int g = 0; g < 4; ++g)
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int col = g * LSTM_HS + u0 + 8 * k;
-        sc2[g][k] = make_float2(sc_s[col], sc_s[col + 1]);
-        bi2[g][k] = make_float2(sc_s[LSTM_NCOL + col], sc_s[LSTM_NCOL + col + 1]);
-      }
-    // byte offsets of this thread's ih values inside a gate box (64-byte swizzle): one half2 per (k, rowsel)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = i >> 1, row = ra + (i & 1) * 8;
-      ih_off[i] = row * 64 + (((2 * hh + k) ^ ((row >> 1) & 3)) << 4) + 4 * (lane & 3);
+      tmem_st_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (g * LT_TMEM_KB + kb) * 32, v);
     }
-    // step 0 reads h_0 (or zeros) from buffer 1 of each half, staged by this CTA's own compute threads
-    const int chunks_per_row = H >> 4;
-    for (int hf = 0; hf < halves; ++hf)
-      for (int id = tid; id < L64_ROWS * chunks_per_row; id += L2_COMPUTE) {
-        const int r = id / chunks_per_row, cc = id % chunks_per_row;
-        const int row = row0 + hf * L64_ROWS + r;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (p.h0 && row < B) v = __ldcg(reinterpret_cast<const uint4*>(p.h0 + (size_t)row * H + cc * 16));
-        *reinterpret_cast<uint4*>(h_s + (2 * hf + 1) * L64_HBUF + cc * L64_CHUNK + r * 16) = v;
-      }
+    tmem_st_wait();
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
+      c[i] = (p.c0 && hid_ok && i < rows_live) ? __half2float(p.c0[(long long)(row0 + r_lo + i) * H + hid]) : 0.f;
+    // step 0 reads h_0 (or zeros) from buffer 1, staged by this CTA's own threads
+    if constexpr (G < R)                           // the rows of the MMA that no batch row uses
+      for (int id = tid; id < 2 * L::HBUF / 16; id += 32 * CW)
+        if (((id >> 3) & (R - 1)) >= G) *reinterpret_cast<uint4*>(h_s + id * 16) = make_uint4(0, 0, 0, 0);
+    const int chunks = H >> 4;
+    for (int id = tid; id < G * chunks; id += 32 * CW) {
+      const int r = id / chunks, cc = id % chunks;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (p.h0 && row0 + r < B) v = __ldcg(reinterpret_cast<const uint4*>(p.h0 + (size_t)(row0 + r) * H + cc * 16));
+      *reinterpret_cast<uint4*>(h_s + L::HBUF + (cc >> 3) * L::KB_BYTES + r * 128 + (((cc & 7) ^ (r & 7)) << 4)) = v;
+    }
     fence_proxy_async_smem();
+  } else if (warp == CW + 3 && lane == 0) {
+    if (p.slices > LT_TMEM_KB) {
+      mbar_arrive_expect_tx(w_full, 4 * LSTM_KB_BYTES);
+      for (int g = 0; g < 4; ++g) tma_load_2d(w_s + g * LSTM_KB_BYTES, &tm_w, w_full, LT_TMEM_KB * 128, g * H + hid0);
+    }
+    for (int s = 0; s < LT_STAGES && s < p.T; ++s) issue_ih(s, s);
   }
-  __syncthreads();                       // h_0 is staged before the first MMAs read it
+  tc_fence_before();
+  __syncthreads();                                 // W_hh is in tensor memory and h_0 staged before the first MMAs read them
+  tc_fence_after();
 
-  if (warp == 8) {
-    // ------------------------------ MMA warp: one thread issues the MMAs and the ih loads ------------------------------
-    if (lane == 0) {
-      bool ok = rank_ok && mbar_wait(w_full, 0, abort_flag, ST_TIMEOUT_LSTM, 0x10, budget);
-      constexpr uint32_t idesc = umma_idesc(1, 0, 0, L64_ROWS, LSTM_NCOL);
-      const uint64_t b_base = umma_smem_desc_sw128(smem_u32(w_s));
-      const int ksteps = H >> 5;                        // one K step (32 bytes of h) per hidden slice
-      for (int s = 0; ok && s < p.T; ++s) {
-        for (int hf = 0; ok && hf < halves; ++hf) {
-          // gates of step s, half hf: h_{s-1} sits in buffer (s + 1) & 1 (step 0: h_0 or zeros, staged locally)
-          LPROF2(1, 4 * hf + 0);
-          const int hb = 2 * hf + ((s + 1) & 1);
-          const uint64_t a_desc = umma_smem_desc_kchunks(smem_u32(h_s + hb * L64_HBUF), L64_CHUNK);
-          if (s > 0) {
-            if (!mbar_wait_cluster(&h_ready[hb], (uint32_t)((s - 1) >> 1) & 1u, abort_flag, ST_TIMEOUT_LSTM, 0x40, budget)) { ok = false; break; }
-            if (s + 2 < p.T) mbar_arrive_expect_tx(&h_ready[hb], p.slices * L64_PIECE);   // its next use: h_{s+1}, read by step s + 2
+  if (warp < CW) {
+    // ------------------------------ gate math ------------------------------
+    // sigmoid(x) = 0.5 + 0.5 tanh(x / 2): the halving of the three sigmoid gates is folded into scale, ih and bias (exact)
+    float sc[4], bi[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const float half = g == 2 ? 1.0f : 0.5f;
+      sc[g] = hid_ok ? __ldg(p.s_hh + g * H + hid) * (1.0f / 448.0f) * half : 0.f;
+      bi[g] = hid_ok && p.bias ? __ldg(p.bias + g * H + hid) * half : 0.f;
+    }
+    const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + LT_ACC_COL + r_lo;
+    const uint8_t* ih_t = ih_s + r_lo * (LT_HS * 2) + u * 2;
+    uint8_t* own = h_s + slc * L::KB_BYTES + (u & 15);               // + row * 128 + swizzled chunk
+    const int ck = u >> 4;
+    // all-gather: half of the warp's rows x its 32 bytes at a time, one 16-byte store per lane (peer, row, chunk)
+    const bool sends = lane < (p.slices - 1) * RPT;
+    const uint32_t to = (uint32_t)(lane / RPT < slc ? lane / RPT : lane / RPT + 1);
+    uint32_t snd_off[2];                                              // source offset in the buffer, rows of the first / second half
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const int r = r_lo + hf * (RPT / 2) + ((lane >> 1) & (RPT / 2 - 1));
+      snd_off[hf] = slc * L::KB_BYTES + r * 128 + (((2 * q + (lane & 1)) ^ (r & 7)) << 4);
+    }
+    const uint32_t snd_dst = sends ? mapa_shared(smem_u32(h_s), to) : 0u, snd_bar = sends ? mapa_shared(smem_u32(h_ready), to) : 0u;
+    int st = 0; uint32_t st_ph = 0;
+    for (int s = 0; s < p.T; ++s) {
+      // ih + bias of this step, before the accumulators are there
+      bool ok = mbar_wait(&ih_full[st], st_ph, abort_flag, ST_TIMEOUT_LSTM, 0x20, budget);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      float2 x[4][RPT / 2];
+      const uint8_t* ihb = ih_t + st * L::IH_BYTES;
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+#pragma unroll
+        for (int i = 0; i < RPT / 2; ++i) {
+          const float half = g == 2 ? 1.0f : 0.5f;
+          const float2 f = make_float2(__half2float(*reinterpret_cast<const __half*>(ihb + g * L::IH_GATE + (2 * i) * (LT_HS * 2))),
+                                       __half2float(*reinterpret_cast<const __half*>(ihb + g * L::IH_GATE + (2 * i + 1) * (LT_HS * 2))));
+          x[g][i] = __ffma2_rn(f, make_float2(half, half), make_float2(bi[g], bi[g]));
+        }
+      if (++st == LT_STAGES) { st = 0; st_ph ^= 1; }
+
+      ok = mbar_wait(mma_done, s & 1, abort_flag, ST_TIMEOUT_LSTM, 0x30, budget);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      tc_fence_after();
+      uint32_t acc[4][RPT];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) tmem_ld_32x32b(t_row + g * R, acc[g]);
+      tmem_ld_wait(acc[0], acc[1], acc[2], acc[3]);
+      uint8_t* dst = own + (s & 1) * L::HBUF;
+      float2 hv[RPT / 2];
+      uint32_t h8[RPT / 2];
+      // half of this thread's rows at a time, so that the first half is on its way while the second is computed
+      constexpr int PAIRS = RPT / 4;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+        for (int i = hf * PAIRS; i < (hf + 1) * PAIRS; ++i) {
+          float2 t[4];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            const float2 pre = __ffma2_rn(make_float2(__uint_as_float(acc[g][2 * i]), __uint_as_float(acc[g][2 * i + 1])),
+                                          make_float2(sc[g], sc[g]), x[g][i]);
+            t[g] = make_float2(tanh_f(pre.x), tanh_f(pre.y));
+            if (g != 2) t[g] = __ffma2_rn(make_float2(0.5f, 0.5f), t[g], make_float2(0.5f, 0.5f));
           }
-          for (int ks = 0; ks < ksteps; ++ks) {
-            if (ks == 0) { tc_fence_after(); LPROF2(1, 4 * hf + 1); }
-            umma_f8(tmem_base + hf * LSTM_NCOL, a_desc + (uint64_t)(ks * (2 * L64_CHUNK >> 4)),
-                    b_base + (uint64_t)((ks >> 2) * (LSTM_KB_BYTES >> 4) + 2 * (ks & 3)), idesc, ks != 0);
-          }
-          if (!ok) break;
-          LPROF2(1, 4 * hf + 2);
-          umma_commit(&mma_done[hf]);
-          // every slice's piece of h_{s-1} is here, our own included, and that one was sent after the compute warps'
-          // barrier of step s - 1: the ih tile of step s - 1 has been consumed and its buffer can take step s + 1
-          if (s > 0 && s + 1 < p.T) issue_ih(hf, s + 1);
-          LPROF2(1, 4 * hf + 3);
+          const float2 cn = __ffma2_rn(t[1], make_float2(c[2 * i], c[2 * i + 1]), __fmul2_rn(t[0], t[2]));
+          hv[i] = __fmul2_rn(t[3], make_float2(tanh_f(cn.x), tanh_f(cn.y)));
+          const float2 cr = __half22float2(__float22half2_rn(cn));        // the cell state is carried in fp16
+          c[2 * i] = cr.x; c[2 * i + 1] = cr.y;
+          h8[i] = __nv_cvt_float2_to_fp8x2(__fmul2_rn(hv[i], make_float2(448.f, 448.f)), __NV_SATFINITE, __NV_E4M3);
+          if (!hid_ok || 2 * i >= rows_live) h8[i] = 0u;
+          else if (2 * i + 1 >= rows_live) h8[i] &= 0xffu;
+          const int r = r_lo + 2 * i;
+          dst[r * 128 + ((ck ^ (r & 7)) << 4)] = (uint8_t)h8[i];
+          dst[(r + 1) * 128 + ((ck ^ ((r + 1) & 7)) << 4)] = (uint8_t)(h8[i] >> 8);
+        }
+        if (hf == 1) { fence_proxy_async_smem(); tc_fence_before(); }      // the stores above before the MMAs read them
+        __syncwarp();
+        if (hf == 1 && lane == 0) mbar_arrive(&own_ready[s & 1]);
+        if (sends && s + 1 < p.T) {
+          const uint32_t off = (s & 1) * L::HBUF + snd_off[hf];
+          st_async_v4(snd_dst + off, *reinterpret_cast<const uint4*>(h_s + off), snd_bar + 8 * (s & 1));
         }
       }
-      if (!ok) abort_flag.set(1);
-    }
-  } else if (warp == 9) {
-    // ------------------------------ send warp: the all-gather of h through distributed shared memory ------------------------------
-    // One bulk copy per destination CTA (lane = destination rank), issued when the compute warps have staged the piece;
-    // its bytes are counted by the destination's barrier of that half and buffer.  A copy costs the SM about 220 clocks,
-    // one after the other whichever threads issue them: twelve are ~2700 clocks, which no compute warp pays here and
-    // which pass while the other half is computed.
-    for (int s = 0; s + 1 < p.T; ++s) {
-      bool ok = true;
-      for (int hf = 0; hf < halves; ++hf) {
-        const int ib = 2 * hf + (s & 1);
-        ok = mbar_wait(&staged[hf], s & 1, abort_flag, ST_TIMEOUT_LSTM, 0x60, budget);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        if (lane < p.slices) {
-          const uint32_t dst = mapa_shared(smem_u32(h_s + ib * L64_HBUF + slc * L64_PIECE), (uint32_t)lane);
-          bulk_copy_to_cluster(dst, stg_s + ib * L64_PIECE, L64_PIECE, mapa_shared(smem_u32(&h_ready[ib]), (uint32_t)lane));
-        }
-      }
-      if (!ok) break;
-    }
-  } else {
-    // ------------------------------ compute warps: the halves take turns ------------------------------
-    bool ok = true;
-    for (int s = 0; ok && s < p.T; ++s) {
-      for (int hf = 0; hf < halves; ++hf) {
-        if (tid == 0) LPROF2(0, 4 * hf + 0);
-        const int ib = 2 * hf + (s & 1);
-        bool mine = mbar_wait(&ih_full[ib], (s >> 1) & 1, abort_flag, ST_TIMEOUT_LSTM, 0x20, budget) &&
-                    mbar_wait(&mma_done[hf], s & 1, abort_flag, ST_TIMEOUT_LSTM, 0x30, budget);
-        mine = __all_sync(0xffffffffu, mine);
-        uint8_t* stg = stg_s + ib * L64_PIECE;
-        uint8_t* h16_s = h16_base + (halves == 2 ? hf : (s & 1)) * L64_H16_BYTES;
-        if (tid == 0) LPROF2(0, 4 * hf + 1);
-        if (mine) {
-          tc_fence_after();
-          uint32_t acc[4][8];
-          const uint32_t t_row = tmem_base + hf * LSTM_NCOL + ((uint32_t)(q * 32) << 16);
+      // the layer's outputs, off the critical path: 32 (E4M3) / 64 (fp16) contiguous bytes per warp and row
+      if (hid_ok) {
+        const size_t o = ((size_t)step_t(s) * B + row0 + r_lo) * H + hid;
+        if (p.h8_out) {
 #pragma unroll
-          for (int g = 0; g < 4; ++g) tmem_ld_16x256b_x2(t_row + g * LSTM_HS + hh * 16, acc[g]);
-          tmem_ld_wait(acc[0], acc[1], acc[2], acc[3]);
-          const uint8_t* ihb = ih_s + ib * L64_IH_BYTES;
-          float hv[8];
-#pragma unroll
-          for (int kr = 0; kr < 4; ++kr) {              // (k, rowsel): two adjacent hidden units of one row
-            const int k = kr >> 1, rs = kr & 1;
-            float pre[4][2];
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const float2 f = __half22float2(*reinterpret_cast<const __half2*>(ihb + g * L64_IH_GATE + ih_off[kr]));
-              pre[g][0] = fmaf(__uint_as_float(acc[g][4 * k + 2 * rs + 0]), sc2[g][k].x, f.x + bi2[g][k].x);
-              pre[g][1] = fmaf(__uint_as_float(acc[g][4 * k + 2 * rs + 1]), sc2[g][k].y, f.y + bi2[g][k].y);
-            }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const int i = 4 * k + 2 * rs + j;
-              const float ig = sigmoid_f(pre[0][j]), fg = sigmoid_f(pre[1][j]), gg = tanh_f(pre[2][j]), og = sigmoid_f(pre[3][j]);
-              const float cprev = hf ? c[1][i] : c[0][i];
-              const float cn = fmaf(fg, cprev, ig * gg);
-              hv[i] = og * tanh_f(cn);
-              const float cr = __half2float(__float2half_rn(cn));       // the cell state is carried in fp16
-              if (hf) c[1][i] = cr; else c[0][i] = cr;
-            }
-          }
-          // stage this thread's bytes of the CTA's piece: chunk hh, 2 bytes per (k, rowsel); rows past the batch as zeros
-#pragma unroll
-          for (int kr = 0; kr < 4; ++kr) {
-            const int k = kr >> 1, rs = kr & 1, i = 4 * k + 2 * rs;
-            const int r = ra + rs * 8;
-            const bool live = row0 + hf * L64_ROWS + r < B;
-            const uint32_t b2 = live ? (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(hv[i] * 448.f, hv[i + 1] * 448.f), __NV_SATFINITE, __NV_E4M3) : 0u;
-            *reinterpret_cast<uint16_t*>(stg + hh * L64_CHUNK + r * 16 + 8 * k + 2 * (lane & 3)) = (uint16_t)b2;
-            if (p.h_out)    // fp16 image: rows of 64 bytes, 16-byte pieces XOR-swizzled by the row pair like the ih boxes
-              *reinterpret_cast<uint32_t*>(h16_s + r * 64 + (((2 * hh + k) ^ ((r >> 1) & 3)) << 4) + 4 * (lane & 3)) = pack_half2(hv[i], hv[i + 1]);
-          }
-          fence_proxy_async_smem();                     // the staging stores before the bulk copies read them
-        }
-        tc_fence_before();
-        if (tid == 0) LPROF2(0, 4 * hf + 2);
-        ok = named_barrier_and(1, L2_COMPUTE, mine) != 0;    // all compute warps go on, or all leave, together
-        if (tid == 0) LPROF2(0, 4 * hf + 3);
-        if (!ok) break;
-        if (tid == 0 && s + 1 < p.T) mbar_arrive(&staged[hf]);   // the send warp takes it from here
-        // the layer's outputs, from the staged images: whole 32-byte (E4M3) / 64-byte (fp16) runs per row
-        const size_t trow = (size_t)step_t(s) * B + row0 + hf * L64_ROWS;
-        const int rows_live = B - (row0 + hf * L64_ROWS);
-        if (p.h8_out && tid >= 128) {                   // (the upper compute warps: the lower ones issue the sends)
-          const int r = (tid - 128) >> 1, cch = tid & 1;
-          if (r < rows_live)
-            *reinterpret_cast<uint4*>(p.h8_out + (trow + r) * H + hid0 + 16 * cch) = *reinterpret_cast<const uint4*>(stg + cch * L64_CHUNK + r * 16);
+          for (int i = 0; i < RPT; ++i)
+            if (i < rows_live) p.h8_out[o + (size_t)i * H] = (uint8_t)(h8[i >> 1] >> (8 * (i & 1)));
         }
         if (p.h_out) {
-          const int r = tid >> 2, pc = tid & 3;
-          if (r < rows_live)
-            *reinterpret_cast<uint4*>(p.h_out + (trow + r) * H + hid0 + 8 * pc) =
-                *reinterpret_cast<const uint4*>(h16_s + r * 64 + ((pc ^ ((r >> 1) & 3)) << 4));
+#pragma unroll
+          for (int i = 0; i < RPT; ++i)
+            if (i < rows_live) p.h_out[o + (size_t)i * H] = __float2half_rn((i & 1) ? hv[i >> 1].y : hv[i >> 1].x);
         }
       }
     }
-    if (p.c_last) {
+    if (p.c_last && hid_ok) {
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf)
+      for (int i = 0; i < RPT; ++i)
+        if (i < rows_live) p.c_last[(long long)(row0 + r_lo + i) * H + hid] = __float2half_rn(c[i]);
+    }
+  } else {
+    // ------------------------------ MMA issue, one gate per warp ------------------------------
+    if (lane == 0) {
+      const int g = warp - CW;
+      constexpr uint32_t idesc = umma_idesc(1, 0, 0, LT_HS, R);
+      const uint32_t d = tmem_base + LT_ACC_COL + g * R;
+      const uint32_t a0 = tmem_base + g * LT_TMEM_KB * 32;
+      const uint64_t b_base[2] = {umma_smem_desc_sw128(smem_u32(h_s)), umma_smem_desc_sw128(smem_u32(h_s + L::HBUF))};
+      const uint64_t a_smem = umma_smem_desc_sw128(smem_u32(w_s + g * LSTM_KB_BYTES));
+      const int ksteps = H >> 5;                   // 32 bytes of K per MMA
+      bool ok = rank_ok;
+      int st = 0;
+      if (ok && p.slices > LT_TMEM_KB) ok = mbar_wait(w_full, 0, abort_flag, ST_TIMEOUT_LSTM, 0x10, budget);
+      // The loop exists once per (row group size, rank): with every descriptor offset a constant of straight-line code an
+      // MMA costs this thread 69 clocks, with offsets computed at run time 120 to 170.
+      auto run = [&](auto slices_tag, auto rank_tag) {
+        constexpr int SLICES = decltype(slices_tag)::value, RANK = decltype(rank_tag)::value;
+        for (int s = 0; s < p.T; ++s) {
+          const int hb = (s + 1) & 1;              // h_{s-1}
+          const uint32_t ph = (uint32_t)((s - 1) >> 1) & 1u;
+          // (the accumulators may be overwritten and this CTA's piece read once every gate warp has reported)
+          if (s > 0 && !mbar_wait(&own_ready[hb], ph, abort_flag, ST_TIMEOUT_LSTM, 0x40, budget)) return false;
+          tc_fence_after();
+          const uint64_t b = hb ? b_base[1] : b_base[0];
+          // K blocks in the order RANK, RANK + 1, ..., wrapping: this CTA's own piece of h is here first
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = row0 + hf * L64_ROWS + cell_row(i);
-          if (hf < halves && row < B) p.c_last[(long long)row * H + hid0 + cell_u(i)] = __float2half_rn(c[hf][i]);
+          for (int n = 0; n < SLICES; ++n) {
+            const int kb = (RANK + n) % SLICES;
+            if (n == 1 && s > 0) {                 // the other CTAs' pieces
+              if (!mbar_wait_cluster(&h_ready[hb], ph, abort_flag, ST_TIMEOUT_LSTM, 0x41, budget)) return false;
+              if (g == 0 && s + 2 < p.T) mbar_arrive_expect_tx(&h_ready[hb], peer_bytes);   // its next use: h_{s+1}, read by step s + 2
+              fence_proxy_async_smem();            // the peers' stores before the MMAs read them
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              if (kb == SLICES - 1 && 4 * kb + k >= ksteps) break;
+              const uint64_t bd = b + (uint64_t)(kb * (L::KB_BYTES >> 4) + 2 * k);
+              if (kb < LT_TMEM_KB) umma_f8_ta(d, a0 + kb * 32 + k * 8, bd, idesc, (n | k) != 0);
+              else umma_f8(d, a_smem + 2 * k, bd, idesc, (n | k) != 0);
+            }
+          }
+          umma_commit(mma_done);
+          // the gate warps have read the ih tile of step s - 1 (their reports above came after that): its stage is free
+          if (g == 3 && s > 0) {
+            if (s - 1 + LT_STAGES < p.T) issue_ih(s - 1 + LT_STAGES, st);
+            if (++st == LT_STAGES) st = 0;
+          }
         }
+        return true;
+      };
+      auto run_rank = [&](auto slices_tag) {
+        constexpr int SLICES = decltype(slices_tag)::value;
+        if constexpr (SLICES > 3) if (slc == 3) return run(slices_tag, std::integral_constant<int, 3>{});
+        if constexpr (SLICES > 2) if (slc == 2) return run(slices_tag, std::integral_constant<int, 2>{});
+        if constexpr (SLICES > 1) if (slc == 1) return run(slices_tag, std::integral_constant<int, 1>{});
+        return run(slices_tag, std::integral_constant<int, 0>{});
+      };
+      if (ok) {
+        if (p.slices == 1) ok = run_rank(std::integral_constant<int, 1>{});
+        else if (p.slices == 2) ok = run_rank(std::integral_constant<int, 2>{});
+        else if (p.slices == 3) ok = run_rank(std::integral_constant<int, 3>{});
+        else ok = run_rank(std::integral_constant<int, 4>{});
+      }
+      if (!ok) {                                   // loads in flight land before the CTA exits
+        abort_flag.set(1);
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) { }
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) { tc_fence_after(); tmem_dealloc(tmem_base, 2 * LSTM_NCOL); }
-  cluster_sync_all();                    // nobody leaves while another CTA of the cluster may still store into it
+  if (warp == CW) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+  cluster_sync_all();                              // nobody leaves while another CTA of the cluster may still copy into it
 }
+
 
 // ---- host -------------------------------------------------------------------------------------------------
 size_t lstm_scratch_bytes(long long B, int H) {
   const size_t hbuf = ((size_t)2 * B * H + 255) & ~(size_t)255;
   const size_t flags = (size_t)((B + LSTM_ROWS - 1) / LSTM_ROWS) * (H / LSTM_HS) * sizeof(unsigned int);
   return hbuf + ((flags + 255) & ~(size_t)255);
+}
+
+using LtKernel = void (*)(const CUtensorMap, const CUtensorMap, const uint8_t*, long long, const LstmParams);
+// The forms of the transposed kernel: batch rows per group, and what a step costs (B200, us at H = 128 / 384 / 512).
+//   8 rows   0.72 / 1.09 / -      12 rows   0.90 / 1.27 / -      16 rows   1.07 / 1.38 / 1.83      32 rows   1.77 / 2.21 / 2.68
+struct LtForm { int rows, threads, smem[LT_MAX_SLICES + 1], cost; LtKernel kernel; };
+template <int R, int G, int CW>
+static constexpr LtForm lt_make_form(int cost) {
+  LtForm f{G, 32 * (CW + 4), {}, cost, lstm_tmem_kernel<R, G, CW>};
+  // (at least 120 KiB: one CTA per SM, it takes all of tensor memory)
+  for (int n = 1; n <= LT_MAX_SLICES; ++n) f.smem[n] = LtSmem<R, G>::bytes(n) > 120 * 1024 ? LtSmem<R, G>::bytes(n) : 120 * 1024;
+  return f;
+}
+constexpr int LT_FORMS = 4;
+static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 8, 8>(10), lt_make_form<16, 12, 12>(12), lt_make_form<16, 16, 8>(13),
+                                          lt_make_form<32, 32, 16>(21)};
+
+static cudaLaunchConfig_t lt_config(const LtForm& f, int slices, long long groups, cudaStream_t st, cudaLaunchAttribute* attr) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = slices; attr->val.clusterDim.y = 1; attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(groups * slices)); cfg.blockDim = dim3(f.threads);
+  cfg.dynamicSmemBytes = f.smem[slices]; cfg.stream = st;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Row groups (clusters) of a form that can be resident at once on device `dev`; 0 = cannot run there.  Asked once.
+static int lt_capacity(int form, int slices, int dev) {
+  static std::atomic<int> cap[LT_FORMS][64][LT_MAX_SLICES + 1];
+  std::atomic<int>& slot = cap[form][dev][slices];
+  int c = slot.load(std::memory_order_acquire);
+  if (c == 0) {
+    const LtForm& f = kLtForms[form];
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = lt_config(f, slices, 1, nullptr, &attr);
+    // (the attribute is per kernel: it is set to what the largest row group needs)
+    cudaError_t e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem[LT_MAX_SLICES]);
+    int n = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, f.kernel, &cfg);
+    (void)cudaGetLastError();
+    c = e == cudaSuccess && n > 0 ? n : -1;
+    if (getenv("GSB200_LSTM_VERBOSE") || c < 0)
+      fprintf(stderr, "gigaslop_b200: LSTM, groups of %d rows on clusters of %d CTAs: %d can be resident (%s)\n", f.rows, slices, n, cudaGetErrorName(e));
+    slot.store(c, std::memory_order_release);
+  }
+  return c > 0 ? c : 0;
+}
+
+// The form with the least waves x cost, row groups limited to `max_ctas` CTAs at a time (0 = the whole GPU); -1 = none.
+// Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows (43 groups,
+// 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (1.12 us per step and 512 rows; 12 rows in two
+// waves 1.28).
+static int lt_choose(long long B, int H, int dev, int max_ctas) {
+  const int slices = (H + LT_HS - 1) / LT_HS;
+  int best = -1;
+  long long best_cost = 0;
+  for (int i = 0; i < LT_FORMS; ++i) {
+    int cap = lt_capacity(i, slices, dev);
+    if (cap > 0 && max_ctas > 0 && cap > max_ctas / slices) cap = max_ctas / slices > 0 ? max_ctas / slices : 1;
+    if (cap <= 0) continue;
+    const long long groups = (B + kLtForms[i].rows - 1) / kLtForms[i].rows;
+    const long long cost = (groups + cap - 1) / cap * kLtForms[i].cost;
+    if (best < 0 || cost < best_cost) { best = i; best_cost = cost; }
+  }
+  return best;
+}
+
+static int32_t launch_lt(const LtForm& f, const LstmLayerArgs& a, LstmParams p, cudaStream_t st) {
+  p.slices = (a.H + LT_HS - 1) / LT_HS;
+  CUtensorMap tw, tih;
+  if (!tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w_hh, (uint64_t)4 * a.H, (uint64_t)a.H, (uint64_t)a.ld_w, 128, LT_HS,
+               CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !tmap_2d(&tih, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.ih, (uint64_t)a.T * a.B, (uint64_t)4 * a.H, (uint64_t)a.ld_ih, LT_HS,
+               f.rows, CU_TENSOR_MAP_SWIZZLE_NONE))
+    return GSB200_ERR_BAD_ARG;
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = lt_config(f, p.slices, (a.B + f.rows - 1) / f.rows, st, &attr);
+  return cuda_status(cudaLaunchKernelEx(&cfg, f.kernel, tw, tih, a.w_hh, a.ld_w, p), "lstm launch");
+}
+
+// In the environment, GSB200_LSTM_ROWS128=1 selects the older cluster kernel (one 128-row tile per CTA, a thread per row) and
+// GSB200_LSTM_NO_CLUSTER=1 the cooperative kernel with global scratch: bit 1 resp. bit 0.
+static int lstm_env() {
+  static std::atomic<int> env_state{-1};
+  int env = env_state.load(std::memory_order_relaxed);
+  if (env < 0) {
+    const char* e1 = getenv("GSB200_LSTM_NO_CLUSTER");
+    const char* e2 = getenv("GSB200_LSTM_ROWS128");
+    env = ((e1 && e1[0] == '1') ? 1 : 0) | ((e2 && e2[0] == '1') ? 2 : 0);
+    env_state.store(env, std::memory_order_relaxed);
+  }
+  return env;
+}
+
+// CTAs of one recurrence launch (what a projection beside it has to leave alone).
+static int lstm_layer_ctas(long long B, int H, int max_ctas) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int form = dev >= 0 && dev < 64 && lstm_env() == 0 ? lt_choose(B, H, dev, max_ctas) : -1;
+  if (form < 0) return (int)((B + LSTM_ROWS - 1) / LSTM_ROWS) * (H / LSTM_HS);
+  const int slices = (H + LT_HS - 1) / LT_HS, cap = lt_capacity(form, slices, dev);
+  const long long groups = (B + kLtForms[form].rows - 1) / kLtForms[form].rows;
+  return (int)(groups < cap ? groups : cap) * slices;
 }
 
 int32_t launch_lstm_layer(const LstmLayerArgs& a, void* scratch, size_t scratch_bytes, cudaStream_t st) {
@@ -880,91 +1021,72 @@ int32_t launch_lstm_layer(const LstmLayerArgs& a, void* scratch, size_t scratch_
   // is what bounds it, not the cap a caller may have set for the GEMM grids
   if (grid > sm_count_physical()) return GSB200_ERR_UNSUPPORTED;
 
-  static std::atomic<int> attr_done[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return GSB200_ERR_DEVICE;
-  if (!attr_done[dev].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(lstm_recurrent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LSTM_SMEM_BYTES);
-    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(lstm)");
-    attr_done[dev].store(1, std::memory_order_release);
-  }
+  if (a.ld_w < a.H || a.ld_w % 16 != 0) return GSB200_ERR_BAD_ARG;
 
   LstmParams p{};
   p.T = (int)a.T; p.B = (int)a.B; p.H = a.H; p.reverse = a.reverse ? 1 : 0;
   p.k_blocks = (a.H + 127) / 128; p.slices = slices;
   p.s_hh = a.s_hh; p.bias = a.bias; p.h0 = a.h0; p.c0 = a.c0;
   p.h_out = a.h_out; p.h8_out = a.h8_out; p.c_last = a.c_last;
+
+  // The transposed form; the others are for a device that cannot host its clusters, and for the environment switches.
+  const int env = lstm_env();
+  if (env == 0) {
+    const int form = lt_choose(a.B, a.H, dev, a.max_ctas);
+    if (form >= 0) return launch_lt(kLtForms[form], a, p, st);
+  }
+
+  static std::atomic<int> attr_done[64];
+  if (!attr_done[dev].load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(lstm_recurrent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LSTM_SMEM_BYTES);
+    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(lstm)");
+    attr_done[dev].store(1, std::memory_order_release);
+  }
   const size_t hbuf_bytes = ((size_t)2 * a.B * a.H + 255) & ~(size_t)255;
   p.hbuf = static_cast<uint8_t*>(scratch);
   p.flags = reinterpret_cast<unsigned int*>(static_cast<uint8_t*>(scratch) + hbuf_bytes);
 
-  if (a.ld_w < a.H || a.ld_w % 16 != 0) return GSB200_ERR_BAD_ARG;
   CUtensorMap tw, tih;
   if (!tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w_hh, (uint64_t)4 * a.H, (uint64_t)a.H, (uint64_t)a.ld_w, 128,
                LSTM_HS, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !tmap_2d(&tih, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.ih, (uint64_t)a.T * a.B, (uint64_t)4 * a.H,
                (uint64_t)a.ld_ih, LSTM_HS, LSTM_ROWS, CU_TENSOR_MAP_SWIZZLE_64B))
     return GSB200_ERR_BAD_ARG;
-  // Cluster forms first (h exchanged through distributed shared memory): H <= 384, the slices of a 128-row group in one
-  // cluster of H / 32 CTAs (more than 8 needs the non-portable cluster size).  The default runs a CTA's rows as two
-  // interleaved 64-row halves.  In the environment, GSB200_LSTM_ROWS128=1 selects the older cluster kernel (one
-  // 128-row tile per CTA, a thread per row) and GSB200_LSTM_NO_CLUSTER=1 the cooperative kernel with global scratch; a
-  // device that cannot host a cluster of that size falls back the same way.  What the device can host is asked once per
-  // (device, kernel, cluster size); a refusal is reported on stderr once and only switches off that combination.
-  static std::atomic<int> env_state{-1};
-  int env = env_state.load(std::memory_order_relaxed);
-  if (env < 0) {
-    const char* e1 = getenv("GSB200_LSTM_NO_CLUSTER");
-    const char* e2 = getenv("GSB200_LSTM_ROWS128");
-    env = ((e1 && e1[0] == '1') ? 1 : 0) | ((e2 && e2[0] == '1') ? 2 : 0);
-    env_state.store(env, std::memory_order_relaxed);
-  }
+  // Cluster kernel on 128-row tiles: H <= 384, the slices of a row group in one cluster of H / 32 CTAs (more than 8 needs
+  // the non-portable cluster size).  What the device can host is asked once per (device, cluster size).
   if (!(env & 1) && p.k_blocks <= LSTMC_MAX_KB && slices <= 16) {
-    static std::atomic<int> cluster_state[2][64][17];       // [64-row form][device][cluster size]: 0 unknown, 1 usable, -1 not
-    auto try_cluster = [&](bool rows64, int cgrid, const CUtensorMap& tih_k) -> bool {
-      void (*kern)(const CUtensorMap, const CUtensorMap, const LstmParams) = rows64 ? lstm_cluster2_kernel : lstm_cluster_kernel;
-      const int smem_bytes = rows64 ? L2_SMEM_BYTES : LSTMC_SMEM_BYTES;
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(cgrid); cfg.blockDim = dim3(rows64 ? L2_THREADS : LSTM_THREADS);
-      cfg.dynamicSmemBytes = smem_bytes; cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = slices; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr; cfg.numAttrs = 1;
-      std::atomic<int>& slot = cluster_state[rows64 ? 1 : 0][dev][slices];
-      int state = slot.load(std::memory_order_acquire);
-      if (state == 0) {
-        cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-        if (ce == cudaSuccess && slices > 8) ce = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        int max_clusters = 0;
-        if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg);
-        state = (ce == cudaSuccess && max_clusters >= 1) ? 1 : -1;
-        if (getenv("GSB200_LSTM_VERBOSE"))
-          fprintf(stderr, "gigaslop_b200: LSTM cluster form (%s), cluster of %d: %d clusters can be resident (%d CTAs asked)\n",
-                  rows64 ? "two 64-row halves" : "128-row tile", slices, max_clusters, cgrid);
-        if (state < 0) {
-          cudaGetLastError();
-          fprintf(stderr, "gigaslop_b200: device %d cannot host a cluster of %d LSTM CTAs (%s: %s)\n", dev, slices,
-                  rows64 ? "two 64-row halves" : "128-row tile", ce == cudaSuccess ? "no active cluster fits" : cudaGetErrorName(ce));
-        }
-        slot.store(state, std::memory_order_release);
+    static std::atomic<int> cluster_state[64][17];       // [device][cluster size]: 0 unknown, 1 usable, -1 not
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(LSTM_THREADS);
+    cfg.dynamicSmemBytes = LSTMC_SMEM_BYTES; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = slices; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    std::atomic<int>& slot = cluster_state[dev][slices];
+    int state = slot.load(std::memory_order_acquire);
+    if (state == 0) {
+      cudaError_t ce = cudaFuncSetAttribute(lstm_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LSTMC_SMEM_BYTES);
+      if (ce == cudaSuccess && slices > 8) ce = cudaFuncSetAttribute(lstm_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      int max_clusters = 0;
+      if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveClusters(&max_clusters, lstm_cluster_kernel, &cfg);
+      state = (ce == cudaSuccess && max_clusters >= 1) ? 1 : -1;
+      if (state < 0) {
+        cudaGetLastError();
+        fprintf(stderr, "gigaslop_b200: device %d cannot host a cluster of %d LSTM CTAs (%s)\n", dev, slices,
+                ce == cudaSuccess ? "no active cluster fits" : cudaGetErrorName(ce));
       }
-      if (state != 1) return false;
-      cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, tw, tih_k, p);
-      if (ce == cudaSuccess) return true;
+      slot.store(state, std::memory_order_release);
+    }
+    if (state == 1) {
+      cudaError_t ce = cudaLaunchKernelEx(&cfg, lstm_cluster_kernel, tw, tih, p);
+      if (ce == cudaSuccess) return GSB200_OK;
       cudaGetLastError();
       fprintf(stderr, "gigaslop_b200: cluster launch of the LSTM layer failed (%s); trying the next form\n", cudaGetErrorName(ce));
-      return false;
-    };
-    if (!(env & 2) && slices <= L2_MAX_SLICES) {          // two interleaved 64-row halves per CTA: ih boxes of 64 rows
-      CUtensorMap tih64;
-      if (tmap_2d(&tih64, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.ih, (uint64_t)a.T * a.B, (uint64_t)4 * a.H,
-                  (uint64_t)a.ld_ih, LSTM_HS, L64_ROWS, CU_TENSOR_MAP_SWIZZLE_64B) &&
-          try_cluster(true, grid, tih64))
-        return GSB200_OK;
     }
-    if (try_cluster(false, grid, tih)) return GSB200_OK;
   }
   // the cooperative kernel exchanges h through the scratch; its step counters start at zero
   cudaError_t e = cudaMemsetAsync(p.flags, 0, (size_t)grid * sizeof(unsigned int), st);
@@ -1050,10 +1172,15 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
   if ((long long)T * B > 0x7fffffffll) return GSB200_ERR_BAD_ARG;
   for (int l = 0; l < n_layers; ++l)
     if (!layers[l].w_ih || !layers[l].s_ih || !layers[l].w_hh || !layers[l].s_hh) return GSB200_ERR_BAD_ARG;
-  const bool overlap = aux != nullptr && aux != st && n_layers > 1;
-  int nb = overlap ? (time_blocks > 0 ? time_blocks : 8) : 1;
-  if (nb > T) nb = (int)T;
+  bool overlap = aux != nullptr && aux != st && n_layers > 1;
   if (ws_bytes < lstm_stack_workspace_bytes(T, B, H, overlap ? 1 : 0)) return GSB200_ERR_BAD_ARG;
+  // Left to choose (time_blocks = 0) the layers run one after the other, each on the whole GPU: the recurrence with fewer
+  // rows per CTA gains what hiding the projection would.  Five layers, T = 2000, B = 512, H = 384: 16.4 ms, in eight blocks
+  // with the recurrence on 96 SMs and the projection on 52 16.3; three layers, T = 1000: B = 512, H = 512 7.1 against
+  // 9.3 ms, H = 256 3.7 / 4.3, H = 128 2.73 / 2.80, B = 200, H = 384 3.75 / 3.89.
+  overlap = overlap && time_blocks > 0;
+  int nb = overlap ? time_blocks : 1;
+  if (nb > T) nb = (int)T;
   int32_t rc = ensure_device();
   if (rc != GSB200_OK) return rc;
 
@@ -1095,9 +1222,9 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
   rc = project(0, 0, T, st, 0);
   if (rc != GSB200_OK) return rc;
 
-  const int groups = (int)((B + LSTM_ROWS - 1) / LSTM_ROWS);
-  const int lstm_ctas = groups * (H / LSTM_HS);
-  int gemm_cap = sm_count_physical() - lstm_ctas;
+  // overlapped: the recurrence takes up to two thirds of the GPU, the projection what is left
+  const int max_ctas = overlap ? sm_count_physical() * 2 / 3 : 0;
+  int gemm_cap = sm_count_physical() - lstm_layer_ctas(B, H, max_ctas);
   if (gemm_cap < 8) gemm_cap = 8;
   cudaError_t ce = cudaSuccess;
   for (int l = 0; l < n_layers; ++l) {
@@ -1119,6 +1246,7 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
       a.h_out = last ? h_out + (size_t)t0 * B * H : nullptr;
       a.h8_out = h8_l + (size_t)t0 * B * H;
       a.c_last = k + 1 < nb ? cst[k & 1] : nullptr;
+      a.max_ctas = max_ctas;
       a.T = t1 - t0; a.B = B; a.H = H; a.reverse = rev ? 1 : 0;
       rc = launch_lstm_layer(a, scratch, scratch_bytes, st);
       if (rc != GSB200_OK) return rc;

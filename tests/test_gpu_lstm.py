@@ -167,3 +167,48 @@ def test_gemm_sm_cap_does_not_reject_the_lstm():
         assert L.gsb200_set_sm_limit(0) == 0
     assert torch.equal(got, want)
     assert g.device_status()[0] == 0
+
+
+# (T, B, H): every form of the transposed kernel and the edges of its tiles: 8, 12, 16 and 32 rows per group; a ragged last
+# group; fewer hidden units than a slice; a partial last slice; one to four CTAs per row group; one and two steps
+TMEM_SHAPES = [(1, 1, 32), (2, 9, 128), (9, 70, 128), (6, 17, 192), (5, 130, 416), (12, 512, 384), (7, 509, 384), (5, 512, 512),
+               (4, 500, 480), (6, 1024, 384), (5, 1000, 256)]
+
+
+def test_transposed_kernel_forms_match_the_cooperative_kernel(tmp_path):
+    """The recurrence picks rows per CTA by how many row groups the GPU holds at once; every form gives the bytes of the
+    cooperative kernel (forced in a child process through the environment)."""
+    import os
+    import subprocess
+    import sys
+    g = need_lib()
+    cases = []
+    for i, (T, B, H) in enumerate(TMEM_SHAPES):
+        gen = torch.Generator().manual_seed(900 + i)
+        L = make_layer(gen, H, 64)
+        cases.append(dict(T=T, B=B, reverse=i % 2 == 1, ih=(torch.randn(T * B, 4 * H, generator=gen) * 0.5).half(), W=L["W_hh"], s=L["s_hh"],
+                          b=L["b"] if i % 3 else None,
+                          h0=((torch.rand(B, H, generator=gen) * 2 - 1) * 448).to(torch.float8_e4m3fn) if i % 4 else None,
+                          c0=(torch.randn(B, H, generator=gen) * 0.3).half() if i % 4 else None))
+    inp, out = tmp_path / "in.pt", tmp_path / "out.pt"
+    torch.save(cases, inp)
+    code = (
+        "import sys, torch; sys.path.insert(0, %r); import gigaslop_b200 as g\n"
+        "cu = lambda t: None if t is None else t.cuda()\n"
+        "res = []\n"
+        "for d in torch.load(%r):\n"
+        "    r = g.lstm_layer(cu(d['ih']), cu(d['W']), cu(d['s']), d['T'], d['B'], bias=cu(d['b']), reverse=d['reverse'], h0=cu(d['h0']),\n"
+        "                     c0=cu(d['c0']), want_c=True)\n"
+        "    res.append([t.cpu().view(torch.uint8) for t in r])\n"
+        "torch.save(res, %r)\n"
+    ) % (os.path.dirname(os.path.dirname(os.path.abspath(__file__))), str(inp), str(out))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, GSB200_LSTM_NO_CLUSTER="1"), capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    cu = lambda t: None if t is None else t.cuda()
+    for d, want, shape in zip(cases, torch.load(out), TMEM_SHAPES):
+        got = g.lstm_layer(cu(d["ih"]), cu(d["W"]), cu(d["s"]), d["T"], d["B"], bias=cu(d["b"]), reverse=d["reverse"],
+                           h0=cu(d["h0"]), c0=cu(d["c0"]), want_c=True)
+        for a, b, what in zip(got, want, ("h fp16", "h e4m3", "c")):
+            assert torch.equal(a.cpu().view(torch.uint8), b), f"{what} at {shape}"
+    assert g.device_status()[0] == 0
