@@ -65,11 +65,19 @@ class LstmLayer(C.Structure):
 
 
 _lib = None
+native = None       # the native call path (csrc/binding.cpp), loaded and bound with the library
+
+# the entry points the native call path uses, in the order of its `Entry`
+NATIVE_ENTRIES = ["gsb200_ptq_int8", "gsb200_ptq_fp8", "gsb200_ptq_mxfp8", "gsb200_gemm_i8_f16", "gsb200_gemm_fp8_f16",
+                  "gsb200_gemm_i8_rotary_f16", "gsb200_gemm_fp8_rotary_f16", "gsb200_dual_gemm_i8_silu_f16",
+                  "gsb200_dual_gemm_fp8_silu_f16", "gsb200_dual_gemm_fp8_silu_mxfp8", "gsb200_mx_tiled_scale_bytes",
+                  "gsb200_mx_scales_to_tiled", "gsb200_gemm_mxfp8_f16", "gsb200_dual_gemm_mxfp8_silu_f16",
+                  "gsb200_fac_gemm_fp8_f16", "gsb200_factored_lstm_step"]
 
 
 def lib():
     """The loaded library (loads on first use; raises if it was never built)."""
-    global _lib
+    global _lib, native
     if _lib is None:
         if not os.path.exists(LIB_PATH):
             raise RuntimeError(
@@ -80,6 +88,14 @@ def lib():
             fn = getattr(handle, name)      # AttributeError if the symbol is not exported
             fn.restype = res
             fn.argtypes = args
+        import torch  # noqa: F401  (the extension links against the libraries torch has loaded)
+        try:
+            from . import _native
+        except ImportError as e:
+            raise RuntimeError("gigaslop_b200/_native.so is missing or does not load: build it with "
+                               "`python -m gigaslop_b200.build`") from e
+        _native.bind([C.cast(getattr(handle, n), C.c_void_p).value for n in NATIVE_ENTRIES])
+        native = _native
         _lib = handle
     return _lib
 

@@ -1,4 +1,4 @@
-"""Build recipe for libgigaslop_b200.so (nvcc, sm_100a only, in-tree output)."""
+"""Build recipe for libgigaslop_b200.so (nvcc, sm_100a only) and _native.so (g++), both in-tree."""
 import os
 import shutil
 import subprocess
@@ -8,6 +8,8 @@ ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libgigaslop_b200.so")
 PTXAS_LOG = os.path.join(PKG, "libgigaslop_b200.ptxas.txt")    # ptxas -v of the last build: registers and spills per kernel
 SRC = os.path.join(PKG, "csrc", "lib.cu")
+NATIVE = os.path.join(PKG, "_native.so")                       # native call path of the Python operators
+NATIVE_SRC = os.path.join(PKG, "csrc", "binding.cpp")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "-lineinfo",
               "-shared", "-Xcompiler", "-fPIC", "-Xptxas=-v"]
 
@@ -22,7 +24,7 @@ def _nvcc():
 def sources():
     d = os.path.join(PKG, "csrc")
     inc = os.path.join(ROOT, "include", "gigaslop_b200")
-    out = [os.path.join(d, f) for f in sorted(os.listdir(d))]
+    out = [os.path.join(d, f) for f in sorted(os.listdir(d)) if not f.endswith(".cpp")]
     for base, _, files in os.walk(inc):
         out += [os.path.join(base, f) for f in files]
     return out
@@ -40,6 +42,8 @@ def build(force=False, verbose=False, defines=(), out=None):
     spill bytes per kernel) is kept beside the library; ``kernel_resources()`` parses it.  ``defines`` / ``out``
     build a variant (``-DGSB200_DIAG`` for the tuning diagnostics) somewhere else."""
     target = out or LIB
+    if out is None:
+        build_native(force)
     if out is None and not force and not is_stale():
         return LIB
     cmd = [_nvcc(), *NVCC_FLAGS, *["-D" + d for d in defines], "-I" + os.path.join(ROOT, "include"), "-o", target, SRC]
@@ -51,6 +55,26 @@ def build(force=False, verbose=False, defines=(), out=None):
     if verbose:
         print(r.stdout)
     return target
+
+
+def build_native(force=False):
+    """Compile _native.so (CPython extension on torch's C++ headers) if missing or older than its sources."""
+    deps = [NATIVE_SRC, os.path.join(ROOT, "include", "gigaslop_b200", "gigaslop_b200.h")]
+    if not force and os.path.exists(NATIVE) and all(os.path.getmtime(f) <= os.path.getmtime(NATIVE) for f in deps):
+        return NATIVE
+    import sysconfig
+    import torch
+    t = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = [sysconfig.get_paths()["include"], os.path.join(ROOT, "include"), os.path.join(t, "include"),
+           os.path.join(t, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *["-I" + i for i in inc], "-o", NATIVE, NATIVE_SRC,
+           "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("compiling the native binding failed:\n" + r.stdout[-4000:])
+    return NATIVE
 
 
 def kernel_resources(log=None):

@@ -3,6 +3,11 @@ and streams; every byte of compute happens in libgigaslop_b200.so.
 
 Function names and argument meaning follow the reference's host helpers
 (``quantize_tensor``, ``fp8_quantize_per_token``) and kernels.
+
+An operator first offers the call to the native path (``_lib.native``, csrc/binding.cpp), which takes it when every
+argument is a plain CUDA tensor of the current device that passes the operator's checks, and answers None otherwise;
+then the ``_checked_*`` function of the same operator decides: it raises what is wrong with the arguments, or makes the
+call through ctypes.
 """
 import functools
 
@@ -66,10 +71,19 @@ def _dt(t):
     raise TypeError("activations must be float16 or float32")
 
 
-@_on_device
 def quantize_tensor(t, dim=-1, out=None, out_scale=None):
     """Per-row symmetric absmax INT8 quantiser; same contract as the reference's
     ``quantize_tensor`` (cute/bench_quant_i8.py:15-31): returns (int8 [M,K], fp32 dequant scale [M])."""
+    n = _lib.native
+    if n is not None and (dim == -1 or dim == 1):
+        r = n.quantize(0, t, out, out_scale)
+        if r is not None:
+            return r
+    return _checked_quantize_tensor(t, dim, out, out_scale)
+
+
+@_on_device
+def _checked_quantize_tensor(t, dim, out, out_scale):
     if dim not in (-1, t.dim() - 1):
         raise ValueError("only per-row (last-dim) quantisation is on the hot path")
     _need_cuda(t)
@@ -82,10 +96,19 @@ def quantize_tensor(t, dim=-1, out=None, out_scale=None):
     return q, s
 
 
-@_on_device
 def fp8_quantize_per_token(x, torch_formulation=True, out=None, out_scale=None):
     """Per-row E4M3 quantiser (fly/rdna_fp8_preshuffle_gemm.py:57-70); ``torch_formulation=False``
     selects the device-kernel arithmetic of fly/rdna_fp8_per_token_quantize.py."""
+    n = _lib.native
+    if n is not None:
+        r = n.quantize(2 if torch_formulation else 1, x, out, out_scale)
+        if r is not None:
+            return r
+    return _checked_fp8_quantize_per_token(x, torch_formulation, out, out_scale)
+
+
+@_on_device
+def _checked_fp8_quantize_per_token(x, torch_formulation, out, out_scale):
     _need_cuda(x)
     x = _rowmajor(x, "x")
     M, K = x.shape
@@ -129,15 +152,33 @@ def _gemm_f16(fn, name, A, B, scale_a, scale_b, out, flags, dtypes):
     return C
 
 
-@_on_device
 def gemm_i8(A, B, scale_a, scale_b, out=None, flags=0):
     """W8A8 GEMM with per-token x per-channel dequant to fp16 (cute/ampere_gemm_i8_quant_rmem.py)."""
+    n = _lib.native
+    if n is not None:
+        r = n.gemm(0, A, B, scale_a, scale_b, out, flags)
+        if r is not None:
+            return r
+    return _checked_gemm_i8(A, B, scale_a, scale_b, out, flags)
+
+
+@_on_device
+def _checked_gemm_i8(A, B, scale_a, scale_b, out, flags):
     return _gemm_f16(lib().gsb200_gemm_i8_f16, "gemm_i8", A, B, scale_a, scale_b, out, flags, _I8)
 
 
-@_on_device
 def gemm_fp8(A, B, scale_a, scale_b, out=None, flags=0):
     """FP8 GEMM, ``B`` K-major ``[N,K]`` (fly/rdna_fp8_preshuffle_gemm.py compile_fp8_gemm)."""
+    n = _lib.native
+    if n is not None:
+        r = n.gemm(1, A, B, scale_a, scale_b, out, flags)
+        if r is not None:
+            return r
+    return _checked_gemm_fp8(A, B, scale_a, scale_b, out, flags)
+
+
+@_on_device
+def _checked_gemm_fp8(A, B, scale_a, scale_b, out, flags):
     return _gemm_f16(lib().gsb200_gemm_fp8_f16, "gemm_fp8", A, B, scale_a, scale_b, out, flags, _F8)
 
 
@@ -156,10 +197,19 @@ def _rotary(fn, name, A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim,
     return C
 
 
-@_on_device
 def gemm_i8_rotary(A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim, rotary_dim, seqlen,
                    row_offset=0, out=None, flags=0):
     """QKV GEMM + rotary epilogue (cute/ampere_gemm_i8_rotary.py TensorOpGemmI8Rotary)."""
+    n = _lib.native
+    if n is not None:
+        r = n.rotary(0, A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags)
+        if r is not None:
+            return r
+    return _checked_gemm_i8_rotary(A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags)
+
+
+@_on_device
+def _checked_gemm_i8_rotary(A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags):
     return _rotary(lib().gsb200_gemm_i8_rotary_f16, "gemm_i8_rotary", A, B, scale_a, scale_b, sin_buf, cos_buf,
                    nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags, _I8)
 
@@ -191,10 +241,19 @@ def quantize_gemm_i8_rotary(x, B, scale_b, sin_buf, cos_buf, nhead, head_dim, ro
     return C
 
 
-@_on_device
 def gemm_fp8_rotary(A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim, rotary_dim, seqlen,
                     row_offset=0, out=None, flags=0):
     """FP8 QKV GEMM + rotary (fly/rdna_fp8_gemm_rotary.py compile_fp8_gemm_rotary)."""
+    n = _lib.native
+    if n is not None:
+        r = n.rotary(1, A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags)
+        if r is not None:
+            return r
+    return _checked_gemm_fp8_rotary(A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags)
+
+
+@_on_device
+def _checked_gemm_fp8_rotary(A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags):
     return _rotary(lib().gsb200_gemm_fp8_rotary_f16, "gemm_fp8_rotary", A, B, scale_a, scale_b, sin_buf, cos_buf,
                    nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags, _F8)
 
@@ -211,23 +270,50 @@ def _dual(fn, name, A, Bg, Bu, scale_a, sbg, sbu, out, flags, dtypes):
     return C
 
 
-@_on_device
 def dual_gemm_i8_silu(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out=None, flags=0):
     """``silu(A.Bg^T) * (A.Bu^T)`` (cute/ampere_dual_gemm_i8_silu.py TensorOpDualGemmI8Silu)."""
+    n = _lib.native
+    if n is not None:
+        r = n.dual(0, A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, flags)
+        if r is not None:
+            return r
+    return _checked_dual_gemm_i8_silu(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, flags)
+
+
+@_on_device
+def _checked_dual_gemm_i8_silu(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, flags):
     return _dual(lib().gsb200_dual_gemm_i8_silu_f16, "dual_gemm_i8_silu", A, B_gate, B_up, scale_a,
                  scale_b_gate, scale_b_up, out, flags, _I8)
 
 
-@_on_device
 def dual_gemm_fp8_silu(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out=None, flags=0):
     """FP8 SwiGLU dual GEMM (fly/rdna_fp8_dual_gemm_silu.py compile_fp8_dual_gemm_silu)."""
+    n = _lib.native
+    if n is not None:
+        r = n.dual(1, A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, flags)
+        if r is not None:
+            return r
+    return _checked_dual_gemm_fp8_silu(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, flags)
+
+
+@_on_device
+def _checked_dual_gemm_fp8_silu(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, flags):
     return _dual(lib().gsb200_dual_gemm_fp8_silu_f16, "dual_gemm_fp8_silu", A, B_gate, B_up, scale_a,
                  scale_b_gate, scale_b_up, out, flags, _F8)
 
 
-@_on_device
 def mxfp8_quantize(x, out=None, out_scale=None):
     """Activations [M,K] fp16/fp32 -> (float8_e4m3fn [M,K], uint8 E8M0 scales [M,K/32]); one scale per 32 elements."""
+    n = _lib.native
+    if n is not None:
+        r = n.quantize_mx(x, out, out_scale)
+        if r is not None:
+            return r
+    return _checked_mxfp8_quantize(x, out, out_scale)
+
+
+@_on_device
+def _checked_mxfp8_quantize(x, out, out_scale):
     _need_cuda(x)
     x = _rowmajor(x, "x")
     M, K = x.shape
@@ -238,10 +324,19 @@ def mxfp8_quantize(x, out=None, out_scale=None):
     return q, s
 
 
-@_on_device
 def dual_gemm_fp8_silu_mxfp8(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out=None, out_scale=None, flags=0):
     """FP8 SwiGLU dual GEMM emitting MXFP8 (elements + E8M0 scale per 32 output columns); the interface of
     fp8_dual_silu_mxfp8_wrapper (fly/export_fp8_dual_gemm_silu_mxfp8.py:206-236)."""
+    n = _lib.native
+    if n is not None:
+        r = n.dual_mx(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, out_scale, flags)
+        if r is not None:
+            return r
+    return _checked_dual_gemm_fp8_silu_mxfp8(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, out_scale, flags)
+
+
+@_on_device
+def _checked_dual_gemm_fp8_silu_mxfp8(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, out_scale, flags):
     M, N, K = _check_ab(A, B_gate, _F8)
     _check_ab(A, B_up, _F8)
     _need_cuda(scale_a, scale_b_gate, scale_b_up)
@@ -267,18 +362,26 @@ def gemm_f16(A, B, scale_a=None, scale_b=None, out=None, flags=0):
     return C
 
 
-@_on_device
 def fp8_down_proj(x_fp8, scale_x, dn_fp8_rc, scale_dn, out=None):
     """``x_down_f16[M,R] = (x_fp8 . dn_fp8^T) * sx[m] * s_dn`` with a single scalar weight scale
     (compile_fp8_down_proj, fly/rdna_fp8_factored_gemm.py:442-651); ``dn`` K-major ``[R, C]``."""
     return gemm_fp8(x_fp8, dn_fp8_rc, scale_x, scale_dn, out=out, flags=_lib.FLAG_SCALAR_SCALE_B)
 
 
-@_on_device
 def fp8_factored_gemm(x_fp8, scale_x, dn_fp8_rc, scale_dn, up_f16_nr, bias, out=None):
     """Hoisted low-rank input projection ``ih = f16(f16((x . dn^T) * sx * s_dn) . up^T + bias)`` in one call
     (compile_fp8_factored_gemm, fly/rdna_fp8_factored_gemm.py:86-435).  ``dn`` ``[R, C]`` E4M3 and ``up``
     ``[N, R]`` fp16, both K-major; the intermediate lives inside ``out`` between the two launches."""
+    n = _lib.native
+    if n is not None:
+        r = n.fac_gemm(x_fp8, scale_x, dn_fp8_rc, scale_dn, up_f16_nr, bias, out)
+        if r is not None:
+            return r
+    return _checked_fp8_factored_gemm(x_fp8, scale_x, dn_fp8_rc, scale_dn, up_f16_nr, bias, out)
+
+
+@_on_device
+def _checked_fp8_factored_gemm(x_fp8, scale_x, dn_fp8_rc, scale_dn, up_f16_nr, bias, out):
     _need_cuda(x_fp8, scale_x, dn_fp8_rc, scale_dn, up_f16_nr, bias)
     _rowmajor(x_fp8, "x"); _rowmajor(dn_fp8_rc, "dn"); _rowmajor(up_f16_nr, "up")
     if x_fp8.dtype != torch.float8_e4m3fn or dn_fp8_rc.dtype != torch.float8_e4m3fn or up_f16_nr.dtype != torch.float16:
@@ -296,10 +399,19 @@ def fp8_factored_gemm(x_fp8, scale_x, dn_fp8_rc, scale_dn, up_f16_nr, bias, out=
     return ih
 
 
-@_on_device
 def factored_lstm_step(h_fp8_out, c_inout, hh_down, up_hh, bias_hh, x_down, up_ih, bias_ih):
     """One step of the low-rank hard-gate LSTM cell; argument order of fp8_factored_lstm_wrapper
     (fly/export_fp8_factored_lstm.py:158-182).  ``up_hh`` ``[4H, K_hh]`` and ``up_ih`` ``[4H, R]`` fp16 K-major."""
+    n = _lib.native
+    if n is not None:
+        r = n.fac_step(h_fp8_out, c_inout, hh_down, up_hh, bias_hh, x_down, up_ih, bias_ih)
+        if r is not None:
+            return h_fp8_out, c_inout
+    return _checked_factored_lstm_step(h_fp8_out, c_inout, hh_down, up_hh, bias_hh, x_down, up_ih, bias_ih)
+
+
+@_on_device
+def _checked_factored_lstm_step(h_fp8_out, c_inout, hh_down, up_hh, bias_hh, x_down, up_ih, bias_ih):
     _need_cuda(h_fp8_out, c_inout, hh_down, up_hh, x_down, up_ih)
     B, K_hh = hh_down.shape
     H = up_hh.shape[0] // 4
@@ -314,9 +426,18 @@ def factored_lstm_step(h_fp8_out, c_inout, hh_down, up_hh, bias_hh, x_down, up_i
     return h_fp8_out, c_inout
 
 
-@_on_device
 def mx_scales_to_tiled(scales, K):
     """Row-major E8M0 scales ``[rows, K/32]`` -> the 128 x 4 tile order the block-scaled GEMMs take."""
+    n = _lib.native
+    if n is not None:
+        r = n.mx_tile(scales, K)
+        if r is not None:
+            return r
+    return _checked_mx_scales_to_tiled(scales, K)
+
+
+@_on_device
+def _checked_mx_scales_to_tiled(scales, K):
     _need_cuda(scales)
     rows = scales.shape[0]
     out = torch.empty(int(lib().gsb200_mx_tiled_scale_bytes(rows, K)), dtype=torch.uint8, device=scales.device)
@@ -325,9 +446,18 @@ def mx_scales_to_tiled(scales, K):
     return out
 
 
-@_on_device
 def gemm_mxfp8(A, sfa_tiled, B, sfb_tiled, out=None):
     """Block-scaled MXFP8 GEMM ``A[M,K] . B[N,K]^T`` (E8M0 scale per 32 K elements on both operands) -> fp16."""
+    n = _lib.native
+    if n is not None:
+        r = n.mx_gemm(A, sfa_tiled, B, sfb_tiled, out)
+        if r is not None:
+            return r
+    return _checked_gemm_mxfp8(A, sfa_tiled, B, sfb_tiled, out)
+
+
+@_on_device
+def _checked_gemm_mxfp8(A, sfa_tiled, B, sfb_tiled, out):
     M, N, K = _check_ab(A, B, _F8)
     C = out if out is not None else torch.empty((M, N), dtype=torch.float16, device=A.device)
     check(lib().gsb200_gemm_mxfp8_f16(A.data_ptr(), A.stride(0), sfa_tiled.data_ptr(), B.data_ptr(), B.stride(0),
@@ -335,9 +465,18 @@ def gemm_mxfp8(A, sfa_tiled, B, sfb_tiled, out=None):
     return C
 
 
-@_on_device
 def dual_gemm_mxfp8_silu(A, sfa_tiled, B_gate, B_up, sfb_gate_tiled, sfb_up_tiled, out=None):
     """Block-scaled MXFP8 SwiGLU dual GEMM ``silu(A.Bg^T) * (A.Bu^T)`` -> fp16."""
+    n = _lib.native
+    if n is not None:
+        r = n.mx_dual(A, sfa_tiled, B_gate, B_up, sfb_gate_tiled, sfb_up_tiled, out)
+        if r is not None:
+            return r
+    return _checked_dual_gemm_mxfp8_silu(A, sfa_tiled, B_gate, B_up, sfb_gate_tiled, sfb_up_tiled, out)
+
+
+@_on_device
+def _checked_dual_gemm_mxfp8_silu(A, sfa_tiled, B_gate, B_up, sfb_gate_tiled, sfb_up_tiled, out):
     M, N, K = _check_ab(A, B_gate, _F8)
     _check_ab(A, B_up, _F8)
     C = out if out is not None else torch.empty((M, N), dtype=torch.float16, device=A.device)

@@ -1,0 +1,104 @@
+"""The native call path of the operators (csrc/binding.cpp): it takes plain CUDA tensors only and leaves every other
+call to the Python function, and what it takes gives the bytes of the ctypes path."""
+import pytest
+import torch
+
+import oracle
+from util import need_lib
+
+
+def test_native_path_declines_what_is_not_plain():
+    from gigaslop_b200 import _lib
+    _lib.lib()
+    n = _lib.native
+    x = torch.zeros(4, 64, dtype=torch.float16)
+    w = torch.zeros(8, 64, dtype=torch.int8)
+    s = torch.zeros(8)
+    assert n.quantize(0, x, None, None) is None                  # CPU tensors
+    assert n.quantize(0, "x", None, None) is None and n.quantize(0, x) is None
+    assert n.gemm(0, w, w, s, s, None, 0) is None
+    assert n.gemm(0, w, w, s, s, None, 1 << 40) is None and n.gemm(0, w, w, s, s, None, 0.0) is None
+    assert n.quantize(0, torch.nn.Parameter(x), None, None) is None
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode():
+        assert n.quantize(0, torch.empty(4, 64, dtype=torch.float16, device="cuda"), None, None) is None
+    with pytest.raises(RuntimeError):
+        need_lib().quantize_tensor(x)
+
+
+@pytest.mark.gpu
+def test_native_path_gives_the_bytes_of_the_checked_path(monkeypatch):
+    g = need_lib()
+    from gigaslop_b200 import _lib
+    gen = torch.Generator().manual_seed(5)
+    M, K, nh = 77, 256, 4
+    x = torch.randn(M, K, generator=gen).half().cuda()
+    xs = torch.randn(M, 2 * K, generator=gen).half().cuda()[:, :K]             # strided rows
+    w = torch.randint(-127, 128, (3 * K, K), generator=gen, dtype=torch.int8).cuda()
+    w8 = ((torch.rand(3 * K, K, generator=gen) * 2 - 1) * 400).to(torch.float8_e4m3fn).cuda()
+    sw = (1e-3 + 1e-2 * torch.rand(3 * K, generator=gen)).cuda()
+    sin, cos = [t.cuda() for t in oracle.rope_tables(M, 32, 64)]
+    up = torch.randn(128, 64, generator=gen).half().cuda()
+    bias = torch.randn(128, generator=gen).cuda()
+    one = torch.full((1,), 2e-3, device="cuda")
+    H, R, B = 64, 64, 33
+    fac = lambda *shape: (torch.randn(*shape, generator=gen) * 0.2).half().cuda()
+    hh, uhh, xd, uih = fac(B, R), fac(4 * H, R), fac(B, R), fac(4 * H, R)
+    qi, si = g.quantize_tensor(x)
+    q8, s8 = g.fp8_quantize_per_token(x)
+    qm, sm = g.mxfp8_quantize(x)
+    wm, swm = g.mxfp8_quantize(torch.randn(3 * K, K, generator=gen).half().cuda())
+    swm = g.mx_scales_to_tiled(swm, K)
+    tm = g.mx_scales_to_tiled(sm, K)
+
+    def step():
+        h, c = torch.zeros(B, H, dtype=torch.uint8, device="cuda"), torch.zeros(B, H, device="cuda")
+        return g.factored_lstm_step(h, c, hh, uhh, None, xd, uih, bias[:1].expand(4 * H).contiguous())
+
+    buf = lambda *shape, dtype=torch.float16: torch.empty(*shape, dtype=dtype, device="cuda")
+    rope = (sin, cos, nh, 64, 64, M, 3)
+    calls = {
+        "quantize_tensor": lambda: g.quantize_tensor(xs), "quantize_tensor f32": lambda: g.quantize_tensor(x.float(), 1, buf(M, K, dtype=torch.int8)),
+        "fp8": lambda: g.fp8_quantize_per_token(xs), "fp8 kernel": lambda: g.fp8_quantize_per_token(x, False, out_scale=buf(M, dtype=torch.float32)),
+        "mxfp8": lambda: g.mxfp8_quantize(xs), "tile": lambda: g.mx_scales_to_tiled(sm, K),
+        "gemm_i8": lambda: g.gemm_i8(qi, w, si, sw), "gemm_i8 out": lambda: g.gemm_i8(qi, w, si, sw, buf(M, 4 * K)[:, :3 * K]),
+        "gemm_fp8": lambda: g.gemm_fp8(q8, w8, s8, sw), "down": lambda: g.fp8_down_proj(q8, s8, w8[:64], one),
+        "rotary i8": lambda: g.gemm_i8_rotary(qi, w, si, sw, *rope), "rotary fp8": lambda: g.gemm_fp8_rotary(q8, w8, s8, sw, *rope),
+        "silu i8": lambda: g.dual_gemm_i8_silu(qi, w[:K], w[K:2 * K], si, sw[:K], sw[K:2 * K]),
+        "silu fp8": lambda: g.dual_gemm_fp8_silu(q8, w8[:K], w8[K:2 * K], s8, sw[:K], sw[K:2 * K]),
+        "silu mx": lambda: g.dual_gemm_fp8_silu_mxfp8(q8, w8[:K], w8[K:2 * K], s8, sw[:K], sw[K:2 * K]),
+        "gemm mx": lambda: g.gemm_mxfp8(qm, tm, wm, swm), "dual mx": lambda: g.dual_gemm_mxfp8_silu(qm, tm, wm, wm, swm, swm),
+        "factored": lambda: g.fp8_factored_gemm(q8, s8, w8[:64], one, up, bias), "step": step,
+    }
+    flat = lambda r: [t.cpu().contiguous().view(torch.uint8) for t in (r if isinstance(r, tuple) else (r,))]
+    taken = []
+
+    class Spy:                                                   # every one of these calls is one the native path takes
+        def __getattr__(self, name):
+            fn = getattr(_lib_native, name)
+            return lambda *a: taken.append((name, r := fn(*a))) or r
+
+    _lib_native = _lib.native
+    monkeypatch.setattr(_lib, "native", Spy())
+    native = {k: flat(f()) for k, f in calls.items()}
+    assert len(taken) == len(calls) and all(r is not None for _, r in taken), [n for n, r in taken if r is None]
+    monkeypatch.setattr(_lib, "native", None)
+    for k, f in calls.items():
+        for a, b in zip(native[k], flat(f())):
+            assert torch.equal(a, b), k
+    # a view handed in as `out` comes back as the same object, on both paths
+    out = buf(M, 3 * K)
+    assert g.gemm_i8(qi, w, si, sw, out) is out
+    monkeypatch.undo()
+    assert g.gemm_i8(qi, w, si, sw, out) is out
+    # another stream: the launch goes to the stream that is current at the call
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        r = g.gemm_i8(qi, w, si, sw)
+    side.synchronize()
+    assert torch.equal(flat(r)[0], native["gemm_i8"][0])
+    with pytest.raises(ValueError):
+        g.gemm_i8(qi[:, ::2], w, si, sw)
+    with pytest.raises(TypeError):
+        g.gemm_fp8(qi, w, si, sw)
