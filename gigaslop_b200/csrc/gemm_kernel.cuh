@@ -122,7 +122,7 @@ struct GemmParams {
   int m_blocks, n_blocks, k_blocks;
   int n_groups;                // WRES: number of row-block groups (grid = n_groups * n_blocks)
   int m_major;                 // STREAM: a CTA walks all column blocks of a row block before the next (ARES always does)
-  int ares_split;              // ARES: CTAs that share each row block of the last, incomplete round (1 = no sharing)
+  int ares_split;              // ARES: shares that each row block of the last, incomplete round is cut into (1 = none)
   void* C;                     // output base (direct-store path and int32 output)
   uint8_t* out_scale;          // EPI_SILU_MX: E8M0 scales [M, N/32]
   long long ld_scale;          //              row stride of out_scale in bytes
@@ -229,20 +229,21 @@ struct TileWalk {
   int visit;       // row-block-major walks: how many row blocks this CTA has left behind
   // Row blocks cta, cta + grid, ... while whole rounds last.  The row blocks left over (fewer than CTAs) would
   // keep some SMs busy for a whole row block while the others idle: with the activation-stationary schedule each of
-  // them is shared by p.ares_split CTAs, which take consecutive column blocks of it (each loads the A block).
+  // them is cut into p.ares_split shares of consecutive column blocks (none empty; the host sees to that), which are
+  // dealt to the CTAs in turn (each loads the A block).
   __device__ __forceinline__ void set_visit(const GemmParams& p) {
     const int grid = ncta(), full = p.m_blocks / grid, rem = p.m_blocks - full * grid;
     m = p.m_blocks;                                   // nothing left unless one of the cases below applies
     n_lo = 0; n_hi = p.n_blocks;
     if (visit < full) {
       m = cta() + visit * grid;
-    } else if (visit == full && rem > 0) {
+    } else {
       const int S = (SCHED == SCHED_ARES && p.ares_split > 1) ? p.ares_split : 1;
       const int per = (p.n_blocks + S - 1) / S;
-      const int c = cta();
-      if (c < rem * S && (c % S) * per < p.n_blocks) {
-        m = full * grid + c / S;
-        n_lo = (c % S) * per;
+      const int u = cta() + (visit - full) * grid;
+      if (u < rem * S) {
+        m = full * grid + u / S;
+        n_lo = (u % S) * per;
         n_hi = n_lo + per < p.n_blocks ? n_lo + per : p.n_blocks;
       }
     }

@@ -102,3 +102,24 @@ def test_variant_setter_rejects_other_values():
     assert g.lib().gsb200_set_gemm_variant(16, 0) != 0
     assert g.lib().gsb200_set_gemm_variant(8, 2) != 0
     assert g.lib().gsb200_set_gemm_variant(-1, -1) == 0
+
+
+@pytest.mark.parametrize("head_dim,rotary_dim", [(64, 64), (128, 128), (128, 64), (64, 32)])
+@pytest.mark.parametrize("M,K", [(1, 512), (129, 512), (2300, 512), (12000, 512), (19100, 256), (333, 1024), (5000, 768)])
+def test_rotary_row_blocks_in_shares_give_the_same_bytes(head_dim, rotary_dim, M, K):
+    """A row block's column blocks may be dealt to several CTAs (few row blocks, or the last round of many): the bytes are
+    those of whole row blocks per CTA, which GSB200_FLAG_OWN_ROW_BLOCKS asks for."""
+    g = need_lib()
+    gen = torch.Generator().manual_seed(M + K + head_dim)
+    nhead = 512 // head_dim
+    N, seqlen = 3 * nhead * head_dim, 700
+    A = torch.randint(-127, 128, (M, K), generator=gen, dtype=torch.int8).cuda()
+    B = torch.randint(-127, 128, (N, K), generator=gen, dtype=torch.int8).cuda()
+    sa, sb = (1e-3 + 1e-2 * torch.rand(M, generator=gen)).cuda(), (1e-3 + 1e-2 * torch.rand(N, generator=gen)).cuda()
+    ang = torch.rand(seqlen, rotary_dim // 2, generator=gen) * 6.28
+    sn, cs = ang.sin().cuda(), ang.cos().cuda()
+    args = (A, B, sa, sb, sn, cs, nhead, head_dim, rotary_dim, seqlen, 55)
+    a, b = g.gemm_i8_rotary(*args), g.gemm_i8_rotary(*args, flags=8)
+    torch.cuda.synchronize()
+    assert torch.equal(a, b)
+    assert g.device_status()[0] == 0
