@@ -104,7 +104,7 @@ static cudaError_t set_attr() {
   cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<KIND, EPI, SCHED_STREAM>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES);
   if (e != cudaSuccess) return e;
-  constexpr int RES = (EPI == EPI_ROTARY || EPI == EPI_ROTARY_GEN || EPI == EPI_BIAS) ? SCHED_ARES : SCHED_WRES;
+  constexpr int RES = (EPI == EPI_ROTARY || EPI == EPI_ROTARY_GEN || EPI == EPI_ROTARY_HD || EPI == EPI_BIAS) ? SCHED_ARES : SCHED_WRES;
   return cudaFuncSetAttribute(gemm_tcgen05_kernel<KIND, EPI, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               GEMM_SMEM_BYTES);
 }
@@ -121,7 +121,7 @@ static cudaError_t set_attr() {
 //   shared-memory traffic per tile.
 template <int KIND, int EPI, bool PAIR, int EW>
 struct Variant {
-  static constexpr int RES = (EPI == EPI_ROTARY || EPI == EPI_ROTARY_GEN || EPI == EPI_BIAS) ? SCHED_ARES : SCHED_WRES;
+  static constexpr int RES = (EPI == EPI_ROTARY || EPI == EPI_ROTARY_GEN || EPI == EPI_ROTARY_HD || EPI == EPI_BIAS) ? SCHED_ARES : SCHED_WRES;
   static constexpr int THREADS = 32 * (FRONT_WARPS + EW);
   using Fn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
   static Fn kernel(bool resident) {
@@ -243,7 +243,8 @@ int32_t ensure_device() {
       set_attr<KIND_I8, EPI_I32>(),     set_attr<KIND_I8, EPI_DEQUANT>(), set_attr<KIND_I8, EPI_ROTARY>(),
       set_attr<KIND_I8, EPI_SILU>(),    set_attr<KIND_F8, EPI_DEQUANT>(), set_attr<KIND_F8, EPI_ROTARY>(),
       set_attr<KIND_F8, EPI_SILU>(),    set_attr<KIND_F8, EPI_SILU_MX>(), set_attr<KIND_F16, EPI_DEQUANT>(),
-      set_attr<KIND_F16, EPI_BIAS>(),   set_attr<KIND_I8, EPI_ROTARY_GEN>(), set_attr<KIND_F8, EPI_ROTARY_GEN>()};
+      set_attr<KIND_F16, EPI_BIAS>(),   set_attr<KIND_I8, EPI_ROTARY_GEN>(), set_attr<KIND_F8, EPI_ROTARY_GEN>(),
+      set_attr<KIND_I8, EPI_ROTARY_HD>(), set_attr<KIND_F8, EPI_ROTARY_HD>()};
   for (cudaError_t er : errs)
     if (er != cudaSuccess) return cuda_status(er, "cudaFuncSetAttribute");
   {
@@ -286,7 +287,7 @@ static cudaError_t launch_inst(const CUtensorMap& ta, const CUtensorMap& tb0, co
   // resident-operand schedule: rotary and the bias epilogue keep A (activation-stationary: one CTA reads a row
   // block's A completely before it writes any of that row block's output, which is what lets the low-rank
   // projection keep its intermediate inside the output buffer), the others keep W (weight-stationary)
-  constexpr int RES = (EPI == EPI_ROTARY || EPI == EPI_ROTARY_GEN || EPI == EPI_BIAS) ? SCHED_ARES : SCHED_WRES;
+  constexpr int RES = (EPI == EPI_ROTARY || EPI == EPI_ROTARY_GEN || EPI == EPI_ROTARY_HD || EPI == EPI_BIAS) ? SCHED_ARES : SCHED_WRES;
   if (resident) gemm_tcgen05_kernel<KIND, EPI, RES><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(ta, tb0, tb1, tc, p);
   else gemm_tcgen05_kernel<KIND, EPI, SCHED_STREAM><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(ta, tb0, tb1, tc, p);
   return cudaGetLastError();
@@ -330,6 +331,7 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
   }
   int rot_cols = 0;
   bool general_rotary = false;
+  int rot_geo = -1;                                     // EPI_ROTARY_HD
   if (a.epi == EPI_ROTARY) {
     if (!a.sin_tab || !a.cos_tab || !aligned16(a.sin_tab) || !aligned16(a.cos_tab)) return GSB200_ERR_BAD_ARG;
     if (a.seqlen < 1 || a.nhead < 1 || a.row_offset < 0) return GSB200_ERR_BAD_ARG;
@@ -341,6 +343,11 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
     if (a.head_dim != 64 || a.rotary_dim != 64) {
       if (fused) return GSB200_ERR_UNSUPPORTED;         // the fused quantiser is built for the 64 / 64 epilogue only
       general_rotary = true;
+      // Heads of 128 and half-rotated heads leave through staged boxes like the 64 / 64 epilogue, with the sin / cos row in
+      // registers; the general one reads it per use and stores 32 bytes per thread and row (M = 20001, K = 512, FP8, heads
+      // of 128: 49.2 us, staged 27.1).
+      if (a.rotary_dim == a.head_dim) rot_geo = 0;
+      else if (2 * a.rotary_dim == a.head_dim) rot_geo = a.head_dim == 128 ? 1 : 2;
     }
   }
   int32_t rc = ensure_device();
@@ -359,6 +366,7 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
   p.sin_tab = a.sin_tab; p.cos_tab = a.cos_tab;
   p.seqlen = a.seqlen > 0 ? a.seqlen : 1;
   p.rot_cols = rot_cols;
+  p.rot_geo = rot_geo;
   p.head_dim = a.head_dim; p.rot_half = a.rotary_dim / 2;
   p.row_offset = (int)(a.row_offset % p.seqlen);
   p.direct_store = (a.flags & GSB200_DIAG_FLAG_MASK & GSB200_DIAG_FLAG_DIRECT_STORE) ? 1 : 0;
@@ -374,7 +382,8 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
   ok = ok && make_map_2d(&tb1, u8, 1, dual ? a.B1 : a.B0, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)a.ldb, BK, BN / 2);
   if (a.epi != EPI_I32 && a.epi != EPI_SILU_MX)
     ok = ok && make_map_2d(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.C, (uint64_t)a.M, (uint64_t)a.N,
-                           (uint64_t)a.ldc, OUT_BOX_COLS, OUT_BOX_ROWS, CU_TENSOR_MAP_SWIZZLE_128B);
+                           (uint64_t)a.ldc, rot_geo >= 0 ? 32 : OUT_BOX_COLS, rot_geo >= 0 ? 32 : OUT_BOX_ROWS,
+                           rot_geo >= 0 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
   else
     tc = ta;
   if (fused) ta = tb0;                            // never used by the fused kernel
@@ -485,6 +494,8 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
         if (fused) {
           gemm_tcgen05_kernel<KIND_I8, EPI_ROTARY, SCHED_ARES, true><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(ta, tb0, tb1, tc, p);
           e = cudaGetLastError();
+        } else if (rot_geo >= 0) {
+          e = launch_inst<KIND_I8, EPI_ROTARY_HD>(ta, tb0, tb1, tc, p, grid, resident, st);
         } else if (general_rotary) {
           e = launch_inst<KIND_I8, EPI_ROTARY_GEN>(ta, tb0, tb1, tc, p, grid, resident, st);
         } else {
@@ -498,7 +509,8 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
     switch (a.epi) {
       case EPI_DEQUANT: e = launch_inst<KIND_F8, EPI_DEQUANT>(ta, tb0, tb1, tc, p, grid, resident, st); break;
       case EPI_ROTARY:
-        e = general_rotary ? launch_inst<KIND_F8, EPI_ROTARY_GEN>(ta, tb0, tb1, tc, p, grid, resident, st)
+        e = rot_geo >= 0 ? launch_inst<KIND_F8, EPI_ROTARY_HD>(ta, tb0, tb1, tc, p, grid, resident, st)
+          : general_rotary ? launch_inst<KIND_F8, EPI_ROTARY_GEN>(ta, tb0, tb1, tc, p, grid, resident, st)
                            : launch_inst<KIND_F8, EPI_ROTARY>(ta, tb0, tb1, tc, p, grid, resident, st);
         break;
       case EPI_SILU: e = launch_inst<KIND_F8, EPI_SILU>(ta, tb0, tb1, tc, p, grid, resident, st); break;

@@ -5,7 +5,8 @@
 //   EPI_I32      raw int32 accumulators                       (bit-exact tier)
 //   EPI_DEQUANT  f16( acc * sA[m] * sB[n] )                   per-token x per-channel dequant
 //   EPI_ROTARY   dequant, then rotate-half on the Q|K columns  (QKV projection; heads of 64, all of it rotated)
-//   EPI_ROTARY_GEN  the same for heads of 64 or 128 columns of which the first 32, 64, 96 or 128 are rotated
+//   EPI_ROTARY_HD   the same for heads of 128 with all or the first half rotated and heads of 64 with the first half rotated
+//   EPI_ROTARY_GEN  the same for what is left: heads of 128 columns of which the first 32 or 96 are rotated
 //   EPI_SILU     f16( silu(gate) * up ), gate|up in one UMMA   (SwiGLU dual GEMM)
 //   EPI_SILU_MX  the same product emitted as MXFP8: E4M3 elements + one E8M0 scale per 32 output columns
 //   EPI_BIAS     f16( acc * sA[m] + b[n] )                    second GEMM of the low-rank input projection
@@ -47,7 +48,7 @@
 
 namespace gsb {
 
-enum : int { EPI_I32 = 0, EPI_DEQUANT = 1, EPI_ROTARY = 2, EPI_SILU = 3, EPI_SILU_MX = 4, EPI_BIAS = 5, EPI_ROTARY_GEN = 6 };
+enum : int { EPI_I32 = 0, EPI_DEQUANT = 1, EPI_ROTARY = 2, EPI_SILU = 3, EPI_SILU_MX = 4, EPI_BIAS = 5, EPI_ROTARY_GEN = 6, EPI_ROTARY_HD = 7 };
 enum : int { KIND_I8 = 0, KIND_F8 = 1, KIND_F16 = 2 };   // F16: fp16 operands (K counted in bytes = 2 per element), f32 accumulate
 enum : int { SCHED_STREAM = 0, SCHED_WRES = 1, SCHED_ARES = 2 };
 
@@ -136,6 +137,7 @@ struct GemmParams {
   int seqlen;                  // runtime sequence length: angle row = (row + row_offset) % seqlen
   int rot_cols;                // 2 * nhead * head_dim: the Q and K columns
   int head_dim;                // EPI_ROTARY_GEN: 64 or 128 (EPI_ROTARY: 64)
+  int rot_geo;                 // EPI_ROTARY_HD: 0 = heads of 128, all rotated; 1 = heads of 128, 64 rotated; 2 = heads of 64, 32 rotated
   int rot_half;                // EPI_ROTARY_GEN: rotary_dim / 2, a multiple of 16 (EPI_ROTARY: 32); also the width of a sin / cos row
   int row_offset;              // global row index of this shard's row 0
   const __half* x_f16;         // fused activation quantiser: fp16 activations [M, K] (the int8 A operand is then made on chip)
@@ -895,6 +897,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 #pragma unroll
     for (int pc = 0; pc < 8; ++pc) stg_off[pc] = (lane & 15) * 128 + ((pc ^ (lane & 7)) << 4);
 
+    // EPI_ROTARY_HD: where this warp's two items of a tile lie.  An item is two 32-column output boxes; it is worked on as
+    // two chunks of 16 + 16 accumulator columns (ca .. ca + 15 and ca + hd_boff ...) that rotate together, or are only
+    // dequantised.
+    //   geometry 0  heads of 128, all rotated: item i is the warp's half of both halves of head i (the sin / cos rows stay 32
+    //               values per thread); geometry 1  heads of 128, 64 rotated: the first or the second 64 columns of head
+    //               `half`; geometry 2  heads of 64, 32 rotated: a head; chunk 0 its rotated columns, chunk 1 the others
+    constexpr bool HD = EPI == EPI_ROTARY_HD, ROT = EPI == EPI_ROTARY || HD;
+    const int geo = HD ? p.rot_geo : 1;
+    const int wrot0 = HD && geo == 0 ? 0 : wout0;                          // from here on the warp's columns of a tile may be rotated
+    const int trig_ld = HD ? (geo == 0 ? 64 : geo == 1 ? 32 : 16) : 32, trig_col = HD && geo == 0 ? 32 * half : 0;
+    [[maybe_unused]] const int hd_a0 = geo == 0 ? 32 * half : 128 * half, hd_item = geo == 0 ? 128 : 64;
+    [[maybe_unused]] const int hd_boff = geo == 0 ? 64 : geo == 1 ? 32 : 16, hd_chunk = geo == 2 ? 32 : 16;
+
     GP_DECL(e_total); GP_DECL(e_acc); GP_DECL(e_read); GP_DECL(e_ld); GP_BEGIN(gp_e0);
     Walk tw; tw.start(p);
     if constexpr (EPI != EPI_I32) {
@@ -921,30 +936,31 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           cur_m_blk = m_blk;
           if constexpr (FUSEQ) new_row_block = true; else sa = sa_next;
         }
-        if constexpr (EPI == EPI_ROTARY) {
+        if constexpr (ROT) {
           // The angle rows cost 16 scattered 16-byte loads per thread.  Once this warp's columns lie past the
           // rotated ones (the V part of a QKV projection, walked last), the rows of the NEXT row block are
           // fetched already, a tile or more before they are needed; otherwise at the row block's first tile.
           int want = m_blk;
-          if (n0 + wout0 >= p.rot_cols && tw.valid(p)) want = nxt_m;
+          if (n0 + wrot0 >= p.rot_cols && tw.valid(p)) want = nxt_m;
           if (want != trig_m_blk) {
             trig_m_blk = want;
             trig_scaled = false;
             const long long r = (long long)want * BM + q * 32 + lane;
             const int pos = r < p.M ? (int)((r + p.row_offset) % p.seqlen) : 0;
-            const float* s4 = p.sin_tab + (long long)pos * 32;
-            const float* c4 = p.cos_tab + (long long)pos * 32;
+            const float* s4 = p.sin_tab + (long long)pos * trig_ld + trig_col;
+            const float* c4 = p.cos_tab + (long long)pos * trig_ld + trig_col;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {     // straight into the registers that hold them: nothing waits for the data here
               asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
                            : "=f"(sn2[2 * j].x), "=f"(sn2[2 * j].y), "=f"(sn2[2 * j + 1].x), "=f"(sn2[2 * j + 1].y) : "l"(s4 + 4 * j));
               asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
                            : "=f"(cs2[2 * j].x), "=f"(cs2[2 * j].y), "=f"(cs2[2 * j + 1].x), "=f"(cs2[2 * j + 1].y) : "l"(c4 + 4 * j));
+              if (HD && j == 3 && p.rot_geo == 2) break;      // rows of 16
             }
           }
           // The rotated columns use sin and cos premultiplied by the token scale: folded in once per row block,
           // at the first tile in which this warp rotates (rows fetched ahead have arrived by then).
-          if (!FUSEQ && trig_m_blk == m_blk && !trig_scaled && n0 + wout0 < p.rot_cols) {
+          if (!FUSEQ && trig_m_blk == m_blk && !trig_scaled && n0 + wrot0 < p.rot_cols) {
             trig_scaled = true;
             const float2 s2 = pk2(sa, sa);
 #pragma unroll
@@ -1285,6 +1301,71 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                 GP_END(e_ld, gp_l1);
                 if (c + 64 < WACC) ldh(c + 64, 0, xa0, xa1); else release();
                 emit(xb0, xb1, c, 1);
+              }
+            } else if constexpr (HD) {
+              const uint32_t sc_t = sc_addr - acol0 * 4, t_t = t_row - acol0;           // of the tile's column 0
+              auto ldh = [&](int i, int hh, uint32_t (&x0)[16], uint32_t (&x1)[16]) {
+                const uint32_t t = t_t + hd_a0 + i * hd_item + hh * hd_chunk;
+                tmem_ld_32x32b_x16(t, x0);
+                tmem_ld_32x32b_x16(t + hd_boff, x1);
+              };
+              auto emit = [&](const uint32_t (&v0)[16], const uint32_t (&v1)[16], int i, int hh) {
+                const int n = n0 + hd_a0 + i * hd_item;
+                if (n >= p.N) return;
+                if (hh == 0) pair_begin();
+                const uint32_t s0 = sc_t + (hd_a0 + i * hd_item + hh * hd_chunk) * 4, s1 = s0 + hd_boff * 4;
+                // 16-byte piece j (0, 1) of the chunk's first / second 16 columns
+                auto put32 = [&](int part, int j, uint4 o) {
+                  const int box = geo == 2 ? hh : part, piece = geo == 2 ? 2 * part + j : 2 * hh + j;
+                  *reinterpret_cast<uint4*>(out_buf + (box ? buf_b : buf_a) * OUT_BUF_BYTES + lane * 64 + ((piece ^ ((lane >> 1) & 3)) << 4)) = o;
+                };
+                if (n < p.rot_cols && (geo == 0 || (geo == 1 ? i == 0 : hh == 0))) {
+#pragma unroll
+                  for (int j = 0; j < 16; j += 8) {
+                    const float4 a_lo = lds_f4_ro(s0 + 4 * j), a_hi = lds_f4_ro(s0 + 4 * j + 16);
+                    const float4 b_lo = lds_f4_ro(s1 + 4 * j), b_hi = lds_f4_ro(s1 + 4 * j + 16);
+                    const float2 sb0[4] = {{a_lo.x, a_lo.y}, {a_lo.z, a_lo.w}, {a_hi.x, a_hi.y}, {a_hi.z, a_hi.w}};
+                    const float2 sb1[4] = {{b_lo.x, b_lo.y}, {b_lo.z, b_lo.w}, {b_hi.x, b_hi.y}, {b_hi.z, b_hi.w}};
+                    uint32_t o0[4], o1[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {        // the arithmetic of EPI_ROTARY
+                      const float2 y0 = fmul2(pk2(acc_to_float<KIND>(v0[j + 2 * k]), acc_to_float<KIND>(v0[j + 2 * k + 1])), sb0[k]);
+                      const float2 y1 = fmul2(pk2(acc_to_float<KIND>(v1[j + 2 * k]), acc_to_float<KIND>(v1[j + 2 * k + 1])), sb1[k]);
+                      const float2 c2 = cs2[hh * 8 + (j >> 1) + k], s2 = sn2[hh * 8 + (j >> 1) + k];
+                      const float2 qa = fmul2(y1, s2), ta = fmul2(y1, c2);
+                      o0[k] = pack_half2_from(__ffma2_rn(y0, c2, make_float2(-qa.x, -qa.y)));
+                      o1[k] = pack_half2_from(__ffma2_rn(y0, s2, ta));
+                    }
+                    put32(0, j >> 3, make_uint4(o0[0], o0[1], o0[2], o0[3]));
+                    put32(1, j >> 3, make_uint4(o1[0], o1[1], o1[2], o1[3]));
+                  }
+                } else {
+#pragma unroll
+                  for (int j = 0; j < 16; j += 8) {
+                    put32(0, j >> 3, dequant_piece<KIND>(&v0[j], sa2, lds_f4_ro(s0 + 4 * j), lds_f4_ro(s0 + 4 * j + 16)));
+                    put32(1, j >> 3, dequant_piece<KIND>(&v1[j], sa2, lds_f4_ro(s1 + 4 * j), lds_f4_ro(s1 + 4 * j + 16)));
+                  }
+                }
+                if (hh == 1) {
+                  fence_proxy_async_smem();
+                  __syncwarp();
+                  if (lane == 0) {                       // boxes of 32 rows x 32 columns; the map clips the rows past M
+                    tma_store_2d(&tm_c, out_buf + buf_a * OUT_BUF_BYTES, n, row_base); tma_store_commit();
+                    tma_store_2d(&tm_c, out_buf + buf_b * OUT_BUF_BYTES, n + (geo == 0 ? 64 : 32), row_base); tma_store_commit();
+                  }
+                  obuf = (buf_b + 1 == OUT_BUFS) ? 0 : buf_b + 1;
+                }
+              };
+              uint32_t xa0[16], xa1[16], xb0[16], xb1[16];
+              ldh(0, 0, xa0, xa1);
+#pragma unroll 1
+              for (int i = 0; i < 2; ++i) {
+                tmem_ld_wait(xa0, xa1);
+                ldh(i, 1, xb0, xb1);
+                emit(xa0, xa1, i, 0);
+                tmem_ld_wait(xb0, xb1);
+                if (i == 0) ldh(1, 0, xa0, xa1); else release();
+                emit(xb0, xb1, i, 1);
               }
             } else {   // EPI_SILU: gate at local column c, up at BN/2 accumulator columns on; a chunk is one 32-column output box
               auto emit = [&](const uint32_t (&g)[32], const uint32_t (&u)[32], int c, int which) {
