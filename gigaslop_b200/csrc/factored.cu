@@ -52,9 +52,11 @@ factored_lstm_step_kernel(const __grid_constant__ CUtensorMap tm_hh, const __gri
     prefetch_tmap(&tm_hh); prefetch_tmap(&tm_xd); prefetch_tmap(&tm_uhh); prefetch_tmap(&tm_uih);
   }
   if (warp == 0) { tmem_alloc(tmem_slot, FS_NCOL); tmem_relinquish(); }
+  pdl_trigger();
+  pdl_wait();
   if (tid < FS_NCOL) {
     const int n = (tid >> 5) * p.H + hid0 + (tid & 31);
-    bias_s[tid] = (p.bias_hh ? __ldg(p.bias_hh + n) : 0.f) + (p.bias_ih ? __ldg(p.bias_ih + n) : 0.f);
+    bias_s[tid] = (p.bias_hh ? ldg_f_here(p.bias_hh + n) : 0.f) + (p.bias_ih ? ldg_f_here(p.bias_ih + n) : 0.f);
   }
   tc_fence_before();
   __syncthreads();
@@ -175,8 +177,9 @@ int32_t launch_factored_lstm_step(uint8_t* h_out, float* c, const __half* hh_dow
   FacStepParams p{};
   p.B = (int)B; p.H = H; p.kb_hh = K_hh / 64; p.kb_ih = R / 64;
   p.bias_hh = bias_hh; p.bias_ih = bias_ih; p.c = c; p.h_out = h_out;
-  factored_lstm_step_kernel<<<(unsigned)grid, FS_THREADS, FS_SMEM_BYTES, st>>>(t_hh, t_xd, t_uhh, t_uih, p);
-  return cuda_status(cudaGetLastError(), "factored lstm step launch");
+  const cudaError_t e = launch_dependent(factored_lstm_step_kernel, (unsigned)grid, FS_THREADS, FS_SMEM_BYTES, st, t_hh, t_xd, t_uhh,
+                                         t_uih, p);
+  return cuda_status(e, "factored lstm step launch");
 }
 
 }  // namespace gsb

@@ -128,16 +128,18 @@ struct Variant {
     return resident ? (Fn)gemm_tcgen05_kernel<KIND, EPI, RES, false, PAIR, EW>
                     : (Fn)gemm_tcgen05_kernel<KIND, EPI, SCHED_STREAM, false, PAIR, EW>;
   }
-  static cudaLaunchConfig_t config(int grid, cudaStream_t st, cudaLaunchAttribute* attr) {
-    attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = PAIR ? 2 : 1; attr->val.clusterDim.y = 1; attr->val.clusterDim.z = 1;
+  static cudaLaunchConfig_t config(int grid, cudaStream_t st, cudaLaunchAttribute (&attr)[2]) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = PAIR ? 2 : 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3(THREADS, 1, 1);
     cfg.dynamicSmemBytes = GEMM_SMEM_BYTES;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cfg;
   }
   // Scheduling units (CTAs, or CTA pairs) that can be resident at once on the current device; 0 = this variant must
@@ -158,8 +160,8 @@ struct Variant {
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (PAIR) {
-          cudaLaunchAttribute attr;
-          cudaLaunchConfig_t cfg = config(2 * (sms / 2), nullptr, &attr);
+          cudaLaunchAttribute attr[2];
+          cudaLaunchConfig_t cfg = config(2 * (sms / 2), nullptr, attr);
           int n = 0;
           if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0) c = n;
         } else if (sms > 0) {
@@ -175,8 +177,8 @@ struct Variant {
   }
   static cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb0, const CUtensorMap& tb1, const CUtensorMap& tc,
                             const GemmParams& p, int grid, bool resident, cudaStream_t st) {
-    cudaLaunchAttribute attr;
-    cudaLaunchConfig_t cfg = config(grid, st, &attr);
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = config(grid, st, attr);
     return cudaLaunchKernelEx(&cfg, kernel(resident), ta, tb0, tb1, tc, p);
   }
 };
@@ -288,9 +290,8 @@ static cudaError_t launch_inst(const CUtensorMap& ta, const CUtensorMap& tb0, co
   // block's A completely before it writes any of that row block's output, which is what lets the low-rank
   // projection keep its intermediate inside the output buffer), the others keep W (weight-stationary)
   constexpr int RES = (EPI == EPI_ROTARY || EPI == EPI_ROTARY_GEN || EPI == EPI_ROTARY_HD || EPI == EPI_BIAS) ? SCHED_ARES : SCHED_WRES;
-  if (resident) gemm_tcgen05_kernel<KIND, EPI, RES><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(ta, tb0, tb1, tc, p);
-  else gemm_tcgen05_kernel<KIND, EPI, SCHED_STREAM><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(ta, tb0, tb1, tc, p);
-  return cudaGetLastError();
+  return launch_dependent(resident ? gemm_tcgen05_kernel<KIND, EPI, RES> : gemm_tcgen05_kernel<KIND, EPI, SCHED_STREAM>, grid,
+                          GEMM_THREADS, GEMM_SMEM_BYTES, st, ta, tb0, tb1, tc, p);
 }
 
 int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
@@ -492,8 +493,8 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
       case EPI_DEQUANT: e = launch_inst<KIND_I8, EPI_DEQUANT>(ta, tb0, tb1, tc, p, grid, resident, st); break;
       case EPI_ROTARY:
         if (fused) {
-          gemm_tcgen05_kernel<KIND_I8, EPI_ROTARY, SCHED_ARES, true><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(ta, tb0, tb1, tc, p);
-          e = cudaGetLastError();
+          e = launch_dependent(gemm_tcgen05_kernel<KIND_I8, EPI_ROTARY, SCHED_ARES, true>, grid, GEMM_THREADS, GEMM_SMEM_BYTES, st, ta, tb0,
+                               tb1, tc, p);
         } else if (rot_geo >= 0) {
           e = launch_inst<KIND_I8, EPI_ROTARY_HD>(ta, tb0, tb1, tc, p, grid, resident, st);
         } else if (general_rotary) {

@@ -358,11 +358,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     if constexpr (PAIR) { tmem_alloc_pair(tmem_slot, TMEM_COLS); tmem_relinquish_pair(); }
     else { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
   }
+  pdl_wait();
   // Channel scales normally arrive by bulk copy from the producer; without a per-channel vector (none given,
   // or one scalar for all columns) every buffer is filled with the constant once, here.
   const bool copy_scales = EPI != EPI_I32 && p.scale_b0 != nullptr && !p.scale_b_scalar;
   if (EPI != EPI_I32 && !copy_scales) {
-    const float v = p.scale_b0 ? __ldg(p.scale_b0) : 1.f;
+    const float v = p.scale_b0 ? ldg_f_here(p.scale_b0) : 1.f;
     for (int i = threadIdx.x; i < Map::SCALE_BUFS * BN; i += NTHREADS) scale_base[i] = v;
   }
   tc_fence_before();
@@ -608,7 +609,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           raw[j][0] = raw[j][1] = make_uint4(0u, 0u, 0u, 0u);
           if (row < p.M && lane < kvec) {
             const uint4* src = reinterpret_cast<const uint4*>(p.x_f16 + row * p.ldx + lane * 16);
-            raw[j][0] = __ldg(src); raw[j][1] = __ldg(src + 1);
+            raw[j][0] = __ldcg(src); raw[j][1] = __ldcg(src + 1);
           }
         }
         // the four rows go through every stage together, so that their shuffle and reciprocal chains overlap
@@ -708,9 +709,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           const float* c4 = p.cos_tab + (long long)pos * 32;
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+            asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                          : "=f"(sn2[2 * k].x), "=f"(sn2[2 * k].y), "=f"(sn2[2 * k + 1].x), "=f"(sn2[2 * k + 1].y) : "l"(s4 + 4 * k));
-            asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+            asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                          : "=f"(cs2[2 * k].x), "=f"(cs2[2 * k].y), "=f"(cs2[2 * k + 1].x), "=f"(cs2[2 * k + 1].y) : "l"(c4 + 4 * k));
           }
         }
@@ -915,7 +916,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     if constexpr (EPI != EPI_I32) {
       if (tw.valid(p)) {
         const int r = rowblk(tw.m) * BM + q * 32 + lane;
-        if (r < p.M) sa_next = p.scale_a ? __ldg(p.scale_a + r) : 1.f;
+        if (r < p.M) sa_next = p.scale_a ? ldg_f_here(p.scale_a + r) : 1.f;
       }
     }
     for (int it = 0; tw.valid(p); ++it) {
@@ -951,9 +952,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             const float* c4 = p.cos_tab + (long long)pos * trig_ld + trig_col;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {     // straight into the registers that hold them: nothing waits for the data here
-              asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+              asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                            : "=f"(sn2[2 * j].x), "=f"(sn2[2 * j].y), "=f"(sn2[2 * j + 1].x), "=f"(sn2[2 * j + 1].y) : "l"(s4 + 4 * j));
-              asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+              asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                            : "=f"(cs2[2 * j].x), "=f"(cs2[2 * j].y), "=f"(cs2[2 * j + 1].x), "=f"(cs2[2 * j + 1].y) : "l"(c4 + 4 * j));
               if (HD && j == 3 && p.rot_geo == 2) break;      // rows of 16
             }
@@ -1093,8 +1094,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                 float4 sv[4], cv[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                  sv[i] = row_ok ? __ldg(reinterpret_cast<const float4*>(srow + u) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                  cv[i] = row_ok ? __ldg(reinterpret_cast<const float4*>(crow + u) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                  sv[i] = row_ok ? ldg_f4_here(srow + u + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                  cv[i] = row_ok ? ldg_f4_here(crow + u + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
                 tmem_ld_wait(x0, x1);
 #pragma unroll

@@ -127,6 +127,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     prefetch_tmap(&tm_a); prefetch_tmap(&tm_b0); prefetch_tmap(&tm_b1); prefetch_tmap(&tm_c);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, MX_TMEM_COLS); tmem_relinquish(); }
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -382,9 +383,11 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
 // (K % 128 == 0, so a row holds whole groups of four).  Consecutive threads write consecutive words; the 32 rows of a
 // lane group lie ld bytes apart, and the other words of their sectors are picked up from L1 by the threads of the
 // neighbouring tiles.  With a thread per byte the launch took 10.5 us (mean of 65536 x 512 and x 2048; 4.3 us now).
-__global__ void mx_scales_to_tiled_kernel(const uint8_t* __restrict__ src, long long ld, long long rows, int kt,
+__global__ void mx_scales_to_tiled_kernel(const uint8_t* src, long long ld, long long rows, int kt,
                                           uint8_t* __restrict__ dst, unsigned words, bool word_loads, bool word_stores) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (i >= words) return;
   const unsigned tile = i >> 7, in = i & 127;              // 128 words per tile
   const unsigned rb = tile / (unsigned)kt, kb = tile % (unsigned)kt;
@@ -392,7 +395,7 @@ __global__ void mx_scales_to_tiled_kernel(const uint8_t* __restrict__ src, long 
   uint32_t v = 0x7f7f7f7fu;                                // padding rows: scale 1.0 on zero data
   if (row < rows) {
     const uint8_t* s = src + row * ld + kb * 4;
-    if (word_loads) v = __ldg(reinterpret_cast<const uint32_t*>(s));
+    if (word_loads) v = __ldcg(reinterpret_cast<const uint32_t*>(s));
     else v = s[0] | (uint32_t)s[1] << 8 | (uint32_t)s[2] << 16 | (uint32_t)s[3] << 24;
   }
   uint8_t* d = dst + (size_t)i * 4;
@@ -411,9 +414,9 @@ int32_t launch_mx_scales_to_tiled(const uint8_t* src, long long ld, long long ro
   if (words > 0xffffff00ll) return GSB200_ERR_BAD_ARG;
   const bool word_loads = ld % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 3) == 0;
   const bool word_stores = (reinterpret_cast<uintptr_t>(dst) & 3) == 0;
-  mx_scales_to_tiled_kernel<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(src, ld, rows, K / 128, dst, (unsigned)words,
-                                                                          word_loads, word_stores);
-  return cuda_status(cudaGetLastError(), "mx scale re-tiling launch");
+  const cudaError_t e = launch_dependent(mx_scales_to_tiled_kernel, (unsigned)((words + 255) / 256), 256, 0, st, src, ld, rows,
+                                         K / 128, dst, (unsigned)words, word_loads, word_stores);
+  return cuda_status(e, "mx scale re-tiling launch");
 }
 
 int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t* sfa, const uint8_t* B0,
@@ -463,19 +466,20 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
   p.k_blocks = K / MX_BK;
   p.sfa = sfa; p.sfb0 = sfb0; p.sfb1 = sfb1;
   const long long tiles = (long long)p.m_blocks * p.n_blocks;
+  cudaError_t e;
   if (wst) {                                                        // weight-stationary form
     int groups = sm_count() / p.n_blocks;
     if (groups > p.m_blocks) groups = p.m_blocks;
     p.n_groups = groups;
     const int grid = groups * p.n_blocks;
-    if (dual) mx_gemm_kernel<true, true><<<grid, MX_THREADS, MxSmem<true>::BYTES, st>>>(ta, tb0, tb1, tc, p);
-    else mx_gemm_kernel<false, true><<<grid, MX_THREADS, MxSmem<true>::BYTES, st>>>(ta, tb0, tb1, tc, p);
-    return cuda_status(cudaGetLastError(), "mx gemm launch");
+    if (dual) e = launch_dependent(mx_gemm_kernel<true, true>, grid, MX_THREADS, MxSmem<true>::BYTES, st, ta, tb0, tb1, tc, p);
+    else e = launch_dependent(mx_gemm_kernel<false, true>, grid, MX_THREADS, MxSmem<true>::BYTES, st, ta, tb0, tb1, tc, p);
+    return cuda_status(e, "mx gemm launch");
   }
   const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-  if (dual) mx_gemm_kernel<true, false><<<grid, MX_THREADS, MxSmem<false>::BYTES, st>>>(ta, tb0, tb1, tc, p);
-  else mx_gemm_kernel<false, false><<<grid, MX_THREADS, MxSmem<false>::BYTES, st>>>(ta, tb0, tb1, tc, p);
-  return cuda_status(cudaGetLastError(), "mx gemm launch");
+  if (dual) e = launch_dependent(mx_gemm_kernel<true, false>, grid, MX_THREADS, MxSmem<false>::BYTES, st, ta, tb0, tb1, tc, p);
+  else e = launch_dependent(mx_gemm_kernel<false, false>, grid, MX_THREADS, MxSmem<false>::BYTES, st, ta, tb0, tb1, tc, p);
+  return cuda_status(e, "mx gemm launch");
 }
 
 }  // namespace gsb

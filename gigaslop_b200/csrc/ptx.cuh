@@ -59,6 +59,19 @@ struct AbortFlag {
   }
 };
 
+// ---- programmatic dependent launch --------------------------------------------
+// The kernels that follow one another in a stream are launched with programmatic stream serialization (launch_dependent):
+// a kernel may start while the one before it drains.  None of them touches global memory before pdl_wait, which returns when
+// the kernel before it is complete and its writes are visible; at least one block of a grid has to wait.  Data another kernel
+// may have written is not read through the non-coherent path (ld.global.nc): that is for data constant over the kernel's
+// life.  pdl_trigger lets the successor's CTAs become resident as this kernel's leave.  The quantisers (after their wait) and
+// the LSTM step do that: the GEMM behind them sets up its barriers and tensor memory meanwhile.  The GEMMs do not: a
+// quantiser that starts beside their last tiles costs more than it gains (us per pass, no overlap / quantisers trigger /
+// GEMMs too: QKV of 65536 rows 84.3 / 79.7 / 83.8, feed-forward 246 / 239 / 249, of 256 rows 28.7 / 22 / 22, of 9001 rows
+// 54.6 / 46 / 47).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -581,16 +594,16 @@ __device__ __forceinline__ uint32_t named_barrier_and(uint32_t id, uint32_t nthr
 // are not ordered against unrelated shared-memory stores.  Only for data that is read-only while the address
 // value is live; derive the address from the result of the synchronisation that published the data, which
 // keeps the reads behind it.
-// Read-only global loads that stay where they are written (volatile): used to start a load a whole tile
+// Global loads that stay where they are written (volatile): used to start a load a whole tile
 // before its value is needed; the compiler would otherwise be free to sink it to the point of use.
 __device__ __forceinline__ float4 ldg_f4_here(const float* p) {
   float4 v;
-  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ float ldg_f_here(const float* p) {
   float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
   return v;
 }
 __device__ __forceinline__ float4 lds_f4_ro(uint32_t addr) {

@@ -9,6 +9,7 @@
 #include <cuda_fp8.h>
 
 #include "capi_internal.h"
+#include "ptx.cuh"
 
 namespace gsb {
 
@@ -19,7 +20,7 @@ __device__ __forceinline__ void load8(const Tin* p, float (&v)[8]);
 
 template <>
 __device__ __forceinline__ void load8<__half>(const __half* p, float (&v)[8]) {
-  const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
+  const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(p));
   const __half2* h = reinterpret_cast<const __half2*>(&raw);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -29,8 +30,8 @@ __device__ __forceinline__ void load8<__half>(const __half* p, float (&v)[8]) {
 }
 template <>
 __device__ __forceinline__ void load8<float>(const float* p, float (&v)[8]) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-  const float4 b = __ldg(reinterpret_cast<const float4*>(p + 4));
+  const float4 a = __ldcg(reinterpret_cast<const float4*>(p));
+  const float4 b = __ldcg(reinterpret_cast<const float4*>(p + 4));
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
@@ -114,6 +115,8 @@ ptq_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q, lo
            float* __restrict__ scale, long long M, int K) {
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * QUANT_WARPS + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_trigger();
   if (row >= M) return;
   const Tin* xr = x + row * ldx;
   uint8_t* qr = q + row * ldq;
@@ -131,7 +134,7 @@ ptq_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q, lo
     for (int i = 0; i < NV; ++i) {
       const int v = lane + 32 * i;
       raw[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (v < nvec) raw[i] = __ldg(reinterpret_cast<const uint4*>(xr + v * 8));
+      if (v < nvec) raw[i] = __ldcg(reinterpret_cast<const uint4*>(xr + v * 8));
       const __half2* h = reinterpret_cast<const __half2*>(&raw[i]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -228,11 +231,12 @@ static cudaError_t launch_fmt(const void* x, long long ldx, void* q, long long l
   const unsigned blocks = (unsigned)((M + QUANT_WARPS - 1) / QUANT_WARPS);
   const Tin* xp = static_cast<const Tin*>(x);
   uint8_t* qp = static_cast<uint8_t*>(q);
-  if (K <= 512) ptq_kernel<Tin, FMT, 2><<<blocks, QUANT_WARPS * 32, 0, st>>>(xp, ldx, qp, ldq, scale, M, K);
-  else if (K <= 1024) ptq_kernel<Tin, FMT, 4><<<blocks, QUANT_WARPS * 32, 0, st>>>(xp, ldx, qp, ldq, scale, M, K);
-  else if (K <= 2048) ptq_kernel<Tin, FMT, 8><<<blocks, QUANT_WARPS * 32, 0, st>>>(xp, ldx, qp, ldq, scale, M, K);
-  else ptq_kernel<Tin, FMT, 0><<<blocks, QUANT_WARPS * 32, 0, st>>>(xp, ldx, qp, ldq, scale, M, K);
-  return cudaGetLastError();
+  cudaError_t e;
+  if (K <= 512) e = launch_dependent(ptq_kernel<Tin, FMT, 2>, blocks, QUANT_WARPS * 32, 0, st, xp, ldx, qp, ldq, scale, M, K);
+  else if (K <= 1024) e = launch_dependent(ptq_kernel<Tin, FMT, 4>, blocks, QUANT_WARPS * 32, 0, st, xp, ldx, qp, ldq, scale, M, K);
+  else if (K <= 2048) e = launch_dependent(ptq_kernel<Tin, FMT, 8>, blocks, QUANT_WARPS * 32, 0, st, xp, ldx, qp, ldq, scale, M, K);
+  else e = launch_dependent(ptq_kernel<Tin, FMT, 0>, blocks, QUANT_WARPS * 32, 0, st, xp, ldx, qp, ldq, scale, M, K);
+  return e;
 }
 
 // ---- MXFP8 activation quantiser: E4M3 elements + one E8M0 scale per 32 consecutive elements of a row -------
@@ -247,6 +251,8 @@ ptq_mx_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q,
               uint8_t* __restrict__ scales, long long lds, long long M, int K) {
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * QUANT_WARPS + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_trigger();
   if (row >= M) return;
   const Tin* xr = x + row * ldx;
   constexpr bool HALF = sizeof(Tin) == 2;
@@ -260,7 +266,7 @@ ptq_mx_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q,
 #pragma unroll
       for (int w = 0; w < WORDS; ++w) {
         raw[i][w] = make_uint4(0u, 0u, 0u, 0u);
-        if (v < nvec) raw[i][w] = __ldg(reinterpret_cast<const uint4*>(xr + v * 8) + w);
+        if (v < nvec) raw[i][w] = __ldcg(reinterpret_cast<const uint4*>(xr + v * 8) + w);
       }
     }
 #pragma unroll
@@ -300,13 +306,13 @@ ptq_mx_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q,
 }
 
 template <typename Tin>
-static void launch_mx_rows(const void* x, long long ldx, uint8_t* q, long long ldq, uint8_t* scales, long long lds, long long M,
+static cudaError_t launch_mx_rows(const void* x, long long ldx, uint8_t* q, long long ldq, uint8_t* scales, long long lds, long long M,
                            int K, cudaStream_t st) {
   const unsigned blocks = (unsigned)((M + QUANT_WARPS - 1) / QUANT_WARPS);
   const Tin* xp = static_cast<const Tin*>(x);
-  if (K <= 256) ptq_mx_kernel<Tin, 1><<<blocks, QUANT_WARPS * 32, 0, st>>>(xp, ldx, q, ldq, scales, lds, M, K);
-  else if (K <= 512) ptq_mx_kernel<Tin, 2><<<blocks, QUANT_WARPS * 32, 0, st>>>(xp, ldx, q, ldq, scales, lds, M, K);
-  else ptq_mx_kernel<Tin, 4><<<blocks, QUANT_WARPS * 32, 0, st>>>(xp, ldx, q, ldq, scales, lds, M, K);
+  if (K <= 256) return launch_dependent(ptq_mx_kernel<Tin, 1>, blocks, QUANT_WARPS * 32, 0, st, xp, ldx, q, ldq, scales, lds, M, K);
+  if (K <= 512) return launch_dependent(ptq_mx_kernel<Tin, 2>, blocks, QUANT_WARPS * 32, 0, st, xp, ldx, q, ldq, scales, lds, M, K);
+  return launch_dependent(ptq_mx_kernel<Tin, 4>, blocks, QUANT_WARPS * 32, 0, st, xp, ldx, q, ldq, scales, lds, M, K);
 }
 
 int32_t launch_ptq_mx(const void* x, int x_dtype, long long ldx, uint8_t* q, long long ldq, uint8_t* scales,
@@ -319,9 +325,9 @@ int32_t launch_ptq_mx(const void* x, int x_dtype, long long ldx, uint8_t* q, lon
   if ((ldx * esz) % 16 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(q) & 7))
     return GSB200_ERR_BAD_ARG;
   if ((M + QUANT_WARPS - 1) / QUANT_WARPS > 0x7fffffffll) return GSB200_ERR_BAD_ARG;
-  if (x_dtype == GSB200_F16) launch_mx_rows<__half>(x, ldx, q, ldq, scales, lds, M, K, st);
-  else launch_mx_rows<float>(x, ldx, q, ldq, scales, lds, M, K, st);
-  return cuda_status(cudaGetLastError(), "ptq_mx launch");
+  const cudaError_t e = x_dtype == GSB200_F16 ? launch_mx_rows<__half>(x, ldx, q, ldq, scales, lds, M, K, st)
+                                              : launch_mx_rows<float>(x, ldx, q, ldq, scales, lds, M, K, st);
+  return cuda_status(e, "ptq_mx launch");
 }
 
 int32_t launch_ptq(const void* x, int x_dtype, long long ldx, void* q, long long ldq, float* scale, long long M, int K,
