@@ -553,7 +553,7 @@ lstm_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 }
 
 // ---- transposed form: W_hh in tensor memory, the batch as the N dimension ------------------------------------------
-// gates^T = W_hh . h^T: a CTA owns 128 hidden units and G = 8, 12, 16 or 32 batch rows (N = R = 16 or 32 columns of the
+// gates^T = W_hh . h^T: a CTA owns 128 hidden units and G = 4, 8, 12, 16 or 32 batch rows (N = R = 16 or 32 columns of the
 // MMA; columns without a row multiply zeros).  The four gates of its hidden units are four M = 128 x N = R accumulators, so
 // a cell's four gate values sit in one TMEM lane and one thread has them all.  The A operand, W_hh (4 x 128 rows x up to
 // 384 bytes), is written to tensor memory once per launch (384 of its 512 columns; a fourth K block, H > 384, stays in
@@ -569,7 +569,7 @@ lstm_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 //  * the batch is the small dimension, so B = 512 spreads over 129 SMs (G = 12) instead of 48: the gate math, five
 //    special-function instructions per cell, is 1000 clocks for 2048 cells (G = 16), 600 for 1024.
 //  * W_hh in tensor memory: an MMA from a shared-memory A operand of 128 rows takes 40 clocks, from TMEM 16.
-// B = 512, H = 384: 1.27 us per step (2.57 before), H = 512: 1.83 (4.8), H = 256: 0.96 (2.29), H = 128: 0.73 (2.27).
+// B = 512, H = 384: 1.27 us per step (2.57 before), H = 512: 1.83 (4.8), H = 256: 0.96 (2.29), H = 128: 0.57 (2.27).
 // Clocks of a step (G = 16, H = 384, of ~2650): own K block's MMAs 340, wait for the others' h 300, their MMAs 560, commit
 // to registers 300, gate math and sending 1000, hand-over to the MMA warps 130.
 //   warps 0 .. CW-1   gate math.  Warp w: TMEM lane quarter w % 4 (32 hidden units, one per lane), G / (CW / 4) batch rows
@@ -895,8 +895,9 @@ size_t lstm_scratch_bytes(long long B, int H) {
 }
 
 using LtKernel = void (*)(const CUtensorMap, const CUtensorMap, const uint8_t*, long long, const LstmParams);
-// The forms of the transposed kernel: batch rows per group, and what a step costs (B200, us at H = 128 / 384 / 512).
-//   8 rows   0.72 / 1.09 / -      12 rows   0.90 / 1.27 / -      16 rows   1.07 / 1.38 / 1.83      32 rows   1.77 / 2.21 / 2.68
+// The forms of the transposed kernel: batch rows per group, and what a step costs (B200, us at H = 128 / 256 / 384 / 512).
+//    4 rows  0.57 / 0.79 / 0.91 / 1.2       8 rows  0.72 / 0.96 / 1.09 / 1.40      12 rows  0.90 / 1.14 / 1.27 / 1.58
+//   16 rows  1.07 / 1.25 / 1.38 / 1.77     32 rows  1.77 / 2.11 / 2.21 / 2.68
 struct LtForm { int rows, threads, smem[LT_MAX_SLICES + 1], cost; LtKernel kernel; };
 template <int R, int G, int CW>
 static constexpr LtForm lt_make_form(int cost) {
@@ -905,8 +906,8 @@ static constexpr LtForm lt_make_form(int cost) {
   for (int n = 1; n <= LT_MAX_SLICES; ++n) f.smem[n] = LtSmem<R, G>::bytes(n) > 120 * 1024 ? LtSmem<R, G>::bytes(n) : 120 * 1024;
   return f;
 }
-constexpr int LT_FORMS = 4;
-static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 8, 8>(10), lt_make_form<16, 12, 12>(12), lt_make_form<16, 16, 8>(13),
+constexpr int LT_FORMS = 5;
+static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(8), lt_make_form<16, 8, 8>(10), lt_make_form<16, 12, 12>(12), lt_make_form<16, 16, 8>(13),
                                           lt_make_form<32, 32, 16>(21)};
 
 static cudaLaunchConfig_t lt_config(const LtForm& f, int slices, long long groups, cudaStream_t st, cudaLaunchAttribute* attr) {

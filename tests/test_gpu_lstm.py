@@ -169,10 +169,10 @@ def test_gemm_sm_cap_does_not_reject_the_lstm():
     assert g.device_status()[0] == 0
 
 
-# (T, B, H): every form of the transposed kernel and the edges of its tiles: 8, 12, 16 and 32 rows per group; a ragged last
+# (T, B, H): every form of the transposed kernel and the edges of its tiles: 4, 8, 12, 16 and 32 rows per group; a ragged last
 # group; fewer hidden units than a slice; a partial last slice; one to four CTAs per row group; one and two steps
 TMEM_SHAPES = [(1, 1, 32), (2, 9, 128), (9, 70, 128), (6, 17, 192), (5, 130, 416), (12, 512, 384), (7, 509, 384), (5, 512, 512),
-               (4, 500, 480), (6, 1024, 384), (5, 1000, 256)]
+               (4, 500, 480), (6, 1024, 384), (5, 1000, 256), (6, 300, 256), (5, 203, 384)]
 
 
 def test_transposed_kernel_forms_match_the_cooperative_kernel(tmp_path):
