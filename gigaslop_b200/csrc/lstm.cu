@@ -895,20 +895,20 @@ size_t lstm_scratch_bytes(long long B, int H) {
 }
 
 using LtKernel = void (*)(const CUtensorMap, const CUtensorMap, const uint8_t*, long long, const LstmParams);
-// The forms of the transposed kernel: batch rows per group, and what a step costs (B200, us at H = 128 / 256 / 384 / 512).
-//    4 rows  0.57 / 0.79 / 0.91 / 1.2       8 rows  0.72 / 0.96 / 1.09 / 1.40      12 rows  0.90 / 1.14 / 1.27 / 1.58
-//   16 rows  1.07 / 1.25 / 1.38 / 1.77     32 rows  1.77 / 2.11 / 2.21 / 2.68
-struct LtForm { int rows, threads, smem[LT_MAX_SLICES + 1], cost; LtKernel kernel; };
+// The forms of the transposed kernel: batch rows per group, and what a step takes (ns, measured on B200) on row groups of one
+// to four CTAs, i.e. at H = 128, 256, 384 and 512.
+struct LtForm { int rows, threads, smem[LT_MAX_SLICES + 1], step_ns[LT_MAX_SLICES + 1]; LtKernel kernel; };
 template <int R, int G, int CW>
-static constexpr LtForm lt_make_form(int cost) {
-  LtForm f{G, 32 * (CW + 4), {}, cost, lstm_tmem_kernel<R, G, CW>};
+static constexpr LtForm lt_make_form(int ns1, int ns2, int ns3, int ns4) {
+  LtForm f{G, 32 * (CW + 4), {}, {0, ns1, ns2, ns3, ns4}, lstm_tmem_kernel<R, G, CW>};
   // (at least 120 KiB: one CTA per SM, it takes all of tensor memory)
   for (int n = 1; n <= LT_MAX_SLICES; ++n) f.smem[n] = LtSmem<R, G>::bytes(n) > 120 * 1024 ? LtSmem<R, G>::bytes(n) : 120 * 1024;
   return f;
 }
 constexpr int LT_FORMS = 5;
-static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(8), lt_make_form<16, 8, 8>(10), lt_make_form<16, 12, 12>(12), lt_make_form<16, 16, 8>(13),
-                                          lt_make_form<32, 32, 16>(21)};
+static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(570, 790, 910, 1230), lt_make_form<16, 8, 8>(720, 960, 1090, 1400),
+                                          lt_make_form<16, 12, 12>(900, 1140, 1270, 1580), lt_make_form<16, 16, 8>(1070, 1250, 1380, 1770),
+                                          lt_make_form<32, 32, 16>(1770, 2110, 2210, 2680)};
 
 static cudaLaunchConfig_t lt_config(const LtForm& f, int slices, long long groups, cudaStream_t st, cudaLaunchAttribute* attr) {
   attr->id = cudaLaunchAttributeClusterDimension;
@@ -942,22 +942,23 @@ static int lt_capacity(int form, int slices, int dev) {
   return c > 0 ? c : 0;
 }
 
-// The form with the least waves x cost, row groups limited to `max_ctas` CTAs at a time (0 = the whole GPU); -1 = none.
-// Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows (43 groups,
-// 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (1.12 us per step and 512 rows; 12 rows in two
-// waves 1.28).
-static int lt_choose(long long B, int H, int dev, int max_ctas) {
+// The form with the shortest step (times the waves it takes), row groups limited to `max_ctas` CTAs at a time (0 = the whole
+// GPU); -1 = none.  Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows
+// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.24 us per step; 12 rows in two
+// waves 2.57).  *ns = the step.
+static int lt_choose(long long B, int H, int dev, int max_ctas, long long* ns = nullptr) {
   const int slices = (H + LT_HS - 1) / LT_HS;
   int best = -1;
-  long long best_cost = 0;
+  long long best_ns = 0;
   for (int i = 0; i < LT_FORMS; ++i) {
     int cap = lt_capacity(i, slices, dev);
     if (cap > 0 && max_ctas > 0 && cap > max_ctas / slices) cap = max_ctas / slices > 0 ? max_ctas / slices : 1;
     if (cap <= 0) continue;
     const long long groups = (B + kLtForms[i].rows - 1) / kLtForms[i].rows;
-    const long long cost = (groups + cap - 1) / cap * kLtForms[i].cost;
-    if (best < 0 || cost < best_cost) { best = i; best_cost = cost; }
+    const long long t = (groups + cap - 1) / cap * kLtForms[i].step_ns[slices];
+    if (best < 0 || t < best_ns) { best = i; best_ns = t; }
   }
+  if (ns) *ns = best_ns;
   return best;
 }
 
@@ -997,6 +998,29 @@ static int lstm_layer_ctas(long long B, int H, int max_ctas) {
   const int slices = (H + LT_HS - 1) / LT_HS, cap = lt_capacity(form, slices, dev);
   const long long groups = (B + kLtForms[form].rows - 1) / kLtForms[form].rows;
   return (int)(groups < cap ? groups : cap) * slices;
+}
+
+// How many launches to cut a layer's recurrence into so that the next layer's projection runs beside it (1 = not at all).
+// The cut recurrence keeps to `max_ctas` CTAs, which may cost it a form with longer steps, and every launch about 12 us;
+// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 16.2 ms one after the other, 15.3
+// in seven blocks; at B = 512, H = 512 (T = 1000, three layers) 6.9 ms against 9.0, so not cut.
+static int lstm_time_blocks(long long T, long long B, int H, int max_ctas) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || lstm_env() != 0) return 8;
+  long long whole = 0, limited = 0;
+  if (lt_choose(B, H, dev, 0, &whole) < 0 || lt_choose(B, H, dev, max_ctas, &limited) < 0) return 8;
+  const double proj = 10e3 + (double)T * (double)B * 9.0 * H / 5200.0;      // ns: fp16 [rows, 4H] written, E4M3 [rows, H] read at 5.2 TB/s
+  const double rest = proj * 0.6 * sm_count_physical() / (sm_count_physical() - max_ctas);   // ... beside the recurrence
+  double best = 0.98 * ((double)T * (double)whole + proj);                  // cut only for more than 2 %
+  int nb = 1;
+  for (int n = 2; n <= 8 && n <= T; ++n) {
+    double t = (double)T * (double)limited * 1.03;                          // (the projection beside it costs the step 3 %)
+    if (t < rest) t = rest;
+    t += proj / n + 12e3 * n;
+    if (t < best) { best = t; nb = n; }
+  }
+  return nb;
 }
 
 int32_t launch_lstm_layer(const LstmLayerArgs& a, void* scratch, size_t scratch_bytes, cudaStream_t st) {
@@ -1175,13 +1199,8 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
     if (!layers[l].w_ih || !layers[l].s_ih || !layers[l].w_hh || !layers[l].s_hh) return GSB200_ERR_BAD_ARG;
   bool overlap = aux != nullptr && aux != st && n_layers > 1;
   if (ws_bytes < lstm_stack_workspace_bytes(T, B, H, overlap ? 1 : 0)) return GSB200_ERR_BAD_ARG;
-  // Left to choose (time_blocks = 0) the layers run one after the other, each on the whole GPU: the recurrence with fewer
-  // rows per CTA gains what hiding the projection would.  Five layers, T = 2000, B = 512, H = 384: 16.4 ms, in eight blocks
-  // with the recurrence on 96 SMs and the projection on 52 16.3; three layers, T = 1000: B = 512, H = 512 7.1 against
-  // 9.3 ms, H = 256 3.7 / 4.3, H = 128 2.73 / 2.80, B = 200, H = 384 3.75 / 3.89.
-  overlap = overlap && time_blocks > 0;
-  int nb = overlap ? time_blocks : 1;
-  if (nb > T) nb = (int)T;
+  if (!overlap) time_blocks = 1;
+  if (time_blocks > T) time_blocks = (int)T;
   int32_t rc = ensure_device();
   if (rc != GSB200_OK) return rc;
 
@@ -1225,6 +1244,8 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
 
   // overlapped: the recurrence takes up to two thirds of the GPU, the projection what is left
   const int max_ctas = overlap ? sm_count_physical() * 2 / 3 : 0;
+  if (overlap && time_blocks <= 0) time_blocks = lstm_time_blocks(T, B, H, max_ctas);
+  const int blocks_cut = time_blocks;                // launches per layer that has another one behind it
   int gemm_cap = sm_count_physical() - lstm_layer_ctas(B, H, max_ctas);
   if (gemm_cap < 8) gemm_cap = 8;
   cudaError_t ce = cudaSuccess;
@@ -1232,6 +1253,7 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
     const bool last = l == n_layers - 1;
     const bool rev = ((l % 2) == 0) == (reverse_first != 0);
     uint8_t* h8_l = h8[l & 1];
+    const int nb = last ? 1 : blocks_cut;            // (nothing runs beside the last layer: one launch on the whole GPU)
     for (int k = 0; k < nb; ++k) {
       // block k in processing order covers steps [s0, s1); in time that is [t0, t1)
       const long long s0 = T * k / nb, s1 = T * (k + 1) / nb;
@@ -1247,11 +1269,11 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
       a.h_out = last ? h_out + (size_t)t0 * B * H : nullptr;
       a.h8_out = h8_l + (size_t)t0 * B * H;
       a.c_last = k + 1 < nb ? cst[k & 1] : nullptr;
-      a.max_ctas = max_ctas;
+      a.max_ctas = nb > 1 ? max_ctas : 0;
       a.T = t1 - t0; a.B = B; a.H = H; a.reverse = rev ? 1 : 0;
       rc = launch_lstm_layer(a, scratch, scratch_bytes, st);
       if (rc != GSB200_OK) return rc;
-      if (overlap && !last) {
+      if (!last && k + 1 < nb) {
         cudaEvent_t ev;
         ce = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
         if (ce != cudaSuccess) return cuda_status(ce, "lstm stack: event");
@@ -1261,21 +1283,19 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
         if (ce != cudaSuccess) return cuda_status(ce, "lstm stack: event");
         rc = project(l + 1, t0, t1, aux, gemm_cap);
         if (rc != GSB200_OK) return rc;
-      }
-    }
-    if (!last) {
-      if (overlap) {                     // the next layer starts when its whole projection is there
-        cudaEvent_t ev;
-        ce = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-        if (ce != cudaSuccess) return cuda_status(ce, "lstm stack: event");
-        ce = cudaEventRecord(ev, aux);
-        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, ev, 0);
-        cudaEventDestroy(ev);
-        if (ce != cudaSuccess) return cuda_status(ce, "lstm stack: event");
-      } else {
-        rc = project(l + 1, 0, T, st, 0);
+      } else if (!last) {                // nothing left to run beside: the whole GPU, in `st`
+        rc = project(l + 1, t0, t1, st, 0);
         if (rc != GSB200_OK) return rc;
       }
+    }
+    if (nb > 1) {                        // the next layer starts when its whole projection is there
+      cudaEvent_t ev;
+      ce = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+      if (ce != cudaSuccess) return cuda_status(ce, "lstm stack: event");
+      ce = cudaEventRecord(ev, aux);
+      if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, ev, 0);
+      cudaEventDestroy(ev);
+      if (ce != cudaSuccess) return cuda_status(ce, "lstm stack: event");
     }
   }
   return GSB200_OK;

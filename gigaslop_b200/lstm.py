@@ -43,9 +43,9 @@ def lstm_stack_workspace(T, B, H, device, overlap=False):
 def lstm_stack(x_fp8, sx, layers, T, B, reverse_first=True, workspace=None, aux_stream=None, time_blocks=0, out=None):
     """Stack of layers (dicts with W_ih, s_ih, b, W_hh, s_hh); even layers run reversed when ``reverse_first``.
     ``x_fp8`` E4M3 ``[T*B, C]`` with per-row scales ``sx``.  Returns the last layer's fp16 ``h`` ``[T*B, H]``.
-    One call into the library (``gsb200_lstm_stack_fp8``).  With ``aux_stream`` (a ``torch.cuda.Stream``) and
-    ``time_blocks`` > 0 the next layer's hoisted projection runs per time block beside the recurrence of the current
-    layer; ``time_blocks`` = 0 lets the library choose (it runs the layers one after the other); same bytes."""
+    One call into the library (``gsb200_lstm_stack_fp8``).  With ``aux_stream`` (a ``torch.cuda.Stream``) the next
+    layer's hoisted projection runs per time block beside the recurrence of the current layer; ``time_blocks`` = 0 lets
+    the library choose the cut (or none); same bytes."""
     from ._lib import LstmLayer
     H = layers[0]["W_hh"].shape[1]
     C = x_fp8.shape[1]

@@ -260,11 +260,11 @@ int32_t gsb200_lstm_layer_fp8(const void* ih, int64_t ld_ih, const uint8_t* w_hh
  * directions alternate (reverse_first != 0: layers 0, 2, ... walk t = T-1..0).  The reference keeps this loop in
  * its caller and replays two launches per timestep and layer from a graph (fly/bench_factored_lstm.py:82-85,104-121).
  * x [T*B, C] E4M3 with per-row scales sx[T*B]; layer 0 has w_ih [4H, C], the others [4H, H]; h_out fp16 [T*B, H] is
- * the last layer's output.  aux_stream (may be null): a second stream of the caller.  With it and time_blocks > 0 each
- * recurrence is cut into that many launches and the next layer's projection of a block's timesteps runs on aux_stream
+ * the last layer's output.  aux_stream (may be null): a second stream of the caller.  With it each recurrence but the
+ * last layer's is cut into time_blocks launches and the next layer's projection of a block's timesteps runs on aux_stream
  * beside the following block, on the SMs the recurrence leaves idle; the result is the same, bit for bit, and `stream` ends
- * up ordered after all of it.  time_blocks = 0 leaves the choice to the library, which runs the layers one after the other
- * on `stream` (the recurrence then has the whole GPU, which is as fast or faster at every measured shape).
+ * up ordered after all of it.  time_blocks = 0 leaves the choice to the library, which may also run the layers one after
+ * the other on `stream` (the recurrence then has the whole GPU).
  * workspace: gsb200_lstm_stack_workspace_bytes(T, B, H, overlap = aux_stream given) bytes, 256-byte aligned. */
 typedef struct {
   const uint8_t* w_ih; int64_t ld_w_ih; const float* s_ih;   /* input weights E4M3 K-major, per-channel scales [4H] */
