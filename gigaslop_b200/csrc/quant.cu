@@ -20,7 +20,7 @@ __device__ __forceinline__ void load8(const Tin* p, float (&v)[8]);
 
 template <>
 __device__ __forceinline__ void load8<__half>(const __half* p, float (&v)[8]) {
-  const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(p));
+  const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(p));
   const __half2* h = reinterpret_cast<const __half2*>(&raw);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -30,8 +30,8 @@ __device__ __forceinline__ void load8<__half>(const __half* p, float (&v)[8]) {
 }
 template <>
 __device__ __forceinline__ void load8<float>(const float* p, float (&v)[8]) {
-  const float4 a = __ldcg(reinterpret_cast<const float4*>(p));
-  const float4 b = __ldcg(reinterpret_cast<const float4*>(p + 4));
+  const float4 a = __ldcs(reinterpret_cast<const float4*>(p));
+  const float4 b = __ldcs(reinterpret_cast<const float4*>(p + 4));
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
@@ -107,6 +107,15 @@ __device__ __forceinline__ uint2 pack_e4m3_quot(const float (&v)[8], float s, fl
   return make_uint2((w[0] | (w[1] << 16)) ^ 0x80808080u, (w[2] | (w[3] << 16)) ^ 0x80808080u);
 }
 
+// This warp's row.  The rows are walked from the last to the first: the GEMMs walk theirs upwards, so a quantiser starts
+// with the rows its producer wrote last and leaves the rows its consumer reads first written last.  Where a tensor is
+// larger than L2 (126 MB) that is what is found there.  The input is read with the
+// streaming hint, so that it does not push the output out.  Feed-forward passes of 65536 rows: INT8 240.7 -> 234.2 us (walked
+// backwards) -> 229.1 (streaming hint), MXFP8 285 -> 281 -> 276.
+__device__ __forceinline__ long long quant_row() {
+  return (long long)(gridDim.x - 1 - blockIdx.x) * QUANT_WARPS + (threadIdx.x >> 5);
+}
+
 // FMT: 0 = int8, 1 = e4m3 kernel formulation, 2 = e4m3 torch formulation.
 // NV > 0: the row (<= NV*256 elements) is cached in registers.  NV == 0: any K, second pass re-reads.
 template <typename Tin, int FMT, int NV>
@@ -114,7 +123,7 @@ __global__ void __launch_bounds__(QUANT_WARPS * 32)
 ptq_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q, long long ldq,
            float* __restrict__ scale, long long M, int K) {
   const int lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * QUANT_WARPS + (threadIdx.x >> 5);
+  const long long row = quant_row();
   pdl_wait();
   pdl_trigger();
   if (row >= M) return;
@@ -134,7 +143,7 @@ ptq_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q, lo
     for (int i = 0; i < NV; ++i) {
       const int v = lane + 32 * i;
       raw[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (v < nvec) raw[i] = __ldcg(reinterpret_cast<const uint4*>(xr + v * 8));
+      if (v < nvec) raw[i] = __ldcs(reinterpret_cast<const uint4*>(xr + v * 8));
       const __half2* h = reinterpret_cast<const __half2*>(&raw[i]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -250,7 +259,7 @@ __global__ void __launch_bounds__(QUANT_WARPS * 32)
 ptq_mx_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q, long long ldq,
               uint8_t* __restrict__ scales, long long lds, long long M, int K) {
   const int lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * QUANT_WARPS + (threadIdx.x >> 5);
+  const long long row = quant_row();
   pdl_wait();
   pdl_trigger();
   if (row >= M) return;
@@ -266,7 +275,7 @@ ptq_mx_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q,
 #pragma unroll
       for (int w = 0; w < WORDS; ++w) {
         raw[i][w] = make_uint4(0u, 0u, 0u, 0u);
-        if (v < nvec) raw[i][w] = __ldcg(reinterpret_cast<const uint4*>(xr + v * 8) + w);
+        if (v < nvec) raw[i][w] = __ldcs(reinterpret_cast<const uint4*>(xr + v * 8) + w);
       }
     }
 #pragma unroll
