@@ -378,6 +378,148 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, MX_TMEM_COLS); }
 }
 
+// ---- streaming form with 256-column tiles (plain GEMM, K > 512) ---------------------------------------------------
+// With both operands streamed the 128 x 128 form above waits for its operands: 33 KiB per K block and 64 tensor clocks per
+// MMA, while about 55 bytes per clock arrive (600 clocks per K block).  A 128 x 256 tile brings twice the products for 1.5
+// times the bytes.  Its accumulator takes 256 TMEM columns, which leaves room for the scale factors but not for a second
+// stage; the epilogue hands it back once it is in registers (a few hundred clocks of the tile's >= 10^4).
+//   warps 0, 3  producers: K block i of the CTA goes to ring stage i % 4, filled by warp 0 (even) or 3 (odd)
+//   warp 1      MMA issue        warps 4..11  epilogue: lane quarter e % 4, column half e / 4
+// M = 65536, N = 512, K = 2048: 71.8 us with 128 columns, 63.7 with 256; M = 9001 11.3 and 9.9; M = 30000 37.1 and 31.3.
+constexpr int MX2_BN = 256;
+constexpr int MX2_STAGES = 4;
+constexpr int MX2_B_BYTES = MX2_BN * MX_BK;                                      // 32 KiB
+constexpr int MX2_STAGE_BYTES = MX_A_BYTES + MX2_B_BYTES + 4 * MX_SF_BYTES;      // A | W | SFA | SFB0 | SFB1 | pad
+constexpr int MX2_OUT = MX2_STAGES * MX2_STAGE_BYTES;
+constexpr int MX2_BAR = MX2_OUT + MX_EPI_WARPS * MX_OUT_BUF;
+constexpr int MX2_BYTES = MX2_BAR + 256 + 1024;
+static_assert(MX2_STAGE_BYTES % 1024 == 0 && MX2_BYTES <= 227 * 1024, "shared memory budget");
+
+__global__ void __launch_bounds__(MX_THREADS, 1)
+mx_gemm256_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
+                  const __grid_constant__ CUtensorMap tm_c, const MxParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + MX2_BAR);
+  uint64_t* full = bars;                                   // [MX2_STAGES]
+  uint64_t* empty = bars + MX2_STAGES;                     // [MX2_STAGES]
+  uint64_t* acc_full = bars + 2 * MX2_STAGES;
+  uint64_t* acc_empty = acc_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+  const AbortFlag abort_flag{smem_u32(tmem_slot + 1)};
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int num_tiles = p.m_blocks * p.n_blocks;           // (the host keeps this below 2^31)
+  const int nb128_all = (p.N + 127) / 128;                 // scale tile row blocks of W
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < MX2_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(acc_full, 1); mbar_init(acc_empty, MX_EPI_WARPS);
+    abort_flag.set(0);
+    fence_mbar_init();
+    prefetch_tmap(&tm_a); prefetch_tmap(&tm_b); prefetch_tmap(&tm_c);
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, MX_TMEM_COLS); tmem_relinquish(); }
+  pdl_wait();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const unsigned int budget = spin_budget();
+
+  if (warp == 0 || warp == 3) {
+    if (lane == 0) {
+      const int mine = warp == 3 ? 1 : 0;
+      bool ok = true;
+      int i = 0;                                           // K blocks of this CTA so far
+      for (int t = blockIdx.x; ok && t < num_tiles; t += gridDim.x) {
+        const int m_blk = t / p.n_blocks, n_blk = t % p.n_blocks;
+        const int nb128 = 2 * n_blk;
+        const bool two = nb128 + 1 < nb128_all;            // the second 128 columns have scale tiles
+        for (int kb = 0; kb < p.k_blocks; ++kb, ++i) {
+          if ((i & 1) != mine) continue;
+          const int st_i = i & (MX2_STAGES - 1);
+          if (!mbar_wait(&empty[st_i], ((uint32_t)(i / MX2_STAGES) & 1u) ^ 1u, abort_flag, ST_TIMEOUT_PRODUCER, 0xB00 | st_i, budget)) { ok = false; break; }
+          uint8_t* st = smem + st_i * MX2_STAGE_BYTES;
+          uint8_t* sf = st + MX_A_BYTES + MX2_B_BYTES;
+          mbar_arrive_expect_tx(&full[st_i], MX_A_BYTES + MX2_B_BYTES + (two ? 3 : 2) * MX_SF_BYTES);
+          tma_load_2d(st, &tm_a, &full[st_i], kb * MX_BK, m_blk * MX_BM);
+          tma_load_2d(st + MX_A_BYTES, &tm_b, &full[st_i], kb * MX_BK, n_blk * MX2_BN);
+          bulk_load(sf, p.sfa + ((size_t)m_blk * p.k_blocks + kb) * MX_SF_BYTES, MX_SF_BYTES, &full[st_i]);
+          bulk_load(sf + MX_SF_BYTES, p.sfb0 + ((size_t)nb128 * p.k_blocks + kb) * MX_SF_BYTES, MX_SF_BYTES, &full[st_i]);
+          if (two) bulk_load(sf + 2 * MX_SF_BYTES, p.sfb0 + ((size_t)(nb128 + 1) * p.k_blocks + kb) * MX_SF_BYTES, MX_SF_BYTES, &full[st_i]);
+        }
+      }
+      if (!ok) { const long long t0 = clock64(); while (clock64() - t0 < 2000000) { } }
+    }
+  } else if (warp == 1) {
+    // the whole warp walks the loop, one lane of it issues (a single thread: 65.2 us instead of 63.7)
+    bool ok = true;
+    int i = 0, it = 0;
+    for (int t = blockIdx.x; ok && t < num_tiles; t += gridDim.x, ++it) {
+      if (!__all_sync(0xffffffffu, mbar_wait(acc_empty, (uint32_t)(it & 1) ^ 1u, abort_flag, ST_TIMEOUT_MMA, 0xB10, budget))) { ok = false; break; }
+      tc_fence_after();
+      for (int kb = 0; kb < p.k_blocks; ++kb, ++i) {
+        const int st_i = i & (MX2_STAGES - 1);
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[st_i], (uint32_t)(i / MX2_STAGES) & 1u, abort_flag, ST_TIMEOUT_MMA, 0xB20 | st_i, budget))) { ok = false; break; }
+        const uint32_t st = smem_u32(smem + st_i * MX2_STAGE_BYTES);
+        const uint32_t sf = st + MX_A_BYTES + MX2_B_BYTES;
+        const uint32_t sfa_t = tmem_base + MX_SF_COL + st_i * 16, sfb_t = sfa_t + 4;     // a slot per stage
+        tmem_cp_32x128b_warpx4_elect(sfa_t, sf_smem_desc(sf));
+        tmem_cp_32x128b_warpx4_elect(sfb_t, sf_smem_desc(sf + MX_SF_BYTES));
+        tmem_cp_32x128b_warpx4_elect(sfb_t + 4, sf_smem_desc(sf + 2 * MX_SF_BYTES));
+        const uint64_t a_desc = umma_smem_desc_sw128(st);
+        const uint64_t b_desc = umma_smem_desc_sw128(st + MX_A_BYTES);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_mxf8_elect(tmem_base, a_desc + 2 * k, b_desc + 2 * k, umma_idesc_mx(0, 0, MX_BM, MX2_BN, k, k), sfa_t, sfb_t, (kb | k) != 0);
+        umma_commit_elect(&empty[st_i]);
+      }
+      if (ok) umma_commit_elect(acc_full);
+    }
+  } else if (warp >= MX_FRONT_WARPS) {
+    const int e = warp - MX_FRONT_WARPS, q = warp & 3, half = e >> 2;
+    uint8_t* out_buf = smem + MX2_OUT + e * MX_OUT_BUF;
+    int it = 0;
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+      const int m_blk = t / p.n_blocks, n0 = (t % p.n_blocks) * MX2_BN + half * 128;
+      if (!__all_sync(0xffffffffu, mbar_wait(acc_full, (uint32_t)it & 1u, abort_flag, ST_TIMEOUT_EPILOGUE, 0xB30, budget))) break;
+      tc_fence_after();
+      const int row_base = m_blk * MX_BM + q * 32;
+      const uint32_t t_row = tmem_base + half * 128 + ((uint32_t)(q * 32) << 16);
+      uint32_t v[4][32];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) tmem_ld_32x32b_x32(t_row + 32 * b, v[b]);
+      tmem_ld_wait(v[0], v[1]);
+      tmem_ld_wait(v[2], v[3]);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty);
+      if (row_base >= p.M) continue;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int n = n0 + 32 * b;
+        if (n >= p.N) break;
+        if (lane == 0) tma_store_wait_read<0>();             // the previous box has left the buffer
+        __syncwarp();
+#pragma unroll
+        for (int pc = 0; pc < 4; ++pc)
+          *reinterpret_cast<uint4*>(out_buf + lane * 64 + ((pc ^ ((lane >> 1) & 3)) << 4)) =
+              make_uint4(pack_half2(__uint_as_float(v[b][8 * pc]), __uint_as_float(v[b][8 * pc + 1])),
+                         pack_half2(__uint_as_float(v[b][8 * pc + 2]), __uint_as_float(v[b][8 * pc + 3])),
+                         pack_half2(__uint_as_float(v[b][8 * pc + 4]), __uint_as_float(v[b][8 * pc + 5])),
+                         pack_half2(__uint_as_float(v[b][8 * pc + 6]), __uint_as_float(v[b][8 * pc + 7])));
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) { tma_store_2d(&tm_c, out_buf, n, row_base); tma_store_commit(); }
+      }
+    }
+    if (lane == 0) tma_store_wait_all<0>();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, MX_TMEM_COLS); }
+}
+
 // ---- row-major [rows, K/32] scales -> the 128 x 4 tile order --------------------------------------------------
 // A thread moves the four scales of one row and one 128-wide K tile: one word of the tile, four neighbouring source bytes
 // (K % 128 == 0, so a row holds whole groups of four).  Consecutive threads write consecutive words; the 32 rows of a
@@ -443,6 +585,8 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
     cudaError_t e3 = cudaFuncSetAttribute(mx_gemm_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxSmem<true>::BYTES);
     cudaError_t e4 = cudaFuncSetAttribute(mx_gemm_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MxSmem<true>::BYTES);
     if (e1 != cudaSuccess || e2 != cudaSuccess) return cuda_status(e1 != cudaSuccess ? e1 : e2, "cudaFuncSetAttribute(mx gemm)");
+    cudaError_t e5 = cudaFuncSetAttribute(mx_gemm256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MX2_BYTES);
+    if (e5 != cudaSuccess) return cuda_status(e5, "cudaFuncSetAttribute(mx gemm)");
     if (e3 != cudaSuccess || e4 != cudaSuccess) return cuda_status(e3 != cudaSuccess ? e3 : e4, "cudaFuncSetAttribute(mx gemm)");
     attr_done[dev].store(1, std::memory_order_release);
   }
@@ -474,6 +618,17 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
     const int grid = groups * p.n_blocks;
     if (dual) e = launch_dependent(mx_gemm_kernel<true, true>, grid, MX_THREADS, MxSmem<true>::BYTES, st, ta, tb0, tb1, tc, p);
     else e = launch_dependent(mx_gemm_kernel<false, true>, grid, MX_THREADS, MxSmem<true>::BYTES, st, ta, tb0, tb1, tc, p);
+    return cuda_status(e, "mx gemm launch");
+  }
+  // 256-column tiles where their rounds are cheaper: a K block takes about 1.65 times what it takes with 128 columns, so few
+  // tiles and an N just above a multiple of 256 stay with 128 (M = 65536, N = 384, K = 1536: 45.1 us, with 256 columns 46.3).
+  const long long sms = sm_count(), tiles256 = (long long)p.m_blocks * ((N + MX2_BN - 1) / MX2_BN);
+  if (!dual && (tiles256 + sms - 1) / sms * 33 < (tiles + sms - 1) / sms * 20 && tiles256 <= 0x7fffffffll) {
+    CUtensorMap tb;
+    if (!map2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, MX2_BN, CU_TENSOR_MAP_SWIZZLE_128B))
+      return GSB200_ERR_BAD_ARG;
+    p.n_blocks = (N + MX2_BN - 1) / MX2_BN;
+    e = launch_dependent(mx_gemm256_kernel, (int)(tiles256 < sms ? tiles256 : sms), MX_THREADS, MX2_BYTES, st, ta, tb, tc, p);
     return cuda_status(e, "mx gemm launch");
   }
   const int grid = (int)(tiles < sm_count() ? tiles : sm_count());

@@ -122,3 +122,24 @@ def test_mx_ffn_chain():
     ref = oracle.mx_gemm_ref(hq.cpu(), hs.cpu(), Wd[0], Wd[1])         # oracle fed with the device's own MXFP8 activations
     from util import assert_close
     assert_close(y, ref.half(), atol=float(ref.abs().max()) * 2 ** -9, rtol=2e-2, what="MX down-projection")
+
+
+# shapes that take the 256-column tiles (enough tiles, K > 512): column tails with one and with two scale tiles in the last
+# tile, ragged rows, K blocks that do not divide the ring, one and several tiles per CTA
+@pytest.mark.parametrize("M,N,K", [(9001, 384, 640), (9088, 512, 768), (19000, 480, 640), (37889, 512, 1152), (18945, 512, 2048)])
+def test_block_scaled_gemm_256_column_tiles(M, N, K):
+    g = need_lib()
+    gen = torch.Generator().manual_seed(M + N + K)
+    Aq, As = mx_operand(gen, M, K)
+    Wq, Ws = mx_operand(gen, N, K)
+    c = g.gemm_mxfp8(Aq.cuda(), g.mx_scales_to_tiled(As.cuda(), K), Wq.cuda(), g.mx_scales_to_tiled(Ws.cuda(), K))
+    torch.cuda.synchronize()
+    assert g.device_status()[0] == 0
+    # the same rows in a call small enough for the 128-column tiles: the same sums in the same order, the same bytes
+    from util import assert_close
+    for lo in (0, 5000, M - 300):
+        Ar, Sr = Aq[lo:lo + 300].contiguous(), As[lo:lo + 300].contiguous()
+        part = g.gemm_mxfp8(Ar.cuda(), g.mx_scales_to_tiled(Sr.cuda(), K), Wq.cuda(), g.mx_scales_to_tiled(Ws.cuda(), K))
+        ref = oracle.mx_gemm_ref(Ar, Sr, Wq, Ws)
+        assert_close(c[lo:lo + 300], ref.half(), atol=float(ref.abs().max()) * 2 ** -9, rtol=2e-2, what="256-column tiles")
+        assert torch.equal(part, c[lo:lo + 300])
