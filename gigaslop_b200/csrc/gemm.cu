@@ -478,6 +478,15 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
     grid = (int)(sched_tiles < sms ? sched_tiles : sms);
   }
   cudaError_t e = cudaErrorInvalidValue;
+  // The SwiGLU that emits MXFP8, weight-stationary: twelve warps, staged output (M = 65536, K = 512, N = 2048: 145 us with
+  // eight warps and 32-byte stores per thread and row, 114 now; K = 384, N = 1536 109 and 73; M = 9001 26.7 and 20.6; equal at
+  // a few hundred rows).
+  if (a.epi == EPI_SILU_MX && resident && variant_setting(g_variant_ew, "GSB200_GEMM_EW") != 8 &&
+      Variant<KIND_F8, EPI_SILU_MX, false, 12>::capacity(true)) {
+    if (!make_map_2d(&tc, u8, 1, a.C, (uint64_t)a.M, (uint64_t)a.N, (uint64_t)a.ldc, 64, 32, CU_TENSOR_MAP_SWIZZLE_64B)) return GSB200_ERR_BAD_ARG;
+    e = Variant<KIND_F8, EPI_SILU_MX, false, 12>::launch(ta, tb0, tb1, tc, p, grid, true, st);
+    return cuda_status(e, "gemm launch");
+  }
   if (pair || ew12) {
     if (pair) grid *= 2;
     // the twelve-warp form stores a warp's 32 rows x 64 columns as ONE box

@@ -297,7 +297,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using Map = SmemMap<SCHED, PAIR, EW>;
-  static_assert(EW == EPI_WARPS || (EW == 12 && !FUSEQ && (EPI == EPI_DEQUANT || EPI == EPI_ROTARY || EPI == EPI_SILU)),
+  static_assert(EW == EPI_WARPS || (EW == 12 && !FUSEQ && (EPI == EPI_DEQUANT || EPI == EPI_ROTARY || EPI == EPI_SILU || EPI == EPI_SILU_MX)),
                 "twelve epilogue warps: built for the dequant, rotary and SwiGLU epilogues");
   constexpr int NTHREADS = 32 * (FRONT_WARPS + EW);
   // EW = 12: the epilogue's unit of work is an ITEM, 32 rows x 64 output columns.  Every epilogue warp hands every
@@ -782,6 +782,65 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 #pragma unroll
           for (int k = 0; k < 4; ++k) put(4 + k, dequant_piece<KIND>(&vb[8 * k], sa2, lds_f4_ro(sc + 128 + 32 * k), lds_f4_ro(sc + 128 + 32 * k + 16)));
           stage_end();
+        } else if constexpr (EPI == EPI_SILU_MX) {
+          // The arithmetic of the eight-warp form (below), a 32-column block at a time; the elements leave as one 32-row x
+          // 64-byte box (64-byte swizzle) instead of 32 bytes per thread and row, the two scales as one 2-byte store.
+          const uint32_t scg = sc_tile + 64 * c * 4, scu = scg + (BN / 2) * 4;
+          const float2 sah2 = pk2(0.5f * sa, 0.5f * sa);
+          uint32_t ebs = 0;
+#pragma unroll 1
+          for (int blk = 0; blk < 2; ++blk) {
+            float2 o[16];
+            float amax = 0.f;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t g[16], u[16];
+              tmem_ld_32x32b_x16(t_tile + 64 * c + 32 * blk + 16 * h, g);
+              tmem_ld_32x32b_x16(t_tile + BN / 2 + 64 * c + 32 * blk + 16 * h, u);
+              tmem_ld_wait(g, u);
+              if (h == 1 && blk == 1) release();
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const uint32_t off = (32 * blk + 16 * h + 4 * k) * 4;
+                const float4 sg = lds_f4_ro(scg + off), su = lds_f4_ro(scu + off);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                  const float2 s2g = i ? make_float2(sg.z, sg.w) : make_float2(sg.x, sg.y), s2u = i ? make_float2(su.z, su.w) : make_float2(su.x, su.y);
+                  const float2 hv = dequant2<KIND>(g[4 * k + 2 * i], g[4 * k + 2 * i + 1], sah2, s2g);
+                  const float2 uv = dequant2<KIND>(u[4 * k + 2 * i], u[4 * k + 2 * i + 1], sa2, s2u);
+                  const float2 ov = fmul2(silu_from_half2(hv), uv);
+                  o[8 * h + 2 * k + i] = ov;
+                  amax = fmaxf(amax, fmaxf(fabsf(ov.x), fabsf(ov.y)));
+                }
+              }
+            }
+            int eb = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 8;
+            eb = max(0, min(254, eb));
+            ebs |= (uint32_t)eb << (8 * blk);
+            const float inv = __uint_as_float((uint32_t)(254 - eb) << 23);
+            const float2 inv2 = pk2(inv, inv);
+            uint32_t w[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const uint32_t lo = __nv_cvt_float2_to_fp8x2(fmul2(o[2 * k], inv2), __NV_SATFINITE, __NV_E4M3);
+              const uint32_t hi = __nv_cvt_float2_to_fp8x2(fmul2(o[2 * k + 1], inv2), __NV_SATFINITE, __NV_E4M3);
+              w[k] = lo | (hi << 16);
+            }
+            if (blk == 0) stage_begin();
+#pragma unroll
+            for (int pc = 0; pc < 2; ++pc)
+              *reinterpret_cast<uint4*>(out_buf + lane * 64 + (((2 * blk + pc) ^ ((lane >> 1) & 3)) << 4)) =
+                  make_uint4(w[4 * pc], w[4 * pc + 1], w[4 * pc + 2], w[4 * pc + 3]);
+          }
+          stage_end();
+          if (row_base + lane < p.M) {
+            uint8_t* dst = p.out_scale + (long long)(row_base + lane) * p.ld_scale + (n >> 5);
+            if (n + 64 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 1) == 0) *reinterpret_cast<uint16_t*>(dst) = (uint16_t)ebs;
+            else {
+              dst[0] = (uint8_t)ebs;
+              if (n + 64 <= p.N) dst[1] = (uint8_t)(ebs >> 8);
+            }
+          }
         } else if constexpr (EPI == EPI_SILU) {
           // gate columns 64 c .. 64 c + 63 of the tile's first half, the matching up columns BN / 2 further on
           const uint32_t scg = sc_tile + 64 * c * 4, scu = scg + (BN / 2) * 4;

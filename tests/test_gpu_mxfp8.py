@@ -143,3 +143,28 @@ def test_block_scaled_gemm_256_column_tiles(M, N, K):
         ref = oracle.mx_gemm_ref(Ar, Sr, Wq, Ws)
         assert_close(c[lo:lo + 300], ref.half(), atol=float(ref.abs().max()) * 2 ** -9, rtol=2e-2, what="256-column tiles")
         assert torch.equal(part, c[lo:lo + 300])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 32, 128), (129, 96, 512), (333, 480, 96), (2000, 2048, 512), (700, 160, 384), (20000, 512, 128)])
+def test_dual_silu_mxfp8_epilogue_forms_agree(M, N, K):
+    """The twelve-warp form (staged boxes, both scales of an item in one store where aligned) against the eight-warp form:
+    the same bytes, with N ending inside a 64-column item, odd scale rows and an output that is a slice of a wider buffer."""
+    g = need_lib()
+    gen = torch.Generator().manual_seed(M + N + K)
+    A = (torch.randn(M, K, generator=gen) * 100).clamp(-448, 448).to(torch.float8_e4m3fn).cuda()
+    W = [(torch.randn(N, K, generator=gen) * 100).clamp(-448, 448).to(torch.float8_e4m3fn).cuda() for _ in range(2)]
+    sa, sg, su = [(1e-4 + 1e-3 * torch.rand(n, generator=gen)).cuda() for n in (M, N, N)]
+    res = []
+    try:
+        for ew in (8, -1):
+            assert g.lib().gsb200_set_gemm_variant(ew, -1) == 0
+            q = torch.zeros(M, N + 32, dtype=torch.uint8, device="cuda")
+            s = torch.zeros(M, N // 32 + 3, dtype=torch.uint8, device="cuda")
+            g.dual_gemm_fp8_silu_mxfp8(A, W[0], W[1], sa, sg, su, out=q[:, :N], out_scale=s[:, :N // 32])
+            res.append((q, s))
+    finally:
+        g.lib().gsb200_set_gemm_variant(-1, -1)
+    torch.cuda.synchronize()
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    assert int(res[1][0][:, N:].count_nonzero()) == 0 and int(res[1][1][:, N // 32:].count_nonzero()) == 0
+    assert g.device_status()[0] == 0
