@@ -95,7 +95,6 @@ static bool make_map_2d(CUtensorMap* m, CUtensorMapDataType dt, int esz, const v
 // Atomics: the contract allows one host thread per GPU, and two of them may meet here.
 constexpr int kMaxDevices = 64;
 constexpr int kVariantMinRowBlocks = 256;      // 128-row blocks from which the twelve-warp form is the default for the SwiGLU
-constexpr int kPairMinRowBlocks = 16;          // ... and from which the streaming schedule runs as CTA pairs (measured down to M = 2048)
 static std::atomic<int> g_dev_ok[kMaxDevices];       // 0 unknown, 1 ok, -1 unsupported
 static std::atomic<int> g_dev_sms[kMaxDevices];
 
@@ -411,7 +410,8 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
     // Defaults, from measurements at the benchmark's sizes: twelve warps pay for the weight-stationary SwiGLU (the
     // heaviest epilogue per output), pairs for the streaming schedule with any of the three epilogues (K > 512: both
     // operands come from L2 for every tile, a single CTA asks for 96 bytes per clock where about 64 arrive, and a
-    // pair halves the W part: 12-22 % at M = 65536); the activation-stationary rotary kernel takes both together (twelve
+    // pair halves the W part: 12-22 % at M = 65536) from the point where single CTAs would need a second round (up to
+    // there they are faster: M = 9001, N = 512, K = 2048 9.5 us against 10.8); the activation-stationary rotary kernel takes both together (twelve
     // warps alone leave it waiting for operands, pairs alone for its epilogue; together 3 % at config 2 and less
     // power); everywhere else the eight-warp single-CTA kernel is as fast or faster.
     const int ew = variant_setting(g_variant_ew, "GSB200_GEMM_EW"), pm = variant_setting(g_variant_pair, "GSB200_GEMM_PAIR");
@@ -425,7 +425,7 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
     const bool both = rotary_both || huge_dequant_both;
     ew12 = ew < 0 ? ((a.epi == EPI_SILU && resident && big) || both) : ew == 12;
     const bool want_pair = p.k_blocks >= 2 && sms >= 2 &&
-                           (pm < 0 ? ((!resident && p.m_blocks >= kPairMinRowBlocks) || (both && ew12)) : pm == 1);
+                           (pm < 0 ? ((!resident && tiles > sms) || (both && ew12)) : pm == 1);
     if (ew12 && !variant_dispatch(a.kind, a.epi, false, true, false, ta, tb0, tb1, tc, p, 0, resident, st)) ew12 = false;
     if (want_pair) {
       int cap = variant_dispatch(a.kind, a.epi, true, ew12, false, ta, tb0, tb1, tc, p, 0, resident, st);
@@ -450,28 +450,20 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
     // (not for the bias epilogue: the low-rank projection reads its A from inside the output rows it writes, which
     // only works while one CTA owns a row block)
     if (!fused && a.epi == EPI_ROTARY && !(a.flags & GSB200_FLAG_OWN_ROW_BLOCKS)) {
-      if (resident) {
-        // The row blocks of the last, incomplete round are cut into shares of consecutive column blocks, as many as let
-        // the round end soonest; with fewer row blocks than CTAs it is the only round.  K = 512, N = 1536: M = 333 takes
-        // 7.8 us instead of 18.8, M = 2048 8.3 instead of 19.2.
-        const int rem = p.m_blocks % sms;
-        if (rem > 0) {
-          int best = p.n_blocks;                     // tiles a CTA walks in the round: one share, the whole row block
-          for (int S = 2; S <= p.n_blocks && S <= sms; ++S) {
-            const int per = (p.n_blocks + S - 1) / S, shares = (p.n_blocks + per - 1) / per;
-            const long long t = ((long long)rem * shares + sms - 1) / sms * per;
-            if (shares == S && t < best) { best = (int)t; p.ares_split = S; }
-          }
-          if (p.m_blocks < sms) grid = rem * p.ares_split < sms ? rem * p.ares_split : sms;
+      // The row blocks of the last, incomplete round are cut into shares of consecutive column blocks, as many as let the
+      // round end soonest; with fewer row blocks than CTAs it is the only round.  K = 512, N = 1536: M = 333 takes 7.8 us
+      // instead of 18.8, M = 2048 8.3 instead of 19.2.  (Single tiles in turn would balance as well, but a CTA would fetch
+      // sin / cos rows for every tile: 4096 scattered 16-byte reads, as long as the tile's products at K = 768.  A share is
+      // charged half a tile for them.  M = 20001: K = 768 52 -> 37 us, K = 1024 69 -> 53.)
+      const int rem = p.m_blocks % sms;
+      if (rem > 0) {
+        long long best = 2 * p.n_blocks + 1;         // half tiles of a CTA in the round with one share, the whole row block
+        for (int S = 2; S <= p.n_blocks && S <= sms; ++S) {
+          const int per = (p.n_blocks + S - 1) / S, shares = (p.n_blocks + per - 1) / per;
+          const long long t = ((long long)rem * shares + sms - 1) / sms * (2 * per + 1);
+          if (shares == S && t < best) { best = t; p.ares_split = S; }
         }
-      } else if (sched_tiles <= 0x7fffffffll) {
-        // both operands streamed: whole row blocks per CTA (the sin / cos rows are fetched once) only while that keeps the
-        // CTAs about as busy as single tiles do
-        const long long by_row = (long long)((p.m_blocks + sms - 1) / sms) * p.n_blocks, by_tile = (sched_tiles + sms - 1) / sms;
-        if (by_tile * 10 < by_row * 9) {
-          p.m_major = 0;
-          grid = (int)(sched_tiles < sms ? sched_tiles : sms);
-        }
+        if (p.m_blocks < sms) grid = rem * p.ares_split < sms ? rem * p.ares_split : sms;
       }
     }
   } else {

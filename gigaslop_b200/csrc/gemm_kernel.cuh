@@ -123,7 +123,7 @@ struct GemmParams {
   int m_blocks, n_blocks, k_blocks;
   int n_groups;                // WRES: number of row-block groups (grid = n_groups * n_blocks)
   int m_major;                 // STREAM: a CTA walks all column blocks of a row block before the next (ARES always does)
-  int ares_split;              // ARES: shares that each row block of the last, incomplete round is cut into (1 = none)
+  int ares_split;              // row-block-major walks: shares that each row block of the last, incomplete round is cut into (1 = none)
   void* C;                     // output base (direct-store path and int32 output)
   uint8_t* out_scale;          // EPI_SILU_MX: E8M0 scales [M, N/32]
   long long ld_scale;          //              row stride of out_scale in bytes
@@ -230,8 +230,7 @@ struct TileWalk {
   int n_lo, n_hi;  // row-block-major walks: this CTA's column blocks of row block m are [n_lo, n_hi)
   int visit;       // row-block-major walks: how many row blocks this CTA has left behind
   // Row blocks cta, cta + grid, ... while whole rounds last.  The row blocks left over (fewer than CTAs) would
-  // keep some SMs busy for a whole row block while the others idle: with the activation-stationary schedule each of
-  // them is cut into p.ares_split shares of consecutive column blocks (none empty; the host sees to that), which are
+  // keep some SMs busy for a whole row block while the others idle: with the rotary epilogue each of them is cut into p.ares_split shares of consecutive column blocks (none empty; the host sees to that), which are
   // dealt to the CTAs in turn (each loads the A block).
   __device__ __forceinline__ void set_visit(const GemmParams& p) {
     const int grid = ncta(), full = p.m_blocks / grid, rem = p.m_blocks - full * grid;
@@ -240,7 +239,7 @@ struct TileWalk {
     if (visit < full) {
       m = cta() + visit * grid;
     } else {
-      const int S = (SCHED == SCHED_ARES && p.ares_split > 1) ? p.ares_split : 1;
+      const int S = p.ares_split > 1 ? p.ares_split : 1;
       const int per = (p.n_blocks + S - 1) / S;
       const int u = cta() + (visit - full) * grid;
       if (u < rem * S) {
