@@ -6,7 +6,7 @@
 // this library); h feeds the recurrent GEMM as E4M3 at the fixed scale 1/448 (the reference's convention for a
 // value bounded by 1, fly/rdna_fp8_factored_lstm.py:321-326); c and the emitted h are fp16.
 //
-// Three kernels with the same arithmetic, and the same order of the K blocks, so that they give the same bytes:
+// Three kernels with the same arithmetic, and the same order of the sums (K = 0 .. H - 1), so that they give the same bytes:
 //   lstm_tmem_kernel       what runs: W_hh in tensor memory, gates^T = W_hh . h^T, h exchanged between at most four CTAs
 //   lstm_cluster_kernel    H <= 384, 128 batch rows x 32 hidden units per CTA, h through distributed shared memory
 //   lstm_recurrent_kernel  H <= 512, the same tile, h through global memory (cooperative launch)
@@ -207,12 +207,11 @@ lstm_recurrent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     if (tid == 0) {
       tc_fence_after();
       constexpr uint32_t idesc = umma_idesc(1, 0, 0, LSTM_ROWS, LSTM_NCOL);
-      for (int n = 0, kb = hid0 >> 7; n < p.k_blocks; ++n) {        // (the K order of the transposed form)
+      for (int kb = 0; kb < p.k_blocks; ++kb) {
         const uint64_t a_desc = umma_smem_desc_sw128(smem_u32(h_s + kb * LSTM_KB_BYTES));
         const uint64_t b_desc = umma_smem_desc_sw128(smem_u32(w_s + kb * LSTM_KB_BYTES));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) umma_f8(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (n | k) != 0);
-        if (++kb == p.k_blocks) kb = 0;
+        for (int k = 0; k < 4; ++k) umma_f8(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
       }
       umma_commit(mma_done);
     }
@@ -433,11 +432,9 @@ lstm_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     const uint64_t a_desc = buf ? a_base[1] : a_base[0];
     const int ksteps = H >> 5;                        // 32 bytes of K per MMA
     tc_fence_after();
-    for (int n = 0, ks = (hid0 >> 7) * 4; n < ksteps; ++n) {         // (the K order of the transposed form)
+    for (int ks = 0; ks < ksteps; ++ks)
       umma_f8(tmem_base, a_desc + (uint64_t)(ks * (2 * LSTMC_CHUNK >> 4)),
-              b_base + (uint64_t)((ks >> 2) * (LSTM_KB_BYTES >> 4) + 2 * (ks & 3)), idesc, n != 0);
-      if (++ks == ksteps) ks = 0;
-    }
+              b_base + (uint64_t)((ks >> 2) * (LSTM_KB_BYTES >> 4) + 2 * (ks & 3)), idesc, ks != 0);
     umma_commit(mma_done);
   };
   if (tid == LSTMC_MMA_TID && ok && p.T > 0) issue_mmas(1);       // step 0 reads buffer 1
@@ -569,9 +566,13 @@ lstm_cluster_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
 //  * the batch is the small dimension, so B = 512 spreads over 129 SMs (G = 12) instead of 48: the gate math, five
 //    special-function instructions per cell, is 1000 clocks for 2048 cells (G = 16), 600 for 1024.
 //  * W_hh in tensor memory: an MMA from a shared-memory A operand of 128 rows takes 40 clocks, from TMEM 16.
-// B = 512, H = 384: 1.27 us per step (2.57 before), H = 512: 1.83 (4.8), H = 256: 0.96 (2.29), H = 128: 0.57 (2.27).
-// Clocks of a step (G = 16, H = 384, of ~2650): own K block's MMAs 340, wait for the others' h 300, their MMAs 560, commit
-// to registers 300, gate math and sending 1000, hand-over to the MMA warps 130.
+// B = 512, H = 384: 1.34 us per step (2.57 with the 128-row tiles), H = 512: 1.91 (4.8), H = 256: 0.93 (2.29), H = 128: 0.56 (2.27).
+// The K blocks are summed in ascending order on every CTA.  Starting with the CTA's own block, which is there first, takes
+// 1.25 us at H = 384 and 1.81 at H = 512, but sums in an order that depends on the CTA: the last bit of a sum changes, an E4M3
+// rounding of h flips with it, and after five layers of 2000 steps the outputs differ by 5e-3.  There is a
+// barrier per sending CTA, so that the first blocks' MMAs do not wait for the last piece.
+// Clocks of a step before that order (G = 16, H = 384, of ~2650): MMAs 900, wait for the others' h 300 of the 640 it is under
+// way, commit to registers 300, gate math and sending 1000, hand-over to the MMA warps 130.
 //   warps 0 .. CW-1   gate math.  Warp w: TMEM lane quarter w % 4 (32 hidden units, one per lane), G / (CW / 4) batch rows
 //   last four warps   one MMA-issuing thread per gate (an MMA costs the thread that issues it 60 to 70 clocks); the last
 //                     one also issues the TMA loads of the ih tiles
@@ -615,8 +616,8 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
   uint64_t* ih_full = bars;                        // [LT_STAGES]
   uint64_t* own_ready = ih_full + LT_STAGES;      // [2] this CTA's piece of h is in the buffer, its accumulators have been read
-  uint64_t* h_ready = own_ready + 2;               // [2] the other CTAs' pieces have landed (bytes counted)
-  uint64_t* mma_done = h_ready + 2;                // the four gates' accumulators are complete
+  uint64_t* h_ready = own_ready + 2;               // [2][LT_MAX_SLICES] the piece of each other CTA has landed (bytes counted)
+  uint64_t* mma_done = h_ready + 2 * LT_MAX_SLICES;                // the four gates' accumulators are complete
   uint64_t* w_full = mma_done + 1;                 // the fourth K block of W_hh has landed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(w_full + 1);
   const AbortFlag abort_flag{smem_u32(tmem_slot + 1)};
@@ -627,15 +628,19 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const int row0 = grp * G, hid0 = slc * LT_HS;
   const int H = p.H, B = p.B;
   const int kb_tmem = p.k_blocks < LT_TMEM_KB ? p.k_blocks : LT_TMEM_KB;
-  const uint32_t peer_bytes = (uint32_t)(p.slices - 1) * G * LT_HS;
+  constexpr uint32_t PIECE_BYTES = G * LT_HS;      // of h, from one CTA
 
   if (tid == 0) {
     for (int i = 0; i < LT_STAGES; ++i) mbar_init(&ih_full[i], 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&own_ready[i], CW); mbar_init(&h_ready[i], 1); }
+    for (int i = 0; i < 2; ++i) mbar_init(&own_ready[i], CW);
+    for (int i = 0; i < 2 * LT_MAX_SLICES; ++i) mbar_init(&h_ready[i], 1);
     mbar_init(mma_done, 4); mbar_init(w_full, 1);
     // arm the first use of each buffer: h_0 arrives in buffer 0 (if there is a step 1), h_1 in buffer 1
-    if (p.slices > 1 && p.T > 1) mbar_arrive_expect_tx(&h_ready[0], peer_bytes);
-    if (p.slices > 1 && p.T > 2) mbar_arrive_expect_tx(&h_ready[1], peer_bytes);
+    for (int r = 0; r < p.slices; ++r) {
+      if (r == slc) continue;
+      if (p.T > 1) mbar_arrive_expect_tx(&h_ready[r], PIECE_BYTES);
+      if (p.T > 2) mbar_arrive_expect_tx(&h_ready[LT_MAX_SLICES + r], PIECE_BYTES);
+    }
     abort_flag.set(0);
     fence_mbar_init();
     prefetch_tmap(&tm_w); prefetch_tmap(&tm_ih);
@@ -728,7 +733,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       const int r = r_lo + hf * (RPT / 2) + ((lane >> 1) & (RPT / 2 - 1));
       snd_off[hf] = slc * L::KB_BYTES + r * 128 + (((2 * q + (lane & 1)) ^ (r & 7)) << 4);
     }
-    const uint32_t snd_dst = sends ? mapa_shared(smem_u32(h_s), to) : 0u, snd_bar = sends ? mapa_shared(smem_u32(h_ready), to) : 0u;
+    const uint32_t snd_dst = sends ? mapa_shared(smem_u32(h_s), to) : 0u, snd_bar = sends ? mapa_shared(smem_u32(h_ready + slc), to) : 0u;
     int st = 0; uint32_t st_ph = 0;
     for (int s = 0; s < p.T; ++s) {
       // ih + bias of this step, before the accumulators are there
@@ -787,7 +792,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         if (hf == 1 && lane == 0) mbar_arrive(&own_ready[s & 1]);
         if (sends && s + 1 < p.T) {
           const uint32_t off = (s & 1) * L::HBUF + snd_off[hf];
-          st_async_v4(snd_dst + off, *reinterpret_cast<const uint4*>(h_s + off), snd_bar + 8 * (s & 1));
+          st_async_v4(snd_dst + off, *reinterpret_cast<const uint4*>(h_s + off), snd_bar + 8 * LT_MAX_SLICES * (s & 1));
         }
       }
       // the layer's outputs, off the critical path: 32 (E4M3) / 64 (fp16) contiguous bytes per warp and row
@@ -834,21 +839,22 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           if (s > 0 && !mbar_wait(&own_ready[hb], ph, abort_flag, ST_TIMEOUT_LSTM, 0x40, budget)) return false;
           tc_fence_after();
           const uint64_t b = hb ? b_base[1] : b_base[0];
-          // K blocks in the order RANK, RANK + 1, ..., wrapping: this CTA's own piece of h is here first
+          // K blocks in ascending order on every CTA (the order of the sums is part of the result), each as soon as its piece
+          // of h is there
 #pragma unroll
-          for (int n = 0; n < SLICES; ++n) {
-            const int kb = (RANK + n) % SLICES;
-            if (n == 1 && s > 0) {                 // the other CTAs' pieces
-              if (!mbar_wait_cluster(&h_ready[hb], ph, abort_flag, ST_TIMEOUT_LSTM, 0x41, budget)) return false;
-              if (g == 0 && s + 2 < p.T) mbar_arrive_expect_tx(&h_ready[hb], peer_bytes);   // its next use: h_{s+1}, read by step s + 2
-              fence_proxy_async_smem();            // the peers' stores before the MMAs read them
+          for (int kb = 0; kb < SLICES; ++kb) {
+            if (kb != RANK && s > 0) {             // another CTA's piece
+              uint64_t* bar = &h_ready[hb * LT_MAX_SLICES + kb];
+              if (!mbar_wait_cluster(bar, ph, abort_flag, ST_TIMEOUT_LSTM, 0x41, budget)) return false;
+              if (g == 0 && s + 2 < p.T) mbar_arrive_expect_tx(bar, PIECE_BYTES);   // its next use: h_{s+1}, read by step s + 2
+              fence_proxy_async_smem();            // the peer's stores before the MMAs read them
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               if (kb == SLICES - 1 && 4 * kb + k >= ksteps) break;
               const uint64_t bd = b + (uint64_t)(kb * (L::KB_BYTES >> 4) + 2 * k);
-              if (kb < LT_TMEM_KB) umma_f8_ta(d, a0 + kb * 32 + k * 8, bd, idesc, (n | k) != 0);
-              else umma_f8(d, a_smem + 2 * k, bd, idesc, (n | k) != 0);
+              if (kb < LT_TMEM_KB) umma_f8_ta(d, a0 + kb * 32 + k * 8, bd, idesc, (kb | k) != 0);
+              else umma_f8(d, a_smem + 2 * k, bd, idesc, (kb | k) != 0);
             }
           }
           umma_commit(mma_done);
@@ -906,9 +912,9 @@ static constexpr LtForm lt_make_form(int ns1, int ns2, int ns3, int ns4) {
   return f;
 }
 constexpr int LT_FORMS = 5;
-static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(570, 790, 910, 1230), lt_make_form<16, 8, 8>(720, 960, 1090, 1400),
-                                          lt_make_form<16, 12, 12>(900, 1140, 1270, 1580), lt_make_form<16, 16, 8>(1070, 1250, 1380, 1770),
-                                          lt_make_form<32, 32, 16>(1770, 2110, 2210, 2680)};
+static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(570, 790, 980, 1360), lt_make_form<16, 8, 8>(720, 960, 1140, 1540),
+                                          lt_make_form<16, 12, 12>(900, 1140, 1340, 1740), lt_make_form<16, 16, 8>(1070, 1250, 1480, 1930),
+                                          lt_make_form<32, 32, 16>(1770, 2110, 2360, 2900)};
 
 static cudaLaunchConfig_t lt_config(const LtForm& f, int slices, long long groups, cudaStream_t st, cudaLaunchAttribute* attr) {
   attr->id = cudaLaunchAttributeClusterDimension;
@@ -944,8 +950,8 @@ static int lt_capacity(int form, int slices, int dev) {
 
 // The form with the shortest step (times the waves it takes), row groups limited to `max_ctas` CTAs at a time (0 = the whole
 // GPU); -1 = none.  Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows
-// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.24 us per step; 12 rows in two
-// waves 2.57).  *ns = the step.
+// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.36 us per step; 12 rows in two
+// waves 2.68).  *ns = the step.
 static int lt_choose(long long B, int H, int dev, int max_ctas, long long* ns = nullptr) {
   const int slices = (H + LT_HS - 1) / LT_HS;
   int best = -1;
@@ -1002,8 +1008,8 @@ static int lstm_layer_ctas(long long B, int H, int max_ctas) {
 
 // How many launches to cut a layer's recurrence into so that the next layer's projection runs beside it (1 = not at all).
 // The cut recurrence keeps to `max_ctas` CTAs, which may cost it a form with longer steps, and every launch about 12 us;
-// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 16.2 ms one after the other, 15.3
-// in seven blocks; at B = 512, H = 512 (T = 1000, three layers) 6.9 ms against 9.0, so not cut.
+// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 16.9 ms one after the other, 16.3
+// in seven blocks; at B = 512, H = 512 (T = 1000, three layers) 7.3 ms against 8.6, so not cut.
 static int lstm_time_blocks(long long T, long long B, int H, int max_ctas) {
   int dev = 0;
   cudaGetDevice(&dev);

@@ -212,3 +212,26 @@ def test_transposed_kernel_forms_match_the_cooperative_kernel(tmp_path):
         for a, b, what in zip(got, want, ("h fp16", "h e4m3", "c")):
             assert torch.equal(a.cpu().view(torch.uint8), b), f"{what} at {shape}"
     assert g.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("H", [256, 384, 512])
+def test_recurrent_sums_run_from_the_first_k_block_to_the_last(H):
+    """The products W_hh . h are summed over K = 0 .. H - 1 in that order, in every CTA of a row group: a last-bit change of a
+    sum can flip an E4M3 rounding of h, which the recurrence feeds back.  Large products that cancel come first (exactly: all
+    partial sums are multiples of 2^12 and below 2^25), the small sum 0.25 after them; in any order that has the small products
+    before the large ones are cancelled, it is lost below the last bit of a sum of more than 2^23."""
+    g = need_lib()
+    B = 5
+    big = 128 if H > 256 else 64                       # columns of each sign
+    w, h = torch.zeros(4 * H, H), torch.zeros(B, H)
+    w[:, :2 * big] = 448.0
+    h[:, :big], h[:, big:2 * big] = 448.0, -448.0
+    w[:, 2 * big:2 * big + 128], h[:, 2 * big:2 * big + 128] = 2.0 ** -9, 1.0
+    s = torch.full((4 * H,), 4 * 448.0)                # gates = 0.25 * (4 * 448) / 448 = 1
+    h16, _, c = g.lstm_layer(torch.zeros(B, 4 * H, dtype=torch.float16, device="cuda"), w.to(torch.float8_e4m3fn).cuda(), s.cuda(), 1, B,
+                             h0=h.to(torch.float8_e4m3fn).cuda(), want_c=True)
+    one = torch.ones(())
+    want_c = torch.sigmoid(one) * torch.tanh(one)
+    assert_close(c, want_c.expand(B, H), atol=2e-3, rtol=0, what="c")              # (hardware tanh: 2^-11 each)
+    assert_close(h16, (torch.sigmoid(one) * torch.tanh(want_c)).expand(B, H), atol=2e-3, rtol=0, what="h")
+    assert g.device_status()[0] == 0
