@@ -1205,8 +1205,6 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
     if (!layers[l].w_ih || !layers[l].s_ih || !layers[l].w_hh || !layers[l].s_hh) return GSB200_ERR_BAD_ARG;
   bool overlap = aux != nullptr && aux != st && n_layers > 1;
   if (ws_bytes < lstm_stack_workspace_bytes(T, B, H, overlap ? 1 : 0)) return GSB200_ERR_BAD_ARG;
-  if (!overlap) time_blocks = 1;
-  if (time_blocks > T) time_blocks = (int)T;
   int32_t rc = ensure_device();
   if (rc != GSB200_OK) return rc;
 
@@ -1250,8 +1248,10 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
 
   // overlapped: the recurrence takes up to two thirds of the GPU, the projection what is left
   const int max_ctas = overlap ? sm_count_physical() * 2 / 3 : 0;
-  if (overlap && time_blocks <= 0) time_blocks = lstm_time_blocks(T, B, H, max_ctas);
-  const int blocks_cut = time_blocks;                // launches per layer that has another one behind it
+  if (!overlap) time_blocks = 1;
+  else if (time_blocks <= 0) time_blocks = lstm_time_blocks(T, B, H, max_ctas);
+  // launches per layer that has another one behind it; no block may be empty, the one behind it would find no state at the cut
+  const int blocks_cut = time_blocks < T ? time_blocks : (int)T;
   int gemm_cap = sm_count_physical() - lstm_layer_ctas(B, H, max_ctas);
   if (gemm_cap < 8) gemm_cap = 8;
   cudaError_t ce = cudaSuccess;

@@ -235,3 +235,59 @@ def test_recurrent_sums_run_from_the_first_k_block_to_the_last(H):
     assert_close(c, want_c.expand(B, H), atol=2e-3, rtol=0, what="c")              # (hardware tanh: 2^-11 each)
     assert_close(h16, (torch.sigmoid(one) * torch.tanh(want_c)).expand(B, H), atol=2e-3, rtol=0, what="h")
     assert g.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("env_key", [None, "GSB200_LSTM_NO_CLUSTER", "GSB200_LSTM_ROWS128"])
+def test_stack_cut_by_the_library_gives_the_bytes_of_the_uncut_stack(env_key):
+    """aux_stream with time_blocks = 0: the library chooses the cut, whichever kernel runs, and never more blocks than steps
+    (a block without a step leaves the next one without the state at its start)."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = (
+        "import sys, torch; sys.path[:0] = [%r, %r]\n"
+        "import gigaslop_b200 as g; from test_gpu_lstm import make_layer, cuda_layer\n"
+        "for T in (1, 5, 7, 40):\n"
+        "    for B, H, first in ((20, 128, True), (70, 384, False)):\n"
+        "        gen = torch.Generator().manual_seed(T)\n"
+        "        layers = [cuda_layer(make_layer(gen, H, 64 if i == 0 else H)) for i in range(3)]\n"
+        "        x8, sx = g.fp8_quantize_per_token(torch.randn(T * B, 64, generator=gen).half().cuda())\n"
+        "        want = g.lstm_stack(x8, sx, layers, T, B, reverse_first=first)\n"
+        "        for nb in (0, 3, 8, 100):\n"
+        "            got = g.lstm_stack(x8, sx, layers, T, B, reverse_first=first, aux_stream=torch.cuda.Stream(), time_blocks=nb)\n"
+        "            torch.cuda.synchronize()\n"
+        "            assert torch.equal(got, want), (T, B, H, nb)\n"
+        "assert g.device_status()[0] == 0\n"
+    ) % (os.path.dirname(here), here)
+    env = dict(os.environ, **({env_key: "1"} if env_key else {}))
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("T,B,H,cut", [(1000, 512, 384, True), (40, 512, 384, False), (200, 512, 512, False)])
+def test_stack_cut_or_not_and_under_capture(T, B, H, cut):
+    """Both outcomes of the time model, eagerly and replayed from a graph that captured the two streams."""
+    g = need_lib()
+    gen = torch.Generator().manual_seed(12)
+    layers = [cuda_layer(make_layer(gen, H, 64 if i == 0 else H)) for i in range(2)]
+    x8, sx = g.fp8_quantize_per_token(torch.randn(T * B, 64, generator=gen).half().cuda())
+    want = g.lstm_stack(x8, sx, layers, T, B)
+    aux = torch.cuda.Stream()
+    ws = g.lstm.lstm_stack_workspace(T, B, H, x8.device, True)
+    out = torch.empty_like(want)
+    call = lambda: g.lstm_stack(x8, sx, layers, T, B, workspace=ws, aux_stream=aux, out=out)
+    call()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+        with torch.cuda.stream(aux):                   # the capture spread to the second stream where the stack was cut
+            assert torch.cuda.is_current_stream_capturing() == cut
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    assert g.device_status()[0] == 0
