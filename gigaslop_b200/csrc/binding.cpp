@@ -81,12 +81,13 @@ T* ptr(const at::Tensor& t) { return static_cast<T*>(t.data_ptr()); }
 template <typename T>
 T* ptr(const at::Tensor* t) { return t ? static_cast<T*>(t->data_ptr()) : nullptr; }
 
-// The library call without the interpreter lock (as ctypes makes it).
-template <typename F>
-bool call(F&& f) {
+// The library call without the interpreter lock (as ctypes makes it).  Its arguments are values that the caller made with the
+// lock held: taking a tensor's data pointer can allocate and throw (copy-on-write), the entry points do neither.
+template <typename Fn, typename... A>
+bool call(Fn fn, A... a) {
   int32_t rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = f();
+  rc = fn(a...);
   Py_END_ALLOW_THREADS
   return rc == 0;
 }
@@ -127,11 +128,10 @@ OPERATOR(quantize, 4)
   const at::Tensor s = s0 ? *s0 : c.empty({M}, at::kFloat);
   const int32_t dt = f16 ? GSB200_F16 : GSB200_F32;
   const gsb200_stream_t st = c.stream();
-  const bool ok = call([&] {
-    if (kind == 0)
-      return ENTRY(PTQ_INT8, gsb200_ptq_int8)(x->data_ptr(), dt, x->stride(0), ptr<int8_t>(q), q.stride(0), ptr<float>(s), M, (int32_t)K, st);
-    return ENTRY(PTQ_FP8, gsb200_ptq_fp8)(x->data_ptr(), dt, x->stride(0), ptr<uint8_t>(q), q.stride(0), ptr<float>(s), M, (int32_t)K, kind == 2, st);
-  });
+  const bool ok = kind == 0
+      ? call(ENTRY(PTQ_INT8, gsb200_ptq_int8), x->data_ptr(), dt, x->stride(0), ptr<int8_t>(q), q.stride(0), ptr<float>(s), M, (int32_t)K, st)
+      : call(ENTRY(PTQ_FP8, gsb200_ptq_fp8), x->data_ptr(), dt, x->stride(0), ptr<uint8_t>(q), q.stride(0), ptr<float>(s), M, (int32_t)K,
+             kind == 2, st);
   SLOW_UNLESS(ok);
   return pair(result(a[2], q), result(a[3], s));
 OPERATOR_END
@@ -146,10 +146,8 @@ OPERATOR(quantize_mx, 3)
   const at::Tensor q = q0 ? *q0 : c.empty({M, K}, at::kFloat8_e4m3fn);
   const at::Tensor s = s0 ? *s0 : c.empty({M, K / 32}, at::kByte);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call([&] {
-    return ENTRY(PTQ_MXFP8, gsb200_ptq_mxfp8)(x->data_ptr(), f16 ? GSB200_F16 : GSB200_F32, x->stride(0), ptr<uint8_t>(q), q.stride(0),
-                                              ptr<uint8_t>(s), s.stride(0), M, (int32_t)K, st);
-  }));
+  SLOW_UNLESS(call(ENTRY(PTQ_MXFP8, gsb200_ptq_mxfp8), x->data_ptr(), f16 ? GSB200_F16 : GSB200_F32, x->stride(0), ptr<uint8_t>(q),
+                   q.stride(0), ptr<uint8_t>(s), s.stride(0), M, (int32_t)K, st));
   return pair(result(a[1], q), result(a[2], s));
 OPERATOR_END
 
@@ -163,13 +161,11 @@ OPERATOR(gemm, 7)
   const int64_t M = A->size(0), N = B->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  const bool ok = call([&] {
-    if (fp8)
-      return ENTRY(GEMM_FP8, gsb200_gemm_fp8_f16)(ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
-                                                  ptr<float>(sa), ptr<float>(sb), M, (int32_t)N, (int32_t)K, flags, st);
-    return ENTRY(GEMM_I8, gsb200_gemm_i8_f16)(ptr<int8_t>(A), A->stride(0), ptr<int8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
-                                              ptr<float>(sa), ptr<float>(sb), M, (int32_t)N, (int32_t)K, flags, st);
-  });
+  const bool ok = fp8
+      ? call(ENTRY(GEMM_FP8, gsb200_gemm_fp8_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
+             ptr<float>(sa), ptr<float>(sb), M, (int32_t)N, (int32_t)K, flags, st)
+      : call(ENTRY(GEMM_I8, gsb200_gemm_i8_f16), ptr<int8_t>(A), A->stride(0), ptr<int8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
+             ptr<float>(sa), ptr<float>(sb), M, (int32_t)N, (int32_t)K, flags, st);
   SLOW_UNLESS(ok);
   return result(a[5], C);
 OPERATOR_END
@@ -188,15 +184,13 @@ OPERATOR(rotary, 14)
   const int64_t M = A->size(0), N = B->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  const bool ok = call([&] {
-    if (fp8)
-      return ENTRY(ROT_FP8, gsb200_gemm_fp8_rotary_f16)(ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
-                                                        ptr<float>(sa), ptr<float>(sb), ptr<float>(sn), ptr<float>(cs), M, (int32_t)N, (int32_t)K,
-                                                        nhead, head_dim, rotary_dim, seqlen, row_offset, flags, st);
-    return ENTRY(ROT_I8, gsb200_gemm_i8_rotary_f16)(ptr<int8_t>(A), A->stride(0), ptr<int8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
-                                                    ptr<float>(sa), ptr<float>(sb), ptr<float>(sn), ptr<float>(cs), M, (int32_t)N, (int32_t)K,
-                                                    nhead, head_dim, rotary_dim, seqlen, row_offset, flags, st);
-  });
+  const bool ok = fp8
+      ? call(ENTRY(ROT_FP8, gsb200_gemm_fp8_rotary_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
+             ptr<float>(sa), ptr<float>(sb), ptr<float>(sn), ptr<float>(cs), M, (int32_t)N, (int32_t)K, nhead, head_dim, rotary_dim, seqlen,
+             row_offset, flags, st)
+      : call(ENTRY(ROT_I8, gsb200_gemm_i8_rotary_f16), ptr<int8_t>(A), A->stride(0), ptr<int8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
+             ptr<float>(sa), ptr<float>(sb), ptr<float>(sn), ptr<float>(cs), M, (int32_t)N, (int32_t)K, nhead, head_dim, rotary_dim, seqlen,
+             row_offset, flags, st);
   SLOW_UNLESS(ok);
   return result(a[12], C);
 OPERATOR_END
@@ -213,13 +207,11 @@ OPERATOR(dual, 9)
   const int64_t M = A->size(0), N = G->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  const bool ok = call([&] {
-    if (fp8)
-      return ENTRY(DUAL_FP8, gsb200_dual_gemm_fp8_silu_f16)(ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(G), ptr<uint8_t>(U), G->stride(0), C.data_ptr(),
-                                                            C.stride(0), ptr<float>(sa), ptr<float>(sg), ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st);
-    return ENTRY(DUAL_I8, gsb200_dual_gemm_i8_silu_f16)(ptr<int8_t>(A), A->stride(0), ptr<int8_t>(G), ptr<int8_t>(U), G->stride(0), C.data_ptr(),
-                                                        C.stride(0), ptr<float>(sa), ptr<float>(sg), ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st);
-  });
+  const bool ok = fp8
+      ? call(ENTRY(DUAL_FP8, gsb200_dual_gemm_fp8_silu_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(G), ptr<uint8_t>(U), G->stride(0),
+             C.data_ptr(), C.stride(0), ptr<float>(sa), ptr<float>(sg), ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st)
+      : call(ENTRY(DUAL_I8, gsb200_dual_gemm_i8_silu_f16), ptr<int8_t>(A), A->stride(0), ptr<int8_t>(G), ptr<int8_t>(U), G->stride(0),
+             C.data_ptr(), C.stride(0), ptr<float>(sa), ptr<float>(sg), ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st);
   SLOW_UNLESS(ok);
   return result(a[7], C);
 OPERATOR_END
@@ -235,11 +227,9 @@ OPERATOR(dual_mx, 9)
   const at::Tensor q = q0 ? *q0 : c.empty({M, N}, at::kFloat8_e4m3fn);
   const at::Tensor s = s0 ? *s0 : c.empty({M, N / 32}, at::kByte);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call([&] {
-    return ENTRY(DUAL_FP8_MX, gsb200_dual_gemm_fp8_silu_mxfp8)(ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(G), ptr<uint8_t>(U), G->stride(0),
-                                                               ptr<uint8_t>(q), q.stride(0), ptr<uint8_t>(s), s.stride(0), ptr<float>(sa), ptr<float>(sg),
-                                                               ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st);
-  }));
+  SLOW_UNLESS(call(ENTRY(DUAL_FP8_MX, gsb200_dual_gemm_fp8_silu_mxfp8), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(G), ptr<uint8_t>(U),
+                   G->stride(0), ptr<uint8_t>(q), q.stride(0), ptr<uint8_t>(s), s.stride(0), ptr<float>(sa), ptr<float>(sg),
+                   ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st));
   return pair(result(a[6], q), result(a[7], s));
 OPERATOR_END
 
@@ -252,7 +242,7 @@ OPERATOR(mx_tile, 2)
   SLOW_UNLESS(bytes >= 0);
   const at::Tensor out = c.empty({bytes}, at::kByte);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call([&] { return ENTRY(MX_TILE, gsb200_mx_scales_to_tiled)(ptr<uint8_t>(s), s->stride(0), s->size(0), K, ptr<uint8_t>(out), st); }));
+  SLOW_UNLESS(call(ENTRY(MX_TILE, gsb200_mx_scales_to_tiled), ptr<uint8_t>(s), s->stride(0), s->size(0), K, ptr<uint8_t>(out), st));
   return wrap(out);
 OPERATOR_END
 
@@ -264,10 +254,8 @@ OPERATOR(mx_gemm, 5)
   const int64_t M = A->size(0), N = B->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call([&] {
-    return ENTRY(MX_GEMM, gsb200_gemm_mxfp8_f16)(ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(sfa), ptr<uint8_t>(B), B->stride(0), ptr<uint8_t>(sfb),
-                                                 C.data_ptr(), C.stride(0), M, (int32_t)N, (int32_t)K, st);
-  }));
+  SLOW_UNLESS(call(ENTRY(MX_GEMM, gsb200_gemm_mxfp8_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(sfa), ptr<uint8_t>(B), B->stride(0),
+                   ptr<uint8_t>(sfb), C.data_ptr(), C.stride(0), M, (int32_t)N, (int32_t)K, st));
   return result(a[4], C);
 OPERATOR_END
 
@@ -279,10 +267,9 @@ OPERATOR(mx_dual, 7)
   const int64_t M = A->size(0), N = G->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call([&] {
-    return ENTRY(MX_DUAL, gsb200_dual_gemm_mxfp8_silu_f16)(ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(sfa), ptr<uint8_t>(G), ptr<uint8_t>(U), G->stride(0),
-                                                           ptr<uint8_t>(sg), ptr<uint8_t>(su), C.data_ptr(), C.stride(0), M, (int32_t)N, (int32_t)K, st);
-  }));
+  SLOW_UNLESS(call(ENTRY(MX_DUAL, gsb200_dual_gemm_mxfp8_silu_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(sfa), ptr<uint8_t>(G),
+                   ptr<uint8_t>(U), G->stride(0), ptr<uint8_t>(sg), ptr<uint8_t>(su), C.data_ptr(), C.stride(0), M, (int32_t)N, (int32_t)K,
+                   st));
   return result(a[6], C);
 OPERATOR_END
 
@@ -295,11 +282,9 @@ OPERATOR(fac_gemm, 7)
   SLOW_UNLESS(dn->size(1) == Cc && up->size(1) == R && bias->numel() == N && sx->numel() == M && fits(Cc) && fits(R) && fits(N));
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call([&] {
-    return ENTRY(FAC_GEMM, gsb200_fac_gemm_fp8_f16)(ptr<uint8_t>(x), x->stride(0), ptr<float>(sx), ptr<uint8_t>(dn), dn->stride(0), ptr<float>(sdn),
-                                                    up->data_ptr(), up->stride(0), ptr<float>(bias), C.data_ptr(), C.stride(0), M, (int32_t)Cc, (int32_t)R,
-                                                    (int32_t)N, st);
-  }));
+  SLOW_UNLESS(call(ENTRY(FAC_GEMM, gsb200_fac_gemm_fp8_f16), ptr<uint8_t>(x), x->stride(0), ptr<float>(sx), ptr<uint8_t>(dn),
+                   dn->stride(0), ptr<float>(sdn), up->data_ptr(), up->stride(0), ptr<float>(bias), C.data_ptr(), C.stride(0), M,
+                   (int32_t)Cc, (int32_t)R, (int32_t)N, st));
   return result(a[6], C);
 OPERATOR_END
 
@@ -313,10 +298,8 @@ OPERATOR(fac_step, 8)
   const int64_t B = hh->size(0), K = hh->size(1), H = uhh->size(0) / 4, R = xd->size(1);
   SLOW_UNLESS(fits(K) && fits(H) && fits(R));
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call([&] {
-    return ENTRY(FAC_STEP, gsb200_factored_lstm_step)(ptr<uint8_t>(h), ptr<float>(cc), hh->data_ptr(), uhh->data_ptr(), ptr<float>(bhh), xd->data_ptr(),
-                                                      uih->data_ptr(), ptr<float>(bih), B, (int32_t)H, (int32_t)K, (int32_t)R, st);
-  }));
+  SLOW_UNLESS(call(ENTRY(FAC_STEP, gsb200_factored_lstm_step), ptr<uint8_t>(h), ptr<float>(cc), hh->data_ptr(), uhh->data_ptr(),
+                   ptr<float>(bhh), xd->data_ptr(), uih->data_ptr(), ptr<float>(bih), B, (int32_t)H, (int32_t)K, (int32_t)R, st));
   Py_RETURN_TRUE;
 OPERATOR_END
 

@@ -102,3 +102,33 @@ def test_native_path_gives_the_bytes_of_the_checked_path(monkeypatch):
         g.gemm_i8(qi[:, ::2], w, si, sw)
     with pytest.raises(TypeError):
         g.gemm_fp8(qi, w, si, sw)
+
+
+@pytest.mark.gpu
+def test_error_of_a_copy_on_write_tensor_is_raised():
+    """Taking the data pointer of a lazily cloned tensor makes its copy, which can fail: the error is an ordinary exception (it
+    is thrown while the interpreter lock is held).  In a child process, which is given little memory and leaves without
+    freeing the tensor: torch itself aborts there after a copy that failed."""
+    import os
+    import subprocess
+    import sys
+    code = (
+        "import os, sys, torch; sys.path.insert(0, %r)\n"
+        "import gigaslop_b200 as g; from gigaslop_b200 import _lib\n"
+        "g.lib(); assert _lib.native is not None\n"
+        "x = torch.randn(1 << 16, 512, device='cuda').half(); torch.cuda.synchronize(); torch.cuda.empty_cache()\n"
+        "q, s = torch.empty(x.shape, dtype=torch.int8, device='cuda'), torch.empty(len(x), device='cuda')\n"
+        "want = g.quantize_tensor(x)[0].cpu()\n"
+        "assert torch.equal(g.quantize_tensor(torch._lazy_clone(x), out=q, out_scale=s)[0].cpu(), want)\n"
+        "y = torch._lazy_clone(x); torch.cuda.empty_cache()\n"
+        "total = torch.cuda.get_device_properties(0).total_memory\n"
+        "torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (8 << 20)) / total)\n"
+        "try:\n"
+        "    g.quantize_tensor(y, out=q, out_scale=s)\n"
+        "    print('no error')\n"
+        "except torch.OutOfMemoryError:\n"
+        "    print('raised')\n"
+        "sys.stdout.flush(); os._exit(0)\n"
+    ) % os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.split() == ["raised"], r.stdout + r.stderr
