@@ -94,7 +94,7 @@ def lib():
         except ImportError as e:
             raise RuntimeError("gigaslop_b200/_native.so is missing or does not load: build it with "
                                "`python -m gigaslop_b200.build`") from e
-        _native.bind([C.cast(getattr(handle, n), C.c_void_p).value for n in NATIVE_ENTRIES])
+        _native.bind([C.cast(getattr(handle, n), C.c_void_p).value for n in NATIVE_ENTRIES], check)
         native = _native
         _lib = handle
     return _lib

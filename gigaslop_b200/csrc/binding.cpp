@@ -2,7 +2,8 @@
 // interpreter in between.  It takes the plain case only -- ordinary CUDA tensors of one device, that device current, no
 // torch-function or dispatch mode active, every shape, stride and type check of the Python function passed -- and
 // returns None for everything else, upon which the Python function runs its own checks (and raises what it always
-// raised) and calls the library through ctypes.  Nothing is kept between calls.
+// raised) and calls the library through ctypes.  A status other than 0 raises here, with the exception that the Python
+// function makes of it.  Nothing is kept between calls.
 //
 // Why: through Python and ctypes an operator costs the host 17 to 22 us (device checks 3, torch.empty 2 to 4, stream
 // lookup 2, about 15 converted arguments 4, launch 4); small calls never reached the GPU's own time.  Here it is 4 to 6.
@@ -24,6 +25,7 @@ namespace {
 enum Entry { PTQ_INT8, PTQ_FP8, PTQ_MXFP8, GEMM_I8, GEMM_FP8, ROT_I8, ROT_FP8, DUAL_I8, DUAL_FP8, DUAL_FP8_MX, MX_BYTES, MX_TILE, MX_GEMM,
              MX_DUAL, FAC_GEMM, FAC_STEP, N_ENTRIES };
 void* g_entry[N_ENTRIES];
+PyObject* g_check;             // check(status, what), raises
 template <typename Fn>
 Fn entry(Entry e, Fn) { return reinterpret_cast<Fn>(g_entry[e]); }
 #define ENTRY(e, name) entry(e, &name)
@@ -84,12 +86,22 @@ T* ptr(const at::Tensor* t) { return t ? static_cast<T*>(t->data_ptr()) : nullpt
 // The library call without the interpreter lock (as ctypes makes it).  Its arguments are values that the caller made with the
 // lock held: taking a tensor's data pointer can allocate and throw (copy-on-write), the entry points do neither.
 template <typename Fn, typename... A>
-bool call(Fn fn, A... a) {
+int32_t call(Fn fn, A... a) {
   int32_t rc;
   Py_BEGIN_ALLOW_THREADS
   rc = fn(a...);
   Py_END_ALLOW_THREADS
-  return rc == 0;
+  return rc;
+}
+// What the library refuses is refused: the package's own `check` raises.  (Not None: the Python function would allocate, print
+// and launch once more.)
+PyObject* refused(int32_t rc, const char* what) {
+  PyObject* r = PyObject_CallFunction(g_check, "is", (int)rc, what);
+  if (r) {
+    Py_DECREF(r);
+    PyErr_SetString(PyExc_SystemError, "gigaslop_b200: check accepted an error status");
+  }
+  return nullptr;
 }
 
 PyObject* wrap(const at::Tensor& t) { return THPVariable_Wrap(t); }
@@ -109,6 +121,7 @@ PyObject* pair(PyObject* a, PyObject* b) {
 }
 
 #define SLOW_UNLESS(cond) do { if (!(cond)) Py_RETURN_NONE; } while (0)
+#define CHECK(rc, what) do { const int32_t rc_ = (rc); if (rc_ != 0) return refused(rc_, what); } while (0)
 #define OPERATOR(name, n)                                                       \
   PyObject* name(PyObject*, PyObject* const* a, Py_ssize_t nargs) {             \
     HANDLE_TH_ERRORS                                                            \
@@ -128,11 +141,11 @@ OPERATOR(quantize, 4)
   const at::Tensor s = s0 ? *s0 : c.empty({M}, at::kFloat);
   const int32_t dt = f16 ? GSB200_F16 : GSB200_F32;
   const gsb200_stream_t st = c.stream();
-  const bool ok = kind == 0
+  const int32_t rc = kind == 0
       ? call(ENTRY(PTQ_INT8, gsb200_ptq_int8), x->data_ptr(), dt, x->stride(0), ptr<int8_t>(q), q.stride(0), ptr<float>(s), M, (int32_t)K, st)
       : call(ENTRY(PTQ_FP8, gsb200_ptq_fp8), x->data_ptr(), dt, x->stride(0), ptr<uint8_t>(q), q.stride(0), ptr<float>(s), M, (int32_t)K,
              kind == 2, st);
-  SLOW_UNLESS(ok);
+  CHECK(rc, kind == 0 ? "quantize_tensor" : "fp8_quantize_per_token");
   return pair(result(a[2], q), result(a[3], s));
 OPERATOR_END
 
@@ -146,8 +159,8 @@ OPERATOR(quantize_mx, 3)
   const at::Tensor q = q0 ? *q0 : c.empty({M, K}, at::kFloat8_e4m3fn);
   const at::Tensor s = s0 ? *s0 : c.empty({M, K / 32}, at::kByte);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call(ENTRY(PTQ_MXFP8, gsb200_ptq_mxfp8), x->data_ptr(), f16 ? GSB200_F16 : GSB200_F32, x->stride(0), ptr<uint8_t>(q),
-                   q.stride(0), ptr<uint8_t>(s), s.stride(0), M, (int32_t)K, st));
+  CHECK(call(ENTRY(PTQ_MXFP8, gsb200_ptq_mxfp8), x->data_ptr(), f16 ? GSB200_F16 : GSB200_F32, x->stride(0), ptr<uint8_t>(q),
+             q.stride(0), ptr<uint8_t>(s), s.stride(0), M, (int32_t)K, st), "mxfp8_quantize");
   return pair(result(a[1], q), result(a[2], s));
 OPERATOR_END
 
@@ -161,12 +174,12 @@ OPERATOR(gemm, 7)
   const int64_t M = A->size(0), N = B->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  const bool ok = fp8
+  const int32_t rc = fp8
       ? call(ENTRY(GEMM_FP8, gsb200_gemm_fp8_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
              ptr<float>(sa), ptr<float>(sb), M, (int32_t)N, (int32_t)K, flags, st)
       : call(ENTRY(GEMM_I8, gsb200_gemm_i8_f16), ptr<int8_t>(A), A->stride(0), ptr<int8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
              ptr<float>(sa), ptr<float>(sb), M, (int32_t)N, (int32_t)K, flags, st);
-  SLOW_UNLESS(ok);
+  CHECK(rc, fp8 ? "gemm_fp8" : "gemm_i8");
   return result(a[5], C);
 OPERATOR_END
 
@@ -184,14 +197,14 @@ OPERATOR(rotary, 14)
   const int64_t M = A->size(0), N = B->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  const bool ok = fp8
+  const int32_t rc = fp8
       ? call(ENTRY(ROT_FP8, gsb200_gemm_fp8_rotary_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
              ptr<float>(sa), ptr<float>(sb), ptr<float>(sn), ptr<float>(cs), M, (int32_t)N, (int32_t)K, nhead, head_dim, rotary_dim, seqlen,
              row_offset, flags, st)
       : call(ENTRY(ROT_I8, gsb200_gemm_i8_rotary_f16), ptr<int8_t>(A), A->stride(0), ptr<int8_t>(B), B->stride(0), C.data_ptr(), C.stride(0),
              ptr<float>(sa), ptr<float>(sb), ptr<float>(sn), ptr<float>(cs), M, (int32_t)N, (int32_t)K, nhead, head_dim, rotary_dim, seqlen,
              row_offset, flags, st);
-  SLOW_UNLESS(ok);
+  CHECK(rc, fp8 ? "gemm_fp8_rotary" : "gemm_i8_rotary");
   return result(a[12], C);
 OPERATOR_END
 
@@ -207,12 +220,12 @@ OPERATOR(dual, 9)
   const int64_t M = A->size(0), N = G->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  const bool ok = fp8
+  const int32_t rc = fp8
       ? call(ENTRY(DUAL_FP8, gsb200_dual_gemm_fp8_silu_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(G), ptr<uint8_t>(U), G->stride(0),
              C.data_ptr(), C.stride(0), ptr<float>(sa), ptr<float>(sg), ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st)
       : call(ENTRY(DUAL_I8, gsb200_dual_gemm_i8_silu_f16), ptr<int8_t>(A), A->stride(0), ptr<int8_t>(G), ptr<int8_t>(U), G->stride(0),
              C.data_ptr(), C.stride(0), ptr<float>(sa), ptr<float>(sg), ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st);
-  SLOW_UNLESS(ok);
+  CHECK(rc, fp8 ? "dual_gemm_fp8_silu" : "dual_gemm_i8_silu");
   return result(a[7], C);
 OPERATOR_END
 
@@ -227,9 +240,9 @@ OPERATOR(dual_mx, 9)
   const at::Tensor q = q0 ? *q0 : c.empty({M, N}, at::kFloat8_e4m3fn);
   const at::Tensor s = s0 ? *s0 : c.empty({M, N / 32}, at::kByte);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call(ENTRY(DUAL_FP8_MX, gsb200_dual_gemm_fp8_silu_mxfp8), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(G), ptr<uint8_t>(U),
-                   G->stride(0), ptr<uint8_t>(q), q.stride(0), ptr<uint8_t>(s), s.stride(0), ptr<float>(sa), ptr<float>(sg),
-                   ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st));
+  CHECK(call(ENTRY(DUAL_FP8_MX, gsb200_dual_gemm_fp8_silu_mxfp8), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(G), ptr<uint8_t>(U),
+             G->stride(0), ptr<uint8_t>(q), q.stride(0), ptr<uint8_t>(s), s.stride(0), ptr<float>(sa), ptr<float>(sg),
+             ptr<float>(su), M, (int32_t)N, (int32_t)K, flags, st), "dual_gemm_fp8_silu_mxfp8");
   return pair(result(a[6], q), result(a[7], s));
 OPERATOR_END
 
@@ -242,7 +255,7 @@ OPERATOR(mx_tile, 2)
   SLOW_UNLESS(bytes >= 0);
   const at::Tensor out = c.empty({bytes}, at::kByte);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call(ENTRY(MX_TILE, gsb200_mx_scales_to_tiled), ptr<uint8_t>(s), s->stride(0), s->size(0), K, ptr<uint8_t>(out), st));
+  CHECK(call(ENTRY(MX_TILE, gsb200_mx_scales_to_tiled), ptr<uint8_t>(s), s->stride(0), s->size(0), K, ptr<uint8_t>(out), st), "mx_scales_to_tiled");
   return wrap(out);
 OPERATOR_END
 
@@ -254,8 +267,8 @@ OPERATOR(mx_gemm, 5)
   const int64_t M = A->size(0), N = B->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call(ENTRY(MX_GEMM, gsb200_gemm_mxfp8_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(sfa), ptr<uint8_t>(B), B->stride(0),
-                   ptr<uint8_t>(sfb), C.data_ptr(), C.stride(0), M, (int32_t)N, (int32_t)K, st));
+  CHECK(call(ENTRY(MX_GEMM, gsb200_gemm_mxfp8_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(sfa), ptr<uint8_t>(B), B->stride(0),
+             ptr<uint8_t>(sfb), C.data_ptr(), C.stride(0), M, (int32_t)N, (int32_t)K, st), "gemm_mxfp8");
   return result(a[4], C);
 OPERATOR_END
 
@@ -267,9 +280,9 @@ OPERATOR(mx_dual, 7)
   const int64_t M = A->size(0), N = G->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call(ENTRY(MX_DUAL, gsb200_dual_gemm_mxfp8_silu_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(sfa), ptr<uint8_t>(G),
-                   ptr<uint8_t>(U), G->stride(0), ptr<uint8_t>(sg), ptr<uint8_t>(su), C.data_ptr(), C.stride(0), M, (int32_t)N, (int32_t)K,
-                   st));
+  CHECK(call(ENTRY(MX_DUAL, gsb200_dual_gemm_mxfp8_silu_f16), ptr<uint8_t>(A), A->stride(0), ptr<uint8_t>(sfa), ptr<uint8_t>(G),
+             ptr<uint8_t>(U), G->stride(0), ptr<uint8_t>(sg), ptr<uint8_t>(su), C.data_ptr(), C.stride(0), M, (int32_t)N, (int32_t)K,
+             st), "dual_gemm_mxfp8_silu");
   return result(a[6], C);
 OPERATOR_END
 
@@ -282,9 +295,9 @@ OPERATOR(fac_gemm, 7)
   SLOW_UNLESS(dn->size(1) == Cc && up->size(1) == R && bias->numel() == N && sx->numel() == M && fits(Cc) && fits(R) && fits(N));
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call(ENTRY(FAC_GEMM, gsb200_fac_gemm_fp8_f16), ptr<uint8_t>(x), x->stride(0), ptr<float>(sx), ptr<uint8_t>(dn),
-                   dn->stride(0), ptr<float>(sdn), up->data_ptr(), up->stride(0), ptr<float>(bias), C.data_ptr(), C.stride(0), M,
-                   (int32_t)Cc, (int32_t)R, (int32_t)N, st));
+  CHECK(call(ENTRY(FAC_GEMM, gsb200_fac_gemm_fp8_f16), ptr<uint8_t>(x), x->stride(0), ptr<float>(sx), ptr<uint8_t>(dn),
+             dn->stride(0), ptr<float>(sdn), up->data_ptr(), up->stride(0), ptr<float>(bias), C.data_ptr(), C.stride(0), M,
+             (int32_t)Cc, (int32_t)R, (int32_t)N, st), "fp8_factored_gemm");
   return result(a[6], C);
 OPERATOR_END
 
@@ -298,13 +311,15 @@ OPERATOR(fac_step, 8)
   const int64_t B = hh->size(0), K = hh->size(1), H = uhh->size(0) / 4, R = xd->size(1);
   SLOW_UNLESS(fits(K) && fits(H) && fits(R));
   const gsb200_stream_t st = c.stream();
-  SLOW_UNLESS(call(ENTRY(FAC_STEP, gsb200_factored_lstm_step), ptr<uint8_t>(h), ptr<float>(cc), hh->data_ptr(), uhh->data_ptr(),
-                   ptr<float>(bhh), xd->data_ptr(), uih->data_ptr(), ptr<float>(bih), B, (int32_t)H, (int32_t)K, (int32_t)R, st));
+  CHECK(call(ENTRY(FAC_STEP, gsb200_factored_lstm_step), ptr<uint8_t>(h), ptr<float>(cc), hh->data_ptr(), uhh->data_ptr(),
+             ptr<float>(bhh), xd->data_ptr(), uih->data_ptr(), ptr<float>(bih), B, (int32_t)H, (int32_t)K, (int32_t)R, st), "factored_lstm_step");
   Py_RETURN_TRUE;
 OPERATOR_END
 
-// bind(addresses): the entry points' addresses in the order of `Entry`
-PyObject* bind(PyObject*, PyObject* seq) {
+// bind(addresses, check): the entry points' addresses in the order of `Entry`, and what turns a status into an exception
+PyObject* bind(PyObject*, PyObject* args) {
+  PyObject *seq, *check;
+  if (!PyArg_ParseTuple(args, "OO:bind", &seq, &check)) return nullptr;
   PyObject* f = PySequence_Fast(seq, "bind takes a sequence of addresses");
   if (!f) return nullptr;
   if (PySequence_Fast_GET_SIZE(f) != N_ENTRIES) {
@@ -317,11 +332,14 @@ PyObject* bind(PyObject*, PyObject* seq) {
     if (PyErr_Occurred()) { Py_DECREF(f); return nullptr; }
   }
   Py_DECREF(f);
+  Py_INCREF(check);
+  Py_XDECREF(g_check);
+  g_check = check;
   Py_RETURN_NONE;
 }
 
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {{"bind", bind, METH_O, nullptr}, METHOD(quantize), METHOD(quantize_mx), METHOD(gemm), METHOD(rotary), METHOD(dual),
+PyMethodDef methods[] = {{"bind", bind, METH_VARARGS, nullptr}, METHOD(quantize), METHOD(quantize_mx), METHOD(gemm), METHOD(rotary), METHOD(dual),
                          METHOD(dual_mx), METHOD(mx_tile), METHOD(mx_gemm), METHOD(mx_dual), METHOD(fac_gemm), METHOD(fac_step),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -132,3 +132,37 @@ def test_error_of_a_copy_on_write_tensor_is_raised():
     ) % os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.split() == ["raised"], r.stdout + r.stderr
+
+
+@pytest.mark.gpu
+def test_call_that_the_library_refuses_is_made_once(monkeypatch):
+    """A refusal raises from the native path: the Python function does not allocate, print and launch a second time."""
+    g = need_lib()
+    from gigaslop_b200 import ops
+    entered = []
+    for name in dir(ops):
+        if name.startswith("_checked_"):
+            monkeypatch.setattr(ops, name, lambda *a, _n=name: entered.append(_n))
+    z = lambda *shape, dtype=torch.float16: torch.zeros(*shape, dtype=dtype, device="cuda")
+    f8 = lambda *shape: z(*shape, dtype=torch.uint8).view(torch.float8_e4m3fn)
+    i8, f32 = lambda *shape: z(*shape, dtype=torch.int8), lambda *shape: z(*shape, dtype=torch.float32)
+    x, w, s, tab = 24, 64, f32(192), f32(8, 32)                   # K = 24: not a multiple of 16 (nor of 32, 64 or 128)
+    calls = {
+        "quantize_tensor": lambda: g.quantize_tensor(z(4, 4)), "fp8_quantize_per_token": lambda: g.fp8_quantize_per_token(z(4, 4)),
+        "mxfp8_quantize": lambda: g.mxfp8_quantize(z(4, 40)), "gemm_i8": lambda: g.gemm_i8(i8(4, x), i8(w, x), s, s),
+        "gemm_fp8": lambda: g.gemm_fp8(f8(4, x), f8(w, x), s, s),
+        "gemm_i8_rotary": lambda: g.gemm_i8_rotary(i8(4, x), i8(192, x), s, s, tab, tab, 1, 64, 64, 8),
+        "gemm_fp8_rotary": lambda: g.gemm_fp8_rotary(f8(4, x), f8(192, x), s, s, tab, tab, 1, 64, 64, 8),
+        "dual_gemm_i8_silu": lambda: g.dual_gemm_i8_silu(i8(4, x), i8(w, x), i8(w, x), s, s, s),
+        "dual_gemm_fp8_silu": lambda: g.dual_gemm_fp8_silu(f8(4, x), f8(w, x), f8(w, x), s, s, s),
+        "dual_gemm_fp8_silu_mxfp8": lambda: g.dual_gemm_fp8_silu_mxfp8(f8(4, x), f8(w, x), f8(w, x), s, s, s),
+        "mx_scales_to_tiled": lambda: g.mx_scales_to_tiled(z(4, 3, dtype=torch.uint8), 96),
+        "gemm_mxfp8": lambda: g.gemm_mxfp8(f8(4, x), f8(512), f8(w, x), f8(512)),
+        "dual_gemm_mxfp8_silu": lambda: g.dual_gemm_mxfp8_silu(f8(4, x), f8(512), f8(w, x), f8(w, x), f8(512), f8(512)),
+        "fp8_factored_gemm": lambda: g.fp8_factored_gemm(f8(4, 64), f32(4), f8(12, 64), f32(1), z(64, 12), f32(64)),
+        "factored_lstm_step": lambda: g.factored_lstm_step(f8(4, 64), f32(4, 64), z(4, x), z(256, x), None, z(4, x), z(256, x), None),
+    }
+    for name, call in calls.items():
+        with pytest.raises(RuntimeError, match=rf"gigaslop_b200\.{name}: .* \(status -"):
+            call()
+        assert not entered, name
