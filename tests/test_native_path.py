@@ -26,6 +26,26 @@ def test_native_path_declines_what_is_not_plain():
         need_lib().quantize_tensor(x)
 
 
+def run_python(code):
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    return subprocess.run([sys.executable, "-c", f"import sys; sys.path.insert(0, {root!r})\n" + code], capture_output=True, text=True,
+                          timeout=120)
+
+
+def test_package_works_without_the_native_path():
+    """The extension is a shortcut: without it the library loads, with a warning, and every call goes through ctypes."""
+    r = run_python("import warnings; sys.modules['gigaslop_b200._native'] = None\n"
+                   "import gigaslop_b200 as g; from gigaslop_b200 import _lib\n"
+                   "with warnings.catch_warnings(record=True) as w:\n"
+                   "    warnings.simplefilter('always'); g.lib(); g.lib()\n"
+                   "assert [x.category for x in w] == [RuntimeWarning] and '_native.so' in str(w[0].message), w\n"
+                   "assert _lib.native is None and g.mx_scales_to_tiled and g.lib().gsb200_mx_tiled_scale_bytes(128, 128) == 512\n")
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 @pytest.mark.gpu
 def test_native_path_gives_the_bytes_of_the_checked_path(monkeypatch):
     g = need_lib()
