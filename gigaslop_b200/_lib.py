@@ -91,7 +91,10 @@ def lib():
             fn.argtypes = args
         import torch  # noqa: F401  (the extension links against the libraries torch has loaded)
         try:
-            from . import _native
+            from . import _native, build
+            made_for = getattr(_native, "TARGET", "another version of this package")
+            if made_for != build.native_target():
+                raise ImportError(f"built for {made_for}, this is {build.native_target()}")
             _native.bind([C.cast(getattr(handle, n), C.c_void_p).value for n in NATIVE_ENTRIES], check)
             native = _native
         except ImportError as e:            # a shortcut, not a part that is needed: every call can go through ctypes

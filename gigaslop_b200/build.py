@@ -57,10 +57,25 @@ def build(force=False, verbose=False, defines=(), out=None):
     return target
 
 
-def build_native(force=False):
-    """Compile _native.so (CPython extension on torch's C++ headers) if missing or older than its sources."""
+def native_target():
+    """What _native.so is built for: it looks into torch's tensors, whose layout belongs to a release (and a C++ ABI) of torch."""
+    import platform
+    import torch
+    return f"torch {torch.__version__}, C++11 ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, Python {platform.python_version()}"
+
+
+def native_is_stale():
+    """_native.so is missing, older than its sources, or built for another torch or Python (the text it carries says which)."""
     deps = [NATIVE_SRC, os.path.join(ROOT, "include", "gigaslop_b200", "gigaslop_b200.h")]
-    if not force and os.path.exists(NATIVE) and all(os.path.getmtime(f) <= os.path.getmtime(NATIVE) for f in deps):
+    if not os.path.exists(NATIVE) or any(os.path.getmtime(f) > os.path.getmtime(NATIVE) for f in deps):
+        return True
+    with open(NATIVE, "rb") as f:
+        return native_target().encode() + b"\0" not in f.read()
+
+
+def build_native(force=False):
+    """Compile _native.so (CPython extension on torch's C++ headers) if it is stale."""
+    if not force and not native_is_stale():
         return NATIVE
     import sysconfig
     import torch
@@ -69,7 +84,7 @@ def build_native(force=False):
     inc = [sysconfig.get_paths()["include"], os.path.join(ROOT, "include"), os.path.join(t, "include"),
            os.path.join(t, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *["-I" + i for i in inc], "-o", NATIVE, NATIVE_SRC,
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DGSB200_NATIVE_TARGET="{native_target()}"', *["-I" + i for i in inc], "-o", NATIVE, NATIVE_SRC,
            "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:

@@ -346,4 +346,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__native() {
+  PyObject* m = PyModule_Create(&module);
+  // (the loader compares it before the first call)
+  if (m && PyModule_AddStringConstant(m, "TARGET", GSB200_NATIVE_TARGET) != 0) { Py_DECREF(m); return nullptr; }
+  return m;
+}

@@ -46,6 +46,22 @@ def test_package_works_without_the_native_path():
     assert r.returncode == 0, r.stdout + r.stderr
 
 
+def test_native_path_belongs_to_one_torch(monkeypatch):
+    """The extension looks into torch's tensors: one built for another torch is rebuilt, and not used."""
+    from gigaslop_b200 import build
+    build.build_native()
+    assert not build.native_is_stale()
+    monkeypatch.setattr(torch, "__version__", "99.0")
+    assert build.native_is_stale()
+    r = run_python("import warnings, torch; torch.__version__ = '99.0'\n"
+                   "import gigaslop_b200 as g; from gigaslop_b200 import _lib\n"
+                   "with warnings.catch_warnings(record=True) as w:\n"
+                   "    warnings.simplefilter('always'); g.lib()\n"
+                   "assert len(w) == 1 and 'torch 99.0' in str(w[0].message), w\n"
+                   "assert _lib.native is None\n")
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 @pytest.mark.gpu
 def test_native_path_gives_the_bytes_of_the_checked_path(monkeypatch):
     g = need_lib()
