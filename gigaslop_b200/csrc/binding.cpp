@@ -235,7 +235,8 @@ OPERATOR(dual_mx, 9)
   int32_t flags;
   SLOW_UNLESS(c.rows(a[0], A) && c.rows(a[1], G) && c.rows(a[2], U) && c.tensor(a[3], sa) && c.tensor(a[4], sg) && c.tensor(a[5], su) &&
               c.out_rows(a[6], q0) && c.out_rows(a[7], s0) && int32(a[8], flags));
-  SLOW_UNLESS(is_f8(A) && is_f8(G) && is_f8(U) && A->size(1) == G->size(1) && A->size(1) == U->size(1) && fits(G->size(0)) && fits(A->size(1)));
+  SLOW_UNLESS(is_f8(A) && is_f8(G) && is_f8(U) && A->size(1) == G->size(1) && G->sizes() == U->sizes() && G->stride(0) == U->stride(0) &&
+              fits(G->size(0)) && fits(A->size(1)));
   const int64_t M = A->size(0), N = G->size(0), K = A->size(1);
   const at::Tensor q = q0 ? *q0 : c.empty({M, N}, at::kFloat8_e4m3fn);
   const at::Tensor s = s0 ? *s0 : c.empty({M, N / 32}, at::kByte);
@@ -276,7 +277,8 @@ OPERATOR_END
 OPERATOR(mx_dual, 7)
   const at::Tensor *A, *sfa, *G, *U, *sg, *su, *C0;
   SLOW_UNLESS(c.rows(a[0], A) && c.tensor(a[1], sfa) && c.rows(a[2], G) && c.rows(a[3], U) && c.tensor(a[4], sg) && c.tensor(a[5], su) && c.out_rows(a[6], C0));
-  SLOW_UNLESS(is_f8(A) && is_f8(G) && is_f8(U) && A->size(1) == G->size(1) && A->size(1) == U->size(1) && fits(G->size(0)) && fits(A->size(1)));
+  SLOW_UNLESS(is_f8(A) && is_f8(G) && is_f8(U) && A->size(1) == G->size(1) && G->sizes() == U->sizes() && G->stride(0) == U->stride(0) &&
+              fits(G->size(0)) && fits(A->size(1)));
   const int64_t M = A->size(0), N = G->size(0), K = A->size(1);
   const at::Tensor C = C0 ? *C0 : c.empty({M, N}, at::kHalf);
   const gsb200_stream_t st = c.stream();

@@ -258,11 +258,16 @@ def _checked_gemm_fp8_rotary(A, B, scale_a, scale_b, sin_buf, cos_buf, nhead, he
                    nhead, head_dim, rotary_dim, seqlen, row_offset, out, flags, _F8)
 
 
-def _dual(fn, name, A, Bg, Bu, scale_a, sbg, sbu, out, flags, dtypes):
+def _check_dual(A, Bg, Bu, dtypes):
     M, N, K = _check_ab(A, Bg, dtypes)
     _check_ab(A, Bu, dtypes)
-    if Bu.shape != Bg.shape or Bu.stride(0) != Bg.stride(0):
+    if Bu.shape != Bg.shape or Bu.stride(0) != Bg.stride(0):      # the library describes both with one N and one stride
         raise ValueError("gate and up weights must share shape and row stride")
+    return M, N, K
+
+
+def _dual(fn, name, A, Bg, Bu, scale_a, sbg, sbu, out, flags, dtypes):
+    M, N, K = _check_dual(A, Bg, Bu, dtypes)
     _need_cuda(scale_a, sbg, sbu)
     C = out if out is not None else torch.empty((M, N), dtype=torch.float16, device=A.device)
     check(fn(A.data_ptr(), A.stride(0), Bg.data_ptr(), Bu.data_ptr(), Bg.stride(0), C.data_ptr(), C.stride(0),
@@ -337,8 +342,7 @@ def dual_gemm_fp8_silu_mxfp8(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up,
 
 @_on_device
 def _checked_dual_gemm_fp8_silu_mxfp8(A, B_gate, B_up, scale_a, scale_b_gate, scale_b_up, out, out_scale, flags):
-    M, N, K = _check_ab(A, B_gate, _F8)
-    _check_ab(A, B_up, _F8)
+    M, N, K = _check_dual(A, B_gate, B_up, _F8)
     _need_cuda(scale_a, scale_b_gate, scale_b_up)
     q = out if out is not None else torch.empty((M, N), dtype=torch.float8_e4m3fn, device=A.device)
     s = out_scale if out_scale is not None else torch.empty((M, N // 32), dtype=torch.uint8, device=A.device)
@@ -477,8 +481,7 @@ def dual_gemm_mxfp8_silu(A, sfa_tiled, B_gate, B_up, sfb_gate_tiled, sfb_up_tile
 
 @_on_device
 def _checked_dual_gemm_mxfp8_silu(A, sfa_tiled, B_gate, B_up, sfb_gate_tiled, sfb_up_tiled, out):
-    M, N, K = _check_ab(A, B_gate, _F8)
-    _check_ab(A, B_up, _F8)
+    M, N, K = _check_dual(A, B_gate, B_up, _F8)
     C = out if out is not None else torch.empty((M, N), dtype=torch.float16, device=A.device)
     check(lib().gsb200_dual_gemm_mxfp8_silu_f16(A.data_ptr(), A.stride(0), sfa_tiled.data_ptr(), B_gate.data_ptr(),
                                                 B_up.data_ptr(), B_gate.stride(0), sfb_gate_tiled.data_ptr(),

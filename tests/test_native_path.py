@@ -202,3 +202,28 @@ def test_call_that_the_library_refuses_is_made_once(monkeypatch):
         with pytest.raises(RuntimeError, match=rf"gigaslop_b200\.{name}: .* \(status -"):
             call()
         assert not entered, name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+def test_gate_and_up_weights_share_shape_and_stride(native, monkeypatch):
+    """The library describes both weights with the gate's row count and stride: an up weight with fewer rows would be read past
+    its end, one with another stride misread.  All four SwiGLU operators raise for both."""
+    g = need_lib()
+    from gigaslop_b200 import _lib
+    if not native:
+        monkeypatch.setattr(_lib, "native", None)
+    z = lambda *shape: torch.zeros(*shape, dtype=torch.uint8, device="cuda")
+    s, M, N, K = torch.ones(256, device="cuda"), 8, 256, 128
+    sf = lambda rows: z(g.lib().gsb200_mx_tiled_scale_bytes(rows, K))
+    f8 = torch.float8_e4m3fn
+    for up in (z(N // 2, K), z(2 * N, K), z(N, 2 * K)[:, :K]):
+        a, gate = z(M, K), z(N, K)
+        with pytest.raises(ValueError):
+            g.dual_gemm_i8_silu(a.view(torch.int8), gate.view(torch.int8), up.view(torch.int8), s, s, s)
+        with pytest.raises(ValueError):
+            g.dual_gemm_fp8_silu(a.view(f8), gate.view(f8), up.view(f8), s, s, s)
+        with pytest.raises(ValueError):
+            g.dual_gemm_fp8_silu_mxfp8(a.view(f8), gate.view(f8), up.view(f8), s, s, s)
+        with pytest.raises(ValueError):
+            g.dual_gemm_mxfp8_silu(a.view(f8), sf(M), gate.view(f8), up.view(f8), sf(N), sf(N))
