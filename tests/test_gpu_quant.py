@@ -119,3 +119,75 @@ def test_bounded_wait_gives_up_and_reports():
     q, s = g.quantize_tensor(x)
     q_ref, _ = oracle.quantize_tensor(x.cpu().float())
     assert torch.equal(q.cpu(), q_ref)
+
+
+def _rows_with_nan_and_inf(K, dtype):
+    """Rows of N(0, 1) values: finite ones between rows that hold a NaN (of either sign), an infinity, both, or nothing else."""
+    gen = torch.Generator().manual_seed(K)
+    nan, inf = float("nan"), float("inf")
+    x = torch.randn(24, K, generator=gen)
+    last = K - 1
+    for row, put in enumerate([{}, {0: nan}, {}, {last: -nan}, {K // 2: inf}, {}, {3: -inf}, {1: nan, 2: inf}, {last: inf, 0: -inf, 7: nan}]):
+        for i, v in put.items():
+            x[row, i] = v
+    x[9], x[10], x[11] = nan, inf, 0.0
+    x[12, :8], x[12, 8:] = nan, 0.0
+    x[13, ::2], x[13, 1::2] = inf, -0.0
+    return x.to(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("K", [8, 512, 1024, 2048, 2304])
+def test_fp8_quantiser_rows_with_nan_and_infinity(dtype, K):
+    """A NaN does not take part in the row maximum; an infinity does (scale infinity: the row's finite values become zeros).
+    What is not a number after the scaling is -448 in the torch formulation (the clamp) and NaN in the kernel formulation."""
+    g = need_lib()
+    x = _rows_with_nan_and_inf(K, dtype)
+    xf = x.float()
+    amax = torch.where(xf.isnan(), torch.zeros(()), xf.abs()).amax(dim=1, keepdim=True).clamp(min=1e-12)
+    scale = amax / 448.0
+    for torch_form in (True, False):
+        v = xf / scale if torch_form else xf * (torch.full_like(amax, 448.0) / amax)
+        q_ref = v.clamp(-448.0, 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
+        q_ref[v.isnan()] = 0xFE if torch_form else 0x7F
+        q, s = g.fp8_quantize_per_token(x.cuda(), torch_formulation=torch_form)
+        assert_bitexact(s, scale.squeeze(1), f"scale, torch_formulation={torch_form}")
+        assert_bitexact(q.view(torch.uint8), q_ref, f"bytes, torch_formulation={torch_form}")
+
+
+@pytest.mark.parametrize("K", [512, 1024, 2048, 2304])
+def test_fp8_quantiser_at_the_limits_of_fp32(K):
+    """Quotients without a division: row maxima up to the largest fp32 number and down to (and below) the floor of 1e-12, with
+    elements far smaller than the maximum, subnormals and both zeros among them."""
+    g = need_lib()
+    gen = torch.Generator().manual_seed(K + 1)
+    rows = []
+    for top in (3.4028234e38, 3e38, 2.0 ** 100, 448.0, 1.0, 1e-11, 1e-12, 9e-13, 1e-30, 1.2e-38, 1e-45):
+        for binades in (12, 140, 140):
+            x = (torch.rand(K, generator=gen) * 2 - 1) * top
+            x = x * torch.exp2(-torch.randint(0, binades, (K,), generator=gen).double()).float()
+            x[0], x[1], x[2], x[3] = top, 0.0, -0.0, 1e-45
+            x[4:12] = -top * torch.tensor([1.0, 0.5, 0.4999, 2 ** -6, 2 ** -9, 2 ** -10, 2 ** -10 * 1.0001, 2 ** -17])
+            rows.append(x)
+    x = torch.stack(rows)
+    q_ref, s_ref = oracle.fp8_quantize_per_token(x)
+    q, s = g.fp8_quantize_per_token(x.cuda())
+    assert_bitexact(s, s_ref, "fp8 scale")
+    assert_bitexact(q, q_ref, "fp8 bytes")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("K", [32, 512, 2048, 2304])
+def test_mx_quantiser_blocks_with_nan_and_infinity(dtype, K):
+    """Per block of 32: a NaN does not take part in the maximum and stays a NaN; an infinity gives the scale 2^120 and saturates."""
+    g = need_lib()
+    x = _rows_with_nan_and_inf(K, dtype)
+    blk = x.float().view(len(x), K // 32, 32)
+    amax = torch.where(blk.isnan(), torch.zeros(()), blk.abs()).amax(dim=-1)
+    byte = (((amax.view(torch.int32) >> 23) & 0xFF) - 8).clamp(0, 254)
+    v = blk * torch.ldexp(torch.ones_like(amax), 127 - byte).unsqueeze(-1)
+    q_ref = v.clamp(-448.0, 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
+    q_ref[v.isnan()] = 0x7F
+    q, s = g.mxfp8_quantize(x.cuda())
+    assert_bitexact(s, byte.to(torch.uint8), "E8M0 scales")
+    assert_bitexact(q.view(torch.uint8), q_ref.view(len(x), K), "bytes")
