@@ -145,11 +145,8 @@ def test_error_of_a_copy_on_write_tensor_is_raised():
     """Taking the data pointer of a lazily cloned tensor makes its copy, which can fail: the error is an ordinary exception (it
     is thrown while the interpreter lock is held).  In a child process, which is given little memory and leaves without
     freeing the tensor: torch itself aborts there after a copy that failed."""
-    import os
-    import subprocess
-    import sys
-    code = (
-        "import os, sys, torch; sys.path.insert(0, %r)\n"
+    r = run_python(
+        "import os, torch\n"
         "import gigaslop_b200 as g; from gigaslop_b200 import _lib\n"
         "g.lib(); assert _lib.native is not None\n"
         "x = torch.randn(1 << 16, 512, device='cuda').half(); torch.cuda.synchronize(); torch.cuda.empty_cache()\n"
@@ -164,9 +161,7 @@ def test_error_of_a_copy_on_write_tensor_is_raised():
         "    print('no error')\n"
         "except torch.OutOfMemoryError:\n"
         "    print('raised')\n"
-        "sys.stdout.flush(); os._exit(0)\n"
-    ) % os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+        "sys.stdout.flush(); os._exit(0)\n")
     assert r.returncode == 0 and r.stdout.split() == ["raised"], r.stdout + r.stderr
 
 
@@ -227,3 +222,46 @@ def test_gate_and_up_weights_share_shape_and_stride(native, monkeypatch):
             g.dual_gemm_fp8_silu_mxfp8(a.view(f8), gate.view(f8), up.view(f8), s, s, s)
         with pytest.raises(ValueError):
             g.dual_gemm_mxfp8_silu(a.view(f8), sf(M), gate.view(f8), up.view(f8), sf(N), sf(N))
+
+
+@pytest.mark.gpu
+def test_native_path_declines_one_argument_that_is_not_plain():
+    """CUDA operands throughout, so that nothing but the one argument named is the reason."""
+    need_lib()
+    from gigaslop_b200 import _lib
+    n = _lib.native
+    x = torch.randn(4, 64, device="cuda").half()
+    a, w = torch.ones(4, 64, dtype=torch.int8, device="cuda"), torch.ones(8, 64, dtype=torch.int8, device="cuda")
+    sa, sw = torch.ones(4, device="cuda"), torch.ones(8, device="cuda")
+    assert n.gemm(0, a, w, sa, sw, None, 0) is not None and n.quantize(0, x, None, None) is not None
+
+    class Sub(torch.Tensor):
+        pass
+
+    declined = {
+        "flags beyond 32 bits": (0, a, w, sa, sw, None, 1 << 40), "flags beyond 64 bits": (0, a, w, sa, sw, None, 1 << 80),
+        "float flags": (0, a, w, sa, sw, None, 0.0), "K mismatch": (0, a[:, :32], w, sa, sw, None, 0),
+        "1-D operand": (0, a[0], w, sa, sw, None, 0), "inner stride": (0, a[:, ::2], w[:, :32], sa, sw, None, 0),
+        "wrong type": (0, a.float(), w, sa, sw, None, 0), "INT8 for FP8": (1, a, w, sa, sw, None, 0),
+        "subclass": (0, a.as_subclass(Sub), w, sa, sw, None, 0), "CPU scale": (0, a, w, sa.cpu(), sw, None, 0),
+        "CPU output": (0, a, w, sa, sw, torch.empty(4, 8, dtype=torch.float16), 0), "not a tensor": (0, a, w, [1.0], sw, None, 0),
+        "conjugate view": (0, a, w, torch.ones(4, dtype=torch.complex64, device="cuda").conj(), sw, None, 0),
+        "negative view": (0, a, w, torch.ones(4, dtype=torch.complex64, device="cuda").conj().imag, sw, None, 0),
+        "an argument too few": (0, a, w, sa, sw, None),
+    }
+    for what, args in declined.items():
+        assert n.gemm(*args) is None, what
+    assert n.quantize(0, x.double(), None, None) is None
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    for mode in (TorchFunctionMode, TorchDispatchMode):
+        with mode():
+            assert n.gemm(0, a, w, sa, sw, None, 0) is None, mode.__name__
+    seen = []
+
+    def batched(t):
+        seen.append(n.quantize(0, t, None, None))
+        return t
+
+    torch.vmap(batched)(x[None])
+    assert seen == [None]
