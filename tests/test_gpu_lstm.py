@@ -32,8 +32,8 @@ def check_h(got, ref, what, tol=0.03, mean_tol=3e-3):
 
 @pytest.mark.parametrize("T,B,H,reverse,init", [(12, 130, 64, False, False), (40, 256, 384, True, True),
                                                 (7, 128, 32, False, True), (25, 512, 384, False, False),
-                                                # H > 384: the cooperative kernel (h through global scratch), four K blocks,
-                                                # zero-padded K pieces of W and h when H % 128 != 0
+                                                # H > 384: four K blocks (the fourth of W_hh in shared memory), zero-padded
+                                                # K pieces of W and h when H % 128 != 0
                                                 (10, 256, 512, False, True), (8, 130, 416, True, True),
                                                 (20, 512, 512, True, False), (6, 300, 448, False, False)])
 def test_recurrent_kernel_vs_oracle(T, B, H, reverse, init):
@@ -73,7 +73,7 @@ def test_two_layer_stack_vs_oracle():
 
 
 def test_three_layer_stack_h512_forward_first():
-    """H = 512 (cooperative kernel), three layers, first layer forward, ragged batch."""
+    """H = 512 (four CTAs per row group), three layers, first layer forward, ragged batch."""
     g = need_lib()
     gen = torch.Generator().manual_seed(56)
     T, B, C, H = 9, 200, 128, 512
@@ -114,10 +114,9 @@ def test_lstm_rejects_unsupported_shapes():
 
 @pytest.mark.parametrize("env_key", ["GSB200_LSTM_NO_CLUSTER", "GSB200_LSTM_ROWS128"])
 def test_cluster_and_cooperative_kernels_agree(tmp_path, env_key):
-    """The recurrence has three kernels: the cluster form on 64-row groups (the default while twice the CTAs fit the
-    GPU), the cluster form on 128-row groups (h exchanged through distributed shared memory, H <= 384) and the
-    cooperative form with global scratch (any H <= 512, and the fallback).  Same arithmetic per cell, so the same
-    bytes: the other two forms are forced in a child process through the environment."""
+    """The recurrence has two kernels: the transposed form on clusters of up to four CTAs and the cooperative form on 128-row
+    tiles with global scratch (the fallback).  Same arithmetic per cell and same order of the sums, so the same bytes: the
+    other form is forced in a child process through the environment, by either of its two switches."""
     import os
     import subprocess
     import sys
