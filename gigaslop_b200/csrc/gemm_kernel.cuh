@@ -283,7 +283,6 @@ struct TileWalk {
 };
 
 // Register budgets of the twelve-epilogue-warp form (512 threads compiled at 128 registers: 128 x 56 + 384 x 152 = 65536).
-constexpr int EW12_THREADS = 32 * (FRONT_WARPS + 12);
 constexpr int EW12_FRONT_REGS = 56;
 constexpr int EW12_EPI_REGS = 152;
 constexpr int EW12_REG_POOL_NEEDED = 32 * (FRONT_WARPS * EW12_FRONT_REGS + 12 * EW12_EPI_REGS);

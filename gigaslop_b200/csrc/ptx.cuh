@@ -31,20 +31,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ uint32_t lane_id() {
-  uint32_t l; asm volatile("mov.u32 %0, %%laneid;" : "=r"(l)); return l;
-}
-
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(pred));
-  return pred != 0;
-}
-
 // ---- abort flag -------------------------------------------------------------
 // One int in the CTA's shared memory that any role sets when a bounded wait gives up; the other roles poll it
 // and unwind.  Held as its 32-bit shared-window address (one register in every waiting role; a generic pointer
@@ -64,8 +50,8 @@ struct AbortFlag {
 // a kernel may start while the one before it drains.  None of them touches global memory before pdl_wait, which returns when
 // the kernel before it is complete and its writes are visible; at least one block of a grid has to wait.  Data another kernel
 // may have written is not read through the non-coherent path (ld.global.nc): that is for data constant over the kernel's
-// life.  pdl_trigger lets the successor's CTAs become resident as this kernel's leave.  The quantisers (after their wait) and
-// the LSTM step do that: the GEMM behind them sets up its barriers and tensor memory meanwhile.  The GEMMs do not: a
+// life.  pdl_trigger lets the successor's CTAs become resident as this kernel's leave.  The quantisers (after their wait), the
+// scale re-tiler and the LSTM cell (before theirs) do that: the GEMM behind them sets up its barriers and tensor memory meanwhile.  The GEMMs do not: a
 // quantiser that starts beside their last tiles costs more than it gains (us per pass, no overlap / quantisers trigger /
 // GEMMs too: QKV of 65536 rows 84.3 / 79.7 / 83.8, feed-forward 246 / 239 / 249, of 256 rows 28.7 / 22 / 22, of 9001 rows
 // 54.6 / 46 / 47).
@@ -97,31 +83,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(smem_u32(bar)), "r"(parity), "r"(kTryWaitSuspendNs)
-      : "memory");
-  return ok != 0;
-}
-
-// Non-blocking test of a phase (no suspend): for a thread that polls several barriers in turn.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// One try_wait that may keep the thread suspended for up to `ns` nanoseconds (woken early when the phase completes).
-__device__ __forceinline__ bool mbar_try_wait_ns(uint64_t* bar, uint32_t parity, uint32_t ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
       : "memory");
   return ok != 0;
 }
@@ -163,22 +124,7 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_addr, uint32_t rank) {
   uint32_t r; asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank)); return r;
 }
-__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t cluster_addr) {
-  uint4 v;
-  asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(cluster_addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint4 v) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
-               ::"r"(cluster_addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-// Arrive on an mbarrier of another CTA of the cluster; release at cluster scope, so what this thread wrote (and
-// what a CTA barrier ordered before it) is visible to whoever acquires the barrier's completion.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The same arrive with the default ordering (release at CTA scope): enough where what the waiter needs is ordered by
+// Arrive on an mbarrier of another CTA of the cluster, with the default ordering (release at CTA scope): enough where what the waiter needs is ordered by
 // other means (tcgen05 fences around a tensor-memory hand-over), and much cheaper than a cluster-scope release.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
@@ -218,7 +164,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
 // ---- TMA --------------------------------------------------------------------
 // Untiled bulk copy global -> shared that reports its bytes to an mbarrier.  Both addresses 16-byte aligned,
@@ -250,13 +195,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uint64_t* bar, int32_t c0, int32_t c1,
-                                            int32_t c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
 // 2-D tiled store shared -> global (bulk async-group completion).
@@ -318,26 +256,6 @@ __device__ __forceinline__ uint64_t umma_smem_desc_sw128(uint32_t smem_addr) {
   d |= (uint64_t)1 << 46;                            // [46,48) descriptor version (Blackwell)
   d |= (uint64_t)2 << 61;                            // [61,64) layout: SWIZZLE_128B
   return d;
-}
-
-// Descriptor for an unswizzled K-major operand kept as [16-byte K chunk][row][16 bytes]: the 8 x 16-byte core
-// matrices of one K chunk follow each other every 128 bytes (stride byte offset), the next K chunk starts
-// `chunk_bytes` further on (leading byte offset).  One 32-byte K step of an 8-bit MMA spans two chunks, so stepping
-// along K adds 2 * chunk_bytes >> 4 to the start-address field.
-__device__ __forceinline__ uint64_t umma_smem_desc_kchunks(uint32_t smem_addr, uint32_t chunk_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((chunk_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)(128 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  return d;                                          // layout bits [61,64) = 0: no swizzle
-}
-// Bulk copy from this CTA's shared memory into the shared memory of a CTA of the cluster; the bytes are reported
-// to an mbarrier of the destination CTA (both destination addresses are cluster addresses from mapa_shared).
-__device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst_cluster_addr, const void* src, uint32_t bytes,
-                                                     uint32_t mbar_cluster_addr) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst_cluster_addr), "r"(smem_u32(src)), "r"(bytes), "r"(mbar_cluster_addr) : "memory");
 }
 
 // 16 bytes from registers into the shared memory of a CTA of the cluster, reported to an mbarrier of that CTA (both are
@@ -434,15 +352,9 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on ONE mbarrier, given as a shared::cluster address (this CTA's or the pair's other CTA's), when all MMAs
-// this thread issued before are done.  A barrier in each CTA takes two of these.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr)
-               : "memory");
-}
-// The same arrival delivered to the barrier at this shared-memory offset in BOTH CTAs of the pair with one instruction
-// (a commit costs its thread about 58 clocks, and the thread that issues a pair's MMAs has few to spare).  This is
-// the multicast of an mbarrier ARRIVAL; no data moves and no load is involved.
+// Arrive, when all MMAs this thread issued before are done, on the barrier at this shared-memory offset in BOTH CTAs of
+// the pair: one instruction, because a commit costs its thread about 58 clocks and the thread that issues a pair's MMAs
+// has few to spare.  This is the multicast of an mbarrier ARRIVAL; no data moves and no load is involved.
 __device__ __forceinline__ void umma_commit_pair_both(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(smem_u32(bar)), "h"((uint16_t)3)
@@ -518,16 +430,6 @@ __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// 16 lanes x 256 bit, twice (16 consecutive 32-bit columns): the layout of an M = 64 accumulator, whose 64 rows sit in
-// the lower 16 lanes of each 32-lane quarter.  Thread i of the warp gets rows i / 4 and i / 4 + 8 of its quarter's 16:
-// v[4k + 0..1] = columns col + 8k + 2 (i % 4) + {0, 1} of row i / 4, v[4k + 2..3] = the same columns of row i / 4 + 8.
-__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[8], uint32_t (&b)[8], uint32_t (&c)[8], uint32_t (&d)[8]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
@@ -567,8 +469,6 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[16], uint32_t (&b)[16
 // compiler (64-bit inline-asm operands cost extra moves) and nothing is contracted into a fused multiply-add.
 __device__ __forceinline__ float2 pk2(float lo, float hi) { return make_float2(lo, hi); }
 __device__ __forceinline__ float2 fmul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 fsub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 __device__ __forceinline__ uint32_t pack_half2_from(float2 v) {
   __half2 h = __float22half2_rn(v);
   return *reinterpret_cast<uint32_t*>(&h);
@@ -591,28 +491,6 @@ __device__ __forceinline__ void stg_v8(void* p, uint4 a, uint4 b) {
 }
 
 // ---- misc -----------------------------------------------------------------------
-__device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-// Barrier over `nthreads` threads that also ANDs a predicate: every participant gets the same answer,
-// so a group of warps can agree to leave a loop together (nobody is left waiting at a later barrier).
-// Returns 1 when every participant passed a true predicate, else 0.
-__device__ __forceinline__ uint32_t named_barrier_and(uint32_t id, uint32_t nthreads, bool pred) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %3, 0;\n\t"
-      "bar.red.and.pred q, %1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"(id), "r"(nthreads), "r"((uint32_t)pred)
-      : "memory");
-  return r;
-}
-// Shared-memory reads the compiler may schedule freely: not volatile and without a memory clobber, so they
-// are not ordered against unrelated shared-memory stores.  Only for data that is read-only while the address
-// value is live; derive the address from the result of the synchronisation that published the data, which
-// keeps the reads behind it.
 // Global loads that stay where they are written (volatile): used to start a load a whole tile
 // before its value is needed; the compiler would otherwise be free to sink it to the point of use.
 __device__ __forceinline__ float4 ldg_f4_here(const float* p) {
@@ -625,6 +503,10 @@ __device__ __forceinline__ float ldg_f_here(const float* p) {
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
   return v;
 }
+// Shared-memory reads the compiler may schedule freely: not volatile and without a memory clobber, so they
+// are not ordered against unrelated shared-memory stores.  Only for data that is read-only while the address
+// value is live; derive the address from the result of the synchronisation that published the data, which
+// keeps the reads behind it.
 __device__ __forceinline__ float4 lds_f4_ro(uint32_t addr) {
   float4 v;
   asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
