@@ -58,7 +58,7 @@ struct LstmLayerArgs {
   const uint8_t* h0; const __half* c0;      // [B, H] initial state or null
   __half* h_out; uint8_t* h8_out; __half* c_last;
   long long T, B; int H; int reverse;
-  int max_ctas = 0;                          // CTAs the recurrence may occupy at a time (0 = the whole GPU)
+  int max_ctas = 0;                          // CTAs the recurrence should get by with, where a form can (0 = the whole GPU)
 };
 size_t lstm_scratch_bytes(long long B, int H);
 int32_t launch_lstm_layer(const LstmLayerArgs& a, void* scratch, size_t scratch_bytes, cudaStream_t st);

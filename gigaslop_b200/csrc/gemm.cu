@@ -94,7 +94,7 @@ static bool make_map_2d(CUtensorMap* m, CUtensorMapDataType dt, int esz, const v
 // ---- per-device state -------------------------------------------------------------------------
 // Atomics: the contract allows one host thread per GPU, and two of them may meet here.
 constexpr int kMaxDevices = 64;
-constexpr int kVariantMinRowBlocks = 256;      // 128-row blocks from which the twelve-warp form is the default for the SwiGLU
+constexpr int kVariantMinRowBlocks = 256;      // 128-row blocks from which the twelve-warp form is the default for the SwiGLU (see launch_gemm)
 static std::atomic<int> g_dev_ok[kMaxDevices];       // 0 unknown, 1 ok, -1 unsupported
 static std::atomic<int> g_dev_sms[kMaxDevices];
 
@@ -413,7 +413,12 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
     // pair halves the W part: 12-22 % at M = 65536) from the point where single CTAs would need a second round (up to
     // there they are faster: M = 9001, N = 512, K = 2048 9.5 us against 10.8); the activation-stationary rotary kernel takes both together (twelve
     // warps alone leave it waiting for operands, pairs alone for its epilogue; together 3 % at config 2 and less
-    // power); everywhere else the eight-warp single-CTA kernel is as fast or faster.
+    // power); elsewhere the eight-warp single-CTA kernel.  Where the SwiGLU's line could lie (INT8, eight against twelve
+    // warps, us): K = 512, N = 2048 equal from 2 row blocks (6.0 / 5.9) over 64 (18.1 / 18.2) and 128 (30.3 / 30.2) to 256
+    // (57.0 / 56.6); K = 384, N = 1536 equal up to 48 row blocks (11.0 / 10.7), then twelve ahead: 64 14.2 / 13.4, 128 22.1 /
+    // 20.6, 256 39.6 / 38.1; K = 256, N = 1024 twelve ahead from 48 (8.6 / 8.0), 128 16.2 / 14.8, 256 26.9 / 24.2.  FP8 the
+    // same.  So for K < 512 the line lies higher than it need.  The general rotary epilogues exist with eight warps and
+    // single CTAs only.
     const int ew = variant_setting(g_variant_ew, "GSB200_GEMM_EW"), pm = variant_setting(g_variant_pair, "GSB200_GEMM_PAIR");
     const bool big = p.m_blocks >= kVariantMinRowBlocks;
     // twelve warps AND pairs, or neither (so not when the caller has fixed one of the two)
@@ -454,7 +459,7 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
       // round end soonest; with fewer row blocks than CTAs it is the only round.  K = 512, N = 1536: M = 333 takes 7.8 us
       // instead of 18.8, M = 2048 8.3 instead of 19.2.  (Single tiles in turn would balance as well, but a CTA would fetch
       // sin / cos rows for every tile: 4096 scattered 16-byte reads, as long as the tile's products at K = 768.  A share is
-      // charged half a tile for them.  M = 20001: K = 768 52 -> 37 us, K = 1024 69 -> 53.)
+      // charged half a tile for them.  M = 20001: K = 768 52 -> 38 us, K = 1024 69 -> 55.)
       const int rem = p.m_blocks % sms;
       if (rem > 0) {
         long long best = 2 * p.n_blocks + 1;         // half tiles of a CTA in the round with one share, the whole row block
@@ -471,8 +476,8 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
   }
   cudaError_t e = cudaErrorInvalidValue;
   // The SwiGLU that emits MXFP8, weight-stationary: twelve warps, staged output (M = 65536, K = 512, N = 2048: 145 us with
-  // eight warps and 32-byte stores per thread and row, 114 now; K = 384, N = 1536 109 and 73; M = 9001 26.7 and 20.6; equal at
-  // a few hundred rows).
+  // eight warps and 32-byte stores per thread and row, 114 now; K = 384, N = 1536 109 and 73; M = 9001 26.7 and 20.6; 2 to 8 row
+  // blocks 6.1 and 5.8, 6.4 and 6.2).  The eight-warp form is the variant override's.
   if (a.epi == EPI_SILU_MX && resident && variant_setting(g_variant_ew, "GSB200_GEMM_EW") != 8 &&
       Variant<KIND_F8, EPI_SILU_MX, false, 12>::capacity(true)) {
     if (!make_map_2d(&tc, u8, 1, a.C, (uint64_t)a.M, (uint64_t)a.N, (uint64_t)a.ldc, 64, 32, CU_TENSOR_MAP_SWIZZLE_64B)) return GSB200_ERR_BAD_ARG;

@@ -230,8 +230,9 @@ struct TileWalk {
   int n_lo, n_hi;  // row-block-major walks: this CTA's column blocks of row block m are [n_lo, n_hi)
   int visit;       // row-block-major walks: how many row blocks this CTA has left behind
   // Row blocks cta, cta + grid, ... while whole rounds last.  The row blocks left over (fewer than CTAs) would
-  // keep some SMs busy for a whole row block while the others idle: with the rotary epilogue each of them is cut into p.ares_split shares of consecutive column blocks (none empty; the host sees to that), which are
-  // dealt to the CTAs in turn (each loads the A block).
+  // keep some SMs busy for a whole row block while the others idle: with the rotary epilogue each of them is cut into
+  // p.ares_split shares of consecutive column blocks (none empty; the host sees to that), which are dealt to the CTAs
+  // in turn (each loads the A block).
   __device__ __forceinline__ void set_visit(const GemmParams& p) {
     const int grid = ncta(), full = p.m_blocks / grid, rem = p.m_blocks - full * grid;
     m = p.m_blocks;                                   // nothing left unless one of the cases below applies
@@ -1109,7 +1110,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             emit(vb, c + 32);
           }
         } else if constexpr (EPI == EPI_ROTARY_GEN) {
-          // Any head of 64 or 128 columns with its first 2 * rot_half columns rotated: x0 = columns [0, rot_half) of
+          // Heads of 128 columns with the first 32 or 96 rotated (what EPI_ROTARY and EPI_ROTARY_HD leave; the code takes any
+          // head of 64 or 128 with its first 2 * rot_half columns rotated): x0 = columns [0, rot_half) of
           // the head, x1 = [rot_half, 2 rot_half), the rest of the head and every V column only dequantised
           // (cute/ampere_gemm_i8_rotary.py:362-393).  Same arithmetic, rounded at the same points, as EPI_ROTARY; 16
           // columns of x0 and the matching 16 of x1 at a time, sin / cos rows read per use, 32-byte stores straight

@@ -688,8 +688,10 @@ static int lt_capacity(int form, int slices, int dev) {
   return c > 0 ? c : 0;
 }
 
-// The form with the shortest step (times the waves it takes), row groups limited to `max_ctas` CTAs at a time (0 = the whole
-// GPU); -1 = none.  Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows
+// The form with the shortest step (times the waves it takes) if the recurrence is to leave the SMs past `max_ctas` to a
+// projection beside it (0 = it has the whole GPU); -1 = none.  `max_ctas` only steers this choice, in which groups past it wait
+// for a next wave: a launch brings all its row groups, and where no form holds them in `max_ctas` CTAs they take more SMs
+// (lstm_layer_ctas counts what a launch does occupy).  Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows
 // (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.36 us per step; 12 rows in two
 // waves 2.68).  *ns = the step.
 static int lt_choose(long long B, int H, int dev, int max_ctas, long long* ns = nullptr) {
@@ -746,7 +748,7 @@ static int lstm_layer_ctas(long long B, int H, int max_ctas) {
 }
 
 // How many launches to cut a layer's recurrence into so that the next layer's projection runs beside it (1 = not at all).
-// The cut recurrence keeps to `max_ctas` CTAs, which may cost it a form with longer steps, and every launch about 12 us;
+// The cut recurrence is steered to `max_ctas` CTAs, which may cost it a form with longer steps, and every launch about 12 us;
 // it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 16.9 ms one after the other, 16.3
 // in seven blocks; at B = 512, H = 512 (T = 1000, three layers) 7.3 ms against 8.6, so not cut.
 static int lstm_time_blocks(long long T, long long B, int H, int max_ctas) {

@@ -109,9 +109,10 @@ __device__ __forceinline__ uint2 pack_e4m3_quot(const float (&v)[8], float s, fl
 
 // This warp's row.  The rows are walked from the last to the first: the GEMMs walk theirs upwards, so a quantiser starts
 // with the rows its producer wrote last and leaves the rows its consumer reads first written last.  Where a tensor is
-// larger than L2 (126 MB) that is what is found there.  The input is read with the
-// streaming hint, so that it does not push the output out.  Feed-forward passes of 65536 rows: INT8 240.7 -> 234.2 us (walked
-// backwards) -> 229.1 (streaming hint), MXFP8 285 -> 281 -> 276.
+// larger than L2 (126 MB) that is what is found there.  The input is read with the streaming hint, so that it does not push
+// the output out.  Feed-forward passes of 65536 rows, a few back to back at the full clock: INT8 240.7 -> 234.2 us (walked
+// backwards) -> 229.1 (streaming hint), MXFP8 285 -> 281 -> 276.  (In runs of a second the power cap takes the clock from 1965
+// to about 1510 MHz and the INT8 pass to 268 us.)
 __device__ __forceinline__ long long quant_row() {
   return (long long)(gridDim.x - 1 - blockIdx.x) * QUANT_WARPS + (threadIdx.x >> 5);
 }

@@ -4,10 +4,10 @@ and streams; every byte of compute happens in libgigaslop_b200.so.
 Function names and argument meaning follow the reference's host helpers
 (``quantize_tensor``, ``fp8_quantize_per_token``) and kernels.
 
-An operator first offers the call to the native path (``_lib.native``, csrc/binding.cpp), which takes it when every
-argument is a plain CUDA tensor of the current device that passes the operator's checks, and answers None otherwise;
-then the ``_checked_*`` function of the same operator decides: it raises what is wrong with the arguments, or makes the
-call through ctypes.
+An operator that has a ``_checked_*`` function first offers the call to the native path (``_lib.native``, csrc/binding.cpp),
+which takes it when every argument is a plain CUDA tensor of the current device that passes the operator's checks, and
+answers None otherwise; then the ``_checked_*`` function decides: it raises what is wrong with the arguments, or makes the
+call through ctypes.  The others (``gemm_i8_i32``, ``gemm_f16``, ``quantize_gemm_i8_rotary``) go through ctypes always.
 """
 import functools
 
