@@ -7,6 +7,7 @@
 #include "capi_internal.h"
 #include "diag.h"
 #include "gemm_kernel.cuh"
+#include "gemm_small.cuh"
 
 namespace gsb {
 
@@ -374,6 +375,16 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
   p.x_f16 = a.x_f16; p.ldx = a.ldx; p.scale_a_out = a.scale_a_out;
   const long long tiles = (long long)p.m_blocks * p.n_blocks;
   if (tiles > 0x7fffffffll) return GSB200_ERR_BAD_ARG;
+
+  // Few tiles: the form with small ones, gemm_small.cuh (unless the caller has fixed a variant or the schedule of the persistent
+  // kernel).
+  if (!fused && !(a.flags & (GSB200_DIAG_FLAG_MASK | GSB200_FLAG_OWN_ROW_BLOCKS)) && (a.kind == KIND_I8 || a.kind == KIND_F8) &&
+      (a.epi == EPI_DEQUANT || a.epi == EPI_SILU || a.epi == EPI_SILU_MX || (a.epi == EPI_ROTARY && (!general_rotary || rot_geo >= 0))) &&
+      variant_setting(g_variant_ew, "GSB200_GEMM_EW") < 0 && variant_setting(g_variant_pair, "GSB200_GEMM_PAIR") < 0) {
+    bool taken = false;
+    rc = launch_gemm_small(a, p, general_rotary ? rot_geo : 3, st, &taken);
+    if (taken || rc != GSB200_OK) return rc;
+  }
 
   CUtensorMap ta, tb0, tb1, tc;
   const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;

@@ -647,8 +647,9 @@ struct LtForm { int rows, threads, smem[LT_MAX_SLICES + 1], step_ns[LT_MAX_SLICE
 template <int R, int G, int CW>
 static constexpr LtForm lt_make_form(int ns1, int ns2, int ns3, int ns4) {
   LtForm f{G, 32 * (CW + 4), {}, {0, ns1, ns2, ns3, ns4}, lstm_tmem_kernel<R, G, CW>};
-  // (at least 120 KiB: one CTA per SM, it takes all of tensor memory)
-  for (int n = 1; n <= LT_MAX_SLICES; ++n) f.smem[n] = LtSmem<R, G>::bytes(n) > 120 * 1024 ? LtSmem<R, G>::bytes(n) : 120 * 1024;
+  // (at least 212 KiB: it takes all of tensor memory, and no CTA of another stream that wants some, a few-tile GEMM's, may sit
+  // beside it waiting)
+  for (int n = 1; n <= LT_MAX_SLICES; ++n) f.smem[n] = LtSmem<R, G>::bytes(n) > 212 * 1024 ? LtSmem<R, G>::bytes(n) : 212 * 1024;
   return f;
 }
 constexpr int LT_FORMS = 5;
