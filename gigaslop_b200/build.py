@@ -85,7 +85,7 @@ def build_native(force=False):
            os.path.join(t, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DGSB200_NATIVE_TARGET="{native_target()}"', *["-I" + i for i in inc], "-o", NATIVE, NATIVE_SRC,
-           "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+           "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError("compiling the native binding failed:\n" + r.stdout[-4000:])

@@ -265,3 +265,28 @@ def test_native_path_declines_one_argument_that_is_not_plain():
 
     torch.vmap(batched)(x[None])
     assert seen == [None]
+
+
+@pytest.mark.gpu
+def test_outputs_are_what_torch_empty_makes():
+    """Outputs come from torch's CUDA allocation function without the dispatcher: ordinary tensors, inference tensors under
+    inference mode, and the dispatcher's (filled) ones in the deterministic mode -- with the same bytes in each."""
+    g = need_lib()
+    x = torch.randn(300, 512, generator=torch.Generator().manual_seed(2)).half().cuda()
+    q, s = g.quantize_tensor(x)
+    for t in (q, s):
+        e = torch.empty(t.shape, dtype=t.dtype, device="cuda")
+        assert type(t) is torch.Tensor and t.stride() == e.stride() and t.storage_offset() == 0 and t.device == e.device
+        assert t.untyped_storage().nbytes() == e.untyped_storage().nbytes() and t._version == 0 and not t.is_inference()
+        assert torch._C._dispatch_keys(t) == torch._C._dispatch_keys(e)
+    with torch.inference_mode():
+        qi, si = g.quantize_tensor(x)
+        assert qi.is_inference() and si.is_inference() and torch.equal(qi, q) and torch.equal(si, s)
+    try:
+        torch.use_deterministic_algorithms(True)
+        qd, sd = g.quantize_tensor(x)
+        assert torch.equal(qd, q) and torch.equal(sd, s)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    e, se = g.quantize_tensor(x[:0])
+    assert e.shape == (0, 512) and se.shape == (0,)
