@@ -520,6 +520,187 @@ mx_gemm256_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, MX_TMEM_COLS); }
 }
 
+// ---- weight-stationary form with 256-column tiles (K <= 512) ---------------------------------------------------------
+// The 128 x 128 weight-stationary form above is bound by shared memory: 224 KiB (dual) pass through it per tile, 1790 clocks, and
+// its 32 column slices leave 20 SMs idle.  With 256 accumulator columns (dual: 128 gate | 128 up) an MMA takes 128 clocks and
+// reads 12 KiB for them (96 instead of 128 bytes per clock), A passes through L2 and shared memory half as often, and N = 2048
+// is 16 slices, 144 CTAs.  TMEM holds one such accumulator beside the scale factors; the next tile's MMAs begin when the
+// epilogue has it in registers.
+// M = 65536, us (graph of launches): dual K = 512, N = 2048 130.5 -> 120; K = 384, N = 1536 83 -> 77; K = 256, N = 1024 48.4 ->
+// 41.9; K = 128, N = 512 25.3 -> 19.3; plain K = 512, N = 2048 74.7 -> 72.5.  The large ones run at about 1.58 GHz under the power
+// cap (190 k clocks at K = 512); there, scale tiles copied to TMEM a K block ahead (131), a warp of its own for them (118) and
+// warp-converged producers (121) change little or lose.
+//   warps 0, 3  producers: K block i of the CTA goes to ring stage i % 4, filled by warp 0 (even) or 3 (odd); warp 0 also loads
+//               the resident slice, K block by K block
+//   warp 1      MMA issue        warps 4..11  epilogue: lane quarter e % 4, column half e / 4 (of gate and up)
+constexpr int MXV_BN = 256;
+constexpr int MXV_STAGES = 4;
+constexpr int MXV_W_KB = MXV_BN * MX_BK;                                  // 32 KiB: W rows of one K block (dual: 128 gate | 128 up)
+constexpr int MXV_A = MXW_MAX_KB * MXV_W_KB;                              // ring of A blocks
+constexpr int MXV_SFA = MXV_A + MXV_STAGES * MX_A_BYTES;                  // their scale tiles
+constexpr int MXV_OUT = MXV_SFA + MXV_STAGES * MX_SF_BYTES;               // staging: per epilogue warp 32 rows x 64 fp16
+constexpr int MXV_OUT_BUF = 4096;
+// The W scale tiles (two per K block) land in the staging boxes: they are copied to TMEM before the first MMAs, whose
+// completion the epilogue waits for before it writes there.
+constexpr int MXV_SFB = MXV_OUT;
+constexpr int MXV_BAR = MXV_OUT + MX_EPI_WARPS * MXV_OUT_BUF;
+constexpr int MXV_BYTES = MXV_BAR + 256;                                  // (no room to align the base: it is 1 KiB-aligned by declaration)
+constexpr int MXV_SFA_COL = 256, MXV_SFB_COL = 256 + 4 * MXV_STAGES;      // TMEM columns of the scale factors
+static_assert(MXV_BYTES <= 227 * 1024 && MXV_OUT % 1024 == 0 && MXV_SFB_COL + 8 * MXW_MAX_KB <= MX_TMEM_COLS, "budget");
+
+template <bool DUAL>
+__global__ void __launch_bounds__(MX_THREADS, 1)
+mx_gemm256w_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b0, const __grid_constant__ CUtensorMap tm_b1,
+                   const __grid_constant__ CUtensorMap tm_c, const MxParams p) {
+  extern __shared__ __align__(1024) uint8_t mxv_smem[];
+  uint8_t* smem = mxv_smem;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + MXV_BAR);
+  uint64_t* full = bars;                                   // [MXV_STAGES]
+  uint64_t* empty = full + MXV_STAGES;                     // [MXV_STAGES]
+  uint64_t* w_full = empty + MXV_STAGES;                   // [MXW_MAX_KB] a K block of the resident slice and its scale tiles
+  uint64_t* acc_full = w_full + MXW_MAX_KB;
+  uint64_t* acc_empty = acc_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+  const AbortFlag abort_flag{smem_u32(tmem_slot + 1)};
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int OUT_COLS = DUAL ? MXV_BN / 2 : MXV_BN;
+  if ((smem_u32(smem) & 1023u) != 0) {                     // (cannot happen: the swizzled tiles need it)
+    if (threadIdx.x == 0) atomicOr(&g_status[0], ST_TIMEOUT_MMA);
+    return;
+  }
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < MXV_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int kb = 0; kb < MXW_MAX_KB; ++kb) mbar_init(&w_full[kb], 1);
+    mbar_init(acc_full, 1); mbar_init(acc_empty, MX_EPI_WARPS);
+    abort_flag.set(0);
+    fence_mbar_init();
+    prefetch_tmap(&tm_a); prefetch_tmap(&tm_b0); prefetch_tmap(&tm_b1); prefetch_tmap(&tm_c);
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, MX_TMEM_COLS); tmem_relinquish(); }
+  pdl_wait();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const unsigned int budget = spin_budget();
+  const int ws_n = (int)(blockIdx.x % p.n_blocks), ws_g = (int)(blockIdx.x / p.n_blocks);    // column slice, row-block group
+  const int n0 = ws_n * OUT_COLS;
+  const bool two = DUAL || 2 * ws_n + 1 < (p.N + 127) / 128;      // the second 128 columns have scale tiles
+
+  if (warp == 0 || warp == 3) {
+    if (lane == 0) {
+      const int mine = warp == 3 ? 1 : 0;
+      bool ok = true;
+      int i = 0;                                           // K blocks of A so far
+      for (int m_blk = ws_g; ok && m_blk < p.m_blocks; m_blk += p.n_groups) {
+        // the row block after this one goes to L2 now (one CTA of the column slices asks for it)
+        const int m_pf = m_blk + p.n_groups;
+        if (mine == 1 && m_pf < p.m_blocks && ws_n == (m_pf / p.n_groups) % p.n_blocks)
+          for (int kb = 0; kb < p.k_blocks; ++kb) tma_prefetch_l2_2d(&tm_a, kb * MX_BK, m_pf * MX_BM);
+        for (int kb = 0; kb < p.k_blocks; ++kb, ++i) {
+          if (mine == 0 && i < p.k_blocks) {               // the slice, beside the first row block
+            uint8_t* wb = smem + kb * MXV_W_KB;
+            uint8_t* sf = smem + MXV_SFB + kb * 2 * MX_SF_BYTES;
+            mbar_arrive_expect_tx(&w_full[kb], MXV_W_KB + (two ? 2 : 1) * MX_SF_BYTES);
+            tma_load_2d(wb, &tm_b0, &w_full[kb], kb * MX_BK, n0);
+            tma_load_2d(wb + MXV_W_KB / 2, &tm_b1, &w_full[kb], kb * MX_BK, DUAL ? n0 : n0 + 128);
+            const size_t t0 = ((size_t)(n0 / 128) * p.k_blocks + kb) * MX_SF_BYTES;
+            bulk_load(sf, p.sfb0 + t0, MX_SF_BYTES, &w_full[kb]);
+            if (two) bulk_load(sf + MX_SF_BYTES, DUAL ? p.sfb1 + t0 : p.sfb0 + t0 + (size_t)p.k_blocks * MX_SF_BYTES, MX_SF_BYTES, &w_full[kb]);
+          }
+          if ((i & 1) != mine) continue;
+          const int s = i & (MXV_STAGES - 1);
+          if (!mbar_wait(&empty[s], ((uint32_t)(i / MXV_STAGES) & 1u) ^ 1u, abort_flag, ST_TIMEOUT_PRODUCER, 0xD00 | s, budget)) { ok = false; break; }
+          mbar_arrive_expect_tx(&full[s], MX_A_BYTES + MX_SF_BYTES);
+          tma_load_2d(smem + MXV_A + s * MX_A_BYTES, &tm_a, &full[s], kb * MX_BK, m_blk * MX_BM);
+          bulk_load(smem + MXV_SFA + s * MX_SF_BYTES, p.sfa + ((size_t)m_blk * p.k_blocks + kb) * MX_SF_BYTES, MX_SF_BYTES, &full[s]);
+        }
+      }
+      if (!ok) { const long long t0 = clock64(); while (clock64() - t0 < 2000000) { } }
+    }
+  } else if (warp == 1) {
+    // the whole warp walks the loop, one lane of it issues
+    bool ok = true;
+    int i = 0, it = 0;
+    for (int m_blk = ws_g; ok && m_blk < p.m_blocks; m_blk += p.n_groups, ++it) {
+      if (!__all_sync(0xffffffffu, mbar_wait(acc_empty, (uint32_t)(it & 1) ^ 1u, abort_flag, ST_TIMEOUT_MMA, 0xD10, budget))) { ok = false; break; }
+      tc_fence_after();
+      for (int kb = 0; kb < p.k_blocks; ++kb, ++i) {
+        const int s = i & (MXV_STAGES - 1);
+        const uint32_t sfb_t = tmem_base + MXV_SFB_COL + kb * 8;
+        if (it == 0) {                                     // the slice arrives during the first tile; its scale tiles go to TMEM once
+          if (!__all_sync(0xffffffffu, mbar_wait(&w_full[kb], 0, abort_flag, ST_TIMEOUT_MMA, 0xD20 | kb, budget))) { ok = false; break; }
+          const uint32_t sf = smem_u32(smem + MXV_SFB + kb * 2 * MX_SF_BYTES);
+          tmem_cp_32x128b_warpx4_elect(sfb_t, sf_smem_desc(sf));
+          tmem_cp_32x128b_warpx4_elect(sfb_t + 4, sf_smem_desc(sf + MX_SF_BYTES));
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (uint32_t)(i / MXV_STAGES) & 1u, abort_flag, ST_TIMEOUT_MMA, 0xD30 | s, budget))) { ok = false; break; }
+        const uint32_t sfa_t = tmem_base + MXV_SFA_COL + s * 4;              // a slot per stage
+        tmem_cp_32x128b_warpx4_elect(sfa_t, sf_smem_desc(smem_u32(smem + MXV_SFA + s * MX_SF_BYTES)));
+        const uint64_t a_desc = umma_smem_desc_sw128(smem_u32(smem + MXV_A + s * MX_A_BYTES));
+        const uint64_t b_desc = umma_smem_desc_sw128(smem_u32(smem + kb * MXV_W_KB));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_mxf8_elect(tmem_base, a_desc + 2 * k, b_desc + 2 * k, umma_idesc_mx(0, 0, MX_BM, MXV_BN, k, k), sfa_t, sfb_t, (kb | k) != 0);
+        umma_commit_elect(&empty[s]);
+      }
+      if (ok) umma_commit_elect(acc_full);
+    }
+  } else if (warp >= MX_FRONT_WARPS) {
+    const int e = warp - MX_FRONT_WARPS, q = warp & 3, half = e >> 2;
+    uint8_t* out_buf = smem + MXV_OUT + e * MXV_OUT_BUF;
+    uint8_t* const stg_row = out_buf + lane * 128;         // this thread's 128-byte row of the box, 16-byte pieces in the 128-byte swizzle
+    int it = 0;
+    for (int m_blk = ws_g; m_blk < p.m_blocks; m_blk += p.n_groups, ++it) {
+      if (!__all_sync(0xffffffffu, mbar_wait(acc_full, (uint32_t)it & 1u, abort_flag, ST_TIMEOUT_EPILOGUE, 0xD40, budget))) break;
+      tc_fence_after();
+      const int row_base = m_blk * MX_BM + q * 32;
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
+      uint32_t v[4][32];                                   // dual: 64 gate columns, 64 up columns; plain: 128 columns
+#pragma unroll
+      for (int b = 0; b < 4; ++b) tmem_ld_32x32b_x32(t_row + (DUAL ? half * 64 + (b >> 1) * 128 + (b & 1) * 32 : half * 128 + 32 * b), v[b]);
+      tmem_ld_wait(v[0], v[1]);
+      tmem_ld_wait(v[2], v[3]);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty);
+      if (row_base >= p.M) continue;
+#pragma unroll
+      for (int b = 0; b < (DUAL ? 1 : 2); ++b) {           // one 64-column box
+        const int n = n0 + (DUAL ? half * 64 : half * 128 + 64 * b);
+        if (n >= p.N) break;
+        if (lane == 0) tma_store_wait_read<0>();           // the previous box has left the buffer
+        __syncwarp();
+#pragma unroll
+        for (int pc = 0; pc < 8; ++pc) {                   // 8 columns
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int c = (pc & 3) * 8 + 2 * j;
+            if constexpr (DUAL) {
+              // silu(gate) * up with silu(g) = h + h * tanh(h), h = g / 2
+              const float2 hv = __fmul2_rn(make_float2(__uint_as_float(v[pc >> 2][c]), __uint_as_float(v[pc >> 2][c + 1])), make_float2(0.5f, 0.5f));
+              const float2 uv = make_float2(__uint_as_float(v[2 + (pc >> 2)][c]), __uint_as_float(v[2 + (pc >> 2)][c + 1]));
+              w[j] = pack_half2_from(__fmul2_rn(silu_from_half2(hv), uv));
+            } else {
+              w[j] = pack_half2(__uint_as_float(v[2 * b + (pc >> 2)][c]), __uint_as_float(v[2 * b + (pc >> 2)][c + 1]));
+            }
+          }
+          *reinterpret_cast<uint4*>(stg_row + ((pc ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) { tma_store_2d(&tm_c, out_buf, n, row_base); tma_store_commit(); }
+      }
+    }
+    if (lane == 0) tma_store_wait_all<0>();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, MX_TMEM_COLS); }
+}
+
 // ---- row-major [rows, K/32] scales -> the 128 x 4 tile order --------------------------------------------------
 // A thread moves the four scales of one row and one 128-wide K tile: one word of the tile, four neighbouring source bytes
 // (K % 128 == 0, so a row holds whole groups of four).  Consecutive threads write consecutive words; the 32 rows of a
@@ -587,6 +768,9 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
     if (e1 != cudaSuccess || e2 != cudaSuccess) return cuda_status(e1 != cudaSuccess ? e1 : e2, "cudaFuncSetAttribute(mx gemm)");
     cudaError_t e5 = cudaFuncSetAttribute(mx_gemm256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MX2_BYTES);
     if (e5 != cudaSuccess) return cuda_status(e5, "cudaFuncSetAttribute(mx gemm)");
+    cudaError_t e6 = cudaFuncSetAttribute(mx_gemm256w_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MXV_BYTES);
+    if (e6 == cudaSuccess) e6 = cudaFuncSetAttribute(mx_gemm256w_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MXV_BYTES);
+    if (e6 != cudaSuccess) return cuda_status(e6, "cudaFuncSetAttribute(mx gemm)");
     if (e3 != cudaSuccess || e4 != cudaSuccess) return cuda_status(e3 != cudaSuccess ? e3 : e4, "cudaFuncSetAttribute(mx gemm)");
     attr_done[dev].store(1, std::memory_order_release);
   }
@@ -611,6 +795,26 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
   p.sfa = sfa; p.sfb0 = sfb0; p.sfb1 = sfb1;
   const long long tiles = (long long)p.m_blocks * p.n_blocks;
   cudaError_t e;
+  // 256-column weight-stationary tiles where their rounds are cheaper: a tile takes about 1.5 times what a 128-column one does
+  // (dual, K = 512, N = 2048: M = 4096 12.5 us with 128 columns, 11.9 with 256; M = 1024 6.8 and 5.9; M = 128, one round of either,
+  // 5.3 and 5.5).
+  if (K / MX_BK <= MXW_MAX_KB) {
+    const int out256 = dual ? 128 : 256, nb = (N + out256 - 1) / out256, sms = sm_count();
+    const int g256 = sms / nb, g128 = wst ? sms / p.n_blocks : 0;
+    if (g256 > 0 && (g128 == 0 || (p.m_blocks + g256 - 1) / g256 * 15 < (p.m_blocks + g128 - 1) / g128 * 10)) {
+      CUtensorMap tw0, tw1, to;
+      if (!map2d(&tw0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
+          !map2d(&tw1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dual ? B1 : B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
+          !map2d(&to, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B))
+        return GSB200_ERR_BAD_ARG;
+      p.n_blocks = nb;
+      p.n_groups = g256 < p.m_blocks ? g256 : p.m_blocks;
+      const int grid = p.n_groups * nb;
+      e = dual ? launch_dependent(mx_gemm256w_kernel<true>, grid, MX_THREADS, MXV_BYTES, st, ta, tw0, tw1, to, p)
+               : launch_dependent(mx_gemm256w_kernel<false>, grid, MX_THREADS, MXV_BYTES, st, ta, tw0, tw1, to, p);
+      return cuda_status(e, "mx gemm launch");
+    }
+  }
   if (wst) {                                                        // weight-stationary form
     int groups = sm_count() / p.n_blocks;
     if (groups > p.m_blocks) groups = p.m_blocks;

@@ -168,3 +168,23 @@ def test_dual_silu_mxfp8_epilogue_forms_agree(M, N, K):
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
     assert int(res[1][0][:, N:].count_nonzero()) == 0 and int(res[1][1][:, N // 32:].count_nonzero()) == 0
     assert g.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("dual", [True, False])
+@pytest.mark.parametrize("M,N,K", [(9001, 2080, 512), (20000, 544, 384), (40000, 160, 128), (19000, 288, 256)])
+def test_block_scaled_weight_stationary_256_column_tiles(dual, M, N, K):
+    """Many row blocks run on 256-column weight-stationary tiles; a slice of two row blocks (one round) on 128-column ones.  Rows
+    are independent, so the slices must give the same bytes: ragged last tiles in M and N (half of a column tile, one without
+    scale tiles), one to four K blocks through the ring of four."""
+    g = need_lib()
+    gen = torch.Generator(device="cuda").manual_seed(M + N + K)
+    def mx(n):
+        q, s = g.mxfp8_quantize(torch.randn(n, K, generator=gen, device="cuda").half())
+        return q, s, g.mx_scales_to_tiled(s, K)
+    (a, sa, ta), (w, _, tw), (u, _, tu) = mx(M), mx(N), mx(N)
+    run = (lambda x, t: g.dual_gemm_mxfp8_silu(x, t, w, u, tw, tu)) if dual else (lambda x, t: g.gemm_mxfp8(x, t, w, tw))
+    got = run(a, ta)
+    for lo in (0, M // 2 // 128 * 128, (M - 1) // 128 * 128 - 128):
+        hi = min(M, lo + 256)
+        assert_bitexact(got[lo:hi], run(a[lo:hi].contiguous(), g.mx_scales_to_tiled(sa[lo:hi].contiguous(), K)), f"rows {lo}:{hi}")
+    assert g.device_status()[0] == 0
