@@ -176,6 +176,12 @@ int32_t gsb200_fac_gemm_fp8_f16(const uint8_t* x, int64_t ldx, const float* scal
   if (!x || !scale_x || !dn_rc || !scale_dn || !up_nr || !bias || !ih) return GSB200_ERR_BAD_ARG;
   if (R <= 0 || R % 8 != 0 || N < R || ldih < N) return GSB200_ERR_BAD_ARG;
   if (R > 256) return GSB200_ERR_UNSUPPORTED;          // the second GEMM keeps a row block's x_down (2R bytes per row) resident
+  // One launch where x_down fits the chip and every argument is as both products below would have it; what is not, they refuse.
+  const uintptr_t al = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dn_rc) | reinterpret_cast<uintptr_t>(up_nr) |
+                       reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(ih);
+  if ((R == 64 || R == 128) && (al & 15) == 0 && M > 0 && M <= 0x7fffff00ll && C > 0 && C % 16 == 0 && ldx >= C && ldx % 16 == 0 && lddn >= C &&
+      lddn % 16 == 0 && ldup >= R && ldup % 8 == 0 && N % 8 == 0 && ldih % 8 == 0 && ((M + 127) / 128) * ((N + 255) / 256) <= 0x7fffffffll)
+    return launch_lowrank(x, ldx, scale_x, dn_rc, lddn, scale_dn, up_nr, ldup, bias, ih, ldih, M, C, R, N, S(stream));
   // 1. x_down[M,R] = f16((x . dn^T) * sx[m] * s_dn), written into the first R columns of each output row
   int32_t rc = launch_gemm(base_args(KIND_F8, EPI_DEQUANT, x, ldx, dn_rc, nullptr, lddn, ih, ldih, scale_x, scale_dn,
                                      nullptr, M, R, C, GSB200_FLAG_SCALAR_SCALE_B),

@@ -51,6 +51,8 @@ struct GemmArgs {
   int sm_cap;                    // > 0: this launch uses at most so many CTAs (beside the process-wide cap)
 };
 int32_t launch_gemm(const GemmArgs& a, cudaStream_t st);
+int32_t launch_lowrank(const uint8_t* x, long long ldx, const float* sx, const uint8_t* dn, long long lddn, const float* s_dn, const void* up,
+                       long long ldup, const float* bias, void* ih, long long ldih, long long M, int C, int R, int N, cudaStream_t st);
 struct LstmLayerArgs {
   const __half* ih; long long ld_ih;        // [T*B, 4H] fp16 hoisted input projection, row = t*B + b
   const uint8_t* w_hh; long long ld_w;      // [4H, H] E4M3, K-major

@@ -2,6 +2,7 @@
 // word and the inline PTX helpers are shared without relocatable device code.
 #include "quant.cu"
 #include "gemm.cu"
+#include "lowrank.cu"
 #include "lstm.cu"
 #include "factored.cu"
 #include "mx_gemm.cu"

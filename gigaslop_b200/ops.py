@@ -375,7 +375,7 @@ def fp8_down_proj(x_fp8, scale_x, dn_fp8_rc, scale_dn, out=None):
 def fp8_factored_gemm(x_fp8, scale_x, dn_fp8_rc, scale_dn, up_f16_nr, bias, out=None):
     """Hoisted low-rank input projection ``ih = f16(f16((x . dn^T) * sx * s_dn) . up^T + bias)`` in one call
     (compile_fp8_factored_gemm, fly/rdna_fp8_factored_gemm.py:86-435).  ``dn`` ``[R, C]`` E4M3 and ``up``
-    ``[N, R]`` fp16, both K-major; the intermediate lives inside ``out`` between the two launches."""
+    ``[N, R]`` fp16, both K-major; the intermediate needs no memory of the caller."""
     n = _lib.native
     if n is not None:
         r = n.fac_gemm(x_fp8, scale_x, dn_fp8_rc, scale_dn, up_f16_nr, bias, out)
