@@ -306,16 +306,19 @@ lstm_recurrent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 //  * the batch is the small dimension, so B = 512 spreads over 129 SMs (G = 12) instead of 48: the gate math, five
 //    special-function instructions per cell, is 1000 clocks for 2048 cells (G = 16), 600 for 1024.
 //  * W_hh in tensor memory: an MMA from a shared-memory A operand of 128 rows takes 40 clocks, from TMEM 16.
-// B = 512, H = 384: 1.34 us per step (2.57 with the 128-row tiles), H = 512: 1.91 (4.8), H = 256: 0.93 (2.29), H = 128: 0.56 (2.27).
+// B = 512, H = 384: 1.21 us per step (2.57 with the 128-row tiles), H = 512: 1.84 (4.8), H = 256: 0.83 (2.29), H = 128: 0.56 (2.27).
+// Two things made 1.34 / 1.91 / 0.93 of that: an MMA warp walks its loop converged, with one elected lane issuing (a single thread
+// moves the operands of every MMA to uniform registers), and the gate warps report to it through a named barrier instead of an
+// mbarrier (1.22 / 1.84 / 0.84 without).
 // The K blocks are summed in ascending order on every CTA.  Starting with the CTA's own block, which is there first, takes
 // 1.25 us at H = 384 and 1.81 at H = 512, but sums in an order that depends on the CTA: the last bit of a sum changes, an E4M3
 // rounding of h flips with it, and after five layers of 2000 steps the outputs differ by 5e-3.  There is a
 // barrier per sending CTA, so that the first blocks' MMAs do not wait for the last piece.
-// Clocks of a step before that order (G = 16, H = 384, of ~2650): MMAs 900, wait for the others' h 300 of the 640 it is under
-// way, commit to registers 300, gate math and sending 1000, hand-over to the MMA warps 130.
+// Clocks of a step before that order and the converged warps (G = 16, H = 384, of ~2650): MMAs 900, wait for the others' h 300 of
+// the 640 it is under way, commit to registers 300, gate math and sending 1000, hand-over to the MMA warps 130.
 //   warps 0 .. CW-1   gate math.  Warp w: TMEM lane quarter w % 4 (32 hidden units, one per lane), G / (CW / 4) batch rows
-//   last four warps   one MMA-issuing thread per gate (an MMA costs the thread that issues it 60 to 70 clocks); the last
-//                     one also issues the TMA loads of the ih tiles
+//   last four warps   MMA issue, one gate each (the MMAs of a gate add to one accumulator, one after the other); the last one also
+//                     issues the TMA loads of the ih tiles
 // h is kept as K-major rows of 128 bytes with the 128-byte swizzle, one K block per CTA of the row group: a CTA's piece is
 // one K block, written by its own gate warps where its own MMAs read it and sent from there to the others.
 // h_t goes to buffer t & 1; the MMAs of step t read buffer (t + 1) & 1.  Buffer t & 1 may be written in step t: the MMAs of
@@ -355,8 +358,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   uint8_t* w_s = smem + L::W;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
   uint64_t* ih_full = bars;                        // [LT_STAGES]
-  uint64_t* own_ready = ih_full + LT_STAGES;      // [2] this CTA's piece of h is in the buffer, its accumulators have been read
-  uint64_t* h_ready = own_ready + 2;               // [2][LT_MAX_SLICES] the piece of each other CTA has landed (bytes counted)
+  uint64_t* h_ready = ih_full + LT_STAGES;         // [2][LT_MAX_SLICES] the piece of each other CTA has landed (bytes counted)
   uint64_t* mma_done = h_ready + 2 * LT_MAX_SLICES;                // the four gates' accumulators are complete
   uint64_t* w_full = mma_done + 1;                 // the fourth K block of W_hh has landed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(w_full + 1);
@@ -369,10 +371,11 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const int H = p.H, B = p.B;
   const int kb_tmem = p.k_blocks < LT_TMEM_KB ? p.k_blocks : LT_TMEM_KB;
   constexpr uint32_t PIECE_BYTES = G * LT_HS;      // of h, from one CTA
+  // gate warps -> MMA warps, once per step but the last: this CTA's piece of h is in the buffer, its accumulators have been read
+  constexpr int OWN_READY = 1, OWN_THREADS = 32 * (CW + 4);
 
   if (tid == 0) {
     for (int i = 0; i < LT_STAGES; ++i) mbar_init(&ih_full[i], 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&own_ready[i], CW);
     for (int i = 0; i < 2 * LT_MAX_SLICES; ++i) mbar_init(&h_ready[i], 1);
     mbar_init(mma_done, 4); mbar_init(w_full, 1);
     // arm the first use of each buffer: h_0 arrives in buffer 0 (if there is a step 1), h_1 in buffer 1
@@ -478,7 +481,10 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     for (int s = 0; s < p.T; ++s) {
       // ih + bias of this step, before the accumulators are there
       bool ok = mbar_wait(&ih_full[st], st_ph, abort_flag, ST_TIMEOUT_LSTM, 0x20, budget);
-      if (!__all_sync(0xffffffffu, ok)) break;
+      if (!__all_sync(0xffffffffu, ok)) {            // (the MMA warps wait for this warp's report, whatever became of it)
+        if (s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
+        break;
+      }
       float2 x[4][RPT / 2];
       const uint8_t* ihb = ih_t + st * L::IH_BYTES;
 #pragma unroll
@@ -493,7 +499,10 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if (++st == LT_STAGES) { st = 0; st_ph ^= 1; }
 
       ok = mbar_wait(mma_done, s & 1, abort_flag, ST_TIMEOUT_LSTM, 0x30, budget);
-      if (!__all_sync(0xffffffffu, ok)) break;
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
+        break;
+      }
       tc_fence_after();
       uint32_t acc[4][RPT];
 #pragma unroll
@@ -529,7 +538,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         }
         if (hf == 1) { fence_proxy_async_smem(); tc_fence_before(); }      // the stores above before the MMAs read them
         __syncwarp();
-        if (hf == 1 && lane == 0) mbar_arrive(&own_ready[s & 1]);
+        if (hf == 1 && s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
         if (sends && s + 1 < p.T) {
           const uint32_t off = (s & 1) * L::HBUF + snd_off[hf];
           st_async_v4(snd_dst + off, *reinterpret_cast<const uint4*>(h_s + off), snd_bar + 8 * LT_MAX_SLICES * (s & 1));
@@ -557,70 +566,78 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     }
   } else {
     // ------------------------------ MMA issue, one gate per warp ------------------------------
-    if (lane == 0) {
-      const int g = warp - CW;
-      constexpr uint32_t idesc = umma_idesc(1, 0, 0, LT_HS, R);
-      const uint32_t d = tmem_base + LT_ACC_COL + g * R;
-      const uint32_t a0 = tmem_base + g * LT_TMEM_KB * 32;
-      const uint64_t b_base[2] = {umma_smem_desc_sw128(smem_u32(h_s)), umma_smem_desc_sw128(smem_u32(h_s + L::HBUF))};
-      const uint64_t a_smem = umma_smem_desc_sw128(smem_u32(w_s + g * LSTM_KB_BYTES));
-      const int ksteps = H >> 5;                   // 32 bytes of K per MMA
-      bool ok = rank_ok;
-      int st = 0;
-      if (ok && p.slices > LT_TMEM_KB) ok = mbar_wait(w_full, 0, abort_flag, ST_TIMEOUT_LSTM, 0x10, budget);
-      // The loop exists once per (row group size, rank): with every descriptor offset a constant of straight-line code an
-      // MMA costs this thread 69 clocks, with offsets computed at run time 120 to 170.
-      auto run = [&](auto slices_tag, auto rank_tag) {
-        constexpr int SLICES = decltype(slices_tag)::value, RANK = decltype(rank_tag)::value;
-        for (int s = 0; s < p.T; ++s) {
-          const int hb = (s + 1) & 1;              // h_{s-1}
-          const uint32_t ph = (uint32_t)((s - 1) >> 1) & 1u;
-          // (the accumulators may be overwritten and this CTA's piece read once every gate warp has reported)
-          if (s > 0 && !mbar_wait(&own_ready[hb], ph, abort_flag, ST_TIMEOUT_LSTM, 0x40, budget)) return false;
-          tc_fence_after();
-          const uint64_t b = hb ? b_base[1] : b_base[0];
-          // K blocks in ascending order on every CTA (the order of the sums is part of the result), each as soon as its piece
-          // of h is there
+    // The whole warp walks the loop, one lane of it issues: the descriptors then stay in uniform registers.
+    const int g = __shfl_sync(0xffffffffu, warp - CW, 0);
+    constexpr uint32_t idesc = umma_idesc(1, 0, 0, LT_HS, R);
+    const uint32_t d = tmem_base + LT_ACC_COL + g * R;
+    const uint32_t a0 = tmem_base + g * LT_TMEM_KB * 32;
+    const uint64_t b_base[2] = {umma_smem_desc_sw128(smem_u32(h_s)), umma_smem_desc_sw128(smem_u32(h_s + L::HBUF))};
+    const uint64_t a_smem = umma_smem_desc_sw128(smem_u32(w_s + g * LSTM_KB_BYTES));
+    const int ksteps = H >> 5;                     // 32 bytes of K per MMA
+    bool ok = rank_ok;
+    int st = 0;
+    if (ok && p.slices > LT_TMEM_KB) ok = __all_sync(0xffffffffu, mbar_wait(w_full, 0, abort_flag, ST_TIMEOUT_LSTM, 0x10, budget));
+    // The loop exists once per (row group size, rank): every descriptor offset is a constant of straight-line code.
+    auto run = [&](auto slices_tag, auto rank_tag) {
+      constexpr int SLICES = decltype(slices_tag)::value, RANK = decltype(rank_tag)::value;
+      for (int s = 0; s < p.T; ++s) {
+        const int hb = (s + 1) & 1;                // h_{s-1}
+        const uint32_t ph = (uint32_t)((s - 1) >> 1) & 1u;
+        // (the accumulators may be overwritten and this CTA's piece read once every gate warp has reported)
+        __syncwarp();
+        if (s > 0) named_sync<OWN_READY, OWN_THREADS>();
+        tc_fence_after();
+        const uint64_t b = hb ? b_base[1] : b_base[0];
+        // K blocks in ascending order on every CTA (the order of the sums is part of the result), each as soon as its piece
+        // of h is there
 #pragma unroll
-          for (int kb = 0; kb < SLICES; ++kb) {
-            if (kb != RANK && s > 0) {             // another CTA's piece
-              uint64_t* bar = &h_ready[hb * LT_MAX_SLICES + kb];
-              if (!mbar_wait_cluster(bar, ph, abort_flag, ST_TIMEOUT_LSTM, 0x41, budget)) return false;
-              if (g == 0 && s + 2 < p.T) mbar_arrive_expect_tx(bar, PIECE_BYTES);   // its next use: h_{s+1}, read by step s + 2
-              fence_proxy_async_smem();            // the peer's stores before the MMAs read them
-            }
+        for (int kb = 0; kb < SLICES; ++kb) {
+          if (kb != RANK && s > 0) {               // another CTA's piece
+            uint64_t* bar = &h_ready[hb * LT_MAX_SLICES + kb];
+            if (!__all_sync(0xffffffffu, mbar_wait_cluster(bar, ph, abort_flag, ST_TIMEOUT_LSTM, 0x41, budget))) return false;
+            if (g == 0 && lane == 0 && s + 2 < p.T) mbar_arrive_expect_tx(bar, PIECE_BYTES);   // its next use: h_{s+1}, read by step s + 2
+            fence_proxy_async_smem();              // the peer's stores before the MMAs read them
+          }
+          const uint64_t bd = b + (uint64_t)(kb * (L::KB_BYTES >> 4));
+          if (kb < LT_TMEM_KB && (kb < SLICES - 1 || 4 * kb + 3 < ksteps)) {
+            umma_f8_ta_x4_elect(d, a0 + kb * 32, bd, idesc, kb != 0);
+          } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               if (kb == SLICES - 1 && 4 * kb + k >= ksteps) break;
-              const uint64_t bd = b + (uint64_t)(kb * (L::KB_BYTES >> 4) + 2 * k);
-              if (kb < LT_TMEM_KB) umma_f8_ta(d, a0 + kb * 32 + k * 8, bd, idesc, (kb | k) != 0);
-              else umma_f8(d, a_smem + 2 * k, bd, idesc, (kb | k) != 0);
+              if (kb < LT_TMEM_KB) umma_f8_ta_elect(d, a0 + kb * 32 + k * 8, bd + 2 * k, idesc, (kb | k) != 0);
+              else umma_f8_elect(d, a_smem + 2 * k, bd + 2 * k, idesc, (kb | k) != 0);
             }
           }
-          umma_commit(mma_done);
-          // the gate warps have read the ih tile of step s - 1 (their reports above came after that): its stage is free
-          if (g == 3 && s > 0) {
-            if (s - 1 + LT_STAGES < p.T) issue_ih(s - 1 + LT_STAGES, st);
-            if (++st == LT_STAGES) st = 0;
-          }
         }
-        return true;
-      };
-      auto run_rank = [&](auto slices_tag) {
-        constexpr int SLICES = decltype(slices_tag)::value;
-        if constexpr (SLICES > 3) if (slc == 3) return run(slices_tag, std::integral_constant<int, 3>{});
-        if constexpr (SLICES > 2) if (slc == 2) return run(slices_tag, std::integral_constant<int, 2>{});
-        if constexpr (SLICES > 1) if (slc == 1) return run(slices_tag, std::integral_constant<int, 1>{});
-        return run(slices_tag, std::integral_constant<int, 0>{});
-      };
-      if (ok) {
-        if (p.slices == 1) ok = run_rank(std::integral_constant<int, 1>{});
-        else if (p.slices == 2) ok = run_rank(std::integral_constant<int, 2>{});
-        else if (p.slices == 3) ok = run_rank(std::integral_constant<int, 3>{});
-        else ok = run_rank(std::integral_constant<int, 4>{});
+        umma_commit_elect(mma_done);
+        if (__any_sync(0xffffffffu, abort_flag.get())) return false;     // (a gate warp that gave up has reported all the same)
+        // the gate warps have read the ih tile of step s - 1 (their reports above came after that): its stage is free
+        if (g == 3 && s > 0) {
+          if (lane == 0 && s - 1 + LT_STAGES < p.T) issue_ih(s - 1 + LT_STAGES, st);
+          if (++st == LT_STAGES) st = 0;
+        }
       }
-      if (!ok) {                                   // loads in flight land before the CTA exits
-        abort_flag.set(1);
+      return true;
+    };
+    auto run_rank = [&](auto slices_tag) {
+      constexpr int SLICES = decltype(slices_tag)::value;
+      if constexpr (SLICES > 3) if (slc == 3) return run(slices_tag, std::integral_constant<int, 3>{});
+      if constexpr (SLICES > 2) if (slc == 2) return run(slices_tag, std::integral_constant<int, 2>{});
+      if constexpr (SLICES > 1) if (slc == 1) return run(slices_tag, std::integral_constant<int, 1>{});
+      return run(slices_tag, std::integral_constant<int, 0>{});
+    };
+    if (ok) {
+      if (p.slices == 1) ok = run_rank(std::integral_constant<int, 1>{});
+      else if (p.slices == 2) ok = run_rank(std::integral_constant<int, 2>{});
+      else if (p.slices == 3) ok = run_rank(std::integral_constant<int, 3>{});
+      else ok = run_rank(std::integral_constant<int, 4>{});
+    }
+    if (!ok) {                                     // (an MMA warp that still runs finds the abort flag after its next barrier)
+      if (lane == 0) abort_flag.set(1);
+      __syncwarp();
+      named_arrive<OWN_READY, OWN_THREADS>();
+      if (lane == 0) {                             // loads in flight land before the CTA exits
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000) { }
       }
@@ -642,7 +659,7 @@ size_t lstm_scratch_bytes(long long B, int H) {
 
 using LtKernel = void (*)(const CUtensorMap, const CUtensorMap, const uint8_t*, long long, const LstmParams);
 // The forms of the transposed kernel: batch rows per group, and what a step takes (ns, measured on B200) on row groups of one
-// to four CTAs, i.e. at H = 128, 256, 384 and 512.
+// to four CTAs, i.e. at H = 128, 256, 384 and 512.  (16 rows at H = 384 as with 96 CTAs, B = 512; 1400 with 129.)
 struct LtForm { int rows, threads, smem[LT_MAX_SLICES + 1], step_ns[LT_MAX_SLICES + 1]; LtKernel kernel; };
 template <int R, int G, int CW>
 static constexpr LtForm lt_make_form(int ns1, int ns2, int ns3, int ns4) {
@@ -653,9 +670,9 @@ static constexpr LtForm lt_make_form(int ns1, int ns2, int ns3, int ns4) {
   return f;
 }
 constexpr int LT_FORMS = 5;
-static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(570, 790, 980, 1360), lt_make_form<16, 8, 8>(720, 960, 1140, 1540),
-                                          lt_make_form<16, 12, 12>(900, 1140, 1340, 1740), lt_make_form<16, 16, 8>(1070, 1250, 1480, 1930),
-                                          lt_make_form<32, 32, 16>(1770, 2110, 2360, 2900)};
+static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(550, 680, 820, 1240), lt_make_form<16, 8, 8>(710, 830, 1010, 1420),
+                                          lt_make_form<16, 12, 12>(870, 1010, 1210, 1610), lt_make_form<16, 16, 8>(1070, 1190, 1350, 1830),
+                                          lt_make_form<32, 32, 16>(1740, 2050, 2230, 2810)};
 
 static cudaLaunchConfig_t lt_config(const LtForm& f, int slices, long long groups, cudaStream_t st, cudaLaunchAttribute* attr) {
   attr->id = cudaLaunchAttributeClusterDimension;
@@ -693,8 +710,8 @@ static int lt_capacity(int form, int slices, int dev) {
 // projection beside it (0 = it has the whole GPU); -1 = none.  `max_ctas` only steers this choice, in which groups past it wait
 // for a next wave: a launch brings all its row groups, and where no form holds them in `max_ctas` CTAs they take more SMs
 // (lstm_layer_ctas counts what a launch does occupy).  Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows
-// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.36 us per step; 12 rows in two
-// waves 2.68).  *ns = the step.
+// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.23 us per step; 12 rows in two
+// waves 2.42).  *ns = the step.
 static int lt_choose(long long B, int H, int dev, int max_ctas, long long* ns = nullptr) {
   const int slices = (H + LT_HS - 1) / LT_HS;
   int best = -1;
@@ -750,8 +767,8 @@ static int lstm_layer_ctas(long long B, int H, int max_ctas) {
 
 // How many launches to cut a layer's recurrence into so that the next layer's projection runs beside it (1 = not at all).
 // The cut recurrence is steered to `max_ctas` CTAs, which may cost it a form with longer steps, and every launch about 12 us;
-// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 16.9 ms one after the other, 16.3
-// in seven blocks; at B = 512, H = 512 (T = 1000, three layers) 7.3 ms against 8.6, so not cut.
+// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 15.8 ms one after the other, 14.9
+// in six blocks; at B = 512, H = 512 (T = 1000, three layers) 7.1 ms against 8.5, so not cut.
 static int lstm_time_blocks(long long T, long long B, int H, int max_ctas) {
   int dev = 0;
   cudaGetDevice(&dev);

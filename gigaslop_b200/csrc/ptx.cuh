@@ -45,6 +45,14 @@ struct AbortFlag {
   }
 };
 
+// ---- named barriers ------------------------------------------------------------
+// A hand-over between warps of a CTA: N threads in all, some of which only arrive.  Executed by converged warps.  The waiting is
+// not bounded: every warp that others wait for arrives on its way out, too, however it came to leave.
+template <int ID, int N>
+__device__ __forceinline__ void named_arrive() { asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
+template <int ID, int N>
+__device__ __forceinline__ void named_sync() { asm volatile("barrier.cta.sync.aligned %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
+
 // ---- programmatic dependent launch --------------------------------------------
 // The kernels that follow one another in a stream are launched with programmatic stream serialization (launch_dependent):
 // a kernel may start while the one before it drains.  None of them touches global memory before pdl_wait, which returns when
@@ -297,15 +305,6 @@ __device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t a_desc, uint64
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The A operand from tensor memory: lane = row of A, four 8-bit K elements per 32-bit column (8 columns per K = 32 step).
-__device__ __forceinline__ void umma_f8_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(
@@ -379,6 +378,31 @@ __device__ __forceinline__ void umma_mxf8_elect(uint32_t d_tmem, uint64_t a_desc
 __device__ __forceinline__ void tmem_cp_32x128b_warpx4_elect(uint32_t taddr, uint64_t s_desc) {
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n\t}"
                ::"r"(taddr), "l"(s_desc) : "memory");
+}
+// The A operand from tensor memory: lane = row of A, four 8-bit K elements per 32-bit column (8 columns per K = 32 step).
+__device__ __forceinline__ void umma_f8_ta_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// ... the four K steps of a 128-byte K block.
+__device__ __forceinline__ void umma_f8_ta_x4_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q, t;\n\tsetp.ne.b32 p, %10, 0;\n\tsetp.eq.b32 t, 0, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %5, %9, p;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%2], %6, %9, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%3], %7, %9, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%4], %8, %9, t;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(a_tmem + 8), "r"(a_tmem + 16), "r"(a_tmem + 24), "l"(b_desc), "l"(b_desc + 2), "l"(b_desc + 4),
+        "l"(b_desc + 6), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f8_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // shared -> TMEM copy of scale factors (32 lanes x 128 bit, replicated to the 4 lane quarters)
 __device__ __forceinline__ void tmem_cp_32x128b_warpx4(uint32_t taddr, uint64_t s_desc) {
