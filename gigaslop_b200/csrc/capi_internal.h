@@ -48,6 +48,7 @@ struct GemmArgs {
   int flags;
   // fused activation quantiser (KIND_I8 + EPI_ROTARY, K <= 512): fp16 activations instead of A / scale_a
   const __half* x_f16; long long ldx; float* scale_a_out;
+  float scale_a_const = 1.f;     // the scale of every row where scale_a is null (EPI_DEQUANT)
   int sm_cap;                    // > 0: this launch uses at most so many CTAs (beside the process-wide cap)
 };
 int32_t launch_gemm(const GemmArgs& a, cudaStream_t st);

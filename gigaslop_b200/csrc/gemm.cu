@@ -362,7 +362,7 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
   p.k_blocks = (a.K + BK - 1) / BK;
   p.C = a.C; p.ldc = a.ldc;
   p.out_scale = a.out_scale; p.ld_scale = a.ld_scale;
-  p.scale_a = a.scale_a; p.scale_b0 = a.scale_b0; p.scale_b1 = a.scale_b1;
+  p.scale_a = a.scale_a; p.scale_a_const = a.scale_a_const; p.scale_b0 = a.scale_b0; p.scale_b1 = a.scale_b1;
   p.scale_b_scalar = (a.flags & GSB200_FLAG_SCALAR_SCALE_B) ? 1 : 0;
   p.sin_tab = a.sin_tab; p.cos_tab = a.cos_tab;
   p.seqlen = a.seqlen > 0 ? a.seqlen : 1;

@@ -128,7 +128,8 @@ struct GemmParams {
   uint8_t* out_scale;          // EPI_SILU_MX: E8M0 scales [M, N/32]
   long long ld_scale;          //              row stride of out_scale in bytes
   long long ldc;               // output row stride in elements
-  const float* scale_a;        // [M]
+  const float* scale_a;        // [M], or null: scale_a_const for every row
+  float scale_a_const;
   const float* scale_b0;       // [N]   (dual: gate)
   const float* scale_b1;       // [N]   (dual: up)
   int scale_b_scalar;          // scale_b0 points to ONE value used for every column (scalar-quantised weights)
@@ -700,7 +701,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       if (first < ITEMS && m_blk != cur_m_blk) {
         cur_m_blk = m_blk;
         const long long r = (long long)row_base + lane;
-        sa = (r < p.M) ? (p.scale_a ? ldg_f_here(p.scale_a + r) : 1.f) : 0.f;
+        sa = (r < p.M) ? (p.scale_a ? ldg_f_here(p.scale_a + r) : p.scale_a_const) : 0.f;
         if constexpr (EPI == EPI_ROTARY) {
           trig_scaled = false;
           const int pos = r < p.M ? (int)((r + p.row_offset) % p.seqlen) : 0;
@@ -974,7 +975,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     if constexpr (EPI != EPI_I32) {
       if (tw.valid(p)) {
         const int r = rowblk(tw.m) * BM + q * 32 + lane;
-        if (r < p.M) sa_next = p.scale_a ? ldg_f_here(p.scale_a + r) : 1.f;
+        if (r < p.M) sa_next = p.scale_a ? ldg_f_here(p.scale_a + r) : p.scale_a_const;
       }
     }
     for (int it = 0; tw.valid(p); ++it) {
@@ -1028,7 +1029,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         }
         if (!FUSEQ && tw.valid(p) && nxt_m != m_blk) {
           const int r = nxt_m * BM + q * 32 + lane;
-          sa_next = (r < p.M) ? (p.scale_a ? ldg_f_here(p.scale_a + r) : 1.f) : 0.f;
+          sa_next = (r < p.M) ? (p.scale_a ? ldg_f_here(p.scale_a + r) : p.scale_a_const) : 0.f;
         }
       }
 

@@ -42,6 +42,7 @@ struct SgParams {
   int M, N, n_tiles, k_blocks, stages;
   void* C; long long ldc;
   uint8_t* out_scale; long long ld_scale;
+  float scale_a_const;
   const float* scale_a; const float* scale_b0; const float* scale_b1;
   int scale_b_scalar;
   const float* sin_tab; const float* cos_tab;
@@ -98,7 +99,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const bool pairs32 = EPI != EPI_ROTARY || p.rot_geo != 2;
   const int ca = pairs32 ? half * H : half * 32, cb = pairs32 ? NPART + half * H : half * 32 + 16;
   bool rotated = false;
-  float sa = 1.f;
+  float sa = p.scale_a_const;
   // Rotary: the tile's 64 rows of sin and of cos, 8 chunks of 16 bytes each (geometry 2: 4), are fetched by all threads in
   // whole lines during the main loop and handed to the threads that need them through the ring, once the MMAs have read it.
   // (A thread loading its own row's values, 32 scattered rows per instruction: 5.1 instead of 4.4 us at 256 rows, 7.0 instead
@@ -346,7 +347,7 @@ static int32_t launch_gemm_small(const GemmArgs& a, const GemmParams& g, int geo
   p.stages = npart == 32 ? (per_sm == 1 ? SG_MAX_STAGES : per_sm == 2 ? 6 : 4) : (per_sm == 1 ? 8 : per_sm == 2 ? 4 : 3);
   if (p.stages > p.k_blocks) p.stages = p.k_blocks;
   p.C = g.C; p.ldc = g.ldc; p.out_scale = g.out_scale; p.ld_scale = g.ld_scale;
-  p.scale_a = g.scale_a; p.scale_b0 = g.scale_b0; p.scale_b1 = g.scale_b1; p.scale_b_scalar = g.scale_b_scalar;
+  p.scale_a = g.scale_a; p.scale_a_const = g.scale_a_const; p.scale_b0 = g.scale_b0; p.scale_b1 = g.scale_b1; p.scale_b_scalar = g.scale_b_scalar;
   p.sin_tab = g.sin_tab; p.cos_tab = g.cos_tab; p.seqlen = g.seqlen; p.row_offset = g.row_offset; p.rot_cols = g.rot_cols; p.rot_geo = geo;
   const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
   CUtensorMap ta, tb0, tb1;

@@ -389,6 +389,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     prefetch_tmap(&tm_w); prefetch_tmap(&tm_ih);
   }
   if (warp == CW) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -421,7 +422,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         uint4 w = make_uint4(0, 0, 0, 0);
-        if (hid_ok && kb * 128 + i * 16 < H) w = __ldg(reinterpret_cast<const uint4*>(w_hh + (long long)(g * H + hid) * ld_w + kb * 128 + i * 16));
+        if (hid_ok && kb * 128 + i * 16 < H) w = __ldcg(reinterpret_cast<const uint4*>(w_hh + (long long)(g * H + hid) * ld_w + kb * 128 + i * 16));
         v[4 * i] = w.x; v[4 * i + 1] = w.y; v[4 * i + 2] = w.z; v[4 * i + 3] = w.w;
       }
       tmem_st_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (g * LT_TMEM_KB + kb) * 32, v);
@@ -429,7 +430,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     tmem_st_wait();
 #pragma unroll
     for (int i = 0; i < RPT; ++i)
-      c[i] = (p.c0 && hid_ok && i < rows_live) ? __half2float(p.c0[(long long)(row0 + r_lo + i) * H + hid]) : 0.f;
+      c[i] = (p.c0 && hid_ok && i < rows_live) ? __half2float(__ldcg(p.c0 + (long long)(row0 + r_lo + i) * H + hid)) : 0.f;
     // step 0 reads h_0 (or zeros) from buffer 1, staged by this CTA's own threads
     if constexpr (G < R)                           // the rows of the MMA that no batch row uses
       for (int id = tid; id < 2 * L::HBUF / 16; id += 32 * CW)
@@ -460,8 +461,8 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       const float half = g == 2 ? 1.0f : 0.5f;
-      sc[g] = hid_ok ? __ldg(p.s_hh + g * H + hid) * (1.0f / 448.0f) * half : 0.f;
-      bi[g] = hid_ok && p.bias ? __ldg(p.bias + g * H + hid) * half : 0.f;
+      sc[g] = hid_ok ? __ldcg(p.s_hh + g * H + hid) * (1.0f / 448.0f) * half : 0.f;
+      bi[g] = hid_ok && p.bias ? __ldcg(p.bias + g * H + hid) * half : 0.f;
     }
     const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + LT_ACC_COL + r_lo;
     const uint8_t* ih_t = ih_s + r_lo * (LT_HS * 2) + u * 2;
@@ -674,13 +675,15 @@ static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(550, 680, 820, 
                                           lt_make_form<16, 12, 12>(870, 1010, 1210, 1610), lt_make_form<16, 16, 8>(1070, 1190, 1350, 1830),
                                           lt_make_form<32, 32, 16>(1740, 2050, 2230, 2810)};
 
-static cudaLaunchConfig_t lt_config(const LtForm& f, int slices, long long groups, cudaStream_t st, cudaLaunchAttribute* attr) {
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = slices; attr->val.clusterDim.y = 1; attr->val.clusterDim.z = 1;
+static cudaLaunchConfig_t lt_config(const LtForm& f, int slices, long long groups, cudaStream_t st, cudaLaunchAttribute (&attr)[2]) {
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = slices; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(groups * slices)); cfg.blockDim = dim3(f.threads);
   cfg.dynamicSmemBytes = f.smem[slices]; cfg.stream = st;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
   return cfg;
 }
 
@@ -691,8 +694,8 @@ static int lt_capacity(int form, int slices, int dev) {
   int c = slot.load(std::memory_order_acquire);
   if (c == 0) {
     const LtForm& f = kLtForms[form];
-    cudaLaunchAttribute attr;
-    cudaLaunchConfig_t cfg = lt_config(f, slices, 1, nullptr, &attr);
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = lt_config(f, slices, 1, nullptr, attr);
     // (the attribute is per kernel: it is set to what the largest row group needs)
     cudaError_t e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem[LT_MAX_SLICES]);
     int n = 0;
@@ -736,8 +739,8 @@ static int32_t launch_lt(const LtForm& f, const LstmLayerArgs& a, LstmParams p, 
       !tmap_2d(&tih, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.ih, (uint64_t)a.T * a.B, (uint64_t)4 * a.H, (uint64_t)a.ld_ih, LT_HS,
                f.rows, CU_TENSOR_MAP_SWIZZLE_NONE))
     return GSB200_ERR_BAD_ARG;
-  cudaLaunchAttribute attr;
-  cudaLaunchConfig_t cfg = lt_config(f, p.slices, (a.B + f.rows - 1) / f.rows, st, &attr);
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = lt_config(f, p.slices, (a.B + f.rows - 1) / f.rows, st, attr);
   return cuda_status(cudaLaunchKernelEx(&cfg, f.kernel, tw, tih, a.w_hh, a.ld_w, p), "lstm launch");
 }
 
@@ -895,12 +898,7 @@ int32_t launch_lstm_layer_static(const LstmLayerArgs& a, cudaStream_t st) {
 // projection of layer l + 1 over the same timesteps runs on the auxiliary stream, on the SMs the recurrence
 // leaves idle -- ordered by events only, no kernel waits for another kernel.
 //
-// Workspace: [ih 0][ih 1 (overlap only)][h8 0][h8 1][row scales = 1/448][c 0][c 1][layer scratch]
-__global__ void fill_f32_kernel(float* dst, long long n, float v) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = v;
-}
-
+// Workspace: [ih 0][ih 1 (overlap only)][h8 0][h8 1][unused: T B floats][c 0][c 1][layer scratch]
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 size_t lstm_stack_workspace_bytes(long long T, long long B, int H, int overlap) {
@@ -934,25 +932,19 @@ int32_t launch_lstm_stack(const uint8_t* x, long long ldx, const float* sx, int 
   uint8_t* h8[2];
   h8[0] = w; w += align256(rows * H);
   h8[1] = w; w += align256(rows * H);
-  float* row_scale = reinterpret_cast<float*>(w); w += align256(rows * 4);
+  w += align256(rows * 4);
   __half* cst[2];
   cst[0] = reinterpret_cast<__half*>(w); w += align256((size_t)B * H * 2);
   cst[1] = reinterpret_cast<__half*>(w); w += align256((size_t)B * H * 2);
   void* scratch = w;
   const size_t scratch_bytes = align256(lstm_scratch_bytes(B, H));
 
-  if (n_layers > 1) {
-    const long long blocks = ((long long)rows + 255) / 256;
-    fill_f32_kernel<<<(unsigned)blocks, 256, 0, st>>>(row_scale, (long long)rows, 1.0f / 448.0f);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_status(e, "lstm stack: row scale fill");
-  }
   // hoisted projection of layer l over timesteps [t0, t1) on stream s, at most sm_cap CTAs (0 = all)
   auto project = [&](int l, long long t0, long long t1, cudaStream_t s, int sm_cap) -> int32_t {
     GemmArgs g{};
     g.kind = KIND_F8; g.epi = EPI_DEQUANT;
     if (l == 0) { g.A = x + (size_t)t0 * B * ldx; g.lda = ldx; g.scale_a = sx + (size_t)t0 * B; g.K = C; }
-    else { g.A = h8[(l - 1) & 1] + (size_t)t0 * B * H; g.lda = H; g.scale_a = row_scale; g.K = H; }
+    else { g.A = h8[(l - 1) & 1] + (size_t)t0 * B * H; g.lda = H; g.scale_a_const = 1.0f / 448.0f; g.K = H; }
     g.B0 = layers[l].w_ih; g.ldb = layers[l].ld_w_ih;
     g.C = ih[l & 1] + (size_t)t0 * B * 4 * H; g.ldc = 4 * H;
     g.scale_b0 = layers[l].s_ih;
