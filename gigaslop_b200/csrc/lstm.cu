@@ -306,10 +306,11 @@ lstm_recurrent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 //  * the batch is the small dimension, so B = 512 spreads over 129 SMs (G = 12) instead of 48: the gate math, five
 //    special-function instructions per cell, is 1000 clocks for 2048 cells (G = 16), 600 for 1024.
 //  * W_hh in tensor memory: an MMA from a shared-memory A operand of 128 rows takes 40 clocks, from TMEM 16.
-// B = 512, H = 384: 1.21 us per step (2.57 with the 128-row tiles), H = 512: 1.84 (4.8), H = 256: 0.83 (2.29), H = 128: 0.56 (2.27).
-// Two things made 1.34 / 1.91 / 0.93 of that: an MMA warp walks its loop converged, with one elected lane issuing (a single thread
-// moves the operands of every MMA to uniform registers), and the gate warps report to it through a named barrier instead of an
-// mbarrier (1.22 / 1.84 / 0.84 without).
+// B = 512, H = 384: 1.12 us per step (2.57 with the 128-row tiles), H = 512: 1.74 (4.8), H = 256: 0.80 (2.29), H = 128: 0.54 (2.27).
+// It was 1.34 / 1.93 / 0.93 / 0.57 before three changes to how its warps wait and issue.  An MMA warp walks its loop converged, with
+// one elected lane issuing (a single thread moves the operands of every MMA to uniform registers): 1.22 / 1.84 / 0.84 / 0.56.  The
+// gate warps report to it through a named barrier instead of an mbarrier: 1.21 / 1.84 / 0.83 / 0.56.  The waits on the chain, for the
+// accumulators and for the other CTAs' h, do not suggest to the hardware how long to stay suspended: the rest.
 // The K blocks are summed in ascending order on every CTA.  Starting with the CTA's own block, which is there first, takes
 // 1.25 us at H = 384 and 1.81 at H = 512, but sums in an order that depends on the CTA: the last bit of a sum changes, an E4M3
 // rounding of h flips with it, and after five layers of 2000 steps the outputs differ by 5e-3.  There is a
@@ -499,7 +500,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         }
       if (++st == LT_STAGES) { st = 0; st_ph ^= 1; }
 
-      ok = mbar_wait(mma_done, s & 1, abort_flag, ST_TIMEOUT_LSTM, 0x30, budget);
+      ok = mbar_wait<true>(mma_done, s & 1, abort_flag, ST_TIMEOUT_LSTM, 0x30, budget);
       if (!__all_sync(0xffffffffu, ok)) {
         if (s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
         break;
@@ -660,7 +661,7 @@ size_t lstm_scratch_bytes(long long B, int H) {
 
 using LtKernel = void (*)(const CUtensorMap, const CUtensorMap, const uint8_t*, long long, const LstmParams);
 // The forms of the transposed kernel: batch rows per group, and what a step takes (ns, measured on B200) on row groups of one
-// to four CTAs, i.e. at H = 128, 256, 384 and 512.  (16 rows at H = 384 as with 96 CTAs, B = 512; 1400 with 129.)
+// to four CTAs, i.e. at H = 128, 256, 384 and 512.  (16 rows at H = 384 as with 96 CTAs, B = 512; 1310 with 129.)
 struct LtForm { int rows, threads, smem[LT_MAX_SLICES + 1], step_ns[LT_MAX_SLICES + 1]; LtKernel kernel; };
 template <int R, int G, int CW>
 static constexpr LtForm lt_make_form(int ns1, int ns2, int ns3, int ns4) {
@@ -671,9 +672,9 @@ static constexpr LtForm lt_make_form(int ns1, int ns2, int ns3, int ns4) {
   return f;
 }
 constexpr int LT_FORMS = 5;
-static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(550, 680, 820, 1240), lt_make_form<16, 8, 8>(710, 830, 1010, 1420),
-                                          lt_make_form<16, 12, 12>(870, 1010, 1210, 1610), lt_make_form<16, 16, 8>(1070, 1190, 1350, 1830),
-                                          lt_make_form<32, 32, 16>(1740, 2050, 2230, 2810)};
+static const LtForm kLtForms[LT_FORMS] = {lt_make_form<16, 4, 4>(530, 645, 775, 1180), lt_make_form<16, 8, 8>(690, 800, 920, 1330),
+                                          lt_make_form<16, 12, 12>(830, 960, 1120, 1550), lt_make_form<16, 16, 8>(1045, 1150, 1240, 1740),
+                                          lt_make_form<32, 32, 16>(1620, 1910, 2060, 2720)};
 
 static cudaLaunchConfig_t lt_config(const LtForm& f, int slices, long long groups, cudaStream_t st, cudaLaunchAttribute (&attr)[2]) {
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -713,8 +714,8 @@ static int lt_capacity(int form, int slices, int dev) {
 // projection beside it (0 = it has the whole GPU); -1 = none.  `max_ctas` only steers this choice, in which groups past it wait
 // for a next wave: a launch brings all its row groups, and where no form holds them in `max_ctas` CTAs they take more SMs
 // (lstm_layer_ctas counts what a launch does occupy).  Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows
-// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.23 us per step; 12 rows in two
-// waves 2.42).  *ns = the step.
+// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.06 us per step; 12 rows in two
+// waves 2.24).  *ns = the step.
 static int lt_choose(long long B, int H, int dev, int max_ctas, long long* ns = nullptr) {
   const int slices = (H + LT_HS - 1) / LT_HS;
   int best = -1;
@@ -770,8 +771,8 @@ static int lstm_layer_ctas(long long B, int H, int max_ctas) {
 
 // How many launches to cut a layer's recurrence into so that the next layer's projection runs beside it (1 = not at all).
 // The cut recurrence is steered to `max_ctas` CTAs, which may cost it a form with longer steps, and every launch about 12 us;
-// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 15.8 ms one after the other, 14.9
-// in six blocks; at B = 512, H = 512 (T = 1000, three layers) 7.1 ms against 8.5, so not cut.
+// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 15.1 ms one after the other, 13.9
+// in five blocks; at B = 512, H = 512 (T = 1000, three layers) 6.8 ms against 8.1, so not cut.
 static int lstm_time_blocks(long long T, long long B, int H, int max_ctas) {
   int dev = 0;
   cudaGetDevice(&dev);

@@ -103,15 +103,32 @@ __device__ __forceinline__ unsigned int spin_budget() {
   return v ? v : kDefaultSpinBudget;
 }
 
+// The same without the hint how long to stay suspended: the thread comes back from a wait sooner.
+__device__ __forceinline__ bool mbar_try_wait_soon(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait.  Returns false if the budget ran out or another role already
 // gave up (abort flag in shared memory); the caller must then unwind.
+// SOON: for a wait on a chain of latencies, the LSTM step's (1205 -> 1125 ns at B = 512, H = 384 together with the cluster form
+// below); the GEMMs' roles wait for longer and lose issue slots to it (SwiGLU of 65536 rows 109.7 -> 113.7 us).
+template <bool SOON = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, AbortFlag abort_flag,
                                           unsigned int fail_code, unsigned int where, unsigned int budget) {
-  if (mbar_try_wait(bar, parity)) return true;
+  auto arrived = [&]() { return SOON ? mbar_try_wait_soon(bar, parity) : mbar_try_wait(bar, parity); };
+  if (arrived()) return true;
   long long t0 = clock64();
   int spins = 0;
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (arrived()) return true;
     if ((++spins & 63) == 0) {
       if (abort_flag.get()) return false;
       if (clock64() - t0 > (long long)budget) {
@@ -142,14 +159,14 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(kTryWaitSuspendNs)
+      : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
   return ok != 0;
 }
-// Bounded wait on a barrier that threads of other CTAs of the cluster arrive at (same contract as mbar_wait).
+// Bounded wait on a barrier that threads of other CTAs of the cluster arrive at (same contract as mbar_wait; without the hint).
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, AbortFlag abort_flag,
                                                   unsigned int fail_code, unsigned int where, unsigned int budget) {
   if (mbar_try_wait_cluster(bar, parity)) return true;
