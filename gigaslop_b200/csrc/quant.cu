@@ -87,12 +87,19 @@ __device__ __forceinline__ uint2 pack_e4m3(const float (&v)[8], float f) {
 // e4m3( clamp(x / s) ) for a row whose values are all finite, without a division per element: with r = 1 / s correctly
 // rounded and q within one ulp of x / s, q + (x - s q) r rounds to the correctly rounded quotient (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  x r itself
-// can be 1.5 ulp off, so the step is made twice.  The residual is inexact only where |x| < 2^-100, and x / s is then far
+// can be 1.5 ulp off, so in general the step is made twice.  For fp16 rows once is enough (HALF): the value that the first step
+// rounds is within 2^-46 of x / s, so its fp32 rounding, and with it the E4M3 byte, can only be wrong where x / s lies that close to
+// m (1 + 2^-24) or m (1 - 2^-25 or 2^-24), m halfway between two E4M3 values, i.e. up to five significant bits.  In integers, X an
+// 11-bit, S a 24-bit significand and m = 16 .. 31: |X 2^k - S (m 2^20 +- 1)| <= 8 needs S = c 2^20 + e, |e| <= 8, and e m = +-c, which
+// leaves m = c = 16, e = -1; but s = fl(amax / 448) of an fp16 amax is never the fp32 number below a power of two (amax / 7 would
+// have to be within 2^-24 of one without being it).  The residual is inexact only where |x| < 2^-100, and x / s is then far
 // below half of the smallest E4M3 value (s >= 2^-49) whatever its last bit; |x| <= 448 s, so the saturating conversion is
 // the clamp.  Everything is carried with the opposite sign, so that a zero keeps its own: the additions round +0 + -0 to
 // +0, and the sign bits are flipped in the packed bytes.
 // With a division per element (about ten instructions) the kernel was issue-bound: M = 131072, K = 1024 took 87.5 us,
-// 4.6 TB/s, and M = 9001, K = 2048 14.0 us; now 69.1 us, 5.8 TB/s, and 9.7 us.
+// 4.6 TB/s, and M = 9001, K = 2048 14.0 us; with the step made twice 64.8 us and 9.9, once 60.0 us (6.7 TB/s) and 8.8.  K = 512: M =
+// 20001 7.3 us twice, 6.5 once, M = 65536 19.0 and 16.5.
+template <bool HALF>
 __device__ __forceinline__ uint2 pack_e4m3_quot(const float (&v)[8], float s, float neg_r) {
   const float2 s2 = make_float2(s, s), n2 = make_float2(neg_r, neg_r);
   uint32_t w[4];
@@ -101,7 +108,7 @@ __device__ __forceinline__ uint2 pack_e4m3_quot(const float (&v)[8], float s, fl
     const float2 x = make_float2(v[2 * i], v[2 * i + 1]);
     float2 q = __fmul2_rn(x, n2);                        // -x / s
     q = __ffma2_rn(__ffma2_rn(q, s2, x), n2, q);
-    q = __ffma2_rn(__ffma2_rn(q, s2, x), n2, q);
+    if constexpr (!HALF) q = __ffma2_rn(__ffma2_rn(q, s2, x), n2, q);
     w[i] = __nv_cvt_float2_to_fp8x2(q, __NV_SATFINITE, __NV_E4M3);
   }
   return make_uint2((w[0] | (w[1] << 16)) ^ 0x80808080u, (w[2] | (w[3] << 16)) ^ 0x80808080u);
@@ -204,7 +211,7 @@ ptq_kernel(const Tin* __restrict__ x, long long ldx, uint8_t* __restrict__ q, lo
     if constexpr (FMT == 0) o = pack_i8(vv, f);
     else if constexpr (FMT == 1) o = pack_e4m3<0>(vv, f);
     else if (bad) o = pack_e4m3<1>(vv, f);       // warp-uniform: only rows with a NaN or an infinity divide
-    else o = pack_e4m3_quot(vv, s, neg_r);
+    else o = pack_e4m3_quot<sizeof(Tin) == 2>(vv, s, neg_r);
     *reinterpret_cast<uint2*>(qr + v * 8) = o;
   };
   if constexpr (HALF_CACHED) {

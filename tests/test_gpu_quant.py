@@ -191,3 +191,29 @@ def test_mx_quantiser_blocks_with_nan_and_infinity(dtype, K):
     q, s = g.mxfp8_quantize(x.cuda())
     assert_bitexact(s, byte.to(torch.uint8), "E8M0 scales")
     assert_bitexact(q.view(torch.uint8), q_ref.view(len(x), K), "bytes")
+
+
+def test_fp8_quotients_of_every_fp16_pair():
+    """The torch formulation divides by amax / 448; the kernel gets the quotient of an fp16 row from one refinement of a product.
+    Every fp16 significand as the row maximum, with every fp16 value up to it: 16 million pairs, scaled to three places in the fp16
+    range (a power of two changes nothing but the exponents)."""
+    g = need_lib()
+    bits = torch.arange(0x3C00, 0x4000, dtype=torch.int32, device="cuda")          # 1 <= amax < 2
+    val = torch.arange(0, 0x4000, dtype=torch.int32, device="cuda")
+    per = -(-len(val) // 511)
+    body = torch.zeros(per * 511, dtype=torch.int32, device="cuda")
+    body[:len(val)] = val
+    body = body.view(per, 511).to(torch.int16).view(torch.float16)
+    for shift in (-13, 0, 14):
+        for chunk in bits.split(128):
+            amax = chunk.to(torch.int16).view(torch.float16)
+            x = torch.empty(len(chunk), per, 512, dtype=torch.float16, device="cuda")
+            x[:, :, 0] = amax[:, None]
+            x[:, :, 1:] = torch.minimum(body[None], amax[:, None, None])
+            x[:, 1::2] *= -1
+            x = (x.view(-1, 512) * 2.0 ** shift)
+            q, s = g.fp8_quantize_per_token(x)
+            ref_s = x.abs().amax(1).float() / torch.full((len(x),), 448.0, device="cuda")     # (a tensor: torch multiplies by 1 / scalar)
+            assert torch.equal(s, ref_s)
+            ref = (x.float() / ref_s[:, None]).clamp(-448.0, 448.0).to(torch.float8_e4m3fn)
+            assert torch.equal(q.view(torch.uint8), ref.view(torch.uint8))
