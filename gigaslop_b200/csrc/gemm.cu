@@ -95,7 +95,6 @@ static bool make_map_2d(CUtensorMap* m, CUtensorMapDataType dt, int esz, const v
 // ---- per-device state -------------------------------------------------------------------------
 // Atomics: the contract allows one host thread per GPU, and two of them may meet here.
 constexpr int kMaxDevices = 64;
-constexpr int kVariantMinRowBlocks = 256;      // 128-row blocks from which the twelve-warp form is the default for the SwiGLU (see launch_gemm)
 static std::atomic<int> g_dev_ok[kMaxDevices];       // 0 unknown, 1 ok, -1 unsupported
 static std::atomic<int> g_dev_sms[kMaxDevices];
 
@@ -418,30 +417,34 @@ int32_t launch_gemm(const GemmArgs& a, cudaStream_t st) {
   const bool variants = !fused && !general_rotary && !p.direct_store && (a.kind == KIND_I8 || a.kind == KIND_F8) &&
                         (a.epi == EPI_DEQUANT || a.epi == EPI_ROTARY || a.epi == EPI_SILU);
   if (variants) {
-    // Defaults, from measurements at the benchmark's sizes: twelve warps pay for the weight-stationary SwiGLU (the
-    // heaviest epilogue per output), pairs for the streaming schedule with any of the three epilogues (K > 512: both
-    // operands come from L2 for every tile, a single CTA asks for 96 bytes per clock where about 64 arrive, and a
-    // pair halves the W part: 12-22 % at M = 65536) from the point where single CTAs would need a second round (up to
-    // there they are faster: M = 9001, N = 512, K = 2048 9.5 us against 10.8); the activation-stationary rotary kernel takes both together (twelve
-    // warps alone leave it waiting for operands, pairs alone for its epilogue; together 3 % at config 2 and less
-    // power); elsewhere the eight-warp single-CTA kernel.  Where the SwiGLU's line could lie (INT8, eight against twelve
-    // warps, us): K = 512, N = 2048 equal from 2 row blocks (6.0 / 5.9) over 64 (18.1 / 18.2) and 128 (30.3 / 30.2) to 256
-    // (57.0 / 56.6); K = 384, N = 1536 equal up to 48 row blocks (11.0 / 10.7), then twelve ahead: 64 14.2 / 13.4, 128 22.1 /
-    // 20.6, 256 39.6 / 38.1; K = 256, N = 1024 twelve ahead from 48 (8.6 / 8.0), 128 16.2 / 14.8, 256 26.9 / 24.2.  FP8 the
-    // same.  So for K < 512 the line lies higher than it need.  The general rotary epilogues exist with eight warps and
-    // single CTAs only.
+    // Defaults, from measurements (graphs of launches, us; INT8, FP8 the same): eight warps on single CTAs, except
+    //  * SwiGLU, weight-stationary: twelve warps from 48 row blocks at K < 512 (eight / twelve: K = 384, N = 1536 48 row blocks 11.2 /
+    //    11.2, 64 14.6 / 13.7, 157 28.8 / 26.6, 256 43.3 / 40.0; K = 256, N = 1024 32 7.1 / 7.1, 48 8.6 / 8.3, 128 16.9 / 15.5, 256 29.3 /
+    //    26.2; K = 128 48 6.7 / 6.6, 128 9.9 / 9.3) and from 160 at K = 512 (128 32.4 / 32.9, 157 38.3 / 38.0, 192 45.5 / 44.7, 256 58.3 / 57.1).
+    //  * rotary, activation-stationary: twelve warps AND pairs (twelve alone leave it waiting for operands, pairs alone for its
+    //    epilogue; both draw less power) from 192 row blocks at K = 512 (neither / both: 157 26.0 / 26.5, 192 30.1 / 29.5, 256 39.9 / 38.6),
+    //    from 256 at K = 384 (224 31.6 / 32.7, 256 32.3 / 30.1), not at K <= 256 (256 21.4 / 21.6, 448 34.9 / 36.0).
+    //  * streaming (K > 512: both operands come from L2 for every tile, a single CTA asks for 96 bytes per clock where about 64
+    //    arrive, and a pair halves the W part): pairs from the point where single CTAs would need a second round (N = 512, K = 2048:
+    //    64 row blocks, one round, 10.6 / 11.8 with pairs, 96 18.8 / 17.4, 256 37.3 / 32.4).  The rotary epilogue's single CTAs share
+    //    out their last round and pairs come later, the later the fewer K blocks a tile has (K = 768: 24 row blocks 10.6 / 12.5, 96
+    //    25.5 / 26.9, 128 37.9 / 34.7; K = 1024: 32 16.6 / 16.9, 48 21.2 / 20.1, 128 59.9 / 49.2): the line goes between these with
+    //    tiles * k_blocks^2 = 230 per SM.
+    // The general rotary epilogues exist with eight warps and single CTAs only.
     const int ew = variant_setting(g_variant_ew, "GSB200_GEMM_EW"), pm = variant_setting(g_variant_pair, "GSB200_GEMM_PAIR");
-    const bool big = p.m_blocks >= kVariantMinRowBlocks;
+    const bool silu_ew12 = a.epi == EPI_SILU && resident && p.m_blocks >= (p.k_blocks < 4 ? 48 : 160);
+    const bool streaming_pair = !resident && tiles > sms && (a.epi != EPI_ROTARY || tiles * p.k_blocks * p.k_blocks > 230ll * sms);
     // twelve warps AND pairs, or neither (so not when the caller has fixed one of the two)
-    const bool rotary_both = a.epi == EPI_ROTARY && resident && big && p.k_blocks >= 2 && sms >= 2 && ew < 0 && pm < 0;
+    const bool rotary_both = a.epi == EPI_ROTARY && resident && p.k_blocks >= 3 && p.m_blocks >= (p.k_blocks == 4 ? 192 : 256) && sms >= 2 &&
+                             ew < 0 && pm < 0;
     // ... and so does the weight-stationary dequant GEMM when its output is far larger than L2 (the hoisted LSTM
     // projection: 3 % at M = 262144, 5 % at a million rows, nothing at 131072)
     const bool huge_dequant_both = a.epi == EPI_DEQUANT && resident && p.m_blocks >= 2048 && p.n_blocks >= 4 &&
                                    p.k_blocks >= 2 && sms >= 2 && ew < 0 && pm < 0;
     const bool both = rotary_both || huge_dequant_both;
-    ew12 = ew < 0 ? ((a.epi == EPI_SILU && resident && big) || both) : ew == 12;
+    ew12 = ew < 0 ? (silu_ew12 || both) : ew == 12;
     const bool want_pair = p.k_blocks >= 2 && sms >= 2 &&
-                           (pm < 0 ? ((!resident && tiles > sms) || (both && ew12)) : pm == 1);
+                           (pm < 0 ? (streaming_pair || (both && ew12)) : pm == 1);
     if (ew12 && !variant_dispatch(a.kind, a.epi, false, true, false, ta, tb0, tb1, tc, p, 0, resident, st)) ew12 = false;
     if (want_pair) {
       int cap = variant_dispatch(a.kind, a.epi, true, ew12, false, ta, tb0, tb1, tc, p, 0, resident, st);

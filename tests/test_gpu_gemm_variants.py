@@ -123,3 +123,27 @@ def test_rotary_row_blocks_in_shares_give_the_same_bytes(head_dim, rotary_dim, M
     torch.cuda.synchronize()
     assert torch.equal(a, b)
     assert g.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("op,row_blocks,K", [("silu", 47, 384), ("silu", 48, 384), ("silu", 48, 128), ("silu", 159, 512), ("silu", 160, 512),
+                                             ("rotary", 191, 512), ("rotary", 192, 512), ("rotary", 256, 384), ("rotary", 256, 256),
+                                             ("rotary", 100, 768), ("rotary", 110, 768), ("rotary", 44, 1024), ("rotary", 46, 1024)])
+def test_both_sides_of_the_lines_between_the_forms(force, op, row_blocks, K):
+    """What the library picks by shape, just below and just above the lines it draws, against eight warps on single CTAs."""
+    g = need_lib()
+    M = 128 * row_blocks - 5
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    i8 = lambda n: torch.randint(-127, 128, (n, K), generator=gen, device="cuda", dtype=torch.int8)
+    sc = lambda n: torch.rand(n, generator=gen, device="cuda") * 1e-2 + 1e-3
+    A, sa = i8(M), sc(M)
+    if op == "silu":
+        G, U, sg, su = i8(256), i8(256), sc(256) * 1e-2, sc(256)
+        run = lambda: g.dual_gemm_i8_silu(A, G, U, sa, sg, su)
+    else:
+        nhead = K // 64
+        W, sw, ang = i8(3 * K), sc(3 * K), torch.randn(500, 32, generator=gen, device="cuda")
+        run = lambda: g.gemm_i8_rotary(A, W, sa, sw, ang.sin(), ang.cos(), nhead, 64, 64, 500, row_offset=3)
+    got = run()
+    force(8, 0)
+    assert_bitexact(got, run())
+    assert g.device_status()[0] == 0
