@@ -81,13 +81,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     prefetch_tmap(&tm_a); prefetch_tmap(&tm_b0); prefetch_tmap(&tm_b1);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 2 * NPART); tmem_relinquish(); }
-  // The grid is at most a wave, so its successor's blocks find room while it runs.
-  pdl_trigger();
-  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // The grid is at most a wave, so its successor's blocks find room while it runs.  They may start only once this CTA has its
+  // tensor memory: a successor's CTA that took some first would hold it until this grid is done, and this one wait for it.
+  pdl_trigger();
+  pdl_wait();
   const unsigned int budget = spin_budget();
 
   // this thread's row; its token scale and sin / cos values are on their way during the main loop

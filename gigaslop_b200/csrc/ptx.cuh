@@ -59,7 +59,7 @@ __device__ __forceinline__ void named_sync() { asm volatile("barrier.cta.sync.al
 // the kernel before it is complete and its writes are visible; at least one block of a grid has to wait.  Data another kernel
 // may have written is not read through the non-coherent path (ld.global.nc): that is for data constant over the kernel's
 // life.  pdl_trigger lets the successor's CTAs become resident as this kernel's leave.  The quantisers (after their wait), the
-// scale re-tiler, the LSTM cell and the few-tile GEMMs (before theirs) do that: the GEMM behind them sets up its barriers and
+// scale re-tiler, the LSTM cell and the few-tile GEMMs (before theirs, with their tensor memory in hand) do that: the GEMM behind them sets up its barriers and
 // tensor memory meanwhile.  The persistent GEMMs do not: a quantiser that starts beside their last tiles costs more than it gains (us per pass, a few
 // back to back at the full clock; no overlap / quantisers trigger / GEMMs too: QKV of 65536 rows 84.3 / 79.7 / 83.8,
 // feed-forward 246 / 239 / 249, of 256 rows 28.7 / 22 / 22, of 9001 rows
