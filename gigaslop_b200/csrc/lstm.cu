@@ -306,7 +306,7 @@ lstm_recurrent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 //  * the batch is the small dimension, so B = 512 spreads over 129 SMs (G = 12) instead of 48: the gate math, five
 //    special-function instructions per cell, is 1000 clocks for 2048 cells (G = 16), 600 for 1024.
 //  * W_hh in tensor memory: an MMA from a shared-memory A operand of 128 rows takes 40 clocks, from TMEM 16.
-// B = 512, H = 384: 1.12 us per step (2.57 with the 128-row tiles), H = 512: 1.74 (4.8), H = 256: 0.80 (2.29), H = 128: 0.54 (2.27).
+// B = 512, H = 384: 1.11 us per step (2.57 with the 128-row tiles), H = 512: 1.74 (4.8), H = 256: 0.80 (2.29), H = 128: 0.54 (2.27).
 // It was 1.34 / 1.93 / 0.93 / 0.57 before three changes to how its warps wait and issue.  An MMA warp walks its loop converged, with
 // one elected lane issuing (a single thread moves the operands of every MMA to uniform registers): 1.22 / 1.84 / 0.84 / 0.56.  The
 // gate warps report to it through a named barrier instead of an mbarrier: 1.21 / 1.84 / 0.83 / 0.56.  The waits on the chain, for the
@@ -538,12 +538,16 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           dst[r * 128 + ((ck ^ (r & 7)) << 4)] = (uint8_t)h8[i];
           dst[(r + 1) * 128 + ((ck ^ ((r + 1) & 7)) << 4)] = (uint8_t)(h8[i] >> 8);
         }
-        if (hf == 1) { fence_proxy_async_smem(); tc_fence_before(); }      // the stores above before the MMAs read them
         __syncwarp();
-        if (hf == 1 && s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
+        // (to the other CTAs first, whose MMAs wait for it longest; B = 256, H = 384 923 ns per step with the report first, 901 so)
         if (sends && s + 1 < p.T) {
           const uint32_t off = (s & 1) * L::HBUF + snd_off[hf];
           st_async_v4(snd_dst + off, *reinterpret_cast<const uint4*>(h_s + off), snd_bar + 8 * LT_MAX_SLICES * (s & 1));
+        }
+        if (hf == 1) {
+          fence_proxy_async_smem(); tc_fence_before();                       // the stores above before this CTA's MMAs read them
+          __syncwarp();
+          if (s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
         }
       }
       // the layer's outputs, off the critical path: 32 (E4M3) / 64 (fp16) contiguous bytes per warp and row
