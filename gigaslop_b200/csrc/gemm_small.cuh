@@ -1,11 +1,12 @@
-// Few-tile form of the 8-bit GEMMs: one 64-row tile per CTA, no persistence.
+// Few-tile form of the 8-bit GEMMs: one tile of 64 or 128 rows per CTA, no persistence.
 //
 // What bounds a GEMM of a few rows is not bandwidth but the chain launch -> first bytes -> MMAs -> epilogue on the few SMs
 // that have a tile.  The persistent kernel's tile is 128 x 256: at K = 512 its MMAs take 2048 clocks and its epilogue about
 // 5000, one after the other when there is only one tile, and the down-projection of 256 rows to 512 columns is four of them.
-// Here a tile is 64 rows x 64 or 128 accumulator columns, so the same work spreads over 8 to 16 times as many SMs: the MMAs of
-// K = 512 take about 900 clocks (issue-bound), a CTA loads 64 KiB instead of 192, and a thread's epilogue is 32 columns, loaded
-// once and stored straight from registers.  us per launch from a graph, persistent kernel -> this one:
+// Here a tile is 64 rows x 64 or 128 accumulator columns (128 x 128 where those are too many), so the same work spreads over 8
+// to 16 times as many SMs: the MMAs of K = 512 take about 900 clocks (issue-bound), a CTA loads 64 KiB instead of 192, and a
+// thread's epilogue is 32 columns, loaded once and stored straight from registers.  us per launch from a graph, persistent
+// kernel -> this one:
 //   dequant N = 512, K = 512    M = 1 5.3 -> 3.0, 256 6.0 -> 3.2, 1024 6.0 -> 3.7, 3072 6.0 -> 4.5
 //   dequant N = 512, K = 2048   M = 64 9.7 -> 5.9, 1024 9.7 -> 6.5, 3072 10.3 -> 7.8      N = 128, K = 1024 (FP8)  M = 256 6.7 -> 4.1
 //   rotary N = 1536, K = 512    M = 64 6.6 -> 3.7, 256 7.5 -> 4.4, 768 8.1 -> 5.2
@@ -14,7 +15,7 @@
 //   n1 = n0 + NPART for the plain epilogue; for the rotary one the two parts are what rotates together (heads of 128 with all
 //   columns rotated: 64 apart).
 //   warp 0 lane 0 loads (TMA, ring of p.stages K blocks), warp 1 lane 0 issues the MMAs, all eight warps do the epilogue: warp w
-//   reads TMEM lane quarter w % 4 (M = 64: row 16 q + l lies in lane 32 q + l, l < 16) and half w / 4 of both parts.
+//   reads TMEM lane quarter w % 4 (64 rows: row 16 q + l lies in lane 32 q + l, l < 16) and half w / 4 of both parts.
 // The arithmetic, its order and its rounding points are those of gemm_kernel.cuh's epilogues: same bytes.
 #pragma once
 #include <cuda_fp8.h>
@@ -26,14 +27,13 @@
 
 namespace gsb {
 
-constexpr int SG_TM = 64;
 constexpr int SG_THREADS = 256;
-constexpr int SG_A_BYTES = SG_TM * BK;               // 8 KiB per K block
 constexpr int SG_MAX_STAGES = 12;
 
-template <int NPART>
+template <int TM, int NPART>
 struct SgSmem {
-  static constexpr int STAGE_BYTES = SG_A_BYTES + 2 * NPART * BK;      // 16 or 24 KiB
+  static constexpr int A_BYTES = TM * BK;                              // per K block
+  static constexpr int STAGE_BYTES = A_BYTES + 2 * NPART * BK;         // 16, 24 or 32 KiB
   static constexpr int TAIL = 2 * NPART * 4 + (2 * SG_MAX_STAGES + 1) * 8 + 16;      // channel scales, barriers, TMEM address, abort flag
   static constexpr int bytes(int stages) { return stages * STAGE_BYTES + ((TAIL + 127) & ~127); }
 };
@@ -50,13 +50,17 @@ struct SgParams {
   int rot_geo;             // rotary: 0 heads of 128, all rotated; 1 heads of 128, 64 rotated; 2 heads of 64, 32 rotated; 3 heads of 64, all rotated
 };
 
-template <int KIND, int EPI, int NPART>
+template <int KIND, int EPI, int TM, int NPART>
 __global__ void __launch_bounds__(SG_THREADS, 2)
 gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b0, const __grid_constant__ CUtensorMap tm_b1,
                   const SgParams p) {
   extern __shared__ __align__(1024) uint8_t sg_smem[];
   constexpr bool DUAL = EPI == EPI_SILU || EPI == EPI_SILU_MX;
-  constexpr int ST = SgSmem<NPART>::STAGE_BYTES, H = NPART / 2;        // H = columns of each part that a warp handles
+  constexpr int ST = SgSmem<TM, NPART>::STAGE_BYTES, H = NPART / 2;    // H = columns of each part that a warp handles
+  constexpr int QR = TM / 4;                                           // rows in a TMEM lane quarter
+  constexpr int SG_A_BYTES = SgSmem<TM, NPART>::A_BYTES;
+  static_assert(TM == 128 || TM == 64, "UMMA M");
+  static_assert(EPI != EPI_ROTARY || TM == 64, "the rotary rows of a tile");
   static_assert(EPI != EPI_SILU_MX || H == 32, "a thread quantises whole blocks of 32 columns");
   static_assert(EPI != EPI_ROTARY || NPART == 32, "rotary parts are 32 columns");
   float* sc_s = reinterpret_cast<float*>(sg_smem + p.stages * ST);     // [2 NPART]
@@ -67,7 +71,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const AbortFlag abort_flag{smem_u32(tmem_slot + 1)};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  const int m0 = (int)(blockIdx.x / p.n_tiles) * SG_TM, tn = (int)(blockIdx.x % p.n_tiles);
+  const int m0 = (int)(blockIdx.x / p.n_tiles) * TM, tn = (int)(blockIdx.x % p.n_tiles);
   int n0, n1;                                          // first W row (= output column) of the two parts
   if constexpr (DUAL) { n0 = n1 = tn * NPART; }
   else if (EPI == EPI_ROTARY && p.rot_geo == 0) { n0 = (tn >> 1) * 128 + (tn & 1) * 32; n1 = n0 + 64; }
@@ -93,8 +97,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 
   // this thread's row; its token scale and sin / cos values are on their way during the main loop
   const int q = warp & 3, half = warp >> 2;
-  const int row = m0 + q * 16 + lane;
-  const bool row_ok = lane < 16 && row < p.M;
+  const int row = m0 + q * QR + lane;
+  const bool row_ok = lane < QR && row < p.M;
   const int rc = row < p.M ? row : p.M - 1;            // (a row that exists, for the load)
   // rotary: the warp's two 16-column chunks ca, cb rotate together (or are only dequantised)
   const bool pairs32 = EPI != EPI_ROTARY || p.rot_geo != 2;
@@ -144,7 +148,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     fetch();
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc = (KIND == KIND_I8) ? umma_idesc(2, 1, 1, SG_TM, 2 * NPART) : umma_idesc(1, 0, 0, SG_TM, 2 * NPART);
+      constexpr uint32_t idesc = (KIND == KIND_I8) ? umma_idesc(2, 1, 1, TM, 2 * NPART) : umma_idesc(1, 0, 0, TM, 2 * NPART);
       int s = 0; uint32_t ph = 0; bool ok = true;
       for (int kb = 0; kb < p.k_blocks; ++kb) {
         if (!mbar_wait(&full[s], ph, abort_flag, ST_TIMEOUT_MMA, 0xC10 | s, budget)) { ok = false; break; }
@@ -284,34 +288,36 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 2 * NPART); }
 }
 
-static long long small_gemm_tiles(const GemmArgs& a, int npart) {
+static long long small_gemm_tiles(const GemmArgs& a, int tm, int npart) {
   const int cols = a.epi == EPI_SILU || a.epi == EPI_SILU_MX ? npart : 2 * npart;
-  return (long long)((a.M + SG_TM - 1) / SG_TM) * ((a.N + cols - 1) / cols);
+  return (long long)((a.M + tm - 1) / tm) * ((a.N + cols - 1) / cols);
 }
 
-template <int KIND, int EPI, int NPART>
+template <int KIND, int EPI, int TM, int NPART>
 static int32_t launch_small_inst(const GemmArgs& a, const SgParams& p, int grid, int dev, const CUtensorMap& ta, const CUtensorMap& tb0,
                                  const CUtensorMap& tb1, cudaStream_t st) {
   static std::atomic<int> attr_done[64];
-  auto k = gemm_small_kernel<KIND, EPI, NPART>;
+  auto k = gemm_small_kernel<KIND, EPI, TM, NPART>;
   if (!attr_done[dev].load(std::memory_order_acquire)) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SgSmem<NPART>::bytes(NPART == 32 ? SG_MAX_STAGES : 8));
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SgSmem<TM, NPART>::bytes(TM == 128 ? 6 : NPART == 32 ? SG_MAX_STAGES : 8));
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(small gemm)");
     attr_done[dev].store(1, std::memory_order_release);
   }
-  return cuda_status(launch_dependent(k, (unsigned)grid, SG_THREADS, (size_t)SgSmem<NPART>::bytes(p.stages), st, ta, tb0, tb1, p), "gemm launch");
+  return cuda_status(launch_dependent(k, (unsigned)grid, SG_THREADS, (size_t)SgSmem<TM, NPART>::bytes(p.stages), st, ta, tb0, tb1, p), "gemm launch");
 }
 
 template <int KIND>
-static int32_t launch_small_kind(const GemmArgs& a, int npart, const SgParams& p, int grid, int dev, const CUtensorMap& ta, const CUtensorMap& tb0,
+static int32_t launch_small_kind(const GemmArgs& a, int tm, int npart, const SgParams& p, int grid, int dev, const CUtensorMap& ta, const CUtensorMap& tb0,
                                  const CUtensorMap& tb1, cudaStream_t st) {
   switch (a.epi) {
-    case EPI_DEQUANT: return launch_small_inst<KIND, EPI_DEQUANT, 32>(a, p, grid, dev, ta, tb0, tb1, st);
-    case EPI_ROTARY: return launch_small_inst<KIND, EPI_ROTARY, 32>(a, p, grid, dev, ta, tb0, tb1, st);
-    case EPI_SILU: return npart == 32 ? launch_small_inst<KIND, EPI_SILU, 32>(a, p, grid, dev, ta, tb0, tb1, st)
-                                      : launch_small_inst<KIND, EPI_SILU, 64>(a, p, grid, dev, ta, tb0, tb1, st);
+    case EPI_DEQUANT: return tm == 64 ? launch_small_inst<KIND, EPI_DEQUANT, 64, 32>(a, p, grid, dev, ta, tb0, tb1, st)
+                                      : launch_small_inst<KIND, EPI_DEQUANT, 128, 64>(a, p, grid, dev, ta, tb0, tb1, st);
+    case EPI_ROTARY: return launch_small_inst<KIND, EPI_ROTARY, 64, 32>(a, p, grid, dev, ta, tb0, tb1, st);
+    case EPI_SILU: return tm == 128 ? launch_small_inst<KIND, EPI_SILU, 128, 64>(a, p, grid, dev, ta, tb0, tb1, st)
+                        : npart == 32 ? launch_small_inst<KIND, EPI_SILU, 64, 32>(a, p, grid, dev, ta, tb0, tb1, st)
+                                      : launch_small_inst<KIND, EPI_SILU, 64, 64>(a, p, grid, dev, ta, tb0, tb1, st);
     default:
-      if constexpr (KIND == KIND_F8) return launch_small_inst<KIND_F8, EPI_SILU_MX, 64>(a, p, grid, dev, ta, tb0, tb1, st);
+      if constexpr (KIND == KIND_F8) return launch_small_inst<KIND_F8, EPI_SILU_MX, 64, 64>(a, p, grid, dev, ta, tb0, tb1, st);
       return GSB200_ERR_BAD_ARG;
   }
 }
@@ -325,6 +331,10 @@ static int32_t launch_small_kind(const GemmArgs& a, int npart, const SgParams& p
 //   registers a thread, two CTAs per SM: M = 512 4.8 / 6.3, M = 768 7.7 / 6.4
 // The rotary form stops at two per SM as well: a launch of a thousand rows and more names its output in a tensor map, which
 // callers may count on finding in the table of maps (gsb200_tensor_map_encodes); this form stores without one.
+// Where the 64-row tiles are too many, 128 x 128 ones (dequant; SwiGLU 128 x (64 + 64)) still fit (us, these / persistent kernel):
+//   dequant, one per SM: N = 512, K = 512, M = 4096 4.5 / 6.1; K = 2048 7.9 / 9.8; N = 1536, K = 512, M = 1500 4.4 / 6.1 (two per SM:
+//   N = 1536, K = 512, M = 2000 5.8 / 6.2, but N = 512, K = 512, M = 6000 6.1 / 6.1 and K = 2048 11.0 / 10.1)
+//   SwiGLU, up to two per SM, K <= 512: N = 2048, K = 512, M = 768 5.3 / 6.2 (64-row tiles, three per SM, 5.7), M = 1024 5.3 / 6.3
 // Under a cap on the SMs a launch may take, one CTA per SM of the cap: more would spread over more SMs.
 static int32_t launch_gemm_small(const GemmArgs& a, const GemmParams& g, int geo, cudaStream_t st, bool* taken) {
   *taken = false;
@@ -334,9 +344,14 @@ static int32_t launch_gemm_small(const GemmArgs& a, const GemmParams& g, int geo
   if (dev < 0 || dev >= 64) return GSB200_OK;
   long long limit = sm_count();
   if (a.sm_cap > 0 && a.sm_cap < limit) limit = a.sm_cap;
-  int npart = a.epi == EPI_SILU_MX ? 64 : 32;
-  long long tiles = small_gemm_tiles(a, npart);
-  if (a.epi == EPI_SILU && tiles > limit) { npart = 64; tiles = small_gemm_tiles(a, npart); }
+  int tm = 64, npart = a.epi == EPI_SILU_MX ? 64 : 32;
+  long long tiles = small_gemm_tiles(a, tm, npart);
+  if (a.epi == EPI_SILU && tiles > limit) { npart = 64; tiles = small_gemm_tiles(a, tm, npart); }
+  const long long tiles128 = small_gemm_tiles(a, 128, 64);
+  if ((a.epi == EPI_DEQUANT && tiles > 3 * limit && tiles128 <= limit) ||
+      (a.epi == EPI_SILU && tiles > 2 * limit && tiles128 <= 2 * limit && g.k_blocks <= RES_MAX_KBLOCKS)) {
+    tm = 128; npart = 64; tiles = tiles128;
+  }
   const long long per_sm = (tiles + limit - 1) / limit;
   const int most = limit < sm_count_physical() ? 1 : a.epi == EPI_ROTARY || a.epi == EPI_SILU_MX ? 2 : 3;
   if (per_sm > most) return GSB200_OK;
@@ -345,20 +360,20 @@ static int32_t launch_gemm_small(const GemmArgs& a, const GemmParams& g, int geo
   p.M = g.M; p.N = g.N; p.k_blocks = g.k_blocks;
   const int cols = dual ? npart : 2 * npart;
   p.n_tiles = (a.N + cols - 1) / cols;
-  p.stages = npart == 32 ? (per_sm == 1 ? SG_MAX_STAGES : per_sm == 2 ? 6 : 4) : (per_sm == 1 ? 8 : per_sm == 2 ? 4 : 3);
+  p.stages = tm == 128 ? (per_sm == 1 ? 6 : 3) : npart == 32 ? (per_sm == 1 ? SG_MAX_STAGES : per_sm == 2 ? 6 : 4) : (per_sm == 1 ? 8 : per_sm == 2 ? 4 : 3);
   if (p.stages > p.k_blocks) p.stages = p.k_blocks;
   p.C = g.C; p.ldc = g.ldc; p.out_scale = g.out_scale; p.ld_scale = g.ld_scale;
   p.scale_a = g.scale_a; p.scale_a_const = g.scale_a_const; p.scale_b0 = g.scale_b0; p.scale_b1 = g.scale_b1; p.scale_b_scalar = g.scale_b_scalar;
   p.sin_tab = g.sin_tab; p.cos_tab = g.cos_tab; p.seqlen = g.seqlen; p.row_offset = g.row_offset; p.rot_cols = g.rot_cols; p.rot_geo = geo;
   const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
   CUtensorMap ta, tb0, tb1;
-  bool ok = tmap_2d(&ta, u8, 1, a.A, (uint64_t)a.M, (uint64_t)a.K, (uint64_t)a.lda, BK, SG_TM, CU_TENSOR_MAP_SWIZZLE_128B) &&
+  bool ok = tmap_2d(&ta, u8, 1, a.A, (uint64_t)a.M, (uint64_t)a.K, (uint64_t)a.lda, BK, (uint32_t)tm, CU_TENSOR_MAP_SWIZZLE_128B) &&
             tmap_2d(&tb0, u8, 1, a.B0, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)a.ldb, BK, npart, CU_TENSOR_MAP_SWIZZLE_128B);
   if (!dual) tb1 = tb0;
   else ok = ok && tmap_2d(&tb1, u8, 1, a.B1, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)a.ldb, BK, npart, CU_TENSOR_MAP_SWIZZLE_128B);
   if (!ok) return GSB200_ERR_BAD_ARG;
-  return a.kind == KIND_I8 ? launch_small_kind<KIND_I8>(a, npart, p, (int)tiles, dev, ta, tb0, tb1, st)
-                           : launch_small_kind<KIND_F8>(a, npart, p, (int)tiles, dev, ta, tb0, tb1, st);
+  return a.kind == KIND_I8 ? launch_small_kind<KIND_I8>(a, tm, npart, p, (int)tiles, dev, ta, tb0, tb1, st)
+                           : launch_small_kind<KIND_F8>(a, tm, npart, p, (int)tiles, dev, ta, tb0, tb1, st);
 }
 
 }  // namespace gsb

@@ -1,4 +1,4 @@
-"""GPU parity of the few-tile GEMM form (64-row tiles, one per CTA) at the edges of its tiles, its ring and its range.
+"""GPU parity of the few-tile GEMM form (tiles of 64 or 128 rows, one per CTA) at the edges of its tiles, its ring and its range.
 
 The persistent kernel, which an override of the variant choice selects, runs the same calls: both must give the same
 bytes, and INT8 results must be the exact-accumulator model's.  Outputs lie inside wider buffers, whose other columns
@@ -43,9 +43,9 @@ def operands(gen, fp8, M, N, K):
 
 
 # one row; tile edges; a column tile cut after its first part and after 8 columns; a ragged K block; rings that are
-# reused (K = 2048 and 3 * 128 with one to three CTAs per SM)
+# reused (K = 2048 and 3 * 128 with one to three CTAs per SM); the last two take 128-row tiles
 SHAPES = [(1, 8, 16), (63, 64, 128), (64, 96, 144), (65, 72, 512), (130, 520, 2048), (777, 1032, 384), (2048, 512, 2048), (3000, 512, 512),
-          (1025, 1536, 640)]
+          (1025, 1536, 640), (3601, 520, 384), (4700, 512, 2048)]
 
 
 @pytest.mark.parametrize("fp8", [False, True])
@@ -62,7 +62,7 @@ def test_dequant(fp8, M, N, K):
 
 
 @pytest.mark.parametrize("fp8", [False, True])
-@pytest.mark.parametrize("M,N,K", [(1, 8, 16), (64, 32, 128), (65, 72, 512), (200, 2048, 512), (330, 1000, 2048), (700, 1544, 384)])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 16), (64, 32, 128), (65, 72, 512), (200, 2048, 512), (330, 1000, 2048), (700, 1544, 384), (1001, 2040, 512)])
 def test_swiglu(fp8, M, N, K):
     g = need_lib()
     gen = torch.Generator().manual_seed(M + 5 * N + 7 * K)
