@@ -797,11 +797,17 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
   cudaError_t e;
   // 256-column weight-stationary tiles where their rounds are cheaper: a tile takes about 1.5 times what a 128-column one does
   // (dual, K = 512, N = 2048: M = 4096 12.5 us with 128 columns, 11.9 with 256; M = 1024 6.8 and 5.9; M = 128, one round of either,
-  // 5.3 and 5.5).
+  // 5.3 and 5.5).  Where the 128-column slices are more than the SMs, the other side is the streaming kernel, which deals its tiles
+  // to all SMs while this form leaves idle what its slices do not fill; a tile here takes 1.5 (dual 1.25) times what a round of 128
+  // columns does there (us, streaming / this one; M = 5000, K = 512: plain N = 18976, 75 slices, 60.0 / 79.0, N = 22016, 86, 68.6 / 81.4, N =
+  // 30016, 118, 92.0 / 84.1; dual N = 9504, 75, 65.5 / 77.8, N = 12000, 94, 80.4 / 81.4, N = 18944, 148, 122 / 87; K = 128: plain N = 22016
+  // 42.2 / 56.1, dual N = 10016 40.8 / 44.9; M = 100, plain N = 22016, a second round there, 6.1 / 6.1, dual N = 9504 6.4 / 5.8).
   if (K / MX_BK <= MXW_MAX_KB) {
     const int out256 = dual ? 128 : 256, nb = (N + out256 - 1) / out256, sms = sm_count();
     const int g256 = sms / nb, g128 = wst ? sms / p.n_blocks : 0;
-    if (g256 > 0 && (g128 == 0 || (p.m_blocks + g256 - 1) / g256 * 15 < (p.m_blocks + g128 - 1) / g128 * 10)) {
+    const long long r256 = g256 > 0 ? (p.m_blocks + g256 - 1) / g256 : 0;
+    const bool better = g128 > 0 ? r256 * 15 < (p.m_blocks + g128 - 1) / g128 * 10ll : r256 * (dual ? 25 : 30) < (tiles + sms - 1) / sms * 20;
+    if (g256 > 0 && better) {
       CUtensorMap tw0, tw1, to;
       if (!map2d(&tw0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
           !map2d(&tw1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dual ? B1 : B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import oracle
-from util import assert_bitexact, need_lib, rand_scales
+from util import assert_bitexact, launches, need_lib, rand_scales
 
 pytestmark = pytest.mark.gpu
 
@@ -187,4 +187,32 @@ def test_block_scaled_weight_stationary_256_column_tiles(dual, M, N, K):
     for lo in (0, M // 2 // 128 * 128, (M - 1) // 128 * 128 - 128):
         hi = min(M, lo + 256)
         assert_bitexact(got[lo:hi], run(a[lo:hi].contiguous(), g.mx_scales_to_tiled(sa[lo:hi].contiguous(), K)), f"rows {lo}:{hi}")
+    assert g.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("dual,N,M,form", [(False, 18976, 100, "mx_gemm256w"), (False, 18976, 1300, "mx_gemm256_k"), (False, 37888, 1300, "mx_gemm256w"),
+                                           (True, 9504, 100, "mx_gemm256w"), (True, 9504, 1300, "mx_gemm_k"), (True, 18944, 1300, "mx_gemm256w")])
+def test_block_scaled_gemm_of_many_column_slices(dual, N, M, form):
+    """More 128-column slices than SMs: 256-column weight-stationary tiles only where they beat the streaming kernel, which has work
+    for every SM.  Either way the bytes are those of the same columns asked for by themselves."""
+    g = need_lib()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are either side of the line for 148 SMs")
+    K = 256
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    def mx(n):
+        q, s = g.mxfp8_quantize(torch.randn(n, K, generator=gen, device="cuda").half())
+        return q, s, g.mx_scales_to_tiled(s, K)
+    (a, _, ta), (w, sw, tw), (u, su, tu) = mx(M), mx(N), mx(N)
+    out = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    run = lambda: g.dual_gemm_mxfp8_silu(a, ta, w, u, tw, tu, out=out) if dual else g.gemm_mxfp8(a, ta, w, tw, out=out)
+    run()
+    names = [n for n, _ in launches(run)]
+    assert len(names) == 1 and form in names[0], names
+    for lo in (0, N // 2 // 128 * 128, (N - 1) // 128 * 128):
+        hi = min(N, lo + 256)
+        part = lambda t: t[lo:hi].contiguous()
+        tiled = lambda s: g.mx_scales_to_tiled(part(s), K)
+        ref = g.dual_gemm_mxfp8_silu(a, ta, part(w), part(u), tiled(sw), tiled(su)) if dual else g.gemm_mxfp8(a, ta, part(w), tiled(sw))
+        assert_bitexact(out[:, lo:hi], ref, f"columns {lo}:{hi}")
     assert g.device_status()[0] == 0

@@ -69,3 +69,28 @@ def rotary_rows(fn, A_rows, sa_rows, B, sb, sn, cs, nhead, head_dim, rotary_dim,
 
 
 SAMPLE_SLICES_64K = [(0, 256), (32768 - 64, 32768 + 64), (65536 - 256, 65536), (12345, 12345 + 77)]
+
+
+def launches(call):
+    """[(kernel name, blocks)] that `call` launches, read from a captured graph; the captured work does not run."""
+    from cuda.bindings import driver as cu
+
+    def ok(res):
+        assert int(res[0]) == 0, res[0]
+        return res[1:] if len(res) > 2 else res[1] if len(res) == 2 else None
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    raw = cu.CUgraph(graph.raw_cuda_graph())
+    n = ok(cu.cuGraphGetNodes(raw, 0))[1]
+    out = []
+    for node in ok(cu.cuGraphGetNodes(raw, n))[0]:
+        if ok(cu.cuGraphNodeGetType(node)) != cu.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        p = ok(cu.cuGraphKernelNodeGetParams(node))
+        name = ok(cu.cuKernelGetName(p.kern)) if int(p.kern) else ok(cu.cuFuncGetName(p.func))
+        out.append((name.decode(), p.gridDimX * p.gridDimY * p.gridDimZ))
+    graph.reset()
+    return out
