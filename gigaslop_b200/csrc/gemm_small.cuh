@@ -329,6 +329,9 @@ static int32_t launch_small_kind(const GemmArgs& a, int tm, int npart, const SgP
 //   dequant N = 1536, K = 512: three per SM, M = 1024, 4.5 / 6.6; a second wave, M = 1536, 7.3 / 6.1
 //   SwiGLU N = 2048, K = 512: three, M = 768, 5.8 / 6.2; a second wave, M = 1024, 8.4 / 6.4.  The one that emits MXFP8 holds 124
 //   registers a thread, two CTAs per SM: M = 512 4.8 / 6.3, M = 768 7.7 / 6.4
+//   SwiGLU over a longer K: three 64 x (64 + 64) tiles move 1.5 times the operand bytes of the SM's share of 128 x 256 ones, and from some K
+//   on that is what counts.  N = 1024, M = 1700, three per SM: K = 640 6.2 / 6.7, 1024 7.6 / 7.6, 1536 9.5 / 9.1, 2048 11.5 / 10.4, 4096 18.9 /
+//   15.7; so three up to K = 1024, and two at any K (M = 1150: K = 1536 7.2 / 8.7, 2048 8.4 / 10.1, 4096 13.4 / 15.2, 8192 23.6 / 31.5)
 // The rotary form stops at two per SM as well: a launch of a thousand rows and more names its output in a tensor map, which
 // callers may count on finding in the table of maps (gsb200_tensor_map_encodes); this form stores without one.
 // Where the 64-row tiles are too many, 128 x 128 ones (dequant; SwiGLU 128 x (64 + 64)) still fit (us, these / persistent kernel):
@@ -353,7 +356,7 @@ static int32_t launch_gemm_small(const GemmArgs& a, const GemmParams& g, int geo
     tm = 128; npart = 64; tiles = tiles128;
   }
   const long long per_sm = (tiles + limit - 1) / limit;
-  const int most = limit < sm_count_physical() ? 1 : a.epi == EPI_ROTARY || a.epi == EPI_SILU_MX ? 2 : 3;
+  const int most = limit < sm_count_physical() ? 1 : a.epi == EPI_ROTARY || a.epi == EPI_SILU_MX || (a.epi == EPI_SILU && g.k_blocks > 8) ? 2 : 3;
   if (per_sm > most) return GSB200_OK;
   *taken = true;
   SgParams p{};

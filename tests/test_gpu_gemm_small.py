@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import oracle
-from util import assert_bitexact, f16_equal_up_to_signed_zero, need_lib, rand_i8, rand_scales
+from util import assert_bitexact, f16_equal_up_to_signed_zero, launches, need_lib, rand_i8, rand_scales
 
 pytestmark = pytest.mark.gpu
 
@@ -71,6 +71,23 @@ def test_swiglu(fp8, M, N, K):
     sa, sg, su = rand_scales(gen, M, 5e-3, 5e-2).cuda(), rand_scales(gen, N).cuda() * 1e-2, rand_scales(gen, N).cuda()
     A, G, U = A.cuda(), G.cuda(), U.cuda()
     both(lambda out: (g.dual_gemm_fp8_silu if fp8 else g.dual_gemm_i8_silu)(A, G, U, sa, sg, su, out=out), M, N)
+
+
+@pytest.mark.parametrize("M,K,kernel", [(700, 1024, "gemm_small"), (700, 1040, "gemm_tcgen05"), (570, 1040, "gemm_small"), (570, 4096, "gemm_small")])
+def test_swiglu_few_tile_form_by_k(M, K, kernel):
+    """Three 64-row tiles per SM (M = 700) only up to K = 1024, two (M = 570) at any K; the same bytes from either kernel."""
+    g = need_lib()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are either side of the line for 148 SMs")
+    gen = torch.Generator().manual_seed(M + K)
+    A, G = operands(gen, False, M, 2048, K)
+    U = operands(gen, False, M, 2048, K)[1]
+    sa, sg, su = rand_scales(gen, M, 5e-3, 5e-2).cuda(), rand_scales(gen, 2048).cuda() * 1e-2, rand_scales(gen, 2048).cuda()
+    A, G, U = A.cuda(), G.cuda(), U.cuda()
+    both(lambda out: g.dual_gemm_i8_silu(A, G, U, sa, sg, su, out=out), M, 2048)
+    out = torch.empty(M, 2048, dtype=torch.float16, device="cuda")
+    names = [n for n, _ in launches(lambda: g.dual_gemm_i8_silu(A, G, U, sa, sg, su, out=out))]
+    assert len(names) == 1 and kernel in names[0], names
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 32, 128), (65, 96, 512), (200, 2048, 512), (500, 1056, 2048)])
