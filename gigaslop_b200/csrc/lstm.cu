@@ -416,15 +416,24 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const int rows_live = min(RPT, max(0, B - (row0 + r_lo)));          // rows of this thread that exist
   float c[RPT];
   if (warp < CW) {
-    // W_hh -> tensor memory: lane = hidden unit, 32 columns = 128 bytes of K; the warps of a lane quarter share the K blocks
+    // W_hh -> tensor memory: lane = hidden unit, 32 columns = 128 bytes of K; the warps of a lane quarter share the K blocks.
+    // A lane reads whole 32-byte sectors of its row (where base and stride allow): of 16-byte pieces the second would have to be
+    // found in L1, and the shared memory that this kernel takes leaves 28 KiB of that.  us per launch of 8 steps, B = 64 / 512: 16-byte
+    // pieces past L1 H = 384 24.0 / 26.9, H = 256 16.9 / 18.8, through L1 17.6 / 24.4 and 14.5 / 17.0, sectors 16.3 / 21.4 and 13.3 / 14.8.
+    const bool w_sectors = ((reinterpret_cast<uintptr_t>(w_hh) | (uintptr_t)ld_w) & 31) == 0;
     for (int blk = warp >> 2; blk < 4 * kb_tmem; blk += CW / 4) {
       const int g = blk / kb_tmem, kb = blk % kb_tmem;
       uint32_t v[32];
+      const uint8_t* src = w_hh + (long long)(g * H + hid) * ld_w + kb * 128;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        uint4 w = make_uint4(0, 0, 0, 0);
-        if (hid_ok && kb * 128 + i * 16 < H) w = __ldcg(reinterpret_cast<const uint4*>(w_hh + (long long)(g * H + hid) * ld_w + kb * 128 + i * 16));
-        v[4 * i] = w.x; v[4 * i + 1] = w.y; v[4 * i + 2] = w.z; v[4 * i + 3] = w.w;
+      for (int i = 0; i < 4; ++i) {                // (H is a multiple of 32)
+        uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+        if (hid_ok && kb * 128 + i * 32 < H) {
+          if (w_sectors) ldg_v8(src + i * 32, lo, hi);
+          else { lo = __ldca(reinterpret_cast<const uint4*>(src + i * 32)); hi = __ldca(reinterpret_cast<const uint4*>(src + i * 32 + 16)); }
+        }
+        v[8 * i] = lo.x; v[8 * i + 1] = lo.y; v[8 * i + 2] = lo.z; v[8 * i + 3] = lo.w;
+        v[8 * i + 4] = hi.x; v[8 * i + 5] = hi.y; v[8 * i + 6] = hi.z; v[8 * i + 7] = hi.w;
       }
       tmem_st_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (g * LT_TMEM_KB + kb) * 32, v);
     }

@@ -290,3 +290,23 @@ def test_stack_cut_or_not_and_under_capture(T, B, H, cut):
         torch.cuda.synchronize()
         assert torch.equal(out, want)
     assert g.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("H", [32, 96, 256, 416, 512])
+def test_recurrence_reads_w_hh_at_any_16_byte_alignment(H):
+    """W_hh is read in 32-byte sectors where base and row stride allow it and in 16-byte pieces elsewhere: the same bytes.  What
+    lies beside the rows must not matter."""
+    g = need_lib()
+    gen = torch.Generator().manual_seed(H)
+    T, B = 9, 70
+    L = cuda_layer(make_layer(gen, H, 64))
+    ih = (torch.randn(T * B, 4 * H, generator=gen) * 0.5).half().cuda()
+    want = g.lstm_layer(ih, L["W_hh"], L["s_hh"], T, B, bias=L["b"], want_c=True)
+    for offset, pad in ((0, 16), (16, 16), (16, 32), (0, 32)):
+        buf = torch.full((4 * H, H + 64), 0x7E, dtype=torch.uint8, device="cuda").view(-1)[offset:offset + 4 * H * (H + pad)].view(4 * H, H + pad)
+        W = buf.view(torch.float8_e4m3fn)[:, :H]
+        W.copy_(L["W_hh"])
+        got = g.lstm_layer(ih, W, L["s_hh"], T, B, bias=L["b"], want_c=True)
+        for a, b in zip(got, want):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8)), (offset, pad)
+    assert g.device_status()[0] == 0
