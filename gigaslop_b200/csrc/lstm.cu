@@ -309,7 +309,7 @@ lstm_recurrent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 // B = 512, H = 384: 1.11 us per step (2.57 with the 128-row tiles), H = 512: 1.74 (4.8), H = 256: 0.80 (2.29), H = 128: 0.54 (2.27).
 // It was 1.34 / 1.93 / 0.93 / 0.57 before three changes to how its warps wait and issue.  An MMA warp walks its loop converged, with
 // one elected lane issuing (a single thread moves the operands of every MMA to uniform registers): 1.22 / 1.84 / 0.84 / 0.56.  The
-// gate warps report to it through a named barrier instead of an mbarrier: 1.21 / 1.84 / 0.83 / 0.56.  The waits on the chain, for the
+// gate warps report to it through named barriers instead of an mbarrier: 1.21 / 1.84 / 0.83 / 0.56.  The waits on the chain, for the
 // accumulators and for the other CTAs' h, do not suggest to the hardware how long to stay suspended: the rest.
 // The K blocks are summed in ascending order on every CTA.  Starting with the CTA's own block, which is there first, takes
 // 1.25 us at H = 384 and 1.81 at H = 512, but sums in an order that depends on the CTA: the last bit of a sum changes, an E4M3
@@ -372,7 +372,16 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const int H = p.H, B = p.B;
   const int kb_tmem = p.k_blocks < LT_TMEM_KB ? p.k_blocks : LT_TMEM_KB;
   constexpr uint32_t PIECE_BYTES = G * LT_HS;      // of h, from one CTA
-  // gate warps -> MMA warps, once per step but the last: this CTA's piece of h is in the buffer, its accumulators have been read
+  // gate warps -> MMA warps, once per step but the last: this CTA's piece of h is in the buffer, its accumulators have been read.
+  // The MMA warps wait without a limit, so an exit has to keep to this:
+  //  * a gate warp that gives up in step s reports for step s, then leaves; an MMA warp that gives up in step s, its barrier passed,
+  //    arrives for the reports of step s, which it would have waited for next, and sets the abort flag before
+  //  * whoever reports for step s has seen the barrier of step s - 2 complete (a gate warp mma_done of step s - 1, an MMA warp the
+  //    barrier itself), but not that of step s - 1.  So two barriers take turns: with one, a gate warp's report for a step it gives up in
+  //    could complete the step before in place of a warp that has yet to arrive, and leave that one waiting for good
+  //  * nobody waits for a report that does not come: let s be the first step a gate warp gives up in.  All report for step s, and an
+  //    MMA warp past that barrier finds the abort flag before it gets to the next.
+  // (us for 300 steps, one barrier / two / an mbarrier: B = 64, H = 384 245 / 246 / 257, H = 256 205 / 209 / 216, H = 64 165 / 170 / 168.)
   constexpr int OWN_READY = 1, OWN_THREADS = 32 * (CW + 4);
 
   if (tid == 0) {
@@ -493,7 +502,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       // ih + bias of this step, before the accumulators are there
       bool ok = mbar_wait(&ih_full[st], st_ph, abort_flag, ST_TIMEOUT_LSTM, 0x20, budget);
       if (!__all_sync(0xffffffffu, ok)) {            // (the MMA warps wait for this warp's report, whatever became of it)
-        if (s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
+        if (s + 1 < p.T) named_arrive<OWN_THREADS>(OWN_READY + (s & 1));
         break;
       }
       float2 x[4][RPT / 2];
@@ -511,7 +520,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 
       ok = mbar_wait<true>(mma_done, s & 1, abort_flag, ST_TIMEOUT_LSTM, 0x30, budget);
       if (!__all_sync(0xffffffffu, ok)) {
-        if (s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
+        if (s + 1 < p.T) named_arrive<OWN_THREADS>(OWN_READY + (s & 1));
         break;
       }
       tc_fence_after();
@@ -556,7 +565,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         if (hf == 1) {
           fence_proxy_async_smem(); tc_fence_before();                       // the stores above before this CTA's MMAs read them
           __syncwarp();
-          if (s + 1 < p.T) named_arrive<OWN_READY, OWN_THREADS>();
+          if (s + 1 < p.T) named_arrive<OWN_THREADS>(OWN_READY + (s & 1));
         }
       }
       // the layer's outputs, off the critical path: 32 (E4M3) / 64 (fp16) contiguous bytes per warp and row
@@ -592,7 +601,8 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     bool ok = rank_ok;
     int st = 0;
     if (ok && p.slices > LT_TMEM_KB) ok = __all_sync(0xffffffffu, mbar_wait(w_full, 0, abort_flag, ST_TIMEOUT_LSTM, 0x10, budget));
-    // The loop exists once per (row group size, rank): every descriptor offset is a constant of straight-line code.
+    // The loop exists once per (row group size, rank): every descriptor offset is a constant of straight-line code.  Returns the step
+    // it gave up in, or -1.
     auto run = [&](auto slices_tag, auto rank_tag) {
       constexpr int SLICES = decltype(slices_tag)::value, RANK = decltype(rank_tag)::value;
       for (int s = 0; s < p.T; ++s) {
@@ -600,7 +610,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         const uint32_t ph = (uint32_t)((s - 1) >> 1) & 1u;
         // (the accumulators may be overwritten and this CTA's piece read once every gate warp has reported)
         __syncwarp();
-        if (s > 0) named_sync<OWN_READY, OWN_THREADS>();
+        if (s > 0) named_sync<OWN_THREADS>(OWN_READY + hb);
         tc_fence_after();
         const uint64_t b = hb ? b_base[1] : b_base[0];
         // K blocks in ascending order on every CTA (the order of the sums is part of the result), each as soon as its piece
@@ -609,7 +619,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         for (int kb = 0; kb < SLICES; ++kb) {
           if (kb != RANK && s > 0) {               // another CTA's piece
             uint64_t* bar = &h_ready[hb * LT_MAX_SLICES + kb];
-            if (!__all_sync(0xffffffffu, mbar_wait_cluster(bar, ph, abort_flag, ST_TIMEOUT_LSTM, 0x41, budget))) return false;
+            if (!__all_sync(0xffffffffu, mbar_wait_cluster(bar, ph, abort_flag, ST_TIMEOUT_LSTM, 0x41, budget))) return s;
             if (g == 0 && lane == 0 && s + 2 < p.T) mbar_arrive_expect_tx(bar, PIECE_BYTES);   // its next use: h_{s+1}, read by step s + 2
             fence_proxy_async_smem();              // the peer's stores before the MMAs read them
           }
@@ -626,14 +636,14 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           }
         }
         umma_commit_elect(mma_done);
-        if (__any_sync(0xffffffffu, abort_flag.get())) return false;     // (a gate warp that gave up has reported all the same)
+        if (__any_sync(0xffffffffu, abort_flag.get())) return s;
         // the gate warps have read the ih tile of step s - 1 (their reports above came after that): its stage is free
         if (g == 3 && s > 0) {
           if (lane == 0 && s - 1 + LT_STAGES < p.T) issue_ih(s - 1 + LT_STAGES, st);
           if (++st == LT_STAGES) st = 0;
         }
       }
-      return true;
+      return -1;
     };
     auto run_rank = [&](auto slices_tag) {
       constexpr int SLICES = decltype(slices_tag)::value;
@@ -642,16 +652,17 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if constexpr (SLICES > 1) if (slc == 1) return run(slices_tag, std::integral_constant<int, 1>{});
       return run(slices_tag, std::integral_constant<int, 0>{});
     };
+    int gave_up = ok ? -1 : 0;
     if (ok) {
-      if (p.slices == 1) ok = run_rank(std::integral_constant<int, 1>{});
-      else if (p.slices == 2) ok = run_rank(std::integral_constant<int, 2>{});
-      else if (p.slices == 3) ok = run_rank(std::integral_constant<int, 3>{});
-      else ok = run_rank(std::integral_constant<int, 4>{});
+      if (p.slices == 1) gave_up = run_rank(std::integral_constant<int, 1>{});
+      else if (p.slices == 2) gave_up = run_rank(std::integral_constant<int, 2>{});
+      else if (p.slices == 3) gave_up = run_rank(std::integral_constant<int, 3>{});
+      else gave_up = run_rank(std::integral_constant<int, 4>{});
     }
-    if (!ok) {                                     // (an MMA warp that still runs finds the abort flag after its next barrier)
+    if (gave_up >= 0) {                            // (before the loop: as in step 0)
       if (lane == 0) abort_flag.set(1);
       __syncwarp();
-      named_arrive<OWN_READY, OWN_THREADS>();
+      named_arrive<OWN_THREADS>(OWN_READY + (gave_up & 1));
       if (lane == 0) {                             // loads in flight land before the CTA exits
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000) { }

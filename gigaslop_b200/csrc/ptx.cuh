@@ -1,8 +1,9 @@
 // Thin inline-PTX wrappers for the sm_100a features the kernels use:
 // mbarrier, TMA (cp.async.bulk.tensor, never with cluster multicast), tcgen05
 // (TMEM allocation, UMMA issue/commit, TMEM loads) and the proxy fences between
-// them.  Every wait is bounded: a wait that gives up records a code in the
-// device status word and lets the kernel unwind instead of spinning forever.
+// them.  Every wait on an mbarrier is bounded: a wait that gives up records a code in the
+// device status word and lets the kernel unwind instead of spinning forever.  Hardware barriers
+// (__syncthreads, named, cluster) have no limit; every warp arrives at them on every way out.
 #pragma once
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -47,11 +48,12 @@ struct AbortFlag {
 
 // ---- named barriers ------------------------------------------------------------
 // A hand-over between warps of a CTA: N threads in all, some of which only arrive.  Executed by converged warps.  The waiting is
-// not bounded: every warp that others wait for arrives on its way out, too, however it came to leave.
-template <int ID, int N>
-__device__ __forceinline__ void named_arrive() { asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
-template <int ID, int N>
-__device__ __forceinline__ void named_sync() { asm volatile("barrier.cta.sync.aligned %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
+// not bounded: every warp that others wait for arrives on its way out, too, however it came to leave, and never twice before a
+// barrier is complete (the extra arrival would stand in for a missing one, whose warp then waits for good).
+template <int N>
+__device__ __forceinline__ void named_arrive(int id) { asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(id), "n"(N) : "memory"); }
+template <int N>
+__device__ __forceinline__ void named_sync(int id) { asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 
 // ---- programmatic dependent launch --------------------------------------------
 // The kernels that follow one another in a stream are launched with programmatic stream serialization (launch_dependent):
