@@ -14,6 +14,7 @@
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/record_function.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -63,10 +64,11 @@ struct Call {
   gsb200_stream_t stream() const { return c10::cuda::getCurrentCUDAStream(device.index()).stream(); }
   // An output.  torch's own CUDA allocation function directly: the way to it through the dispatcher is most of what at::empty
   // costs.  The dispatcher is asked where something may want to see the call: dispatch keys switched on for this
-  // thread (functorch, tracing), or the deterministic mode, in which at::empty fills its result.
+  // thread (functorch, tracing), observers of operator calls (a profiler), or the deterministic mode, in which at::empty
+  // fills its result.
   at::Tensor empty(at::IntArrayRef size, at::ScalarType dt) const {
     const c10::DispatchKeySet on = c10::impl::tls_local_dispatch_key_set().included_;
-    if ((on - c10::default_included_set).empty() && !at::globalContext().deterministicAlgorithms())
+    if ((on - c10::default_included_set).empty() && !at::hasCallbacks() && !at::globalContext().deterministicAlgorithms())
       return at::Tensor(at::detail::empty_cuda(size, dt, device, std::nullopt));
     return at::empty(size, at::TensorOptions().device(device).dtype(dt));
   }

@@ -290,3 +290,15 @@ def test_outputs_are_what_torch_empty_makes():
         torch.use_deterministic_algorithms(False)
     e, se = g.quantize_tensor(x[:0])
     assert e.shape == (0, 512) and se.shape == (0,)
+
+
+@pytest.mark.gpu
+def test_a_profiler_sees_the_outputs_allocated():
+    """Under a profiler of operator calls the outputs come through the dispatcher, so a trace shows them as torch.empty's."""
+    g = need_lib()
+    x = torch.randn(300, 512, generator=torch.Generator().manual_seed(2)).half().cuda()
+    want = g.quantize_tensor(x)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        got = g.quantize_tensor(x)
+    assert sum(e.count for e in prof.key_averages() if e.key == "aten::empty") == 2
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
