@@ -779,13 +779,17 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
     return tmap_2d(m, dt, esz, base, rows, cols, ld, bc, br, sw);
   };
   CUtensorMap ta, tb0, tb1, tc;
-  const uint32_t brows = dual ? 64 : 128;
-  bool ok = map2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B);
-  ok = ok && map2d(&tb0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, brows, CU_TENSOR_MAP_SWIZZLE_128B);
-  ok = ok && map2d(&tb1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dual ? B1 : B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, brows, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (!map2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return GSB200_ERR_BAD_ARG;
+  // W in boxes of `rows` rows, the output in 32 x 32 boxes
+  auto map_w = [&](uint32_t rows) {
+    if (!map2d(&tb0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, rows, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
+    if (!dual) { tb1 = tb0; return true; }
+    return map2d(&tb1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B1, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, rows, CU_TENSOR_MAP_SWIZZLE_128B);
+  };
+  auto map_c = [&]() {
+    return map2d(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+  };
   const bool wst = K / MX_BK <= MXW_MAX_KB && (N + (dual ? 64 : 128) - 1) / (dual ? 64 : 128) <= sm_count();
-  ok = ok && map2d(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
-  if (!ok) return GSB200_ERR_BAD_ARG;
   MxParams p{};
   p.M = (int)M; p.N = N; p.K = K;
   const int out_cols = dual ? 64 : 128;
@@ -808,20 +812,18 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
     const long long r256 = g256 > 0 ? (p.m_blocks + g256 - 1) / g256 : 0;
     const bool better = g128 > 0 ? r256 * 15 < (p.m_blocks + g128 - 1) / g128 * 10ll : r256 * (dual ? 25 : 30) < (tiles + sms - 1) / sms * 20;
     if (g256 > 0 && better) {
-      CUtensorMap tw0, tw1, to;
-      if (!map2d(&tw0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
-          !map2d(&tw1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, dual ? B1 : B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
-          !map2d(&to, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B))
+      if (!map_w(128) || !map2d(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B))
         return GSB200_ERR_BAD_ARG;
       p.n_blocks = nb;
       p.n_groups = g256 < p.m_blocks ? g256 : p.m_blocks;
       const int grid = p.n_groups * nb;
-      e = dual ? launch_dependent(mx_gemm256w_kernel<true>, grid, MX_THREADS, MXV_BYTES, st, ta, tw0, tw1, to, p)
-               : launch_dependent(mx_gemm256w_kernel<false>, grid, MX_THREADS, MXV_BYTES, st, ta, tw0, tw1, to, p);
+      e = dual ? launch_dependent(mx_gemm256w_kernel<true>, grid, MX_THREADS, MXV_BYTES, st, ta, tb0, tb1, tc, p)
+               : launch_dependent(mx_gemm256w_kernel<false>, grid, MX_THREADS, MXV_BYTES, st, ta, tb0, tb1, tc, p);
       return cuda_status(e, "mx gemm launch");
     }
   }
   if (wst) {                                                        // weight-stationary form
+    if (!map_w(dual ? 64 : 128) || !map_c()) return GSB200_ERR_BAD_ARG;
     int groups = sm_count() / p.n_blocks;
     if (groups > p.m_blocks) groups = p.m_blocks;
     p.n_groups = groups;
@@ -834,13 +836,12 @@ int32_t launch_mx_gemm(bool dual, const uint8_t* A, long long lda, const uint8_t
   // tiles and an N just above a multiple of 256 stay with 128 (M = 65536, N = 384, K = 1536: 45.1 us, with 256 columns 46.3).
   const long long sms = sm_count(), tiles256 = (long long)p.m_blocks * ((N + MX2_BN - 1) / MX2_BN);
   if (!dual && (tiles256 + sms - 1) / sms * 33 < (tiles + sms - 1) / sms * 20 && tiles256 <= 0x7fffffffll) {
-    CUtensorMap tb;
-    if (!map2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, B0, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128, MX2_BN, CU_TENSOR_MAP_SWIZZLE_128B))
-      return GSB200_ERR_BAD_ARG;
+    if (!map_w(MX2_BN) || !map_c()) return GSB200_ERR_BAD_ARG;
     p.n_blocks = (N + MX2_BN - 1) / MX2_BN;
-    e = launch_dependent(mx_gemm256_kernel, (int)(tiles256 < sms ? tiles256 : sms), MX_THREADS, MX2_BYTES, st, ta, tb, tc, p);
+    e = launch_dependent(mx_gemm256_kernel, (int)(tiles256 < sms ? tiles256 : sms), MX_THREADS, MX2_BYTES, st, ta, tb0, tc, p);
     return cuda_status(e, "mx gemm launch");
   }
+  if (!map_w(dual ? 64 : 128) || !map_c()) return GSB200_ERR_BAD_ARG;
   const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
   if (dual) e = launch_dependent(mx_gemm_kernel<true, false>, grid, MX_THREADS, MxSmem<false>::BYTES, st, ta, tb0, tb1, tc, p);
   else e = launch_dependent(mx_gemm_kernel<false, false>, grid, MX_THREADS, MxSmem<false>::BYTES, st, ta, tb0, tb1, tc, p);

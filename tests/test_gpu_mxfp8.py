@@ -216,3 +216,20 @@ def test_block_scaled_gemm_of_many_column_slices(dual, N, M, form):
         ref = g.dual_gemm_mxfp8_silu(a, ta, part(w), part(u), tiled(sw), tiled(su)) if dual else g.gemm_mxfp8(a, ta, part(w), tiled(sw))
         assert_bitexact(out[:, lo:hi], ref, f"columns {lo}:{hi}")
     assert g.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("dual,M,N,K,maps", [(False, 1024, 2048, 512, 3), (True, 1024, 2048, 512, 4), (False, 128, 2048, 512, 3), (True, 128, 2048, 512, 4),
+                                             (False, 20000, 512, 1024, 3), (True, 300, 512, 1024, 4)])
+def test_a_block_scaled_call_encodes_the_maps_it_uses(dual, M, N, K, maps):
+    """On buffers not seen before: one tensor map each for A, a weight and the output, whichever kernel runs."""
+    g = need_lib()
+    gen = torch.Generator(device="cuda").manual_seed(M + N + K)
+    def mx(n):
+        q, s = g.mxfp8_quantize(torch.randn(n, K, generator=gen, device="cuda").half())
+        return q, g.mx_scales_to_tiled(s, K)
+    (a, ta), (w, tw), (u, tu) = mx(M), mx(N), mx(N)
+    out = torch.empty(M, N + 8 * (1 + dual), dtype=torch.float16, device="cuda")[:, :N]       # (a stride of this test's own)
+    a, w, u = [torch.empty(t.shape[0], K + 16 * (3 + dual), dtype=t.dtype, device="cuda")[:, :K].copy_(t) for t in (a, w, u)]
+    n0 = int(g.lib().gsb200_tensor_map_encodes())
+    g.dual_gemm_mxfp8_silu(a, ta, w, u, tw, tu, out=out) if dual else g.gemm_mxfp8(a, ta, w, tw, out=out)
+    assert int(g.lib().gsb200_tensor_map_encodes()) - n0 == maps
