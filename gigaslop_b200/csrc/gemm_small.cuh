@@ -70,6 +70,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   const AbortFlag abort_flag{smem_u32(tmem_slot + 1)};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if ((smem_u32(sg_smem) & 1023u) != 0) {              // (cannot happen: the swizzled tiles need it)
+    if (threadIdx.x == 0) atomicOr(&g_status[0], ST_TIMEOUT_MMA);
+    return;
+  }
 
   const int m0 = (int)(blockIdx.x / p.n_tiles) * TM, tn = (int)(blockIdx.x % p.n_tiles);
   int n0, n1;                                          // first W row (= output column) of the two parts
@@ -294,7 +298,7 @@ static long long small_gemm_tiles(const GemmArgs& a, int tm, int npart) {
 }
 
 template <int KIND, int EPI, int TM, int NPART>
-static int32_t launch_small_inst(const GemmArgs& a, const SgParams& p, int grid, int dev, const CUtensorMap& ta, const CUtensorMap& tb0,
+static int32_t launch_small_inst(const SgParams& p, int grid, int dev, const CUtensorMap& ta, const CUtensorMap& tb0,
                                  const CUtensorMap& tb1, cudaStream_t st) {
   static std::atomic<int> attr_done[64];
   auto k = gemm_small_kernel<KIND, EPI, TM, NPART>;
@@ -310,14 +314,14 @@ template <int KIND>
 static int32_t launch_small_kind(const GemmArgs& a, int tm, int npart, const SgParams& p, int grid, int dev, const CUtensorMap& ta, const CUtensorMap& tb0,
                                  const CUtensorMap& tb1, cudaStream_t st) {
   switch (a.epi) {
-    case EPI_DEQUANT: return tm == 64 ? launch_small_inst<KIND, EPI_DEQUANT, 64, 32>(a, p, grid, dev, ta, tb0, tb1, st)
-                                      : launch_small_inst<KIND, EPI_DEQUANT, 128, 64>(a, p, grid, dev, ta, tb0, tb1, st);
-    case EPI_ROTARY: return launch_small_inst<KIND, EPI_ROTARY, 64, 32>(a, p, grid, dev, ta, tb0, tb1, st);
-    case EPI_SILU: return tm == 128 ? launch_small_inst<KIND, EPI_SILU, 128, 64>(a, p, grid, dev, ta, tb0, tb1, st)
-                        : npart == 32 ? launch_small_inst<KIND, EPI_SILU, 64, 32>(a, p, grid, dev, ta, tb0, tb1, st)
-                                      : launch_small_inst<KIND, EPI_SILU, 64, 64>(a, p, grid, dev, ta, tb0, tb1, st);
+    case EPI_DEQUANT: return tm == 64 ? launch_small_inst<KIND, EPI_DEQUANT, 64, 32>(p, grid, dev, ta, tb0, tb1, st)
+                                      : launch_small_inst<KIND, EPI_DEQUANT, 128, 64>(p, grid, dev, ta, tb0, tb1, st);
+    case EPI_ROTARY: return launch_small_inst<KIND, EPI_ROTARY, 64, 32>(p, grid, dev, ta, tb0, tb1, st);
+    case EPI_SILU: return tm == 128 ? launch_small_inst<KIND, EPI_SILU, 128, 64>(p, grid, dev, ta, tb0, tb1, st)
+                        : npart == 32 ? launch_small_inst<KIND, EPI_SILU, 64, 32>(p, grid, dev, ta, tb0, tb1, st)
+                                      : launch_small_inst<KIND, EPI_SILU, 64, 64>(p, grid, dev, ta, tb0, tb1, st);
     default:
-      if constexpr (KIND == KIND_F8) return launch_small_inst<KIND_F8, EPI_SILU_MX, 64, 64>(a, p, grid, dev, ta, tb0, tb1, st);
+      if constexpr (KIND == KIND_F8) return launch_small_inst<KIND_F8, EPI_SILU_MX, 64, 64>(p, grid, dev, ta, tb0, tb1, st);
       return GSB200_ERR_BAD_ARG;
   }
 }

@@ -31,3 +31,18 @@ def test_twelve_warp_gemm_register_pool_covers_its_resplit():
     for name, v in res.items():
         assert 512 * v["registers"] >= 128 * 56 + 384 * 152, (name, v)
         assert 512 * v["registers"] <= 65536, (name, v)
+
+
+def test_every_kernel_with_dynamic_shared_memory_sees_to_its_alignment():
+    """128-byte-swizzled tiles need a base that is a multiple of 1 KiB; dynamic shared memory is not promised to have one.  Every
+    kernel rounds its base up or checks it before it uses it."""
+    import glob
+    import os
+    from gigaslop_b200 import build
+    found = 0
+    for path in sorted(glob.glob(os.path.join(build.PKG, "csrc", "*.cu*"))):
+        for part in open(path).read().split("extern __shared__")[1:]:
+            found += 1
+            head = part[:part.index("__syncthreads")]
+            assert "+ 1023) & ~uintptr_t(1023)" in head or "& 1023u) != 0" in head, (os.path.basename(path), part[:60])
+    assert found >= 10
