@@ -170,12 +170,18 @@ def test_dual_silu_mxfp8_epilogue_forms_agree(M, N, K):
     assert g.device_status()[0] == 0
 
 
-@pytest.mark.parametrize("dual", [True, False])
-@pytest.mark.parametrize("M,N,K", [(9001, 2080, 512), (20000, 544, 384), (40000, 160, 128), (19000, 288, 256)])
-def test_block_scaled_weight_stationary_256_column_tiles(dual, M, N, K):
-    """Many row blocks run on 256-column weight-stationary tiles; a slice of two row blocks (one round) on 128-column ones.  Rows
-    are independent, so the slices must give the same bytes: ragged last tiles in M and N (half of a column tile, one without
-    scale tiles), one to four K blocks through the ring of four."""
+# (which of these the 256-column tiles take on 148 SMs; M = 9001 leaves a row block of 41 rows, M = 3001 one of 57)
+FORM_256W = [(True, 9001, 2080, 512, True), (True, 20000, 544, 384, True), (True, 40000, 160, 128, False), (True, 19000, 288, 256, False),
+             (False, 9001, 2080, 512, True), (False, 20000, 544, 384, False), (False, 40000, 160, 128, True), (False, 19000, 288, 256, False)]
+FORM_256W += [(True, m, n, k, True) for k in (128, 256, 384, 512) for m, n in ((9001, 160), (3001, 544))]
+FORM_256W += [(False, m, n, k, True) for k in (128, 256, 384, 512) for m, n in ((9001, 288), (3001, 800))]
+
+
+@pytest.mark.parametrize("dual,M,N,K,wide", FORM_256W)
+def test_block_scaled_weight_stationary_256_column_tiles(dual, M, N, K, wide):
+    """Many row blocks run on 256-column weight-stationary tiles where their rounds are cheaper; a slice of two row blocks (one
+    round) on 128-column ones.  Rows are independent, so the slices must give the same bytes: ragged last tiles in M and N (half
+    of a column tile, one without scale tiles), one to four K blocks through the ring of four."""
     g = need_lib()
     gen = torch.Generator(device="cuda").manual_seed(M + N + K)
     def mx(n):
@@ -184,6 +190,10 @@ def test_block_scaled_weight_stationary_256_column_tiles(dual, M, N, K):
     (a, sa, ta), (w, _, tw), (u, _, tu) = mx(M), mx(N), mx(N)
     run = (lambda x, t: g.dual_gemm_mxfp8_silu(x, t, w, u, tw, tu)) if dual else (lambda x, t: g.gemm_mxfp8(x, t, w, tw))
     got = run(a, ta)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        few, tf = a[:256].contiguous(), g.mx_scales_to_tiled(sa[:256].contiguous(), K)
+        assert [("mx_gemm256w" in n) for n, _ in launches(lambda: run(a, ta))] == [wide]
+        assert [("mx_gemm256w" in n) for n, _ in launches(lambda: run(few, tf))] == [False]
     for lo in (0, M // 2 // 128 * 128, (M - 1) // 128 * 128 - 128):
         hi = min(M, lo + 256)
         assert_bitexact(got[lo:hi], run(a[lo:hi].contiguous(), g.mx_scales_to_tiled(sa[lo:hi].contiguous(), K)), f"rows {lo}:{hi}")
