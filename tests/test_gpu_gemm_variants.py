@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import oracle
-from util import assert_bitexact, f16_equal_up_to_signed_zero, need_lib, rand_i8, rand_scales
+from util import assert_bitexact, f16_equal_up_to_signed_zero, launches, need_lib, rand_i8, rand_scales
 
 pytestmark = pytest.mark.gpu
 
@@ -146,4 +146,28 @@ def test_both_sides_of_the_lines_between_the_forms(force, op, row_blocks, K):
     got = run()
     force(8, 0)
     assert_bitexact(got, run())
+    assert g.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("row_blocks,N,K,warps", [(47, 1536, 384, 8), (48, 1536, 384, 12), (47, 1024, 128, 8), (48, 1024, 128, 12), (159, 512, 512, 8),
+                                                  (160, 512, 512, 12), (47, 256, 384, 0), (48, 256, 128, 0)])
+def test_swiglu_lines_between_eight_and_twelve_warps(force, row_blocks, N, K, warps):
+    """Which kernel a SwiGLU takes either side of its lines (0: a narrow one, few tiles of 128 x 64, never gets to them), and that
+    the bytes are those of eight warps."""
+    g = need_lib()
+    M = 128 * row_blocks - 5
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    i8 = lambda n: torch.randint(-127, 128, (n, K), generator=gen, device="cuda", dtype=torch.int8)
+    sc = lambda n: torch.rand(n, generator=gen, device="cuda") * 1e-2 + 1e-3
+    A, sa, G, U, sg, su = i8(M), sc(M), i8(N), i8(N), sc(N) * 1e-2, sc(N)
+    out = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    run = lambda: g.dual_gemm_i8_silu(A, G, U, sa, sg, su, out=out)
+    run()
+    got = out.clone()
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        names = [n for n, _ in launches(run)]
+        assert len(names) == 1 and ("gemm_small" if warps == 0 else f"Li{warps}EEEv14CUtensorMap") in names[0], names
+    force(8, 0)
+    run()
+    assert_bitexact(got, out)
     assert g.device_status()[0] == 0
