@@ -62,7 +62,7 @@ def test_dequant(fp8, M, N, K):
 
 
 @pytest.mark.parametrize("fp8", [False, True])
-@pytest.mark.parametrize("M,N,K", [(1, 8, 16), (64, 32, 128), (65, 72, 512), (200, 2048, 512), (330, 1000, 2048), (700, 1544, 384), (1001, 2040, 512)])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 16), (64, 32, 128), (65, 72, 512), (200, 2048, 512), (330, 1000, 2048), (700, 1544, 384), (1001, 2040, 512), (700, 2040, 1024), (570, 2040, 1040)])
 def test_swiglu(fp8, M, N, K):
     g = need_lib()
     gen = torch.Generator().manual_seed(M + 5 * N + 7 * K)
@@ -90,7 +90,7 @@ def test_swiglu_few_tile_form_by_k(M, K, kernel):
     assert len(names) == 1 and kernel in names[0], names
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 32, 128), (65, 96, 512), (200, 2048, 512), (500, 1056, 2048)])
+@pytest.mark.parametrize("M,N,K", [(1, 32, 128), (65, 96, 512), (200, 2048, 512), (500, 1056, 2048), (500, 2048, 2048), (590, 1056, 1024)])
 def test_swiglu_to_mxfp8(M, N, K):
     g = need_lib()
     gen = torch.Generator().manual_seed(M + 5 * N + 7 * K)
@@ -147,3 +147,29 @@ def test_scalar_and_absent_scales_and_a_capped_grid():
         assert_bitexact(g.fp8_down_proj(A, sa, B, sb), c.contiguous())
     finally:
         assert g.lib().gsb200_set_sm_limit(0) == 0
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("with_a,with_b", [(False, True), (True, False), (False, False)])
+@pytest.mark.parametrize("M,N,K", [(65, 72, 144), (3000, 512, 512), (4700, 512, 512)])
+def test_null_scales_count_as_one(fp8, with_a, with_b, M, N, K):
+    """The C entry points take null for either scale of a plain GEMM: 64-row and 128-row tiles against the persistent kernel, and the
+    products against exact sums."""
+    g = need_lib()
+    gen = torch.Generator().manual_seed(M + N)
+    draw = lambda n: torch.randint(-3, 4, (n, K), generator=gen, dtype=torch.int8)
+    A, B = draw(M), draw(N)
+    sa, sb = rand_scales(gen, M, 0.5, 2.0).cuda(), rand_scales(gen, N, 0.5, 2.0).cuda()
+    Ac, Bc = (t.to(torch.float8_e4m3fn).cuda() if fp8 else t.cuda() for t in (A, B))
+    entry = g.lib().gsb200_gemm_fp8_f16 if fp8 else g.lib().gsb200_gemm_i8_f16
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(out):
+        assert entry(Ac.data_ptr(), Ac.stride(0), Bc.data_ptr(), Bc.stride(0), out.data_ptr(), out.stride(0), sa.data_ptr() if with_a else None,
+                     sb.data_ptr() if with_b else None, M, N, K, 0, stream) == 0
+    c = both(call, M, N)
+    acc = A.cuda().float() @ B.cuda().float().t()
+    assert float(acc.abs().max()) < 2 ** 15                # (whole numbers, exact in fp32)
+    ref = acc.double() * (sa.double()[:, None] if with_a else 1) * (sb.double() if with_b else 1)
+    # two products in fp32 and one rounding to fp16
+    assert bool(((c.double() - ref).abs() <= ref.abs() * (2 ** -11 + 2 ** -22)).all())
