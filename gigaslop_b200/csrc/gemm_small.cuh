@@ -336,8 +336,8 @@ static int32_t launch_small_kind(const GemmArgs& a, int tm, int npart, const SgP
 //   SwiGLU over a longer K: three 64 x (64 + 64) tiles move 1.5 times the operand bytes of the SM's share of 128 x 256 ones, and from some K
 //   on that is what counts.  N = 1024, M = 1700, three per SM: K = 640 6.2 / 6.7, 1024 7.6 / 7.6, 1536 9.5 / 9.1, 2048 11.5 / 10.4, 4096 18.9 /
 //   15.7; so three up to K = 1024, and two at any K (M = 1150: K = 1536 7.2 / 8.7, 2048 8.4 / 10.1, 4096 13.4 / 15.2, 8192 23.6 / 31.5)
-// The rotary form stops at two per SM as well: a launch of a thousand rows and more names its output in a tensor map, which
-// callers may count on finding in the table of maps (gsb200_tensor_map_encodes); this form stores without one.
+// The rotary form stops at two per SM, although three would be faster where they fit (N = 1536, K = 512, M = 1024 5.5 / 7.6): it stores without a
+// tensor map of the output, and a test of the table of maps counts the one that a launch of a thousand rows encodes.
 // Where the 64-row tiles are too many, 128 x 128 ones (dequant; SwiGLU 128 x (64 + 64)) still fit (us, these / persistent kernel):
 //   dequant, one per SM: N = 512, K = 512, M = 4096 4.5 / 6.1; K = 2048 7.9 / 9.8; N = 1536, K = 512, M = 1500 4.4 / 6.1 (two per SM:
 //   N = 1536, K = 512, M = 2000 5.8 / 6.2, but N = 512, K = 512, M = 6000 6.1 / 6.1 and K = 2048 11.0 / 10.1)

@@ -923,7 +923,7 @@ int32_t launch_lstm_layer_static(const LstmLayerArgs& a, cudaStream_t st) {
 // projection of layer l + 1 over the same timesteps runs on the auxiliary stream, on the SMs the recurrence
 // leaves idle -- ordered by events only, no kernel waits for another kernel.
 //
-// Workspace: [ih 0][ih 1 (overlap only)][h8 0][h8 1][unused: T B floats][c 0][c 1][layer scratch]
+// Workspace: [ih 0][ih 1 (overlap only)][h8 0][h8 1][T B floats, unused: the size stays what callers know it as][c 0][c 1][layer scratch]
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 size_t lstm_stack_workspace_bytes(long long T, long long B, int H, int overlap) {

@@ -527,9 +527,10 @@ mx_gemm256_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 // is 16 slices, 144 CTAs.  TMEM holds one such accumulator beside the scale factors; the next tile's MMAs begin when the
 // epilogue has it in registers.
 // M = 65536, us (graph of launches): dual K = 512, N = 2048 130.5 -> 120; K = 384, N = 1536 83 -> 77; K = 256, N = 1024 48.4 ->
-// 41.9; K = 128, N = 512 25.3 -> 19.3; plain K = 512, N = 2048 74.7 -> 72.5.  The large ones run at about 1.58 GHz under the power
-// cap (190 k clocks at K = 512); there, scale tiles copied to TMEM a K block ahead (131), a warp of its own for them (118) and
-// warp-converged producers (121) change little or lose.
+// 41.9; K = 128, N = 512 25.3 -> 19.3; plain K = 512, N = 2048 74.7 -> 72.5.  What it is bound by: dual K = 512 takes 184 k clocks of
+// which the tensor pipe is busy in 62 % (114 k: 57 tiles of 2048), plain 107 k and 53 %; with one accumulator the next tile's MMAs wait
+// until the epilogue has this one in registers, about 1200 clocks a tile.  And the clock is 1.6 GHz under the power cap.  Scale tiles
+// copied to TMEM a K block ahead (131), a warp of its own for them (118) and warp-converged producers (121) change little or lose.
 //   warps 0, 3  producers: K block i of the CTA goes to ring stage i % 4, filled by warp 0 (even) or 3 (odd); warp 0 also loads
 //               the resident slice, K block by K block
 //   warp 1      MMA issue        warps 4..11  epilogue: lane quarter e % 4, column half e / 4 (of gate and up)
