@@ -306,11 +306,12 @@ lstm_recurrent_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 //  * the batch is the small dimension, so B = 512 spreads over 129 SMs (G = 12) instead of 48: the gate math, five
 //    special-function instructions per cell, is 1000 clocks for 2048 cells (G = 16), 600 for 1024.
 //  * W_hh in tensor memory: an MMA from a shared-memory A operand of 128 rows takes 40 clocks, from TMEM 16.
-// B = 512, H = 384: 1.11 us per step (2.57 with the 128-row tiles), H = 512: 1.74 (4.8), H = 256: 0.80 (2.29), H = 128: 0.54 (2.27).
-// It was 1.34 / 1.93 / 0.93 / 0.57 before three changes to how its warps wait and issue.  An MMA warp walks its loop converged, with
+// B = 512, H = 384: 1.03 us per step (2.57 with the 128-row tiles), H = 512: 1.74 (4.8), H = 256: 0.78 (2.29), H = 128: 0.54 (2.27).
+// It was 1.34 / 1.93 / 0.93 / 0.57 before four changes to how its warps wait and issue.  An MMA warp walks its loop converged, with
 // one elected lane issuing (a single thread moves the operands of every MMA to uniform registers): 1.22 / 1.84 / 0.84 / 0.56.  The
 // gate warps report to it through named barriers instead of an mbarrier: 1.21 / 1.84 / 0.83 / 0.56.  The waits on the chain, for the
-// accumulators and for the other CTAs' h, do not suggest to the hardware how long to stay suspended: the rest.
+// accumulators and for the other CTAs' h, do not suggest to the hardware how long to stay suspended: 1.12 / 1.73 /
+// 0.82 / 0.56.  The steps are unrolled by two (below): the rest.
 // The K blocks are summed in ascending order on every CTA.  Starting with the CTA's own block, which is there first, takes
 // 1.25 us at H = 384 and 1.81 at H = 512, but sums in an order that depends on the CTA: the last bit of a sum changes, an E4M3
 // rounding of h flips with it, and after five layers of 2000 steps the outputs differ by 5e-3.  There is a
@@ -381,7 +382,11 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   //    could complete the step before in place of a warp that has yet to arrive, and leave that one waiting for good
   //  * nobody waits for a report that does not come: let s be the first step a gate warp gives up in.  All report for step s, and an
   //    MMA warp past that barrier finds the abort flag before it gets to the next.
-  // (us for 300 steps, one barrier / two / an mbarrier: B = 64, H = 384 245 / 246 / 257, H = 256 205 / 209 / 216, H = 64 165 / 170 / 168.)
+  // Both loops over the steps are unrolled by two, so that which barrier and which buffer of h a step uses is a constant: the barriers
+  // in turn would cost up to 2.5 % otherwise, and the gate warps' and MMA warps' addresses are constants, too.  ns per step, B x H, one
+  // barrier / two / two and unrolled (gate warps alone, MMA warps alone): 512 x 384 1109 / 1118 / 1015 (1102, 1057), 64 x 384 772 / 774 / 687
+  // (750, 705), 512 x 256 815 / 823 / 764, 512 x 128 560 / 572 / 531, 70 x 128 550 / 561 / 528, 512 x 512 1746 / 1751 / 1738.  An mbarrier,
+  // whose wait has a limit: 4 % more than one barrier at H = 256 and 384.
   constexpr int OWN_READY = 1, OWN_THREADS = 32 * (CW + 4);
 
   if (tid == 0) {
@@ -498,6 +503,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     }
     const uint32_t snd_dst = sends ? mapa_shared(smem_u32(h_s), to) : 0u, snd_bar = sends ? mapa_shared(smem_u32(h_ready + slc), to) : 0u;
     int st = 0; uint32_t st_ph = 0;
+#pragma unroll 2
     for (int s = 0; s < p.T; ++s) {
       // ih + bias of this step, before the accumulators are there
       bool ok = mbar_wait(&ih_full[st], st_ph, abort_flag, ST_TIMEOUT_LSTM, 0x20, budget);
@@ -605,6 +611,7 @@ lstm_tmem_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     // it gave up in, or -1.
     auto run = [&](auto slices_tag, auto rank_tag) {
       constexpr int SLICES = decltype(slices_tag)::value, RANK = decltype(rank_tag)::value;
+#pragma unroll 2
       for (int s = 0; s < p.T; ++s) {
         const int hb = (s + 1) & 1;                // h_{s-1}
         const uint32_t ph = (uint32_t)((s - 1) >> 1) & 1u;
@@ -685,7 +692,9 @@ size_t lstm_scratch_bytes(long long B, int H) {
 
 using LtKernel = void (*)(const CUtensorMap, const CUtensorMap, const uint8_t*, long long, const LstmParams);
 // The forms of the transposed kernel: batch rows per group, and what a step takes (ns, measured on B200) on row groups of one
-// to four CTAs, i.e. at H = 128, 256, 384 and 512.  (16 rows at H = 384 as with 96 CTAs, B = 512; 1310 with 129.)
+// to four CTAs, i.e. at H = 128, 256, 384 and 512.  (16 rows at H = 384 as with 96 CTAs, B = 512; 1310 with 129.)  Measured before the loops were unrolled by two; now, all
+// SMs taken: 4 rows 540, 623, 697, 1131; 8 700, 775, 851, 1315; 12 767, 928, 1029, 1492; 16 1109, 1206, 1252, 1746; 32 1584, 1911, 2031, 2663.  Only the order
+// of the forms counts, and it is the same (but for 3 % at H = 256 with B past 1184).
 struct LtForm { int rows, threads, smem[LT_MAX_SLICES + 1], step_ns[LT_MAX_SLICES + 1]; LtKernel kernel; };
 template <int R, int G, int CW>
 static constexpr LtForm lt_make_form(int ns1, int ns2, int ns3, int ns4) {
@@ -738,8 +747,8 @@ static int lt_capacity(int form, int slices, int dev) {
 // projection beside it (0 = it has the whole GPU); -1 = none.  `max_ctas` only steers this choice, in which groups past it wait
 // for a next wave: a launch brings all its row groups, and where no form holds them in `max_ctas` CTAs they take more SMs
 // (lstm_layer_ctas counts what a launch does occupy).  Fewer rows per CTA make a shorter step as long as all groups are resident: B = 512, H = 384 takes 12 rows
-// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.06 us per step; 12 rows in two
-// waves 2.24).  *ns = the step.
+// (43 groups, 129 CTAs), B = 512, H = 512 16 rows (128 CTAs), B = 1024, H = 384 32 rows (2.03 us per step; 12 rows in two
+// waves 2.06).  *ns = the step.
 static int lt_choose(long long B, int H, int dev, int max_ctas, long long* ns = nullptr) {
   const int slices = (H + LT_HS - 1) / LT_HS;
   int best = -1;
@@ -795,8 +804,8 @@ static int lstm_layer_ctas(long long B, int H, int max_ctas) {
 
 // How many launches to cut a layer's recurrence into so that the next layer's projection runs beside it (1 = not at all).
 // The cut recurrence is steered to `max_ctas` CTAs, which may cost it a form with longer steps, and every launch about 12 us;
-// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 15.1 ms one after the other, 13.9
-// in five blocks; at B = 512, H = 512 (T = 1000, three layers) 6.8 ms against 8.1, so not cut.
+// it hides the projection up to the last block's.  Five layers, T = 2000, B = 512, H = 384: 14.3 ms one after the other, 13.4
+// to 14.0 in five blocks; at B = 512, H = 512 (T = 1000, three layers) 6.8 ms against 8.0, so not cut.
 static int lstm_time_blocks(long long T, long long B, int H, int max_ctas) {
   int dev = 0;
   cudaGetDevice(&dev);
