@@ -66,10 +66,13 @@ struct Call {
   // costs.  The dispatcher is asked where something may want to see the call: dispatch keys switched on for this
   // thread (functorch, tracing), observers of operator calls (a profiler), or the deterministic mode, in which at::empty
   // fills its result.
-  at::Tensor empty(at::IntArrayRef size, at::ScalarType dt) const {
-    const c10::DispatchKeySet on = c10::impl::tls_local_dispatch_key_set().included_;
-    if ((on - c10::default_included_set).empty() && !at::hasCallbacks() && !at::globalContext().deterministicAlgorithms())
-      return at::Tensor(at::detail::empty_cuda(size, dt, device, std::nullopt));
+  int direct = -1;             // what empty() found for this call
+  at::Tensor empty(at::IntArrayRef size, at::ScalarType dt) {
+    if (direct < 0) {
+      const c10::DispatchKeySet on = c10::impl::tls_local_dispatch_key_set().included_;
+      direct = (on - c10::default_included_set).empty() && !at::hasCallbacks() && !at::globalContext().deterministicAlgorithms() ? 1 : 0;
+    }
+    if (direct) return at::Tensor(at::detail::empty_cuda(size, dt, device, std::nullopt));
     return at::empty(size, at::TensorOptions().device(device).dtype(dt));
   }
 };
